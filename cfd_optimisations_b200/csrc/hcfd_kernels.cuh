@@ -188,38 +188,32 @@ __device__ __forceinline__ float qsqrt<float>(float x) { return x == 0.0f ? 0.0f
 // ---------------------------------------------------------------------------------------
 // flux arithmetic, written with the reference's expression trees
 
-// Flux::EulerFlux (src/Base/Flux.cpp:89-97); ir = 1/U[0], which Rusanov has formed already
-// (the same IEEE quotient, so passing it on changes no bit).
+// One side of the Rusanov flux: Euler flux along n (Flux::EulerFlux, src/Base/Flux.cpp:89-97)
+// and the side's wave speed |u.n| + a.  The reference expands every component over n0 and n1;
+// with m = n.(rho u) and u.n = m / rho formed once, F = (m, u.n rho u + P n0, u.n rho v + P n1,
+// (E + P) u.n): 9 operations in place of 22, equal up to rounding.
 template <class T>
-__device__ __forceinline__ void euler_flux(const T U[4], T ir, T n0, T n1, T gma, T F[4]) {
-    const T gmo = gma - T(1);
-    const T P = gmo * (U[3] - T(0.5) * ir * (U[1] * U[1] + U[2] * U[2]));
-    F[0] = n0 * U[1] + n1 * U[2];
-    F[1] = n0 * (U[1] * U[1] * ir + P) + n1 * U[2] * U[1] * ir;
-    F[2] = n0 * U[1] * U[2] * ir + n1 * (U[2] * U[2] * ir + P);
-    F[3] = n0 * (U[3] + P) * U[1] * ir + n1 * (U[3] + P) * U[2] * ir;
+__device__ __forceinline__ void euler_side(const T U[4], T n0, T n1, T gma, T F[4], T& speed) {
+    const T ir = qrcp(U[0]);
+    const T m = n0 * U[1] + n1 * U[2];
+    const T vn = m * ir;
+    const T P = (gma - T(1)) * (U[3] - T(0.5) * ir * (U[1] * U[1] + U[2] * U[2]));
+    F[0] = m;
+    F[1] = vn * U[1] + n0 * P;
+    F[2] = vn * U[2] + n1 * P;
+    F[3] = vn * (U[3] + P);
+    speed = fabs(vn) + qsqrt(gma * P * ir);
 }
 
-// Flux::Rusanov (src/Base/Flux.cpp:52-81).
+// Flux::Rusanov (src/Base/Flux.cpp:52-81).  The reference takes the largest of |u.n -+ a| over
+// both sides; the larger of |x - a| and |x + a| is |x| + a (the same addition of the same
+// magnitudes), so one maximum is left of three.
 template <class T>
 __device__ __forceinline__ void rusanov(const T UL[4], const T UR[4], T n0, T n1, T gma, T F[4]) {
-    const T gmo = gma - T(1);
-    const T irl = qrcp(UL[0]);
-    const T irr = qrcp(UR[0]);
-    const T nvl = (n0 * UL[1] + n1 * UL[2]) * irl;
-    const T nvr = (n0 * UR[1] + n1 * UR[2]) * irr;
-    const T qql = T(0.5) * (UL[1] * UL[1] + UL[2] * UL[2]) * irl;
-    const T qqr = T(0.5) * (UR[1] * UR[1] + UR[2] * UR[2]) * irr;
-    const T pl = gmo * (UL[3] - qql);
-    const T pr = gmo * (UR[3] - qqr);
-    const T al = qsqrt(gma * pl * irl);
-    const T ar = qsqrt(gma * pr * irr);
-    const T S1 = fmax(fabs(nvl - al), fabs(nvr - ar));
-    const T S2 = fmax(fabs(nvl + al), fabs(nvr + ar));
-    const T S = fmax(S1, S2);
-    T FL[4], FR[4];
-    euler_flux(UL, irl, n0, n1, gma, FL);
-    euler_flux(UR, irr, n0, n1, gma, FR);
+    T FL[4], FR[4], sl, sr;
+    euler_side(UL, n0, n1, gma, FL, sl);
+    euler_side(UR, n0, n1, gma, FR, sr);
+    const T S = fmax(sl, sr);
 #pragma unroll
     for (int v = 0; v < 4; v++) F[v] = T(0.5) * ((FL[v] + FR[v]) - S * (UR[v] - UL[v]));
 }
@@ -241,8 +235,8 @@ __device__ __forceinline__ void face_weights(bool isL, T If, T Af, T& ws, T& wn,
 // Spectral-radius term of one face for the local time step: (|u.n| + a) A_f from the
 // cell's own state (u, v, a precomputed).
 template <class T>
-__device__ __forceinline__ T wave(T u, T v, T a, const FaceGeo<T>& g) {
-    return (fabs(u * g.nx + v * g.ny) + a) * g.Af;
+__device__ __forceinline__ T wave(T u, T v, T a, T nx, T ny, T Af) {
+    return (fabs(u * nx + v * ny) + a) * Af;
 }
 
 template <class T>
@@ -254,19 +248,129 @@ __device__ __forceinline__ void cell_speed(const T U[4], T gma, T& u, T& v, T& a
     a = qsqrt(gma * p * ir);
 }
 
-// Face value of the limiter for one variable, |d| > 1e-9 (d = grad u . r_f):
-//   Barth-Jespersen (Limiter.cpp:67-71): min(1, D1 / d), D1 = u_max - u if d > 0, else u_min - u;
-//   Venkatakrishnan: min(1, (D1^2 + e2 + 2 D1 d) / (D1^2 + 2 d^2 + D1 d + e2)),
-//                    e2 = (K h)^3, h = sqrt(cell area).
-// (Skipping the quotient where it is at least 1 would give the same bits, but measured on the
-// B200 the branch costs more than the division it saves, in both precisions.)
+// Running extremes.  FP64 has no min/max instruction: fmin and fmax, with their NaN rules, cost
+// several times a compare and a select.  A NaN x leaves acc as it is, as fmin and fmax do.
+__device__ __forceinline__ double least(double acc, double x) { return x < acc ? x : acc; }
+__device__ __forceinline__ float least(float acc, float x) { return fminf(acc, x); }
+__device__ __forceinline__ double greatest(double acc, double x) { return x > acc ? x : acc; }
+__device__ __forceinline__ float greatest(float acc, float x) { return fmaxf(acc, x); }
+
+// Numerator and denominator of the limiter on one side of a cell (D >= 0 the room to the
+// neighbours' extreme, d > 0 the increment at a face), phi = min(1, num / den):
+//   Barth-Jespersen (Limiter.cpp:67-71): D / d;
+//   Venkatakrishnan: (D^2 + e2 + 2 D d) / (D^2 + 2 d^2 + D d + e2), e2 = (K h)^3, h = sqrt(cell area).
 template <class T>
-__device__ __forceinline__ T face_limiter(int limiter, T D1, T d, T e2) {
-    if (limiter == LIM_BJ) return fmin(T(1), qdiv(D1, d));
-    const T num = D1 * D1 + e2 + T(2) * D1 * d;
-    const T den = D1 * D1 + T(2) * d * d + D1 * d + e2;
-    return fmin(T(1), qdiv(num, den));
+__device__ __forceinline__ void limiter_terms(int limiter, T D, T d, T e2, T& num, T& den) {
+    num = D;
+    den = d;
+    if (limiter != LIM_BJ) {
+        const T t = D * D + e2;
+        num = t + T(2) * D * d;
+        den = t + d * (D + T(2) * d);
+    }
 }
+
+// Limiter values of a cell's four variables: per variable the smallest face value
+// min(1, limiter(D1, d)) over the cell's faces with |d| > 1e-9, d = grad u . r_f and D1 the room
+// upwards (u_max - u) where d > 0, downwards (u_min - u) where d < 0 (Limiter.cpp:41-76).
+// On one side D1 is the same for every face and min(1, limiter) does not grow with |d| (for
+// Venkatakrishnan it is below 1 only where d > D1 / 2, and falls from there), so the face with
+// the largest |d| on each side decides: two candidates per variable whatever the number of
+// faces.  In FP64, whose quotients are long dependency chains, the smaller candidate is chosen
+// by cross products (both denominators are positive; no overflow below |u| ~ 1e75), and one
+// quotient per variable is formed, and none in a cell where every variable has num >= den (phi =
+// 1).  In FP32 the approximate quotients are cheaper than the choice.  Against a quotient per
+// face and fmin/fmax throughout: see the table of steps in the notes at tile_pass1_kernel.
+template <class T, int W>
+__device__ __forceinline__ void cell_limiter(int limiter, const T u[4], const T umin[4], const T umax[4], const T g[8],
+                                             const T ro[W][2], T e2, T phi[4]) {
+    const T eps = T(1e-9);
+    T num[4], den[4];
+    bool any = false;
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        T up = T(0), dn = T(0);
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            const T d = g[2 * v] * ro[k][0] + g[2 * v + 1] * ro[k][1];
+            up = greatest(up, d);
+            dn = least(dn, d);
+        }
+        T n1, d1, n2, d2;
+        limiter_terms(limiter, umax[v] - u[v], up, e2, n1, d1);
+        limiter_terms(limiter, u[v] - umin[v], -dn, e2, n2, d2);
+        const bool on1 = up > eps, on2 = dn < -eps;
+        if (sizeof(T) == 8) {
+            n1 = on1 ? n1 : T(1);
+            d1 = on1 ? d1 : T(1);
+            const bool second = on2 && n2 * d1 < n1 * d2;
+            num[v] = second ? n2 : n1;
+            den[v] = second ? d2 : d1;
+            any |= num[v] < den[v];
+            phi[v] = T(1);
+        } else {
+            const T q1 = qdiv(n1, d1), q2 = qdiv(n2, d2);
+            phi[v] = fmin(on1 ? fmin(T(1), q1) : T(1), on2 ? q2 : T(1));
+        }
+    }
+    if (sizeof(T) == 8 && any) {
+#pragma unroll
+        for (int v = 0; v < 4; v++) phi[v] = num[v] < den[v] ? num[v] / den[v] : T(1);
+    }
+}
+
+// Pass 1 of one cell, face by face: Green-Gauss gradient, the neighbours' extremes and the
+// wave-speed sum of the CFL time step.  The tiled and the per-cell kernels differ only in where
+// the operands come from.
+template <class T, int W>
+struct Pass1Cell {
+    T u[4], G[8], umin[4], umax[4], ro[W][2], lam, cu, cv, ca;
+
+    __device__ __forceinline__ void begin(int time_mode, T gma) {
+#pragma unroll
+        for (int v = 0; v < 4; v++) { G[2 * v] = T(0); G[2 * v + 1] = T(0); umin[v] = u[v]; umax[v] = u[v]; }
+        lam = T(0);
+        if (time_mode != TM_FIXED) cell_speed(u, gma, cu, cv, ca);
+    }
+    // GaussGreen.cpp:25-28: uf = u_CL If + u_CR (1 - If); +uf Af n into CL, -uf Af n into CR (the
+    // side folded into face_weights); r is this cell's own centre-to-face vector.
+    __device__ __forceinline__ void face(int k, const T un[4], bool isL, T nx, T ny, T Af, T If, T rx, T ry, int time_mode) {
+        T ws, wn, sA;
+        face_weights(isL, If, Af, ws, wn, sA);
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            const T uf = u[v] * ws + un[v] * wn;
+            const T t = uf * sA;
+            G[2 * v] += t * nx;
+            G[2 * v + 1] += t * ny;
+            umin[v] = least(umin[v], un[v]);                 // Limiter.cpp:31-39
+            umax[v] = greatest(umax[v], un[v]);
+        }
+        ro[k][0] = rx;
+        ro[k][1] = ry;
+        if (time_mode != TM_FIXED) lam += wave(cu, cv, ca, nx, ny, Af);
+    }
+    __device__ __forceinline__ void no_face(int k) { ro[k][0] = T(0); ro[k][1] = T(0); }
+    // Gradient (GaussGreen.cpp:33-39), limiter (or the frozen values in phis) and the limited
+    // gradient in out; phis holds the limiter values used.
+    __device__ __forceinline__ void finish(T iv, int limiter, T venkat_K, int lmode, T phis[4], T out[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) G[j] *= iv;
+        if (lmode != LIM_FROZEN) {
+            T e2 = T(0);
+            if (limiter == LIM_VENKAT) {
+                const T kh = venkat_K * qsqrt(qrcp(iv));
+                e2 = kh * kh * kh;
+            }
+            cell_limiter<T, W>(limiter, u, umin, umax, G, ro, e2, phis);
+        }
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            out[2 * v] = phis[v] * G[2 * v];
+            out[2 * v + 1] = phis[v] * G[2 * v + 1];
+        }
+    }
+};
 
 // Two-sum accumulation s + c += x (Knuth), with explicit round-to-nearest adds so that no
 // multiply is fused into the sum.
@@ -370,74 +474,28 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
 #pragma unroll
         for (int k = 0; k < W; k++) s[k] = __ldg(a.slot + (size_t) k * a.Nc + c);
         if (s[0].y >= 0) {
-            T u[4];
-            ld_cell(a.U, a.Nc, c, u);
+            Pass1Cell<T, W> p;
+            ld_cell(a.U, a.Nc, c, p.u);
             const T iv = __ldg(a.iv + c);
-            T G[4][2], umin[4], umax[4], ro[W][2];
-#pragma unroll
-            for (int v = 0; v < 4; v++) { G[v][0] = T(0); G[v][1] = T(0); umin[v] = u[v]; umax[v] = u[v]; }
-            T cu = T(0), cv = T(0), ca = T(0), lam = T(0);
-            if (a.time_mode != TM_FIXED) cell_speed(u, a.gma, cu, cv, ca);
+            p.begin(a.time_mode, a.gma);
 #pragma unroll
             for (int k = 0; k < W; k++) {
-                ro[k][0] = T(0); ro[k][1] = T(0);
-                if (s[k].y < 0) continue;
+                if (s[k].y < 0) { p.no_face(k); continue; }
                 const bool isL = s[k].x >= 0;
                 const int f = isL ? s[k].x : ~s[k].x;
                 FaceGeo<T> g;
                 ld_geo(a.geo, f, g);
                 T un[4];
                 ld_cell(a.U, a.Nc, s[k].y, un);
-                // GaussGreen.cpp:25-28: uf = u_CL If + u_CR (1 - If); +uf Af n into CL,
-                // -uf Af n into CR (the side folded into face_weights).
-                T ws, wn, sA;
-                face_weights(isL, g.If, g.Af, ws, wn, sA);
-#pragma unroll
-                for (int v = 0; v < 4; v++) {
-                    const T uf = u[v] * ws + un[v] * wn;
-                    const T t = uf * sA;
-                    G[v][0] += t * g.nx;
-                    G[v][1] += t * g.ny;
-                    umin[v] = fmin(umin[v], un[v]);        // Limiter.cpp:31-39
-                    umax[v] = fmax(umax[v], un[v]);
-                }
-                ro[k][0] = isL ? g.rLx : g.rRx;
-                ro[k][1] = isL ? g.rLy : g.rRy;
-                if (a.time_mode != TM_FIXED) lam += wave(cu, cv, ca, g);
+                p.face(k, un, isL, g.nx, g.ny, g.Af, g.If, isL ? g.rLx : g.rRx, isL ? g.rLy : g.rRy, a.time_mode);
             }
-            T e2 = T(0);
-            if (a.limiter == LIM_VENKAT) {
-                const T kh = a.venkat_K * qsqrt(qrcp(iv));
-                e2 = kh * kh * kh;
-            }
-            const T eps = T(1e-9);
             const int lmode = limiter_mode(a.stats->steps, a.freeze_after);
             T out[8], phis[4];
             if (lmode == LIM_FROZEN) ld_cell(a.phiF, a.Nc, c, phis);
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const T gx = G[v][0] * iv, gy = G[v][1] * iv;     // GaussGreen.cpp:33-39
-                T phi = T(1);
-                if (lmode == LIM_FROZEN) {
-                    phi = phis[v];
-                } else {
-#pragma unroll
-                    for (int k = 0; k < W; k++) {
-                        if (s[k].y < 0) continue;
-                        const T d = gx * ro[k][0] + gy * ro[k][1];   // Limiter.cpp:50-51
-                        T pf = T(1);                                 // Limiter.cpp:67-71
-                        if (d > eps || d < -eps)
-                            pf = face_limiter(a.limiter, (d > eps) ? umax[v] - u[v] : umin[v] - u[v], d, e2);
-                        phi = fmin(phi, pf);                         // Limiter.cpp:73-74
-                    }
-                }
-                phis[v] = phi;
-                out[2 * v] = phi * gx;
-                out[2 * v + 1] = phi * gy;
-            }
+            p.finish(iv, a.limiter, a.venkat_K, lmode, phis, out);
             if (lmode == LIM_RECORD) st_cell(a.phiF, a.Nc, c, phis);
             st_grad(a.phiG, a.Nc, c, out);
-            if (a.time_mode != TM_FIXED) xmx = iv * lam;
+            if (a.time_mode != TM_FIXED) xmx = iv * p.lam;
         }
     }
     if (a.time_mode != TM_FIXED) {
@@ -519,11 +577,10 @@ __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
                         const T x = isL ? -(g.Af * F[v]) : g.Af * F[v];
                         two_sum(R[v], Rc[v], x);
                     } else {
-                        if (isL) R[v] -= g.Af * F[v];
-                        else     R[v] += g.Af * F[v];
+                        R[v] += (isL ? -g.Af : g.Af) * F[v];
                     }
                 }
-                if (a.time_mode == TM_LOCAL) lam += wave(cu, cv, ca, g);
+                if (a.time_mode == TM_LOCAL) lam += wave(cu, cv, ca, g.nx, g.ny, g.Af);
             }
             T dt;
             if (a.time_mode == TM_LOCAL) dt = T(a.dt_or_cfl) * qrcp(iv * lam);

@@ -622,19 +622,18 @@ __global__ void __launch_bounds__(288) tile_pass1_kernel(const TileArgs<T> a) {
         short cs[8];
         lds_slots(sSlot + c * a.Wp, a.Wp, cs);
         if (cs[0] < 0) continue;
-        T u[4];
-        lds_cell(sU, NL, c, u);
+        Pass1Cell<T, W> p;
+        lds_cell(sU, NL, c, p.u);
         const T iv = sIv[c];
-        T G[4][2], umin[4], umax[4], ro[W][2];
-#pragma unroll
-        for (int v = 0; v < 4; v++) { G[v][0] = T(0); G[v][1] = T(0); umin[v] = u[v]; umax[v] = u[v]; }
-        T cu = T(0), cv = T(0), ca = T(0), lam = T(0);
-        if (s.time_mode != TM_FIXED) cell_speed(u, s.gma, cu, cv, ca);
+        p.begin(s.time_mode, s.gma);
 #pragma unroll
         for (int k = 0; k < W; k++) {
-            ro[k][0] = T(0); ro[k][1] = T(0);
-            if (cs[k] < 0) continue;
-            int e = cs[k] >> 1;
+            if (W > 3 && cs[k] < 0) { p.no_face(k); continue; }
+            // A slot a cell does not use (W = 3: a cell of an open mesh with fewer faces) reads
+            // entry 0 with zero length, the cell itself as its neighbour and r = 0, which adds
+            // nothing, in place of a branch per face.
+            const bool on = W > 3 || cs[k] >= 0;
+            int e = on ? cs[k] >> 1 : 0;
             const bool isL = (cs[k] & 1) == 0;
             if constexpr (kChecked)    // a bad index is replaced by entry 0 / tile cell 0 (no branch)
                 e = index_ok(e < nfl, a.err) ? e : 0;
@@ -642,62 +641,19 @@ __global__ void __launch_bounds__(288) tile_pass1_kernel(const TileArgs<T> a) {
             lds_geo4(sGeo, nfl, e, g);
             int nbl = isL ? meta_lb(sMeta[e]) : meta_la(sMeta[e]);
             if constexpr (kChecked)
-                nbl = index_ok(local_ok(nbl, nb, a.B, si.nh), a.err) ? nbl : 0;
+                nbl = index_ok(!on || local_ok(nbl, nb, a.B, si.nh), a.err) ? nbl : 0;
             T un[4];
-            lds_cell(sU, NL, nbl, un);
-            // GaussGreen.cpp:25-28: uf = u_CL If + u_CR (1 - If), added into CL and taken from
-            // CR.  The side is folded into two weights and a signed length once per face
-            // (face_weights) instead of selecting four left/right states and branching per
-            // variable.
-            T ws, wn, sA;
-            face_weights(isL, g.If, g.Af, ws, wn, sA);
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const T uf = u[v] * ws + un[v] * wn;
-                const T tt = uf * sA;
-                G[v][0] += tt * g.nx;
-                G[v][1] += tt * g.ny;
-                umin[v] = fmin(umin[v], un[v]);                  // Limiter.cpp:31-39
-                umax[v] = fmax(umax[v], un[v]);
-            }
+            lds_cell(sU, NL, on ? nbl : c, un);
             // this cell's own centre-to-face vector: one pair, at its side's plane
             const auto rr = ldp(sGeo, nfl, isL ? 2 : 3, e);
-            ro[k][0] = rr.x;
-            ro[k][1] = rr.y;
-            if (s.time_mode != TM_FIXED) lam += wave(cu, cv, ca, g);
+            p.face(k, un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, on ? rr.x : T(0), on ? rr.y : T(0), s.time_mode);
         }
-        T e2 = T(0);
-        if (s.limiter == LIM_VENKAT) {
-            const T kh = s.venkat_K * qsqrt(qrcp(iv));
-            e2 = kh * kh * kh;
-        }
-        const T eps = T(1e-9);
         T out[8], phis[4];
         if (lmode == LIM_FROZEN) ld_cell(s.phiF, a.ps, base + c, phis);
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-            const T gx = G[v][0] * iv, gy = G[v][1] * iv;
-            T phi = T(1);
-            if (lmode == LIM_FROZEN) {
-                phi = phis[v];
-            } else {
-#pragma unroll
-                for (int k = 0; k < W; k++) {
-                    if (cs[k] < 0) continue;
-                    const T d = gx * ro[k][0] + gy * ro[k][1];
-                    T pf = T(1);                                     // Limiter.cpp:67-71
-                    if (d > eps || d < -eps)
-                        pf = face_limiter(s.limiter, (d > eps) ? umax[v] - u[v] : umin[v] - u[v], d, e2);
-                    phi = fmin(phi, pf);
-                }
-            }
-            phis[v] = phi;
-            out[2 * v] = phi * gx;
-            out[2 * v + 1] = phi * gy;
-        }
+        p.finish(iv, s.limiter, s.venkat_K, lmode, phis, out);
         if (lmode == LIM_RECORD) st_cell(s.phiF, a.ps, base + c, phis);
         st_grad(s.phiG, a.ps, base + c, out);
-        if (s.time_mode != TM_FIXED) xmx = fmax(xmx, iv * lam);
+        if (s.time_mode != TM_FIXED) xmx = fmax(xmx, iv * p.lam);
     }
     if constexpr (ARENA) {
         // per-instance minimum (exact and order-free): each warp carries its minimum across
@@ -812,14 +768,13 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
                 if constexpr (COMP) {                            // Fv holds A_f F here
                     two_sum(R[v], Rc[v], isL ? -Fv : Fv);
                 } else {
-                    if (isL) R[v] -= Af * Fv;
-                    else     R[v] += Af * Fv;
+                    R[v] += (isL ? -Af : Af) * Fv;
                 }
             }
             if (s.time_mode == TM_LOCAL) {                       // the normal only for the local dt
                 FaceGeo<T> g;
                 lds_geo3(sGeo, nf, e, a.rec, g.nx, g.ny, g.Af);
-                lam += wave(cu, cv, ca, g);
+                lam += wave(cu, cv, ca, g.nx, g.ny, g.Af);
             }
         }
         T dt;
