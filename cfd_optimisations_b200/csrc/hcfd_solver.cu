@@ -9,6 +9,7 @@
 // numbering.
 #include "hcfd_internal.hpp"
 #include "hcfd_kernels.cuh"
+#include "hcfd_resident.cuh"
 #include "hcfd_tile.cuh"
 
 #include <algorithm>
@@ -101,6 +102,11 @@ struct hcfd_solver {
     // early take more tiles; without, every CTA takes every grid-th tile
     bool queue1 = true, queue2 = false;
     bool tiled = false;
+    // resident steps (hcfd_resident.cuh): tp[0] holds one tile per SM; d_counter[3] counts the
+    // arrivals at its grid barriers, bar_base of them before the next launch
+    bool resident = false;
+    unsigned char* d_exported = nullptr;
+    unsigned bar_base = 0;
     int cur = 0;                         // which of d_U holds the state
     int block = 256;
     int partial_len = 0;
@@ -139,7 +145,7 @@ void free_all(hcfd_solver* s) {
     for (auto e : s->ev1) cudaEventDestroy(e);
     for (auto e : s->ev2) cudaEventDestroy(e);
     void* ptrs[] = {s->d_fc, s->d_perm, s->d_slot, s->d_geo64, s->d_geoT, s->d_iv, s->d_U[0], s->d_U[1],
-                    s->d_phiG, s->d_phiF, s->d_io, s->d_cp, s->d_dtmin, s->d_partial, s->d_counter, s->d_err, s->d_stats};
+                    s->d_phiG, s->d_phiF, s->d_io, s->d_cp, s->d_dtmin, s->d_partial, s->d_counter, s->d_err, s->d_stats, s->d_exported};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (TiledPass& P : s->tp) {
         void* q[] = {P.d_tgeo, P.d_tmeta, P.d_foff, P.d_hoff, P.d_halo, P.d_cslot, P.d_efid};
@@ -236,11 +242,48 @@ int prof_end(hcfd_solver* s, bool rec, Ev& e, std::vector<cudaEvent_t>& into) {
     return HCFD_OK;
 }
 
+// nsteps steps (phases 3), or one half of one step, of the resident kernel.
+template <class T, int W>
+int launch_resident(hcfd_solver* s, int time_mode, double dt_or_cfl, int nsteps, int phases) {
+    hcfd::TileArgs<T> a = tile_args<T>(s, time_mode, dt_or_cfl, s->tp[0], 1);
+    hcfd::ResidentArgs r;
+    r.exported = s->d_exported;
+    r.bar = s->d_counter + 3;
+    r.bar_base = s->bar_base;
+    r.dtmin = s->d_dtmin;
+    r.partial_first = s->d_partial + s->partial_len;
+    r.nsteps = nsteps;
+    r.phases = phases;
+    void* args[] = {&a, &r};
+    CK(cudaLaunchCooperativeKernel((const void*) hcfd::resident_kernel<T, W, std::is_same<T, float>::value>, dim3(s->grid1),
+                                   dim3(s->tp[0].block), args, s->smem1, s->stream));
+    s->bar_base += (unsigned) s->grid1 * (phases == 3 ? 2u * (unsigned) nsteps - 1u : phases == 2 ? 1u : 0u);
+    return HCFD_OK;
+}
+
+template <class T>
+int launch_resident_w(hcfd_solver* s, int time_mode, double dt_or_cfl, int nsteps) {
+    switch (s->W) {
+    case 3: return launch_resident<T, 3>(s, time_mode, dt_or_cfl, nsteps, 3);
+    case 4: return launch_resident<T, 4>(s, time_mode, dt_or_cfl, nsteps, 3);
+    default: return launch_resident<T, 8>(s, time_mode, dt_or_cfl, nsteps, 3);
+    }
+}
+
 template <class T, int W>
 int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl) {
     Ev e1, e2;
     int rc;
     const bool rec = s->prof && (s->prof_count++ % s->prof_every == 0);
+    if (s->resident) {
+        // per-kernel events: the two halves of the step as launches of their own
+        if (!rec) return launch_resident<T, W>(s, time_mode, dt_or_cfl, 1, 3);
+        if ((rc = prof_begin(s, rec, e1)) || (rc = launch_resident<T, W>(s, time_mode, dt_or_cfl, 1, 1)) ||
+            (rc = prof_end(s, rec, e1, s->ev1)) || (rc = prof_begin(s, rec, e2)) ||
+            (rc = launch_resident<T, W>(s, time_mode, dt_or_cfl, 1, 2)) || (rc = prof_end(s, rec, e2, s->ev2)))
+            return rc;
+        return HCFD_OK;
+    }
     if (s->tiled) {
         const TiledPass& P2 = s->split ? s->tp[1] : s->tp[0];
         const hcfd::TileArgs<T> a1 = tile_args<T>(s, time_mode, dt_or_cfl, s->tp[0], 1);
@@ -299,6 +342,37 @@ int setup_tiled_w(hcfd_solver* s) {
     s->grid1 = std::min(P.ntiles, b1 * s->nsm);
     s->grid2 = std::min(Q.ntiles, b2 * s->nsm);
     return HCFD_OK;
+}
+
+// Whether the resident kernel can hold this mesh, one tile of tp[0] per SM; sets its launch shape.
+template <class T, int W>
+int setup_resident_w(hcfd_solver* s, bool* fits) {
+    const hcfd::TilePlan& P = s->tp[0].plan;
+    const auto kernel = hcfd::resident_kernel<T, W, std::is_same<T, float>::value>;
+    *fits = false;
+    s->smem1 = hcfd::ResidentSmem<T>(P.B, P.Hmax, P.Fmax, P.Wp).total;
+    int maxsm = 0;
+    CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
+    cudaFuncAttributes fa;
+    CK(cudaFuncGetAttributes(&fa, kernel));
+    if (s->smem1 + fa.sharedSizeBytes > (size_t) maxsm) return HCFD_OK;
+    // the attribute is the kernel's, shared by every handle: the largest any handle may need
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm - (int) fa.sharedSizeBytes));
+    s->tp[0].block = std::min((P.B + 31) / 32 * 32, hcfd::kResidentThreads);
+    int nb = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, s->tp[0].block, s->smem1));
+    s->grid1 = s->grid2 = P.ntiles;
+    *fits = nb >= 1 && P.ntiles <= nb * s->nsm;
+    return HCFD_OK;
+}
+
+template <class T>
+int setup_resident(hcfd_solver* s, bool* fits) {
+    switch (s->W) {
+    case 3: return setup_resident_w<T, 3>(s, fits);
+    case 4: return setup_resident_w<T, 4>(s, fits);
+    default: return setup_resident_w<T, 8>(s, fits);
+    }
 }
 
 template <class T>
@@ -403,7 +477,25 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
 
     s->tiled = (p.kernel == HCFD_KERNEL_TILED);
     std::vector<int2> slot;
-    if (s->tiled) {
+    if (s->tiled && !p.tile && !p.tile2 && !p.block) {
+        // Resident steps where the whole mesh fits in the SMs' shared memory, one tile per SM
+        // (no explicit tile or block).  The plan is built only where the cells' own arrays fit.
+        const bool f64 = p.precision == HCFD_FP64;
+        int maxsm = 0, coop = 0;
+        CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
+        CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
+        const int B = std::max(32, ((Nc + s->nsm - 1) / s->nsm + 7) / 8 * 8);
+        const size_t least = f64 ? hcfd::ResidentSmem<double>(B, 0, B * 3 / 2, s->W).total
+                                 : hcfd::ResidentSmem<float>(B, 0, B * 3 / 2, s->W).total;
+        if (coop && least <= (size_t) maxsm) {
+            rc = hcfd::build_tile_plan(*mv, cf_off, cf_con, ghost, perm, s->F_BC, bc_first, B, s->W, s->tp[0].plan, true);
+            if (rc != HCFD_OK) hcfd::clear_error();     // too scattered for one tile per SM: the tiled kernels
+            else if ((rc = f64 ? setup_resident<double>(s.get(), &s->resident) : setup_resident<float>(s.get(), &s->resident)))
+                return rc;
+        }
+        if (!s->resident) s->tp[0] = TiledPass();
+    }
+    if (s->tiled && !s->resident) {
         // Pass 1 on tiles of `tile` cells, pass 2 on tiles of `tile2`.  When neither is given:
         // FP64 224 and 192 cells, FP32 256 and 128 (pass 2's flux work per tile is heavy in
         // FP64, and fewer tile cuts pay; measured on the B200), falling back to smaller
@@ -447,7 +539,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         }
         if (!ok) return fail(HCFD_EINVAL, "tile does not fit in shared memory");
         if (!s->split) s->tp[1] = TiledPass();
-    } else {
+    } else if (!s->tiled) {
         // Per-cell kernels: slot-major table {face or ~face, neighbour}, internal numbering.
         slot.assign((size_t) s->W * Nc, make_int2(-1, -1));
         for (int ci = 0; ci < Nc; ci++) {
@@ -468,7 +560,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
     const bool f32 = p.precision == HCFD_FP32;
     const size_t tsz = f32 ? sizeof(float) : sizeof(double);
     if (s->tiled) {
-        rc = f32 ? setup_tiled<float>(h) : setup_tiled<double>(h);
+        rc = s->resident ? HCFD_OK : f32 ? setup_tiled<float>(h) : setup_tiled<double>(h);
         if (rc) return bail(rc);
         h->partial_len = std::max(h->grid1, h->grid2);
     } else {
@@ -492,7 +584,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         (rc = dalloc((char**) &h->d_U[0], tsz * 4 * Nc)) || (rc = dalloc((char**) &h->d_U[1], tsz * 4 * Nc)) ||
         (rc = dalloc((char**) &h->d_phiG, tsz * 8 * Nc)) || (rc = dalloc(&h->d_io, 4 * (size_t) Nc)) ||
         (p.freeze_limiter_after > 0 && (rc = dalloc((char**) &h->d_phiF, tsz * 4 * Nc))) ||
-        (rc = dalloc(&h->d_cp, Nf)) || (rc = dalloc(&h->d_dtmin, 2)) || (rc = dalloc(&h->d_partial, h->partial_len)) ||
+        (rc = dalloc(&h->d_cp, Nf)) || (rc = dalloc(&h->d_dtmin, 2)) || (rc = dalloc(&h->d_partial, 2 * (size_t) h->partial_len)) ||
         (rc = dalloc(&h->d_counter, 4)) || (rc = dalloc(&h->d_err, 1)) || (rc = dalloc(&h->d_stats, 1)) ||
         (rc = dalloc(&d_fn, 2 * (size_t) Nf)) || (rc = dalloc(&d_fcu, 2 * (size_t) Nf)) ||
         (rc = dalloc(&d_cnoff, Nc + 1)) || (rc = dalloc(&d_cncon, ncn)) || (rc = dalloc(&d_cfoff, Nc + 1)) ||
@@ -513,6 +605,10 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
                 free_tmp();
                 return bail(rc);
             }
+        }
+        if (h->resident && (rc = dalloc(&h->d_exported, niv))) {
+            free_tmp();
+            return bail(rc);
         }
     } else {
         if ((rc = dalloc(&h->d_slot, slot.size())) || (f32 && (rc = dalloc((char**) &h->d_geoT, tsz * 8 * (size_t) Nf)))) {
@@ -545,6 +641,11 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
             if (ce == cudaSuccess) ce = up(T.d_halo, P.halo.data(), 4 * P.halo.size());
             if (ce == cudaSuccess) ce = up(T.d_cslot, P.cslot.data(), 2 * P.cslot.size());
             if (ce == cudaSuccess) ce = up(T.d_efid, P.efid.data(), 4 * P.efid.size());
+        }
+        if (h->resident) {
+            std::vector<unsigned char> ex(niv, 0);
+            for (int ci : h->tp[0].plan.halo) ex[ci] = 1;
+            if (ce == cudaSuccess) ce = up(h->d_exported, ex.data(), ex.size());
         }
     } else {
         if (ce == cudaSuccess) ce = up(h->d_slot, slot.data(), sizeof(int2) * slot.size());
@@ -630,7 +731,8 @@ int hcfd_gpu_initialise(hcfd_solver* s, const double* qic) {
     if (rc) return rc;
     CK(cudaMemsetAsync(s->d_stats, 0, sizeof(hcfd::StepStats), s->stream));
     CK(cudaMemsetAsync(s->d_err, 0, sizeof(unsigned int), s->stream));
-    CK(cudaMemsetAsync(s->d_counter, 0, 4 * sizeof(unsigned int), s->stream));   // ticket, tile queues
+    CK(cudaMemsetAsync(s->d_counter, 0, 4 * sizeof(unsigned int), s->stream));   // ticket, tile queues, grid barriers
+    s->bar_base = 0;
     const unsigned long long inf2[2] = {0x7FF0000000000000ULL, 0x7FF0000000000000ULL};
     CK(cudaMemcpyAsync(s->d_dtmin, inf2, sizeof(inf2), cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));
@@ -660,10 +762,17 @@ int hcfd_gpu_step(hcfd_solver* s, int nsteps, int time_mode, double dt_or_cfl, h
         }
     }
     int n = nsteps;
+    while (s->resident && !s->prof && n > 0) {
+        // bounded launches, so that other streams' work gets its turn on the SMs
+        const int k = std::min(n, 1024);
+        rc = s->fp32() ? launch_resident_w<float>(s, time_mode, dt_or_cfl, k) : launch_resident_w<double>(s, time_mode, dt_or_cfl, k);
+        if (rc) return rc;
+        n -= k;
+    }
     while (n > 0) {
         // pairs of steps without per-kernel events run as the graph; profiled steps run eagerly
         const bool rec = s->prof && (s->prof_count % s->prof_every == 0 || (s->prof_count + 1) % s->prof_every == 0);
-        if (n >= 2 && !rec) {
+        if (n >= 2 && !rec && !s->resident) {
             if (s->graph && (s->g_mode != time_mode || s->g_value != dt_or_cfl || s->g_cur != s->cur)) {
                 cudaGraphExecDestroy(s->graph);
                 s->graph = nullptr;
@@ -990,7 +1099,7 @@ int hcfd_gpu_step_timed(hcfd_solver* s, int nsteps, int time_mode, double dt_or_
     return read_stats(s, nullptr);
 }
 
-int hcfd_gpu_launches_per_step(hcfd_solver* s) { return s ? 2 : 0; }
+int hcfd_gpu_launches_per_step(hcfd_solver* s) { return s ? (s->resident ? 1 : 2) : 0; }
 
 int hcfd_host_pin(void* p, size_t bytes) {
     hcfd::clear_error();

@@ -508,52 +508,96 @@ struct FaceIn {
         const int bc = meta_bc(w);
         const int mx = meta_la(w), my = meta_lb(w);
         const int rp = rplane(rec);
-        FaceGeo<T> g;
-        {
-            const auto n2 = ldp(sGeo, nf, 0, e), rl = ldp(sGeo, nf, rp, e), rr = ldp(sGeo, nf, rp + 1, e);
-            g.nx = n2.x; g.ny = n2.y; g.rLx = rl.x; g.rLy = rl.y; g.rRx = rr.x; g.rRy = rr.y;
-        }
-        nx = g.nx; ny = g.ny; Af = lds_area(sGeo, nf, e, rec);
-        T uL[4], uR[4], gL[8];
-        lds_cell(sU, NL, mx, uL);
-        lds_cell(sU, NL, my, uR);
+        // Ghost on the right: -grad and the same phi as the interior cell with r_R = -r_L
+        // (BoundaryConditions/Base.cpp:29-53, Domain.cpp:84-88): the same increment, so both
+        // sides read the left cell's gradient and r.
+        const bool interior = bc < 0;
+        const auto n2 = ldp(sGeo, nf, 0, e), rl = ldp(sGeo, nf, rp, e), rr = ldp(sGeo, nf, interior ? rp + 1 : rp, e);
+        nx = n2.x; ny = n2.y; Af = lds_area(sGeo, nf, e, rec);
+        T gL[8], gR[8];
+        lds_cell(sU, NL, mx, uoL);
+        lds_cell(sU, NL, my, uqR);
         lds_grad(sG, NL, mx, gL);
-        if (bc >= 0) {
-            // Ghost on the right: -grad and the same phi as the interior cell with r_R = -r_L
-            // (BoundaryConditions/Base.cpp:29-53, Domain.cpp:84-88): the same increment.
+        lds_grad(sG, NL, interior ? my : mx, gR);
 #pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const T du = gL[2 * v] * g.rLx + gL[2 * v + 1] * g.rLy;
-                uoL[v] = uL[v] + du;
-                uqR[v] = uR[v] + du;
-            }
-        } else {
-            T gR[8];
-            lds_grad(sG, NL, my, gR);
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                uoL[v] = uL[v] + (gL[2 * v] * g.rLx + gL[2 * v + 1] * g.rLy);
-                uqR[v] = uR[v] + (gR[2 * v] * g.rRx + gR[2 * v + 1] * g.rRy);
-            }
+        for (int v = 0; v < 4; v++) {
+            uoL[v] += gL[2 * v] * rl.x + gL[2 * v + 1] * rl.y;
+            uqR[v] += gR[2 * v] * rr.x + gR[2 * v + 1] * rr.y;
         }
     }
     __device__ __forceinline__ void flux(T gma, T F[4]) const { rusanov(uoL, uqR, nx, ny, gma, F); }
-    // F over the two r pairs of this entry's staged record: only this thread reads them in
-    // pass 2, and it has read them already.  With AF the product A_f F is stored instead (the
+    // F as two pairs at sF (plane stride nf).  With AF the product A_f F is stored instead (the
     // compensated FP32 sums round that product before adding it, so forming it once per face
     // gives the same bits as forming it in each of the two cells).
     template <bool AF>
-    __device__ __forceinline__ void store(T* sGeo, int nf, int rec, const T F[4]) const {
-        const int rp = rplane(rec);
+    __device__ __forceinline__ void store(T* sF, int nf, const T F[4]) const {
         if (AF) {
-            stp(sGeo, nf, rp, e, F[0] * Af, F[1] * Af);
-            stp(sGeo, nf, rp + 1, e, F[2] * Af, F[3] * Af);
+            stp(sF, nf, 0, e, F[0] * Af, F[1] * Af);
+            stp(sF, nf, 1, e, F[2] * Af, F[3] * Af);
         } else {
-            stp(sGeo, nf, rp, e, F[0], F[1]);
-            stp(sGeo, nf, rp + 1, e, F[2], F[3]);
+            stp(sF, nf, 0, e, F[0], F[1]);
+            stp(sF, nf, 1, e, F[2], F[3]);
         }
     }
 };
+
+// Sum of A_f F over one cell's faces in increasing face order (Flux.cpp:39-42), F as stored by
+// FaceIn::store at sF, and (local time stepping) the cell's wave-speed sum.  One face's flux
+// leaves its left cell and enters its right one.  FP32 sums are compensated; the first term
+// needs no two-sum, 0 + x being exact.
+template <class T, int W, bool COMP>
+__device__ __forceinline__ void cell_flux_sum(const short cs[8], const T* sF, const T* sGeo, int nf, int rec, int time_mode,
+                                              const T u[4], T gma, T R[4], T& lam, unsigned int* err) {
+    T Rc[4];
+#pragma unroll
+    for (int v = 0; v < 4; v++) { R[v] = T(0); Rc[v] = T(0); }
+    T cu = T(0), cv = T(0), ca = T(0);
+    lam = T(0);
+    if (time_mode == TM_LOCAL) cell_speed(u, gma, cu, cv, ca);
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        if (W > 3 && cs[k] < 0) continue;
+        // (W = 3) an unused slot reads entry 0 with weight zero, in place of a branch per face
+        const bool on = W > 3 || cs[k] >= 0;
+        const bool isL = (cs[k] & 1) == 0;
+        int e = on ? cs[k] >> 1 : 0;
+        if constexpr (kChecked) e = index_ok(e < nf, err) ? e : 0;
+        const auto F01 = ldp(sF, nf, 0, e), F23 = ldp(sF, nf, 1, e);
+        const T Fk[4] = {F01.x, F01.y, F23.x, F23.y};
+        if constexpr (COMP) {
+#pragma unroll
+            for (int v = 0; v < 4; v++) {                        // Fk holds A_f F here
+                const T x = !on ? T(0) : isL ? -Fk[v] : Fk[v];
+                if (k == 0) R[v] = x;
+                else two_sum(R[v], Rc[v], x);
+            }
+        } else {
+            const T Af = lds_area(sGeo, nf, e, rec);
+            const T sA = !on ? T(0) : isL ? -Af : Af;
+#pragma unroll
+            for (int v = 0; v < 4; v++) R[v] += sA * Fk[v];
+        }
+        if (time_mode == TM_LOCAL) {                             // the normal only for the local dt
+            T nx, ny, A;
+            lds_geo3(sGeo, nf, e, rec, nx, ny, A);
+            lam += wave(cu, cv, ca, nx, ny, on ? A : T(0));
+        }
+    }
+    if constexpr (COMP)
+#pragma unroll
+        for (int v = 0; v < 4; v++) R[v] += Rc[v];
+}
+
+// U += dt R (Flux.cpp:45-49, Euler.cpp:107-113); returns the density residual R_rho.
+template <class T>
+__device__ __forceinline__ T cell_update(const T u[4], const T R[4], T iv, T dt, T un[4], int& bad) {
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        un[v] = u[v] + dt * (R[v] * iv);
+        bad |= !isfinite(un[v]);
+    }
+    return R[0] * iv;
+}
 
 // Warp-specialised persistent tile loop.  The last warp of the CTA is the producer
 // (producer_loop); the first NT = blockDim.x - 32 threads compute.  Compute iteration i
@@ -610,6 +654,36 @@ struct FaceIn {
     }                                                                                            \
     }
 
+// Pass 1's face loop of tile cell c (its state in p.u), operands from shared memory: nf entries,
+// nb tile cells and nh halo cells of NL staged.
+template <class T, int W>
+__device__ __forceinline__ void tile_faces(Pass1Cell<T, W>& p, const TileArgs<T>& a, const Cell4<T>* sU, const T* sGeo,
+                                           const unsigned* sMeta, const short cs[8], int NL, int nf, int nb, int nh, int c) {
+    p.begin(a.s.time_mode, a.s.gma);
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        if (W > 3 && cs[k] < 0) { p.no_face(k); continue; }
+        // A slot a cell does not use (W = 3: a cell of an open mesh with fewer faces) reads
+        // entry 0 with zero length, the cell itself as its neighbour and r = 0, which adds
+        // nothing, in place of a branch per face.
+        const bool on = W > 3 || cs[k] >= 0;
+        int e = on ? cs[k] >> 1 : 0;
+        const bool isL = (cs[k] & 1) == 0;
+        if constexpr (kChecked)    // a bad index is replaced by entry 0 / tile cell 0 (no branch)
+            e = index_ok(e < nf, a.err) ? e : 0;
+        FaceGeo<T> g;
+        lds_geo4(sGeo, nf, e, g);
+        int nbl = isL ? meta_lb(sMeta[e]) : meta_la(sMeta[e]);
+        if constexpr (kChecked)
+            nbl = index_ok(!on || local_ok(nbl, nb, a.B, nh), a.err) ? nbl : 0;
+        T un[4];
+        lds_cell(sU, NL, on ? nbl : c, un);
+        // this cell's own centre-to-face vector: one pair, at its side's plane
+        const auto rr = ldp(sGeo, nf, isL ? 2 : 3, e);
+        p.face(k, un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, on ? rr.x : T(0), on ? rr.y : T(0), a.s.time_mode);
+    }
+}
+
 template <class T, int W, bool ARENA>
 __global__ void __launch_bounds__(288) tile_pass1_kernel(const TileArgs<T> a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -625,29 +699,7 @@ __global__ void __launch_bounds__(288) tile_pass1_kernel(const TileArgs<T> a) {
         Pass1Cell<T, W> p;
         lds_cell(sU, NL, c, p.u);
         const T iv = sIv[c];
-        p.begin(s.time_mode, s.gma);
-#pragma unroll
-        for (int k = 0; k < W; k++) {
-            if (W > 3 && cs[k] < 0) { p.no_face(k); continue; }
-            // A slot a cell does not use (W = 3: a cell of an open mesh with fewer faces) reads
-            // entry 0 with zero length, the cell itself as its neighbour and r = 0, which adds
-            // nothing, in place of a branch per face.
-            const bool on = W > 3 || cs[k] >= 0;
-            int e = on ? cs[k] >> 1 : 0;
-            const bool isL = (cs[k] & 1) == 0;
-            if constexpr (kChecked)    // a bad index is replaced by entry 0 / tile cell 0 (no branch)
-                e = index_ok(e < nfl, a.err) ? e : 0;
-            FaceGeo<T> g;
-            lds_geo4(sGeo, nfl, e, g);
-            int nbl = isL ? meta_lb(sMeta[e]) : meta_la(sMeta[e]);
-            if constexpr (kChecked)
-                nbl = index_ok(!on || local_ok(nbl, nb, a.B, si.nh), a.err) ? nbl : 0;
-            T un[4];
-            lds_cell(sU, NL, on ? nbl : c, un);
-            // this cell's own centre-to-face vector: one pair, at its side's plane
-            const auto rr = ldp(sGeo, nfl, isL ? 2 : 3, e);
-            p.face(k, un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, on ? rr.x : T(0), on ? rr.y : T(0), s.time_mode);
-        }
+        tile_faces<T, W>(p, a, sU, sGeo, sMeta, cs, NL, nfl, nb, si.nh, c);
         T out[8], phis[4];
         if (lmode == LIM_FROZEN) ld_cell(s.phiF, a.ps, base + c, phis);
         p.finish(iv, s.limiter, s.venkat_K, lmode, phis, out);
@@ -707,7 +759,9 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
     // twice, so that no warp runs both paths one after the other); this saves FP64 work.  In
     // FP32 every warp takes the two-entry path: the flux is cheap there, and measured on the
     // B200 the split costs more than it saves.
-    T* sGeoW = reinterpret_cast<T*>(st + L.geo);
+    // The fluxes go over the r pairs of the staged records, which only the entry's own thread
+    // reads in pass 2, and has read by then.
+    T* sF = reinterpret_cast<T*>(st + L.geo) + 2 * rplane(a.rec) * nf;
     for (int e = threadIdx.x; e < nf; e += 2 * NT) {
         const int base2 = e - (int) threadIdx.x;                 // first entry of this round
         const int pairs = min(NT, max(0, nf - base2 - NT));      // threads with a second entry
@@ -721,8 +775,8 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
             T FA[4], FB[4];
             A.flux(s.gma, FA);
             Bq.flux(s.gma, FB);
-            A.template store<COMP>(sGeoW, nf, a.rec, FA);
-            if (eB != e) Bq.template store<COMP>(sGeoW, nf, a.rec, FB);
+            A.template store<COMP>(sF, nf, FA);
+            if (eB != e) Bq.template store<COMP>(sF, nf, FB);
         } else {
             if constexpr (kChecked)
                 if (!entry_ok(sMeta[e], nb, a.B, si.nh, a.err)) continue;
@@ -730,7 +784,7 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
             A.load(sU, sG, NL, sGeo, sMeta, nf, a.rec, e);
             T FA[4];
             A.flux(s.gma, FA);
-            A.template store<COMP>(sGeoW, nf, a.rec, FA);
+            A.template store<COMP>(sF, nf, FA);
         }
     }
     compute_sync(NT);
@@ -745,50 +799,11 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
         T u[4];
         lds_cell(sU, NL, c, u);
         const T iv = sIv[c];
-        T R[4], Rc[4];
-#pragma unroll
-        for (int v = 0; v < 4; v++) { R[v] = T(0); Rc[v] = T(0); }
-        T cu = T(0), cv = T(0), ca = T(0), lam = T(0);
-        if (s.time_mode == TM_LOCAL) cell_speed(u, s.gma, cu, cv, ca);
-#pragma unroll
-        for (int k = 0; k < W; k++) {
-            if (cs[k] < 0) continue;
-            const bool isL = (cs[k] & 1) == 0;
-            int e = cs[k] >> 1;
-            if constexpr (kChecked)
-                e = index_ok(e < nf, a.err) ? e : 0;
-            const int rp = rplane(a.rec);
-            const auto F01 = ldp(sGeo, nf, rp, e), F23 = ldp(sGeo, nf, rp + 1, e);
-            const T Fk[4] = {F01.x, F01.y, F23.x, F23.y};
-            T Af = T(0);
-            if constexpr (!COMP) Af = lds_area(sGeo, nf, e, a.rec);
-#pragma unroll
-            for (int v = 0; v < 4; v++) {                        // Flux.cpp:39-42
-                const T Fv = Fk[v];
-                if constexpr (COMP) {                            // Fv holds A_f F here
-                    two_sum(R[v], Rc[v], isL ? -Fv : Fv);
-                } else {
-                    R[v] += (isL ? -Af : Af) * Fv;
-                }
-            }
-            if (s.time_mode == TM_LOCAL) {                       // the normal only for the local dt
-                FaceGeo<T> g;
-                lds_geo3(sGeo, nf, e, a.rec, g.nx, g.ny, g.Af);
-                lam += wave(cu, cv, ca, g.nx, g.ny, g.Af);
-            }
-        }
-        T dt;
-        if (s.time_mode == TM_LOCAL) dt = cfl_or_dt * qrcp(iv * lam);
-        else dt = T(dt_used);
-        T un_[4];
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-            T Rv = COMP ? R[v] + Rc[v] : R[v];
-            Rv = Rv * iv;                                        // Flux.cpp:45-49
-            un_[v] = u[v] + dt * Rv;                             // Euler.cpp:107-113
-            if (v == 0) r2 += (double) Rv * (double) Rv;
-            bad |= !isfinite(un_[v]);
-        }
+        T R[4], lam, un_[4];
+        cell_flux_sum<T, W, COMP>(cs, sF, sGeo, nf, a.rec, s.time_mode, u, s.gma, R, lam, a.err);
+        const T dt = s.time_mode == TM_LOCAL ? cfl_or_dt * qrcp(iv * lam) : T(dt_used);
+        const T Rr = cell_update(u, R, iv, dt, un_, bad);
+        r2 += (double) Rr * (double) Rr;
         st_cell(s.Unew, a.ps, base + c, un_);
         // ghost refresh (Euler.cpp:96, :138-142): this cell is its ghosts' only neighbour
 #pragma unroll
