@@ -270,7 +270,7 @@ __device__ __forceinline__ void limiter_terms(int limiter, T D, T d, T e2, T& nu
     }
 }
 
-// Limiter values of a cell's four variables: per variable the smallest face value
+// Limiter values of NVAR of a cell's variables: per variable the smallest face value
 // min(1, limiter(D1, d)) over the cell's faces with |d| > 1e-9, d = grad u . r_f and D1 the room
 // upwards (u_max - u) where d > 0, downwards (u_min - u) where d < 0 (Limiter.cpp:41-76).
 // On one side D1 is the same for every face and min(1, limiter) does not grow with |d| (for
@@ -281,14 +281,14 @@ __device__ __forceinline__ void limiter_terms(int limiter, T D, T d, T e2, T& nu
 // quotient per variable is formed, and none in a cell where every variable has num >= den (phi =
 // 1).  In FP32 the approximate quotients are cheaper than the choice.  Against a quotient per
 // face and fmin/fmax throughout: see the table of steps in the notes at tile_pass1_kernel.
-template <class T, int W>
-__device__ __forceinline__ void cell_limiter(int limiter, const T u[4], const T umin[4], const T umax[4], const T g[8],
-                                             const T ro[W][2], T e2, T phi[4]) {
+template <class T, int W, int NVAR>
+__device__ __forceinline__ void cell_limiter(int limiter, const T* u, const T* umin, const T* umax, const T* g,
+                                             const T ro[W][2], T e2, T* phi) {
     const T eps = T(1e-9);
-    T num[4], den[4];
+    T num[NVAR], den[NVAR];
     bool any = false;
 #pragma unroll
-    for (int v = 0; v < 4; v++) {
+    for (int v = 0; v < NVAR; v++) {
         T up = T(0), dn = T(0);
 #pragma unroll
         for (int k = 0; k < W; k++) {
@@ -315,30 +315,31 @@ __device__ __forceinline__ void cell_limiter(int limiter, const T u[4], const T 
     }
     if (sizeof(T) == 8 && any) {
 #pragma unroll
-        for (int v = 0; v < 4; v++) phi[v] = num[v] < den[v] ? num[v] / den[v] : T(1);
+        for (int v = 0; v < NVAR; v++) phi[v] = num[v] < den[v] ? num[v] / den[v] : T(1);
     }
 }
 
 // Pass 1 of one cell, face by face: Green-Gauss gradient, the neighbours' extremes and the
-// wave-speed sum of the CFL time step.  The tiled and the per-cell kernels differ only in where
-// the operands come from.
-template <class T, int W>
+// wave-speed sum of the CFL time step, for NVAR of the cell's variables (all four, or a pair where
+// two threads share a cell).  The kernels differ only in where the operands come from.
+template <class T, int W, int NVAR = 4>
 struct Pass1Cell {
-    T u[4], G[8], umin[4], umax[4], ro[W][2], lam, cu, cv, ca;
+    T u[NVAR], G[2 * NVAR], umin[NVAR], umax[NVAR], ro[W][2], lam, cu, cv, ca;
 
-    __device__ __forceinline__ void begin(int time_mode, T gma) {
+    // with_lam: the wave-speed sum is wanted (U: the cell's whole state)
+    __device__ __forceinline__ void begin(bool with_lam, T gma, const T U[4]) {
 #pragma unroll
-        for (int v = 0; v < 4; v++) { G[2 * v] = T(0); G[2 * v + 1] = T(0); umin[v] = u[v]; umax[v] = u[v]; }
+        for (int v = 0; v < NVAR; v++) { G[2 * v] = T(0); G[2 * v + 1] = T(0); umin[v] = u[v]; umax[v] = u[v]; }
         lam = T(0);
-        if (time_mode != TM_FIXED) cell_speed(u, gma, cu, cv, ca);
+        if (with_lam) cell_speed(U, gma, cu, cv, ca);
     }
     // GaussGreen.cpp:25-28: uf = u_CL If + u_CR (1 - If); +uf Af n into CL, -uf Af n into CR (the
     // side folded into face_weights); r is this cell's own centre-to-face vector.
-    __device__ __forceinline__ void face(int k, const T un[4], bool isL, T nx, T ny, T Af, T If, T rx, T ry, int time_mode) {
+    __device__ __forceinline__ void face(int k, const T* un, bool isL, T nx, T ny, T Af, T If, T rx, T ry, bool with_lam) {
         T ws, wn, sA;
         face_weights(isL, If, Af, ws, wn, sA);
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
+        for (int v = 0; v < NVAR; v++) {
             const T uf = u[v] * ws + un[v] * wn;
             const T t = uf * sA;
             G[2 * v] += t * nx;
@@ -348,24 +349,24 @@ struct Pass1Cell {
         }
         ro[k][0] = rx;
         ro[k][1] = ry;
-        if (time_mode != TM_FIXED) lam += wave(cu, cv, ca, nx, ny, Af);
+        if (with_lam) lam += wave(cu, cv, ca, nx, ny, Af);
     }
     __device__ __forceinline__ void no_face(int k) { ro[k][0] = T(0); ro[k][1] = T(0); }
     // Gradient (GaussGreen.cpp:33-39), limiter (or the frozen values in phis) and the limited
     // gradient in out; phis holds the limiter values used.
-    __device__ __forceinline__ void finish(T iv, int limiter, T venkat_K, int lmode, T phis[4], T out[8]) {
+    __device__ __forceinline__ void finish(T iv, int limiter, T venkat_K, int lmode, T* phis, T* out) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) G[j] *= iv;
+        for (int j = 0; j < 2 * NVAR; j++) G[j] *= iv;
         if (lmode != LIM_FROZEN) {
             T e2 = T(0);
             if (limiter == LIM_VENKAT) {
                 const T kh = venkat_K * qsqrt(qrcp(iv));
                 e2 = kh * kh * kh;
             }
-            cell_limiter<T, W>(limiter, u, umin, umax, G, ro, e2, phis);
+            cell_limiter<T, W, NVAR>(limiter, u, umin, umax, G, ro, e2, phis);
         }
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
+        for (int v = 0; v < NVAR; v++) {
             out[2 * v] = phis[v] * G[2 * v];
             out[2 * v + 1] = phis[v] * G[2 * v + 1];
         }
@@ -477,7 +478,8 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
             Pass1Cell<T, W> p;
             ld_cell(a.U, a.Nc, c, p.u);
             const T iv = __ldg(a.iv + c);
-            p.begin(a.time_mode, a.gma);
+            const bool with_lam = a.time_mode != TM_FIXED;
+            p.begin(with_lam, a.gma, p.u);
 #pragma unroll
             for (int k = 0; k < W; k++) {
                 if (s[k].y < 0) { p.no_face(k); continue; }
@@ -487,7 +489,7 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
                 ld_geo(a.geo, f, g);
                 T un[4];
                 ld_cell(a.U, a.Nc, s[k].y, un);
-                p.face(k, un, isL, g.nx, g.ny, g.Af, g.If, isL ? g.rLx : g.rRx, isL ? g.rLy : g.rRy, a.time_mode);
+                p.face(k, un, isL, g.nx, g.ny, g.Af, g.If, isL ? g.rLx : g.rRx, isL ? g.rLy : g.rRy, with_lam);
             }
             const int lmode = limiter_mode(a.stats->steps, a.freeze_after);
             T out[8], phis[4];

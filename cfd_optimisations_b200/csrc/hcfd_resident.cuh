@@ -1,27 +1,28 @@
 // Resident step kernel: whole solves of small meshes in one cooperative launch.
 //
-// A step of a mesh of up to ~120,000 cells (FP64; ~230,000 in FP32) takes the tiled kernels
-// far longer than its bytes or operations: two launches, each filling barriers, descriptors
-// and copies before its one tile per CTA and draining after it.  Here every SM holds one tile
-// in shared memory (state, limited gradients, face records, fluxes, slots) for all steps
-// of a call.  What crosses tiles goes through global memory (L2): the state and the limited
-// gradient of the cells that are in another tile's halo, and the CFL minimum; a grid barrier
-// after each of the step's two halves orders it.
+// On a mesh of up to ~140,000 cells (FP64; ~280,000 in FP32) a step of the tiled kernels is
+// two launches, each filling barriers, descriptors and copies before its few tiles per CTA and
+// draining after them, far from its bytes or operations.  Here every SM holds one tile in shared
+// memory (state, limited gradients, face records, fluxes, slots) for all steps of a call.
 //
 //   half 1: gradient, limiter, CFL of the tile's cells (Pass1Cell, as pass 1); the limited
-//           gradients stay in shared memory, those of exported cells are written out too
-//   barrier; halo gradients read
-//   half 2: flux per face entry, sum and update per cell, ghosts (FaceIn, cell_flux_sum,
-//           cell_update, as pass 2); exported cells written out
-//   barrier; halo states read
+//           gradients stay in shared memory
+//   half 2: flux per face entry, then sum and update per cell, ghosts (FaceIn, cell_flux_sum,
+//           cell_update, as pass 2)
+//
+// What crosses tiles goes through L2 as stamped words (see ll_store), with no grid barrier: the
+// state and limited gradient of the cells in another tile's halo, and under a global CFL number
+// each tile's largest iv lam.  A grid barrier (fence, counter, poll) measured 3,500-5,500 cycles
+// and the loads behind it 900-1,400; a stamped word arrives in about 1,400, and the CFL words
+// travel while the fluxes are computed.
 //
 // The arithmetic is that of the tiled kernels, function for function, so a state does not
 // depend on which of them stepped it.
 //
-// The grid must be co-resident (the host launches it cooperatively, one CTA per tile, at most
-// one per SM).  Every spin is bounded: a wait that gives up sets the error word, which every
-// other waiting CTA polls, and all of them leave; copies into shared memory in flight are
-// waited for first.
+// Tiles wait for one another, so the grid must be co-resident: the host launches it
+// cooperatively, one CTA per tile, at most one per SM.  Every wait is bounded; one that gives
+// up sets the error word, which every other wait polls, and all CTAs leave (the copies into a
+// CTA's shared memory are waited for first).
 #pragma once
 #include "hcfd_tile.cuh"
 
@@ -29,69 +30,113 @@ namespace hcfd {
 
 constexpr int kResidentThreads = 512;       // 128 registers a thread, what the two halves need in FP64
 
+// Flags per cell.
+constexpr unsigned char kCellExported = 1, kCellHasGhost = 2, kCellIsGhost = 4;
+
 struct ResidentArgs {
-    const unsigned char* __restrict__ exported;   // [ntiles * B]: the cell is in another tile's halo
-    unsigned int* bar;                            // arrivals at grid barriers, never reset while the handle works
-    unsigned int bar_base;                        // its value before this launch
-    unsigned long long* dtmin;                    // [2], both +inf between launches
+    const unsigned char* __restrict__ flags;      // [ntiles * B]
+    ulonglong2* llU;                              // exchanged states: 8 bytes a word pair, cell-major
+    ulonglong2* llG;                              // exchanged limited gradients
+    ulonglong2* llX;                              // [2][ntiles]: largest iv lam of a tile, by step parity
+    unsigned int epoch;                           // stamp of this launch's first step (later launches' are larger)
+    unsigned long long* dtmin;                    // local time stepping, profiling: +inf between whole steps
     double* partial_first;                        // [grid]: residual partials of the first step since initialise
     int nsteps;
     int phases;                                   // 3: whole steps; 1 or 2: one half of one step (profiling)
+    int refetch;                                  // fluxes overwrite the r vectors, which are fetched again each step
 };
 
-// Shared memory of one tile (all offsets multiples of 128 bytes).
+// Shared memory of one tile (all offsets multiples of 128 bytes).  With `refetch` the fluxes have
+// no room of their own (they take the r vectors' place, as in pass 2).
 template <class T>
 struct ResidentSmem {
-    size_t u, g, geo, flux, meta, cslot, iv, exported, halo, total;
-    __host__ __device__ ResidentSmem(int B, int Hmax, int Fmax, int Wp) {
+    size_t u, g, geo, flux, meta, cslot, iv, dt, flags, halo, total;
+    __host__ __device__ ResidentSmem(int B, int Hmax, int Fmax, int Wp, bool refetch) {
         size_t p = kHeader;
         u = p;        p += align128((size_t) (B + Hmax) * sizeof(Cell4<T>));
         g = p;        p += align128((size_t) (B + Hmax) * sizeof(Grad8<T>));
         geo = p;      p += align128((size_t) Fmax * sizeof(FaceGeo<T>));
-        flux = p;     p += align128((size_t) Fmax * sizeof(Cell4<T>));
+        flux = p;     p += refetch ? 0 : align128((size_t) Fmax * sizeof(Cell4<T>));
         meta = p;     p += align128((size_t) Fmax * 4);
         cslot = p;    p += align128((size_t) B * Wp * sizeof(short));
         iv = p;       p += align128((size_t) B * sizeof(T));
-        exported = p; p += align128((size_t) B);
+        dt = p;       p += align128((size_t) B * sizeof(T));          // local time steps
+        flags = p;    p += align128((size_t) B);
         halo = p;     p += align128((size_t) Hmax * sizeof(int));
         total = p;
     }
 };
 
-// Loads of values that other CTAs wrote during this kernel: from L2, never through L1.
-__device__ __forceinline__ uint4 ld_l2(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
-template <class R>   // 16-byte chunks j of record i, chunk planes of stride ps -> planes of stride NL
-__device__ __forceinline__ void halo_load(R* s, int NL, int l, const R* g, size_t ps, int i) {
-    constexpr int C = sizeof(R) / 16;
-    uint4 x[C];
-#pragma unroll
-    for (int j = 0; j < C; j++) x[j] = ld_l2(reinterpret_cast<const uint4*>(g) + j * ps + i);
-#pragma unroll
-    for (int j = 0; j < C; j++) reinterpret_cast<uint4*>(s)[j * NL + l] = x[j];
+// Stamped words: 8 bytes of payload travel as two 64-bit words, each 32 bits of payload under
+// the step's stamp.  A 64-bit access is single-copy atomic, so a word that carries the stamp
+// carries its payload: no fence, flag or barrier orders the exchange.  A slot is free for the next
+// step when its reader has answered with data of its own that depends on it: neighbours exchange
+// states and gradients in turn, and each needs the other's last answer to go on, so one buffer of
+// each is enough; the CFL words of a step are read by every tile before any tile can publish those
+// of the step after the next, so they take two.
+__device__ __forceinline__ void ll_store(ulonglong2* p, unsigned long long x, unsigned stamp) {
+    const unsigned long long st = (unsigned long long) stamp << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"((x & 0xFFFFFFFFULL) | st), "l"((x >> 32) | st)
+                 : "memory");
 }
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Arrival of thread 0 for its CTA and bounded wait for the whole grid (`target` arrivals since
-// the counter was zeroed; the counter wraps).  False when the wait gave up or another CTA set
-// the error word.  Call between two __syncthreads: the first orders the CTA's writes before the
-// arrival (with the fence), the second the other CTAs' writes before the CTA's reads.
-__device__ __forceinline__ bool grid_arrive_wait(unsigned* bar, unsigned target, unsigned polls, unsigned* err) {
-    __threadfence();
-    atomicAdd(bar, 1u);
-    bool ok = false;
+__device__ __forceinline__ bool ll_load(const ulonglong2* p, unsigned stamp, unsigned long long& x, unsigned polls,
+                                        unsigned* err) {
 #pragma unroll 1
     for (unsigned i = 0; i < polls; i++) {
-        if ((int) (ld_acquire(bar) - target) >= 0) { ok = true; break; }
-        if ((i & 63u) == 63u && *(volatile unsigned*) err) break;
+        unsigned long long a, b;
+        asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+        if ((unsigned) (a >> 32) == stamp && (unsigned) (b >> 32) == stamp) {
+            x = (a & 0xFFFFFFFFULL) | (b << 32);
+            return true;
+        }
+        if ((i & 63u) == 63u && *(volatile unsigned*) err) return false;
     }
-    if (!ok) atomicOr(err, 1u);
-    __threadfence();
+    atomicOr(err, 1u);
+    return false;
+}
+__device__ __forceinline__ unsigned long long payload(double x) { return (unsigned long long) __double_as_longlong(x); }
+__device__ __forceinline__ unsigned long long payload(float x, float y) {
+    return (unsigned long long) __float_as_uint(x) | ((unsigned long long) __float_as_uint(y) << 32);
+}
+// n values (even) from word pair k0 of a cell's record at p.
+template <int n>
+__device__ __forceinline__ void ll_values(ulonglong2* p, int k0, const double* x, unsigned stamp) {
+#pragma unroll
+    for (int i = 0; i < n; i++) ll_store(p + k0 + i, payload(x[i]), stamp);
+}
+template <int n>
+__device__ __forceinline__ void ll_values(ulonglong2* p, int k0, const float* x, unsigned stamp) {
+#pragma unroll
+    for (int i = 0; i < n / 2; i++) ll_store(p + k0 / 2 + i, payload(x[2 * i], x[2 * i + 1]), stamp);
+}
+
+// Halo records of a step into chunk planes of stride NL, from local cell B on: one thread per
+// 8 bytes.  Ghosts in the halo (ids stored complemented) are refreshed by this tile itself.
+template <class R>
+__device__ __forceinline__ bool halo_receive(R* s, int NL, int B, const ulonglong2* ll, const int* sHalo, int nh, unsigned stamp,
+                                             unsigned polls, unsigned* err) {
+    constexpr int K = sizeof(R) / 8;
+    unsigned long long* d = reinterpret_cast<unsigned long long*>(s);
+    bool ok = true;
+    for (int q = threadIdx.x; q < nh * K; q += blockDim.x) {
+        const int h = q / K, k = q % K, ci = sHalo[h];
+        if (ci < 0) continue;
+        unsigned long long x = 0;
+        if (!ll_load(ll + (size_t) ci * K + k, stamp, x, polls, err)) { ok = false; break; }
+        d[2 * ((k >> 1) * NL + B + h) + (k & 1)] = x;
+    }
     return ok;
+}
+
+// Largest of a warp's values >= 0 (their bit patterns order them).
+__device__ __forceinline__ float warp_max_pos(float x) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x)));
+}
+__device__ __forceinline__ double warp_max_pos(double x) {
+    const unsigned long long b = (unsigned long long) __double_as_longlong(x);
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned) (b >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned) (b >> 32) == hi ? (unsigned) b : 0u);
+    return __longlong_as_double((long long) (((unsigned long long) hi << 32) | lo));
 }
 
 // Block sum in a fixed order: per warp by shuffles, then the warps in order.  sm: 32 doubles.
@@ -105,20 +150,22 @@ __device__ __forceinline__ double block_sum(double x, double* sm) {
     return t;
 }
 
-// What bounds it: a chain of latencies, not bytes.  At 26,000 cells (176 a CTA) a step is two
-// barriers, two halo exchanges and two arithmetic chains of ~1,000 cycles each.  One CTA per SM,
-// since the tile takes most of an SM's shared memory at the upper end and the lower end is not
-// short of warps but of latency.
-template <class T, int W, bool COMP>
+// NVAR 2: two threads per cell, each with one pair of variables (gradient, limiter, flux sum and
+// update are independent per variable), for tiles of at most 256 cells, whose steps are a chain
+// of latencies with one or two warps per scheduler; NVAR 4: a thread per cell.
+// One CTA per SM: the tile takes most of an SM's shared memory at the upper end, and at the lower
+// end more CTAs would only add halo.
+template <class T, int W, bool COMP, int NVAR>
 __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const TileArgs<T> a, const ResidentArgs r) {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ double red[32];
+    __shared__ double red[32], red2[32], red3[32];
     __shared__ int s_bad;
     __shared__ bool s_last;
-    const ResidentSmem<T> L(a.B, a.Hmax, a.Fmax, a.Wp);
+    const bool refetch = r.refetch != 0;
+    const ResidentSmem<T> L(a.B, a.Hmax, a.Fmax, a.Wp, refetch);
     const StepArgs<T>& s = a.s;
     const int NT = blockDim.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int NL = a.B + a.Hmax;
+    const int NL = a.B + a.Hmax, Bp = (a.B + 31) & ~31;
     int base, nb, f0, nf, h0, nh, inst;
     tile_info<false>(a, (int) blockIdx.x, base, nb, f0, nf, h0, nh, inst);
     bool good = true;
@@ -131,15 +178,17 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
     Cell4<T>* sU = reinterpret_cast<Cell4<T>*>(smem + L.u);
     Grad8<T>* sG = reinterpret_cast<Grad8<T>*>(smem + L.g);
     T* sGeo = reinterpret_cast<T*>(smem + L.geo);
-    T* sF = reinterpret_cast<T*>(smem + L.flux);
+    T* sF = refetch ? sGeo + 4 * nf : reinterpret_cast<T*>(smem + L.flux);
     unsigned* sMeta = reinterpret_cast<unsigned*>(smem + L.meta);
     short* sSlot = reinterpret_cast<short*>(smem + L.cslot);
     T* sIv = reinterpret_cast<T*>(smem + L.iv);
-    unsigned char* sExp = smem + L.exported;
+    T* sDt = reinterpret_cast<T*>(smem + L.dt);
+    unsigned char* sFlag = smem + L.flags;
     int* sHalo = reinterpret_cast<int*>(smem + L.halo);
     Cell4<T>* gU = const_cast<Cell4<T>*>(s.U);
     unsigned long long* full = reinterpret_cast<unsigned long long*>(smem);
     constexpr int CU = sizeof(Cell4<T>) / 16, CG = sizeof(Grad8<T>) / 16;
+    constexpr int KU = sizeof(Cell4<T>) / 8, KG = sizeof(Grad8<T>) / 8;
 
     // the tile: bulk copies of its contiguous blocks, halo ids and halo states by the threads
     if (tid == 0) {
@@ -171,13 +220,18 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
             }
         }
     }
-    for (int c = tid; c < nb; c += NT) sExp[c] = r.exported[base + c];
+    for (int c = tid; c < nb; c += NT) sFlag[c] = r.flags[base + c];
     for (int h = tid; h < nh; h += NT) {
         int ci = __ldg(a.halo + h0 + h);
         if (!index_ok(ci >= 0 && ci < a.ps, a.err)) ci = 0;
-        sHalo[h] = ci;
-        halo_load(sU, NL, a.B + h, s.U, a.ps, ci);
-        if (r.phases == 2) halo_load(sG, NL, a.B + h, s.phiG, a.ps, ci);
+        sHalo[h] = (r.flags[ci] & kCellIsGhost) ? ~ci : ci;
+        T u[4], g[8];
+        ld_cell(s.U, a.ps, ci, u);
+        st_cell(sU, NL, a.B + h, u);
+        if (r.phases == 2) {
+            ld_grad(s.phiG, a.ps, ci, g);
+            st_grad(sG, NL, a.B + h, g);
+        }
     }
     const long long steps0 = s.stats->steps;
     __syncthreads();
@@ -187,64 +241,86 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         if (tid == 0 && (int) blockIdx.x != a.skip_tile) mbar_drain(full, 0, a.err);
         return;
     }
-
-    unsigned target = r.bar_base;
     if (r.phases == 2) {
-        // no barrier of half 1 stands between these halo reads and the other CTAs' updates
-        target += gridDim.x;
-        if (!__syncthreads_and(tid != 0 || grid_arrive_wait(r.bar, target, a.polls, a.err))) return;
+        // no exchange of half 1 stands between these halo reads and the other CTAs' updates: wait for all tiles
+        if (tid == 0) ll_store(r.llX + blockIdx.x, 0ULL, r.epoch);
+        bool ok = true;
+        unsigned long long x;
+        for (int i = tid; i < (int) gridDim.x && ok; i += NT) ok = ll_load(r.llX + i, r.epoch, x, a.polls, a.err);
+        if (!__syncthreads_and(ok)) return;
     }
+
     double r2 = 0.0, dt_used = s.dt_or_cfl;
     int bad = 0;
-    for (int step = 0; step < r.nsteps; step++) {
+    for (int step = 0;; step++) {
         const bool last_step = step + 1 == r.nsteps;
-        unsigned long long* dtmin = r.dtmin + (step & 1);
+        const unsigned stamp = r.epoch + (unsigned) step;
+        bool ok = true;
         if (r.phases & 1) {
             const int lmode = limiter_mode(steps0 + step, s.freeze_after);
             T xmx = T(0);
-            for (int c = tid; c < nb; c += NT) {
+            for (int w = tid; w < (NVAR == 4 ? nb : Bp + nb); w += NT) {
+                const int j = NVAR == 4 ? 0 : w >= Bp, c = w - j * Bp;
+                if (NVAR != 4 && c >= nb) continue;
                 short cs[8];
                 lds_slots(sSlot + c * a.Wp, a.Wp, cs);
                 if (cs[0] < 0) continue;
-                Pass1Cell<T, W> p;
-                lds_cell(sU, NL, c, p.u);
-                tile_faces<T, W>(p, a, sU, sGeo, sMeta, cs, NL, nf, nb, nh, c);
-                T out[8], phis[4];
+                const bool with_lam = s.time_mode != TM_FIXED && j == 0;
+                Pass1Cell<T, W, NVAR> p;
+                tile_faces(p, a, sU, sGeo, sMeta, cs, NL, nf, nb, nh, c, j, with_lam);
+                T out[2 * NVAR], phis[NVAR];
                 if (lmode == LIM_FROZEN) {
-                    // written by this thread's SM, perhaps in this launch: not through the read-only path
-                    const uint4* q = reinterpret_cast<const uint4*>(s.phiF);
+                    // perhaps written in this launch (by this thread): not through the read-only path
 #pragma unroll
-                    for (int j = 0; j < CU; j++) {
-                        const uint4 x = ld_l2(q + (size_t) j * a.ps + base + c);
-                        memcpy(reinterpret_cast<char*>(phis) + 16 * j, &x, 16);
+                    for (int h = 0; h < NVAR / 2; h++) {
+                        const auto x = __ldcg(pair_at(s.phiF, a.ps, base + c, j + h));
+                        phis[2 * h] = x.x; phis[2 * h + 1] = x.y;
                     }
                 }
                 const T iv = sIv[c];
                 p.finish(iv, s.limiter, s.venkat_K, lmode, phis, out);
-                if (lmode == LIM_RECORD) st_cell(s.phiF, a.ps, base + c, phis);
-                st_grad(sG, NL, c, out);
-                if (sExp[c] || r.phases == 1) st_grad(s.phiG, a.ps, base + c, out);
-                if (s.time_mode != TM_FIXED) xmx = fmax(xmx, iv * p.lam);
+#pragma unroll
+                for (int h = 0; h < NVAR / 2; h++) {
+                    if (lmode == LIM_RECORD) {
+                        auto* q = pair_at(s.phiF, a.ps, base + c, j + h);
+                        q->x = phis[2 * h]; q->y = phis[2 * h + 1];
+                    }
+                    st_grad_pair(sG, NL, c, j + h, out + 4 * h);
+                    if (r.phases == 1) st_grad_pair(s.phiG, a.ps, base + c, j + h, out + 4 * h);
+                }
+                if (sFlag[c] & kCellExported) ll_values<2 * NVAR>(r.llG + (size_t) (base + c) * KG, 4 * j, out, stamp);
+                if (with_lam) {
+                    xmx = fmax(xmx, iv * p.lam);
+                    if (s.time_mode == TM_LOCAL) sDt[c] = T(s.dt_or_cfl) * qrcp(iv * p.lam);
+                }
             }
-            if (s.time_mode != TM_FIXED) {
-                const T m = warp_max(xmx);
+            // the tile's largest iv lam: to every tile under a global CFL number; folded into one
+            // minimum for the statistics under local time stepping
+            const bool fold = r.phases == 1 ? s.time_mode != TM_FIXED : s.time_mode == TM_LOCAL && last_step;
+            if (s.time_mode == TM_GLOBAL || fold) {
+                const T m = warp_max_pos(xmx);
                 if (lane == 0) red[wid] = (double) m;
             }
             __syncthreads();
-            if (s.time_mode != TM_FIXED && wid == 0) {
-                const double m = warp_max(lane < (NT >> 5) ? red[lane] : 0.0);
-                const double d = dt_of_max(T(m));
-                if (lane == 0 && d < 1e300) atomicMin(dtmin, (unsigned long long) __double_as_longlong(d));
+            if ((s.time_mode == TM_GLOBAL || fold) && wid == 0) {
+                const double m = warp_max_pos(lane < (NT >> 5) ? red[lane] : 0.0);
+                if (lane == 0) {
+                    if (!fold) ll_store(r.llX + (size_t) (step & 1) * gridDim.x + blockIdx.x, payload(m), stamp);
+                    else if (m > 0.0) atomicMin(r.dtmin, payload(dt_of_max(T(m))));
+                }
             }
             if (r.phases == 1) return;
-            target += gridDim.x;
-            if (!__syncthreads_and(tid != 0 || grid_arrive_wait(r.bar, target, a.polls, a.err))) return;
-            // the other slot is no longer read: its readers arrived at this barrier after reading it
-            if (blockIdx.x == 0 && tid == 0) r.dtmin[(step + 1) & 1] = 0x7FF0000000000000ULL;
-            for (int h = tid; h < nh; h += NT) halo_load(sG, NL, a.B + h, s.phiG, a.ps, sHalo[h]);
+            ok = halo_receive(sG, NL, a.B, r.llG, sHalo, nh, stamp, a.polls, a.err);
+            if (!__syncthreads_and(ok)) return;
+        } else if (s.time_mode == TM_LOCAL) {        // half 2 alone: the local steps half 1 keeps
+            for (int c = tid; c < nb; c += NT) {
+                short cs[8];
+                T u[4];
+                lds_slots(sSlot + c * a.Wp, a.Wp, cs);
+                lds_cell(sU, NL, c, u);
+                if (cs[0] >= 0) sDt[c] = T(s.dt_or_cfl) * qrcp(sIv[c] * cell_wave_sum<T, W>(cs, sGeo, nf, 8, u, s.gma, a.err));
+            }
         }
-        if (s.time_mode != TM_FIXED) dt_used = s.dt_or_cfl * __longlong_as_double((long long) __ldcg(dtmin));
-        __syncthreads();
         for (int e = tid; e < nf; e += 2 * NT) {
             const int eB = (e + NT < nf) ? e + NT : e;
             if constexpr (kChecked)
@@ -264,29 +340,59 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
             }
             A.template store<COMP>(sF, nf, FA);
         }
-        __syncthreads();
+        if (s.time_mode == TM_GLOBAL && r.phases == 3) {
+            double m = 0.0;
+            for (int i = tid; i < (int) gridDim.x && ok; i += NT) {
+                unsigned long long x = 0;
+                ok = ll_load(r.llX + (size_t) (step & 1) * gridDim.x + i, stamp, x, a.polls, a.err);
+                m = greatest(m, __longlong_as_double((long long) x));
+            }
+            m = warp_max_pos(m);
+            if (lane == 0) red2[wid] = m;
+        }
+        if (!__syncthreads_and(ok)) return;
+        if (r.phases == 2) {
+            if (s.time_mode != TM_FIXED) dt_used = s.dt_or_cfl * __longlong_as_double((long long) __ldcg(r.dtmin));
+        } else if (s.time_mode == TM_GLOBAL) {
+            double m = 0.0;
+            for (int i = 0; i < (NT >> 5); i++) m = greatest(m, red2[i]);
+            dt_used = s.dt_or_cfl * (m > 0.0 ? dt_of_max(T(m)) : __longlong_as_double(0x7FF0000000000000LL));
+        }
         const bool want_r2 = last_step || steps0 + step == 0;
         r2 = 0.0;
-        for (int c = tid; c < nb; c += NT) {
+        for (int w = tid; w < (NVAR == 4 ? nb : Bp + nb); w += NT) {
+            const int j = NVAR == 4 ? 0 : w >= Bp, c = w - j * Bp;
+            if (NVAR != 4 && c >= nb) continue;
             short cs[8];
             lds_slots(sSlot + c * a.Wp, a.Wp, cs);
             if (cs[0] < 0) continue;
-            T u[4], R[4], lam, un[4];
-            lds_cell(sU, NL, c, u);
-            const T iv = sIv[c];
-            cell_flux_sum<T, W, COMP>(cs, sF, sGeo, nf, 8, s.time_mode, u, s.gma, R, lam, a.err);
-            const T dt = s.time_mode == TM_LOCAL ? T(s.dt_or_cfl) * qrcp(iv * lam) : T(dt_used);
-            const T Rr = cell_update(u, R, iv, dt, un, bad);
-            const double q = (double) Rr * (double) Rr;
-            r2 += q;
-            bad |= !isfinite(q);
-            st_cell(sU, NL, c, un);
-            if (last_step || sExp[c]) st_cell(gU, a.ps, base + c, un);
-            // ghost refresh (Euler.cpp:96, :138-142): this cell is its ghosts' only neighbour
+            T u[NVAR], R[NVAR], un[NVAR];
+            lds_vars<NVAR>(sU, NL, c, j, u);
+            cell_flux_sum<T, W, COMP, NVAR>(cs, sF, sGeo, nf, 8, j, R, a.err);
+            const T dt = s.time_mode == TM_LOCAL ? sDt[c] : T(dt_used);
+            const T Rr = cell_update<NVAR>(u, R, sIv[c], dt, un, bad);
+            if (j == 0) {
+                const double q = (double) Rr * (double) Rr;
+                if (want_r2) r2 += q;
+                bad |= !isfinite(q);
+            }
+            if (!last_step && (sFlag[c] & kCellExported)) ll_values<NVAR>(r.llU + (size_t) (base + c) * KU, 2 * j, un, stamp);
+            st_vars<NVAR>(sU, NL, c, j, un);
+            if (last_step) st_vars<NVAR>(gU, a.ps, base + c, j, un);
+        }
+        __syncthreads();
+        // ghost refresh (Euler.cpp:96, :138-142): a cell is its ghosts' only neighbour
+        for (int c = tid; c < nb; c += NT) {
+            if (!(sFlag[c] & kCellHasGhost)) continue;
+            short cs[8];
+            lds_slots(sSlot + c * a.Wp, a.Wp, cs);
+            T un[4];
+            lds_cell(sU, NL, c, un);
 #pragma unroll
             for (int k = 0; k < W; k++) {
                 if (cs[k] < 0 || (cs[k] & 1)) continue;
                 const int e = cs[k] >> 1;
+                if (!index_ok(e < nf, a.err)) continue;
                 const unsigned w = sMeta[e];
                 const int bc = meta_bc(w);
                 if (bc < 0) continue;
@@ -296,23 +402,29 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
                 lds_geo3(sGeo, nf, e, 8, gnx, gny, gA);
                 ghost_state(s.bc.type[bc], un, gnx, gny, s.gma, s.bc.UBC[bc], s.bc.QBC[bc], ug);
                 st_cell(sU, NL, lb, ug);
-                // a ghost of another tile's range is re-read with the halo
-                if (last_step || lb >= a.B) st_cell(gU, a.ps, lb < a.B ? base + lb : sHalo[lb - a.B], ug);
+                if (last_step) st_cell(gU, a.ps, lb < a.B ? base + lb : ~sHalo[lb - a.B], ug);
             }
         }
         if (want_r2) {
-            const double t = block_sum(r2, red);
+            const double t = block_sum(r2, red3);
             if (tid == 0) {
                 if (steps0 + step == 0) r.partial_first[blockIdx.x] = t;
                 if (last_step) s.partial[blockIdx.x] = t;
             }
         }
         if (last_step) break;
-        __syncthreads();
-        target += gridDim.x;
-        if (!__syncthreads_and(tid != 0 || grid_arrive_wait(r.bar, target, a.polls, a.err))) return;
-        for (int h = tid; h < nh; h += NT) halo_load(sU, NL, a.B + h, s.U, a.ps, sHalo[h]);
-        __syncthreads();
+        if (refetch && tid == 0) {
+            // the r vectors back over the fluxes, which every thread has read
+            fence_proxy_async();
+            mbar_arrive_expect_tx(full, nf * 4u * (unsigned) sizeof(T));
+            if (nf) bulk_g2s(sF, a.tgeo + (size_t) f0 * 8 + 4 * (size_t) nf, nf * 4u * (unsigned) sizeof(T), full);
+        }
+        ok = halo_receive(sU, NL, a.B, r.llU, sHalo, nh, stamp, a.polls, a.err);
+        if (refetch && !mbar_wait(full, (unsigned) (step + 1) & 1u, a.polls, a.err, abort_word(smem))) ok = false;
+        if (!__syncthreads_and(ok)) {
+            if (refetch && tid == 0) mbar_drain(full, (unsigned) (step + 1) & 1u, a.err);
+            return;
+        }
     }
 
     // statistics: the last CTA to arrive sums the partials in CTA order
@@ -331,9 +443,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         x += __ldcg(s.partial + i);
         if (steps0 == 0) y += __ldcg(r.partial_first + i);
     }
-    x = block_sum(x, red);
-    if (steps0 == 0) y = block_sum(y, red);
+    x = block_sum(x, red3);
+    if (steps0 == 0) y = block_sum(y, red3);
     if (tid == 0) {
+        if (s.time_mode == TM_LOCAL) dt_used = s.dt_or_cfl * __longlong_as_double((long long) __ldcg(r.dtmin));
         StepStats* st = s.stats;
         st->res2_last = x;
         if (steps0 == 0) st->res2_first = y;
@@ -341,7 +454,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         st->dt_last = dt_used;
         if (!(x == x) || x > 1.7e308) st->nonfinite = 1;
         *s.counter = 0u;
-        r.dtmin[0] = r.dtmin[1] = 0x7FF0000000000000ULL;
+        *r.dtmin = 0x7FF0000000000000ULL;
     }
 }
 

@@ -102,11 +102,14 @@ struct hcfd_solver {
     // early take more tiles; without, every CTA takes every grid-th tile
     bool queue1 = true, queue2 = false;
     bool tiled = false;
-    // resident steps (hcfd_resident.cuh): tp[0] holds one tile per SM; d_counter[3] counts the
-    // arrivals at its grid barriers, bar_base of them before the next launch
-    bool resident = false;
-    unsigned char* d_exported = nullptr;
-    unsigned bar_base = 0;
+    // resident steps (hcfd_resident.cuh): tp[0] holds one tile per SM; d_flags marks its cells,
+    // d_ll holds the words tiles exchange (states, gradients, CFL), epoch is the stamp of the
+    // next launch's first step
+    bool resident = false, refetch = false, pairs = false;
+    unsigned char* d_flags = nullptr;
+    ulonglong2* d_ll = nullptr;
+    size_t ll_words = 0;
+    unsigned epoch = 1;
     int cur = 0;                         // which of d_U holds the state
     int block = 256;
     int partial_len = 0;
@@ -145,7 +148,7 @@ void free_all(hcfd_solver* s) {
     for (auto e : s->ev1) cudaEventDestroy(e);
     for (auto e : s->ev2) cudaEventDestroy(e);
     void* ptrs[] = {s->d_fc, s->d_perm, s->d_slot, s->d_geo64, s->d_geoT, s->d_iv, s->d_U[0], s->d_U[1],
-                    s->d_phiG, s->d_phiF, s->d_io, s->d_cp, s->d_dtmin, s->d_partial, s->d_counter, s->d_err, s->d_stats, s->d_exported};
+                    s->d_phiG, s->d_phiF, s->d_io, s->d_cp, s->d_dtmin, s->d_partial, s->d_counter, s->d_err, s->d_stats, s->d_flags, s->d_ll};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (TiledPass& P : s->tp) {
         void* q[] = {P.d_tgeo, P.d_tmeta, P.d_foff, P.d_hoff, P.d_halo, P.d_cslot, P.d_efid};
@@ -242,22 +245,35 @@ int prof_end(hcfd_solver* s, bool rec, Ev& e, std::vector<cudaEvent_t>& into) {
     return HCFD_OK;
 }
 
+// The resident kernel of a handle's shape.
+template <class T, int W>
+const void* resident_fn(const hcfd_solver* s) {
+    constexpr bool COMP = std::is_same<T, float>::value;
+    return s->pairs ? (const void*) hcfd::resident_kernel<T, W, COMP, 2> : (const void*) hcfd::resident_kernel<T, W, COMP, 4>;
+}
+
 // nsteps steps (phases 3), or one half of one step, of the resident kernel.
 template <class T, int W>
 int launch_resident(hcfd_solver* s, int time_mode, double dt_or_cfl, int nsteps, int phases) {
+    if (s->epoch > 0xF0000000u) {            // stamps start over before they wrap
+        CK(cudaMemsetAsync(s->d_ll, 0, sizeof(ulonglong2) * s->ll_words, s->stream));
+        s->epoch = 1;
+    }
     hcfd::TileArgs<T> a = tile_args<T>(s, time_mode, dt_or_cfl, s->tp[0], 1);
     hcfd::ResidentArgs r;
-    r.exported = s->d_exported;
-    r.bar = s->d_counter + 3;
-    r.bar_base = s->bar_base;
+    r.flags = s->d_flags;
+    r.llU = s->d_ll;
+    r.llG = r.llU + (size_t) s->Nc * (sizeof(hcfd::Cell4<T>) / 8);
+    r.llX = r.llG + (size_t) s->Nc * (sizeof(hcfd::Grad8<T>) / 8);
+    r.epoch = s->epoch;
     r.dtmin = s->d_dtmin;
     r.partial_first = s->d_partial + s->partial_len;
     r.nsteps = nsteps;
     r.phases = phases;
+    r.refetch = s->refetch ? 1 : 0;
     void* args[] = {&a, &r};
-    CK(cudaLaunchCooperativeKernel((const void*) hcfd::resident_kernel<T, W, std::is_same<T, float>::value>, dim3(s->grid1),
-                                   dim3(s->tp[0].block), args, s->smem1, s->stream));
-    s->bar_base += (unsigned) s->grid1 * (phases == 3 ? 2u * (unsigned) nsteps - 1u : phases == 2 ? 1u : 0u);
+    CK(cudaLaunchCooperativeKernel(resident_fn<T, W>(s), dim3(s->grid1), dim3(s->tp[0].block), args, s->smem1, s->stream));
+    s->epoch += (unsigned) nsteps;
     return HCFD_OK;
 }
 
@@ -345,20 +361,27 @@ int setup_tiled_w(hcfd_solver* s) {
 }
 
 // Whether the resident kernel can hold this mesh, one tile of tp[0] per SM; sets its launch shape.
+// Tiles of at most 256 cells take two threads per cell; fluxes take the r vectors' place (fetched
+// again from L2 each step, behind the halo exchange) only where they have no room of their own.
 template <class T, int W>
 int setup_resident_w(hcfd_solver* s, bool* fits) {
     const hcfd::TilePlan& P = s->tp[0].plan;
-    const auto kernel = hcfd::resident_kernel<T, W, std::is_same<T, float>::value>;
+    const int Bp = (P.B + 31) / 32 * 32;
+    s->pairs = 2 * Bp <= hcfd::kResidentThreads;
+    s->tp[0].block = s->pairs ? std::min(hcfd::kResidentThreads, std::max(2 * Bp, (P.Fmax + 31) / 32 * 32))
+                              : std::min(Bp, hcfd::kResidentThreads);
+    const void* kernel = resident_fn<T, W>(s);
     *fits = false;
-    s->smem1 = hcfd::ResidentSmem<T>(P.B, P.Hmax, P.Fmax, P.Wp).total;
     int maxsm = 0;
     CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
     cudaFuncAttributes fa;
     CK(cudaFuncGetAttributes(&fa, kernel));
-    if (s->smem1 + fa.sharedSizeBytes > (size_t) maxsm) return HCFD_OK;
+    const size_t room = (size_t) maxsm - fa.sharedSizeBytes;
+    s->refetch = hcfd::ResidentSmem<T>(P.B, P.Hmax, P.Fmax, P.Wp, false).total > room;
+    s->smem1 = hcfd::ResidentSmem<T>(P.B, P.Hmax, P.Fmax, P.Wp, s->refetch).total;
+    if (s->smem1 > room) return HCFD_OK;
     // the attribute is the kernel's, shared by every handle: the largest any handle may need
-    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm - (int) fa.sharedSizeBytes));
-    s->tp[0].block = std::min((P.B + 31) / 32 * 32, hcfd::kResidentThreads);
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) room));
     int nb = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, s->tp[0].block, s->smem1));
     s->grid1 = s->grid2 = P.ntiles;
@@ -485,8 +508,8 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
         CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
         const int B = std::max(32, ((Nc + s->nsm - 1) / s->nsm + 7) / 8 * 8);
-        const size_t least = f64 ? hcfd::ResidentSmem<double>(B, 0, B * 3 / 2, s->W).total
-                                 : hcfd::ResidentSmem<float>(B, 0, B * 3 / 2, s->W).total;
+        const size_t least = f64 ? hcfd::ResidentSmem<double>(B, 0, B * 3 / 2, s->W, true).total
+                                 : hcfd::ResidentSmem<float>(B, 0, B * 3 / 2, s->W, true).total;
         if (coop && least <= (size_t) maxsm) {
             rc = hcfd::build_tile_plan(*mv, cf_off, cf_con, ghost, perm, s->F_BC, bc_first, B, s->W, s->tp[0].plan, true);
             if (rc != HCFD_OK) hcfd::clear_error();     // too scattered for one tile per SM: the tiled kernels
@@ -606,7 +629,8 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
                 return bail(rc);
             }
         }
-        if (h->resident && (rc = dalloc(&h->d_exported, niv))) {
+        h->ll_words = (size_t) Nc * (tsz / 8.0 * 12) + 2 * (size_t) h->grid1;
+        if (h->resident && ((rc = dalloc(&h->d_flags, niv)) || (rc = dalloc(&h->d_ll, h->ll_words)))) {
             free_tmp();
             return bail(rc);
         }
@@ -643,9 +667,14 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
             if (ce == cudaSuccess) ce = up(T.d_efid, P.efid.data(), 4 * P.efid.size());
         }
         if (h->resident) {
-            std::vector<unsigned char> ex(niv, 0);
-            for (int ci : h->tp[0].plan.halo) ex[ci] = 1;
-            if (ce == cudaSuccess) ce = up(h->d_exported, ex.data(), ex.size());
+            std::vector<unsigned char> fl(niv, 0);
+            for (int ci : h->tp[0].plan.halo) fl[ci] |= hcfd::kCellExported;
+            for (int f = h->F_BC; f < Nf; f++) {
+                fl[fc_int[2 * (size_t) f]] |= hcfd::kCellHasGhost;
+                fl[fc_int[2 * (size_t) f + 1]] |= hcfd::kCellIsGhost;
+            }
+            if (ce == cudaSuccess) ce = up(h->d_flags, fl.data(), fl.size());
+            if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_ll, 0, sizeof(ulonglong2) * h->ll_words, st);
         }
     } else {
         if (ce == cudaSuccess) ce = up(h->d_slot, slot.data(), sizeof(int2) * slot.size());
@@ -731,8 +760,7 @@ int hcfd_gpu_initialise(hcfd_solver* s, const double* qic) {
     if (rc) return rc;
     CK(cudaMemsetAsync(s->d_stats, 0, sizeof(hcfd::StepStats), s->stream));
     CK(cudaMemsetAsync(s->d_err, 0, sizeof(unsigned int), s->stream));
-    CK(cudaMemsetAsync(s->d_counter, 0, 4 * sizeof(unsigned int), s->stream));   // ticket, tile queues, grid barriers
-    s->bar_base = 0;
+    CK(cudaMemsetAsync(s->d_counter, 0, 4 * sizeof(unsigned int), s->stream));   // ticket, tile queues
     const unsigned long long inf2[2] = {0x7FF0000000000000ULL, 0x7FF0000000000000ULL};
     CK(cudaMemcpyAsync(s->d_dtmin, inf2, sizeof(inf2), cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));

@@ -136,6 +136,9 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
+// Orders this thread's (and, behind a barrier, its CTA's) ordinary accesses to shared memory before
+// bulk copies it issues afterwards.
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
     unsigned ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n}"
@@ -542,18 +545,15 @@ struct FaceIn {
 };
 
 // Sum of A_f F over one cell's faces in increasing face order (Flux.cpp:39-42), F as stored by
-// FaceIn::store at sF, and (local time stepping) the cell's wave-speed sum.  One face's flux
-// leaves its left cell and enters its right one.  FP32 sums are compensated; the first term
-// needs no two-sum, 0 + x being exact.
-template <class T, int W, bool COMP>
-__device__ __forceinline__ void cell_flux_sum(const short cs[8], const T* sF, const T* sGeo, int nf, int rec, int time_mode,
-                                              const T u[4], T gma, T R[4], T& lam, unsigned int* err) {
-    T Rc[4];
+// FaceIn::store at sF; one face's flux leaves its left cell and enters its right one.  NVAR 2: the
+// sums of variable pair j alone.  FP32 sums are compensated; the first term needs no two-sum,
+// 0 + x being exact.
+template <class T, int W, bool COMP, int NVAR>
+__device__ __forceinline__ void cell_flux_sum(const short cs[8], const T* sF, const T* sGeo, int nf, int rec, int j, T* R,
+                                              unsigned int* err) {
+    T Rc[NVAR];
 #pragma unroll
-    for (int v = 0; v < 4; v++) { R[v] = T(0); Rc[v] = T(0); }
-    T cu = T(0), cv = T(0), ca = T(0);
-    lam = T(0);
-    if (time_mode == TM_LOCAL) cell_speed(u, gma, cu, cv, ca);
+    for (int v = 0; v < NVAR; v++) { R[v] = T(0); Rc[v] = T(0); }
 #pragma unroll
     for (int k = 0; k < W; k++) {
         if (W > 3 && cs[k] < 0) continue;
@@ -562,11 +562,15 @@ __device__ __forceinline__ void cell_flux_sum(const short cs[8], const T* sF, co
         const bool isL = (cs[k] & 1) == 0;
         int e = on ? cs[k] >> 1 : 0;
         if constexpr (kChecked) e = index_ok(e < nf, err) ? e : 0;
-        const auto F01 = ldp(sF, nf, 0, e), F23 = ldp(sF, nf, 1, e);
-        const T Fk[4] = {F01.x, F01.y, F23.x, F23.y};
+        T Fk[NVAR];
+#pragma unroll
+        for (int h = 0; h < NVAR / 2; h++) {
+            const auto x = ldp(sF, nf, NVAR == 4 ? h : j, e);
+            Fk[2 * h] = x.x; Fk[2 * h + 1] = x.y;
+        }
         if constexpr (COMP) {
 #pragma unroll
-            for (int v = 0; v < 4; v++) {                        // Fk holds A_f F here
+            for (int v = 0; v < NVAR; v++) {                     // Fk holds A_f F here
                 const T x = !on ? T(0) : isL ? -Fk[v] : Fk[v];
                 if (k == 0) R[v] = x;
                 else two_sum(R[v], Rc[v], x);
@@ -575,24 +579,37 @@ __device__ __forceinline__ void cell_flux_sum(const short cs[8], const T* sF, co
             const T Af = lds_area(sGeo, nf, e, rec);
             const T sA = !on ? T(0) : isL ? -Af : Af;
 #pragma unroll
-            for (int v = 0; v < 4; v++) R[v] += sA * Fk[v];
-        }
-        if (time_mode == TM_LOCAL) {                             // the normal only for the local dt
-            T nx, ny, A;
-            lds_geo3(sGeo, nf, e, rec, nx, ny, A);
-            lam += wave(cu, cv, ca, nx, ny, on ? A : T(0));
+            for (int v = 0; v < NVAR; v++) R[v] += sA * Fk[v];
         }
     }
     if constexpr (COMP)
 #pragma unroll
-        for (int v = 0; v < 4; v++) R[v] += Rc[v];
+        for (int v = 0; v < NVAR; v++) R[v] += Rc[v];
+}
+
+// The wave-speed sum of a cell with state u (local time stepping in pass 2).
+template <class T, int W>
+__device__ __forceinline__ T cell_wave_sum(const short cs[8], const T* sGeo, int nf, int rec, const T u[4], T gma,
+                                           unsigned int* err) {
+    T cu, cv, ca, lam = T(0);
+    cell_speed(u, gma, cu, cv, ca);
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        if (cs[k] < 0) continue;
+        int e = cs[k] >> 1;
+        if constexpr (kChecked) e = index_ok(e < nf, err) ? e : 0;
+        T nx, ny, A;
+        lds_geo3(sGeo, nf, e, rec, nx, ny, A);
+        lam += wave(cu, cv, ca, nx, ny, A);
+    }
+    return lam;
 }
 
 // U += dt R (Flux.cpp:45-49, Euler.cpp:107-113); returns the density residual R_rho.
-template <class T>
-__device__ __forceinline__ T cell_update(const T u[4], const T R[4], T iv, T dt, T un[4], int& bad) {
+template <int NVAR, class T>
+__device__ __forceinline__ T cell_update(const T* u, const T* R, T iv, T dt, T* un, int& bad) {
 #pragma unroll
-    for (int v = 0; v < 4; v++) {
+    for (int v = 0; v < NVAR; v++) {
         un[v] = u[v] + dt * (R[v] * iv);
         bad |= !isfinite(un[v]);
     }
@@ -640,7 +657,7 @@ __device__ __forceinline__ T cell_update(const T u[4], const T R[4], T iv, T dt,
         const int t = staged ? si.t : 0;                                                         \
         const bool fin = staged && t < 0;     /* the producer has no more tiles */               \
         if (!PASS2 && fin) break;                                                                \
-        const int base = si.base, nb = si.nb, h0t = si.h0, inst = si.inst;                      \
+        const int base = si.base, nb = si.nb, inst = si.inst;                                   \
         const Cell4<T>* sU = reinterpret_cast<const Cell4<T>*>(st + L.u);                        \
         const T* sGeo = reinterpret_cast<const T*>(st + L.geo);                                  \
         const int nfl = si.nf;                                                                   \
@@ -654,12 +671,55 @@ __device__ __forceinline__ T cell_update(const T u[4], const T R[4], T iv, T dt,
     }                                                                                            \
     }
 
-// Pass 1's face loop of tile cell c (its state in p.u), operands from shared memory: nf entries,
-// nb tile cells and nh halo cells of NL staged.
-template <class T, int W>
-__device__ __forceinline__ void tile_faces(Pass1Cell<T, W>& p, const TileArgs<T>& a, const Cell4<T>* sU, const T* sGeo,
-                                           const unsigned* sMeta, const short cs[8], int NL, int nf, int nb, int nh, int c) {
-    p.begin(a.s.time_mode, a.s.gma);
+// Pair j of a cell's variables (0: rho, rho u; 1: rho v, E) in chunk planes.
+__device__ __forceinline__ double2* pair_at(Cell4<double>* p, size_t ps, int i, int j) {
+    return reinterpret_cast<double2*>(p) + j * ps + i;
+}
+__device__ __forceinline__ float2* pair_at(Cell4<float>* p, size_t, int i, int j) {
+    return reinterpret_cast<float2*>(p) + 2 * (size_t) i + j;
+}
+// Limited gradients of pair j (four values) into chunk planes.
+__device__ __forceinline__ void st_grad_pair(Grad8<double>* p, size_t ps, int i, int j, const double g[4]) {
+    double2* q = reinterpret_cast<double2*>(p) + 2 * j * ps + i;
+    q[0] = make_double2(g[0], g[1]);
+    q[ps] = make_double2(g[2], g[3]);
+}
+__device__ __forceinline__ void st_grad_pair(Grad8<float>* p, size_t ps, int i, int j, const float g[4]) {
+    reinterpret_cast<float4*>(p)[j * ps + i] = make_float4(g[0], g[1], g[2], g[3]);
+}
+template <int NVAR, class T>   // all four variables, or pair j
+__device__ __forceinline__ void st_vars(Cell4<T>* p, size_t ps, int i, int j, const T* u) {
+    if constexpr (NVAR == 4) {
+        st_cell(p, ps, i, u);
+    } else {
+        auto* q = pair_at(p, ps, i, j);
+        q->x = u[0]; q->y = u[1];
+    }
+}
+template <int NVAR, class T>
+__device__ __forceinline__ void lds_vars(const Cell4<T>* p, int ps, int i, int j, T* u) {
+    if constexpr (NVAR == 4) {
+        lds_cell(p, ps, i, u);
+    } else {
+        const auto x = *pair_at(const_cast<Cell4<T>*>(p), ps, i, j);
+        u[0] = x.x; u[1] = x.y;
+    }
+}
+
+// Pass 1's face loop of tile cell c (pair j of its variables when NVAR is 2), operands from shared
+// memory: nf entries, nb tile cells and nh halo cells of NL staged.
+template <class T, int W, int NVAR>
+__device__ __forceinline__ void tile_faces(Pass1Cell<T, W, NVAR>& p, const TileArgs<T>& a, const Cell4<T>* sU, const T* sGeo,
+                                           const unsigned* sMeta, const short cs[8], int NL, int nf, int nb, int nh, int c,
+                                           int j, bool with_lam) {
+    lds_vars<NVAR>(sU, NL, c, j, p.u);
+    if constexpr (NVAR == 4) {
+        p.begin(with_lam, a.s.gma, p.u);
+    } else {
+        T U[4];
+        if (with_lam) lds_cell(sU, NL, c, U);
+        p.begin(with_lam, a.s.gma, U);
+    }
 #pragma unroll
     for (int k = 0; k < W; k++) {
         if (W > 3 && cs[k] < 0) { p.no_face(k); continue; }
@@ -676,11 +736,11 @@ __device__ __forceinline__ void tile_faces(Pass1Cell<T, W>& p, const TileArgs<T>
         int nbl = isL ? meta_lb(sMeta[e]) : meta_la(sMeta[e]);
         if constexpr (kChecked)
             nbl = index_ok(!on || local_ok(nbl, nb, a.B, nh), a.err) ? nbl : 0;
-        T un[4];
-        lds_cell(sU, NL, on ? nbl : c, un);
+        T un[NVAR];
+        lds_vars<NVAR>(sU, NL, on ? nbl : c, j, un);
         // this cell's own centre-to-face vector: one pair, at its side's plane
         const auto rr = ldp(sGeo, nf, isL ? 2 : 3, e);
-        p.face(k, un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, on ? rr.x : T(0), on ? rr.y : T(0), a.s.time_mode);
+        p.face(k, un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, on ? rr.x : T(0), on ? rr.y : T(0), with_lam);
     }
 }
 
@@ -697,9 +757,8 @@ __global__ void __launch_bounds__(288) tile_pass1_kernel(const TileArgs<T> a) {
         lds_slots(sSlot + c * a.Wp, a.Wp, cs);
         if (cs[0] < 0) continue;
         Pass1Cell<T, W> p;
-        lds_cell(sU, NL, c, p.u);
         const T iv = sIv[c];
-        tile_faces<T, W>(p, a, sU, sGeo, sMeta, cs, NL, nfl, nb, si.nh, c);
+        tile_faces(p, a, sU, sGeo, sMeta, cs, NL, nfl, nb, si.nh, c, 0, s.time_mode != TM_FIXED);
         T out[8], phis[4];
         if (lmode == LIM_FROZEN) ld_cell(s.phiF, a.ps, base + c, phis);
         p.finish(iv, s.limiter, s.venkat_K, lmode, phis, out);
@@ -799,10 +858,12 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
         T u[4];
         lds_cell(sU, NL, c, u);
         const T iv = sIv[c];
-        T R[4], lam, un_[4];
-        cell_flux_sum<T, W, COMP>(cs, sF, sGeo, nf, a.rec, s.time_mode, u, s.gma, R, lam, a.err);
-        const T dt = s.time_mode == TM_LOCAL ? cfl_or_dt * qrcp(iv * lam) : T(dt_used);
-        const T Rr = cell_update(u, R, iv, dt, un_, bad);
+        T R[4], un_[4];
+        cell_flux_sum<T, W, COMP, 4>(cs, sF, sGeo, nf, a.rec, 0, R, a.err);
+        T dt = T(dt_used);
+        if (s.time_mode == TM_LOCAL)
+            dt = cfl_or_dt * qrcp(iv * cell_wave_sum<T, W>(cs, sGeo, nf, a.rec, u, s.gma, a.err));
+        const T Rr = cell_update<4>(u, R, iv, dt, un_, bad);
         r2 += (double) Rr * (double) Rr;
         st_cell(s.Unew, a.ps, base + c, un_);
         // ghost refresh (Euler.cpp:96, :138-142): this cell is its ghosts' only neighbour
@@ -815,7 +876,7 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
             if (bc < 0) continue;
             const int lb = meta_lb(w);
             if (!index_ok(local_ok(lb, nb, a.B, si.nh) && bc < MAXBC, a.err)) continue;
-            const int gi = lb < a.B ? base + lb : __ldg(a.halo + h0t + lb - a.B);
+            const int gi = lb < a.B ? base + lb : __ldg(a.halo + si.h0 + lb - a.B);
             if (!index_ok(gi >= 0 && gi < a.ps, a.err)) continue;
             T gnx, gny, gA;
             lds_geo3(sGeo, nf, e, a.rec, gnx, gny, gA);
