@@ -270,61 +270,24 @@ __device__ __forceinline__ void limiter_terms(int limiter, T D, T d, T e2, T& nu
     }
 }
 
-// Limiter values of NVAR of a cell's variables: per variable the smallest face value
-// min(1, limiter(D1, d)) over the cell's faces with |d| > 1e-9, d = grad u . r_f and D1 the room
-// upwards (u_max - u) where d > 0, downwards (u_min - u) where d < 0 (Limiter.cpp:41-76).
-// On one side D1 is the same for every face and min(1, limiter) does not grow with |d| (for
-// Venkatakrishnan it is below 1 only where d > D1 / 2, and falls from there), so the face with
-// the largest |d| on each side decides: two candidates per variable whatever the number of
-// faces.  In FP64, whose quotients are long dependency chains, the smaller candidate is chosen
-// by cross products (both denominators are positive; no overflow below |u| ~ 1e75), and one
-// quotient per variable is formed, and none in a cell where every variable has num >= den (phi =
-// 1).  In FP32 the approximate quotients are cheaper than the choice.  Against a quotient per
-// face and fmin/fmax throughout: see the table of steps in the notes at tile_pass1_kernel.
-template <class T, int W, int NVAR>
-__device__ __forceinline__ void cell_limiter(int limiter, const T* u, const T* umin, const T* umax, const T* g,
-                                             const T ro[W][2], T e2, T* phi) {
-    const T eps = T(1e-9);
-    T num[NVAR], den[NVAR];
-    bool any = false;
-#pragma unroll
-    for (int v = 0; v < NVAR; v++) {
-        T up = T(0), dn = T(0);
-#pragma unroll
-        for (int k = 0; k < W; k++) {
-            const T d = g[2 * v] * ro[k][0] + g[2 * v + 1] * ro[k][1];
-            up = greatest(up, d);
-            dn = least(dn, d);
-        }
-        T n1, d1, n2, d2;
-        limiter_terms(limiter, umax[v] - u[v], up, e2, n1, d1);
-        limiter_terms(limiter, u[v] - umin[v], -dn, e2, n2, d2);
-        const bool on1 = up > eps, on2 = dn < -eps;
-        if (sizeof(T) == 8) {
-            n1 = on1 ? n1 : T(1);
-            d1 = on1 ? d1 : T(1);
-            const bool second = on2 && n2 * d1 < n1 * d2;
-            num[v] = second ? n2 : n1;
-            den[v] = second ? d2 : d1;
-            any |= num[v] < den[v];
-            phi[v] = T(1);
-        } else {
-            const T q1 = qdiv(n1, d1), q2 = qdiv(n2, d2);
-            phi[v] = fmin(on1 ? fmin(T(1), q1) : T(1), on2 ? q2 : T(1));
-        }
-    }
-    if (sizeof(T) == 8 && any) {
-#pragma unroll
-        for (int v = 0; v < NVAR; v++) phi[v] = num[v] < den[v] ? num[v] / den[v] : T(1);
-    }
-}
-
-// Pass 1 of one cell, face by face: Green-Gauss gradient, the neighbours' extremes and the
-// wave-speed sum of the CFL time step, for NVAR of the cell's variables (all four, or a pair where
-// two threads share a cell).  The kernels differ only in where the operands come from.
-template <class T, int W, int NVAR = 4>
+// Pass 1 of one cell for NVAR of its variables (all four, or a pair where two threads share a
+// cell): face by face the Green-Gauss gradient, the neighbours' extremes and the wave-speed sum of
+// the CFL time step; then, with the gradient known, face by face the increments the limiter looks
+// at.  The kernels differ in where the operands come from and in unrolling.
+//
+// Limiter: per variable the smallest face value min(1, limiter(D1, d)) over the cell's faces with
+// |d| > 1e-9, d = grad u . r_f and D1 the room upwards (u_max - u) where d > 0, downwards
+// (u_min - u) where d < 0 (Limiter.cpp:41-76).  On one side D1 is the same for every face and
+// min(1, limiter) does not grow with |d| (for Venkatakrishnan it is below 1 only where d > D1 / 2,
+// and falls from there), so the face with the largest |d| on each side decides: two candidates
+// per variable whatever the number of faces.  In FP64, whose quotients are long dependency
+// chains, the smaller candidate is chosen by cross products (both denominators are positive; no
+// overflow below |u| ~ 1e75), and one quotient per variable is formed, and none in a cell where
+// every variable has num >= den (phi = 1).  In FP32 the approximate quotients are cheaper than
+// the choice.
+template <class T, int NVAR = 4>
 struct Pass1Cell {
-    T u[NVAR], G[2 * NVAR], umin[NVAR], umax[NVAR], ro[W][2], lam, cu, cv, ca;
+    T u[NVAR], G[2 * NVAR], umin[NVAR], umax[NVAR], up[NVAR], dn[NVAR], lam, cu, cv, ca;
 
     // with_lam: the wave-speed sum is wanted (U: the cell's whole state)
     __device__ __forceinline__ void begin(bool with_lam, T gma, const T U[4]) {
@@ -334,8 +297,8 @@ struct Pass1Cell {
         if (with_lam) cell_speed(U, gma, cu, cv, ca);
     }
     // GaussGreen.cpp:25-28: uf = u_CL If + u_CR (1 - If); +uf Af n into CL, -uf Af n into CR (the
-    // side folded into face_weights); r is this cell's own centre-to-face vector.
-    __device__ __forceinline__ void face(int k, const T* un, bool isL, T nx, T ny, T Af, T If, T rx, T ry, bool with_lam) {
+    // side folded into face_weights).
+    __device__ __forceinline__ void face(const T* un, bool isL, T nx, T ny, T Af, T If, bool with_lam) {
         T ws, wn, sA;
         face_weights(isL, If, Af, ws, wn, sA);
 #pragma unroll
@@ -347,23 +310,61 @@ struct Pass1Cell {
             umin[v] = least(umin[v], un[v]);                 // Limiter.cpp:31-39
             umax[v] = greatest(umax[v], un[v]);
         }
-        ro[k][0] = rx;
-        ro[k][1] = ry;
         if (with_lam) lam += wave(cu, cv, ca, nx, ny, Af);
     }
-    __device__ __forceinline__ void no_face(int k) { ro[k][0] = T(0); ro[k][1] = T(0); }
-    // Gradient (GaussGreen.cpp:33-39), limiter (or the frozen values in phis) and the limited
-    // gradient in out; phis holds the limiter values used.
-    __device__ __forceinline__ void finish(T iv, int limiter, T venkat_K, int lmode, T* phis, T* out) {
+    // The gradient (GaussGreen.cpp:33-39), once all faces are in.
+    __device__ __forceinline__ void gradient(T iv) {
 #pragma unroll
         for (int j = 0; j < 2 * NVAR; j++) G[j] *= iv;
+#pragma unroll
+        for (int v = 0; v < NVAR; v++) up[v] = dn[v] = T(0);
+    }
+    // The increments at one face, r this cell's own centre-to-face vector.
+    __device__ __forceinline__ void increment(T rx, T ry) {
+#pragma unroll
+        for (int v = 0; v < NVAR; v++) {
+            const T d = G[2 * v] * rx + G[2 * v + 1] * ry;
+            up[v] = greatest(up[v], d);
+            dn[v] = least(dn[v], d);
+        }
+    }
+    __device__ __forceinline__ void limit(int limiter, T e2, T* phi) const {
+        const T eps = T(1e-9);
+        T num[NVAR], den[NVAR];
+        bool any = false;
+#pragma unroll
+        for (int v = 0; v < NVAR; v++) {
+            T n1, d1, n2, d2;
+            limiter_terms(limiter, umax[v] - u[v], up[v], e2, n1, d1);
+            limiter_terms(limiter, u[v] - umin[v], -dn[v], e2, n2, d2);
+            const bool on1 = up[v] > eps, on2 = dn[v] < -eps;
+            if (sizeof(T) == 8) {
+                n1 = on1 ? n1 : T(1);
+                d1 = on1 ? d1 : T(1);
+                const bool second = on2 && n2 * d1 < n1 * d2;
+                num[v] = second ? n2 : n1;
+                den[v] = second ? d2 : d1;
+                any |= num[v] < den[v];
+                phi[v] = T(1);
+            } else {
+                const T q1 = qdiv(n1, d1), q2 = qdiv(n2, d2);
+                phi[v] = fmin(on1 ? fmin(T(1), q1) : T(1), on2 ? q2 : T(1));
+            }
+        }
+        if (sizeof(T) == 8 && any) {
+#pragma unroll
+            for (int v = 0; v < NVAR; v++) phi[v] = num[v] < den[v] ? num[v] / den[v] : T(1);
+        }
+    }
+    // The limited gradient in out; phis holds the limiter values used (given when frozen).
+    __device__ __forceinline__ void finish(T iv, int limiter, T venkat_K, int lmode, T* phis, T* out) const {
         if (lmode != LIM_FROZEN) {
             T e2 = T(0);
             if (limiter == LIM_VENKAT) {
                 const T kh = venkat_K * qsqrt(qrcp(iv));
                 e2 = kh * kh * kh;
             }
-            cell_limiter<T, W, NVAR>(limiter, u, umin, umax, G, ro, e2, phis);
+            limit(limiter, e2, phis);
         }
 #pragma unroll
         for (int v = 0; v < NVAR; v++) {
@@ -475,22 +476,29 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
 #pragma unroll
         for (int k = 0; k < W; k++) s[k] = __ldg(a.slot + (size_t) k * a.Nc + c);
         if (s[0].y >= 0) {
-            Pass1Cell<T, W> p;
+            Pass1Cell<T> p;
+            T ro[W][2];
             ld_cell(a.U, a.Nc, c, p.u);
             const T iv = __ldg(a.iv + c);
             const bool with_lam = a.time_mode != TM_FIXED;
             p.begin(with_lam, a.gma, p.u);
 #pragma unroll
             for (int k = 0; k < W; k++) {
-                if (s[k].y < 0) { p.no_face(k); continue; }
+                ro[k][0] = T(0); ro[k][1] = T(0);
+                if (s[k].y < 0) continue;
                 const bool isL = s[k].x >= 0;
                 const int f = isL ? s[k].x : ~s[k].x;
                 FaceGeo<T> g;
                 ld_geo(a.geo, f, g);
                 T un[4];
                 ld_cell(a.U, a.Nc, s[k].y, un);
-                p.face(k, un, isL, g.nx, g.ny, g.Af, g.If, isL ? g.rLx : g.rRx, isL ? g.rLy : g.rRy, with_lam);
+                p.face(un, isL, g.nx, g.ny, g.Af, g.If, with_lam);
+                ro[k][0] = isL ? g.rLx : g.rRx;
+                ro[k][1] = isL ? g.rLy : g.rRy;
             }
+            p.gradient(iv);
+#pragma unroll
+            for (int k = 0; k < W; k++) p.increment(ro[k][0], ro[k][1]);
             const int lmode = limiter_mode(a.stats->steps, a.freeze_after);
             T out[8], phis[4];
             if (lmode == LIM_FROZEN) ld_cell(a.phiF, a.Nc, c, phis);

@@ -50,7 +50,7 @@ struct ResidentArgs {
 // no room of their own (they take the r vectors' place, as in pass 2).
 template <class T>
 struct ResidentSmem {
-    size_t u, g, geo, flux, meta, cslot, iv, dt, flags, halo, total;
+    size_t u, g, geo, flux, meta, nbr, iv, dt, flags, halo, total;
     __host__ __device__ ResidentSmem(int B, int Hmax, int Fmax, int Wp, bool refetch) {
         size_t p = kHeader;
         u = p;        p += align128((size_t) (B + Hmax) * sizeof(Cell4<T>));
@@ -58,7 +58,7 @@ struct ResidentSmem {
         geo = p;      p += align128((size_t) Fmax * sizeof(FaceGeo<T>));
         flux = p;     p += refetch ? 0 : align128((size_t) Fmax * sizeof(Cell4<T>));
         meta = p;     p += align128((size_t) Fmax * 4);
-        cslot = p;    p += align128((size_t) B * Wp * sizeof(short));
+        nbr = p;      p += align128((size_t) ((B + 31) & ~31) * Wp * sizeof(unsigned));
         iv = p;       p += align128((size_t) B * sizeof(T));
         dt = p;       p += align128((size_t) B * sizeof(T));          // local time steps
         flags = p;    p += align128((size_t) B);
@@ -139,6 +139,51 @@ __device__ __forceinline__ double warp_max_pos(double x) {
     return __longlong_as_double((long long) (((unsigned long long) hi << 32) | lo));
 }
 
+// Smallest of a warp's values >= 0.
+__device__ __forceinline__ double warp_min_pos(double x) {
+    const unsigned long long b = (unsigned long long) __double_as_longlong(x);
+    const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned) (b >> 32));
+    const unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned) (b >> 32) == hi ? (unsigned) b : 0xffffffffu);
+    return __longlong_as_double((long long) (((unsigned long long) hi << 32) | lo));
+}
+
+// Smallest of n stamped doubles >= 0, by one warp, up to five words a lane in flight at once.
+__device__ __forceinline__ bool ll_least(const ulonglong2* p, int n, unsigned stamp, double& least_out, unsigned polls,
+                                         unsigned* err) {
+    constexpr int U = 5;
+    const int lane = threadIdx.x & 31;
+    double m = __longlong_as_double(0x7FF0000000000000LL);
+    bool ok = true;
+    for (int i0 = 0; i0 < n && ok; i0 += 32 * U) {
+        unsigned i = 0;
+        for (bool all = false; !all; i++) {
+            unsigned long long a[U], b[U];
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                const int at = i0 + 32 * k + lane;
+                a[k] = b[k] = (unsigned long long) stamp << 32 | 0x7FF00000u;
+                if (at < n)
+                    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a[k]), "=l"(b[k]) : "l"(p + at) : "memory");
+                else
+                    a[k] = (unsigned long long) stamp << 32;
+            }
+            all = true;
+            double t = m;
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                all = all && (unsigned) (a[k] >> 32) == stamp && (unsigned) (b[k] >> 32) == stamp;
+                t = least(t, __longlong_as_double((long long) ((a[k] & 0xFFFFFFFFULL) | (b[k] << 32))));
+            }
+            all = __all_sync(0xffffffffu, all);
+            if (all) m = t;
+            else if (i >= polls || ((i & 63u) == 63u && __any_sync(0xffffffffu, *(volatile unsigned*) err))) { ok = false; break; }
+        }
+    }
+    if (!ok) atomicOr(err, 1u);
+    least_out = warp_min_pos(m);
+    return ok;
+}
+
 // Block sum in a fixed order: per warp by shuffles, then the warps in order.  sm: 32 doubles.
 __device__ __forceinline__ double block_sum(double x, double* sm) {
     x = warp_sum(x);
@@ -150,6 +195,76 @@ __device__ __forceinline__ double block_sum(double x, double* sm) {
     return t;
 }
 
+// One face of a tile cell in a word: its entry (bits 0-13), the cell's side (bit 14: right), the
+// local index of the neighbour across it (bits 15-27); kNoFace for an unused slot.  It saves the
+// step loops a trip through the entry's metadata.
+constexpr unsigned kNoFace = 0xFFFFFFFFu;
+__device__ __forceinline__ int nbr_entry(unsigned w) { return (int) (w & 0x3FFFu); }
+__device__ __forceinline__ bool nbr_right(unsigned w) { return (w >> 14) & 1u; }
+__device__ __forceinline__ int nbr_local(unsigned w) { return (int) (w >> 15); }
+
+// Pass 1 of a cell up to the limiter's increments, as tile_faces, its face words at nbr (stride Bp).
+template <class T, int W, int NVAR>
+__device__ __forceinline__ void resident_faces(Pass1Cell<T, NVAR>& p, const Cell4<T>* sU, const T* sGeo, const unsigned* nbr,
+                                               int Bp, int NL, int nf, int c, int j, T iv) {
+    T ro[W][2];
+    unsigned x[W];
+#pragma unroll
+    for (int k = 0; k < W; k++) x[k] = nbr[k * Bp];
+    lds_vars<NVAR>(sU, NL, c, j, p.u);
+    p.begin(false, T(0), nullptr);
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        ro[k][0] = ro[k][1] = T(0);
+        if (W > 3 && x[k] == kNoFace) continue;
+        const bool on = W > 3 || x[k] != kNoFace;     // (W = 3) an unused slot adds nothing, see tile_faces
+        const int e = on ? nbr_entry(x[k]) : 0;
+        const bool isL = !nbr_right(x[k]);
+        FaceGeo<T> g;
+        lds_geo4(sGeo, nf, e, g);
+        T un[NVAR];
+        lds_vars<NVAR>(sU, NL, on ? nbr_local(x[k]) : c, j, un);
+        p.face(un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, false);
+        const auto rr = ldp(sGeo, nf, isL ? 2 : 3, e);
+        ro[k][0] = on ? rr.x : T(0);
+        ro[k][1] = on ? rr.y : T(0);
+    }
+    p.gradient(iv);
+#pragma unroll
+    for (int k = 0; k < W; k++) p.increment(ro[k][0], ro[k][1]);
+}
+
+// The cell's wave-speed sum (as Pass1Cell and cell_wave_sum form it).
+template <class T, int W>
+__device__ __forceinline__ T resident_wave_sum(const Cell4<T>* sU, const T* sGeo, const unsigned* nbr, int Bp, int NL, int nf,
+                                               int c, T gma) {
+    T u[4], cu, cv, ca, lam = T(0);
+    lds_cell(sU, NL, c, u);
+    cell_speed(u, gma, cu, cv, ca);
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        const unsigned x = nbr[k * Bp];
+        if (W > 3 && x == kNoFace) continue;
+        const bool on = W > 3 || x != kNoFace;
+        T nx, ny, A;
+        lds_geo3(sGeo, nf, on ? nbr_entry(x) : 0, 8, nx, ny, A);
+        lam += wave(cu, cv, ca, nx, ny, on ? A : T(0));
+    }
+    return lam;
+}
+
+// A_f F over a cell's faces, as cell_flux_sum.
+template <class T, int W, bool COMP, int NVAR>
+__device__ __forceinline__ void resident_flux_sum(const unsigned* nbr, int Bp, const T* sF, const T* sGeo, int nf, int j, T* R) {
+    short cs[8];
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        const unsigned x = nbr[k * Bp];
+        cs[k] = x == kNoFace ? (short) -1 : (short) ((nbr_entry(x) << 1) | (nbr_right(x) ? 1 : 0));
+    }
+    cell_flux_sum<T, W, COMP, NVAR>(cs, sF, sGeo, nf, 8, j, R, nullptr);
+}
+
 // NVAR 2: two threads per cell, each with one pair of variables (gradient, limiter, flux sum and
 // update are independent per variable), for tiles of at most 256 cells, whose steps are a chain
 // of latencies with one or two warps per scheduler; NVAR 4: a thread per cell.
@@ -158,7 +273,7 @@ __device__ __forceinline__ double block_sum(double x, double* sm) {
 template <class T, int W, bool COMP, int NVAR>
 __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const TileArgs<T> a, const ResidentArgs r) {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ double red[32], red2[32], red3[32];
+    __shared__ double red[32], red3[32], s_dt;
     __shared__ int s_bad;
     __shared__ bool s_last;
     const bool refetch = r.refetch != 0;
@@ -180,7 +295,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
     T* sGeo = reinterpret_cast<T*>(smem + L.geo);
     T* sF = refetch ? sGeo + 4 * nf : reinterpret_cast<T*>(smem + L.flux);
     unsigned* sMeta = reinterpret_cast<unsigned*>(smem + L.meta);
-    short* sSlot = reinterpret_cast<short*>(smem + L.cslot);
+    unsigned* sNbr = reinterpret_cast<unsigned*>(smem + L.nbr);
     T* sIv = reinterpret_cast<T*>(smem + L.iv);
     T* sDt = reinterpret_cast<T*>(smem + L.dt);
     unsigned char* sFlag = smem + L.flags;
@@ -199,8 +314,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         if ((int) blockIdx.x != a.skip_tile) {       // failure injection for tests: nothing armed
             const unsigned bu = nb * 16u * CU, bg = r.phases == 2 ? nb * 16u * CG : 0u;
             const unsigned bf = nf * 8u * (unsigned) sizeof(T), bm = nf * 4u;
-            const unsigned bs = good ? a.B * a.Wp * (unsigned) sizeof(short) : 0u, bi = good ? a.B * (unsigned) sizeof(T) : 0u;
-            mbar_arrive_expect_tx(full, bu + bg + bf + bm + bs + bi);
+            const unsigned bi = good ? a.B * (unsigned) sizeof(T) : 0u;
+            mbar_arrive_expect_tx(full, bu + bg + bf + bm + bi);
             if (good) {
 #pragma unroll
                 for (int j = 0; j < CU; j++)
@@ -215,7 +330,6 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
                     bulk_g2s(sGeo, a.tgeo + (size_t) f0 * 8, bf, full);
                     bulk_g2s(sMeta, a.tmeta + f0, bm, full);
                 }
-                bulk_g2s(sSlot, a.cslot + (size_t) base * a.Wp, bs, full);
                 bulk_g2s(sIv, s.iv + base, bi, full);
             }
         }
@@ -241,6 +355,23 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         if (tid == 0 && (int) blockIdx.x != a.skip_tile) mbar_drain(full, 0, a.err);
         return;
     }
+    for (int c = tid; c < nb; c += NT) {
+        short cs[8];
+        lds_slots(a.cslot + (size_t) (base + c) * a.Wp, a.Wp, cs);
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            unsigned x = kNoFace;
+            if (cs[k] >= 0) {
+                const int e = cs[k] >> 1, side = cs[k] & 1;
+                if (index_ok(e < nf, a.err)) {
+                    const int l = side ? meta_la(sMeta[e]) : meta_lb(sMeta[e]);
+                    if (index_ok(local_ok(l, nb, a.B, nh), a.err)) x = (unsigned) (e | (side << 14) | (l << 15));
+                }
+            }
+            sNbr[k * Bp + c] = x;
+        }
+    }
+    __syncthreads();
     if (r.phases == 2) {
         // no exchange of half 1 stands between these halo reads and the other CTAs' updates: wait for all tiles
         if (tid == 0) ll_store(r.llX + blockIdx.x, 0ULL, r.epoch);
@@ -250,6 +381,24 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         if (!__syncthreads_and(ok)) return;
     }
 
+    // The wave speeds of the coming step, from the state it starts with: local time steps, or the
+    // tile's largest iv lam, left per warp in `red`.  Formed behind the update of the step before,
+    // so that the tiles' words for a global CFL number travel during half 1 and the fluxes.
+    auto wave_speeds = [&]() {
+        if (s.time_mode == TM_FIXED) return;
+        T xmx = T(0);
+        for (int c = tid; c < nb; c += NT) {
+            if (sNbr[c] == kNoFace) continue;
+            const T x = sIv[c] * resident_wave_sum<T, W>(sU, sGeo, sNbr + c, Bp, NL, nf, c, s.gma);
+            xmx = fmax(xmx, x);
+            if (s.time_mode == TM_LOCAL) sDt[c] = T(s.dt_or_cfl) * qrcp(x);
+        }
+        xmx = warp_max_pos(xmx);
+        if (lane == 0) red[wid] = (double) xmx;
+    };
+    wave_speeds();
+    __syncthreads();
+
     double r2 = 0.0, dt_used = s.dt_or_cfl;
     int bad = 0;
     for (int step = 0;; step++) {
@@ -257,17 +406,25 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         const unsigned stamp = r.epoch + (unsigned) step;
         bool ok = true;
         if (r.phases & 1) {
+            // the tile's smallest step at CFL 1: to every tile under a global CFL number; folded into
+            // one minimum for the statistics under local time stepping
+            const bool fold = r.phases == 1 ? s.time_mode != TM_FIXED : s.time_mode == TM_LOCAL && last_step;
+            if ((s.time_mode == TM_GLOBAL || fold) && wid == 0) {
+                const double m = warp_max_pos(lane < (NT >> 5) ? red[lane] : 0.0);
+                const double d = m > 0.0 ? dt_of_max(T(m)) : __longlong_as_double(0x7FF0000000000000LL);
+                if (lane == 0) {
+                    if (!fold) ll_store(r.llX + (size_t) (step & 1) * gridDim.x + blockIdx.x, payload(d), stamp);
+                    else atomicMin(r.dtmin, payload(d));
+                }
+            }
             const int lmode = limiter_mode(steps0 + step, s.freeze_after);
-            T xmx = T(0);
             for (int w = tid; w < (NVAR == 4 ? nb : Bp + nb); w += NT) {
                 const int j = NVAR == 4 ? 0 : w >= Bp, c = w - j * Bp;
                 if (NVAR != 4 && c >= nb) continue;
-                short cs[8];
-                lds_slots(sSlot + c * a.Wp, a.Wp, cs);
-                if (cs[0] < 0) continue;
-                const bool with_lam = s.time_mode != TM_FIXED && j == 0;
-                Pass1Cell<T, W, NVAR> p;
-                tile_faces(p, a, sU, sGeo, sMeta, cs, NL, nf, nb, nh, c, j, with_lam);
+                if (sNbr[c] == kNoFace) continue;
+                const T iv = sIv[c];
+                Pass1Cell<T, NVAR> p;
+                resident_faces<T, W, NVAR>(p, sU, sGeo, sNbr + c, Bp, NL, nf, c, j, iv);
                 T out[2 * NVAR], phis[NVAR];
                 if (lmode == LIM_FROZEN) {
                     // perhaps written in this launch (by this thread): not through the read-only path
@@ -277,7 +434,6 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
                         phis[2 * h] = x.x; phis[2 * h + 1] = x.y;
                     }
                 }
-                const T iv = sIv[c];
                 p.finish(iv, s.limiter, s.venkat_K, lmode, phis, out);
 #pragma unroll
                 for (int h = 0; h < NVAR / 2; h++) {
@@ -288,87 +444,44 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
                     st_grad_pair(sG, NL, c, j + h, out + 4 * h);
                     if (r.phases == 1) st_grad_pair(s.phiG, a.ps, base + c, j + h, out + 4 * h);
                 }
-                if (sFlag[c] & kCellExported) ll_values<2 * NVAR>(r.llG + (size_t) (base + c) * KG, 4 * j, out, stamp);
-                if (with_lam) {
-                    xmx = fmax(xmx, iv * p.lam);
-                    if (s.time_mode == TM_LOCAL) sDt[c] = T(s.dt_or_cfl) * qrcp(iv * p.lam);
-                }
-            }
-            // the tile's largest iv lam: to every tile under a global CFL number; folded into one
-            // minimum for the statistics under local time stepping
-            const bool fold = r.phases == 1 ? s.time_mode != TM_FIXED : s.time_mode == TM_LOCAL && last_step;
-            if (s.time_mode == TM_GLOBAL || fold) {
-                const T m = warp_max_pos(xmx);
-                if (lane == 0) red[wid] = (double) m;
-            }
-            __syncthreads();
-            if ((s.time_mode == TM_GLOBAL || fold) && wid == 0) {
-                const double m = warp_max_pos(lane < (NT >> 5) ? red[lane] : 0.0);
-                if (lane == 0) {
-                    if (!fold) ll_store(r.llX + (size_t) (step & 1) * gridDim.x + blockIdx.x, payload(m), stamp);
-                    else if (m > 0.0) atomicMin(r.dtmin, payload(dt_of_max(T(m))));
-                }
+                if (r.phases == 3 && (sFlag[c] & kCellExported)) ll_values<2 * NVAR>(r.llG + (size_t) (base + c) * KG, 4 * j, out, stamp);
             }
             if (r.phases == 1) return;
+            __syncthreads();
             ok = halo_receive(sG, NL, a.B, r.llG, sHalo, nh, stamp, a.polls, a.err);
             if (!__syncthreads_and(ok)) return;
-        } else if (s.time_mode == TM_LOCAL) {        // half 2 alone: the local steps half 1 keeps
-            for (int c = tid; c < nb; c += NT) {
-                short cs[8];
-                T u[4];
-                lds_slots(sSlot + c * a.Wp, a.Wp, cs);
-                lds_cell(sU, NL, c, u);
-                if (cs[0] >= 0) sDt[c] = T(s.dt_or_cfl) * qrcp(sIv[c] * cell_wave_sum<T, W>(cs, sGeo, nf, 8, u, s.gma, a.err));
-            }
         }
-        for (int e = tid; e < nf; e += 2 * NT) {
-            const int eB = (e + NT < nf) ? e + NT : e;
+#pragma unroll 1
+        for (int e = tid; e < nf; e += NT) {
             if constexpr (kChecked)
-                if (!entry_ok(sMeta[e], nb, a.B, nh, a.err) || !entry_ok(sMeta[eB], nb, a.B, nh, a.err)) continue;
+                if (!entry_ok(sMeta[e], nb, a.B, nh, a.err)) continue;
             FaceIn<T> A;
             T FA[4];
             A.load(sU, sG, NL, sGeo, sMeta, nf, 8, e);
-            if (e - lane + NT < nf) {                // some thread of this warp has a second entry
-                FaceIn<T> Bq;
-                T FB[4];
-                Bq.load(sU, sG, NL, sGeo, sMeta, nf, 8, eB);
-                A.flux(s.gma, FA);
-                Bq.flux(s.gma, FB);
-                if (eB != e) Bq.template store<COMP>(sF, nf, FB);
-            } else {
-                A.flux(s.gma, FA);
-            }
+            A.flux(s.gma, FA);
             A.template store<COMP>(sF, nf, FA);
         }
-        if (s.time_mode == TM_GLOBAL && r.phases == 3) {
-            double m = 0.0;
-            for (int i = tid; i < (int) gridDim.x && ok; i += NT) {
-                unsigned long long x = 0;
-                ok = ll_load(r.llX + (size_t) (step & 1) * gridDim.x + i, stamp, x, a.polls, a.err);
-                m = greatest(m, __longlong_as_double((long long) x));
-            }
-            m = warp_max_pos(m);
-            if (lane == 0) red2[wid] = m;
+        // the smallest of the tiles' CFL words, by the last warp (the one with the fewest fluxes)
+        if (s.time_mode == TM_GLOBAL && r.phases == 3 && wid == (NT >> 5) - 1) {
+            double d;
+            ok = ll_least(r.llX + (size_t) (step & 1) * gridDim.x, (int) gridDim.x, stamp, d, a.polls, a.err);
+            if (lane == 0) s_dt = s.dt_or_cfl * d;
         }
         if (!__syncthreads_and(ok)) return;
         if (r.phases == 2) {
             if (s.time_mode != TM_FIXED) dt_used = s.dt_or_cfl * __longlong_as_double((long long) __ldcg(r.dtmin));
         } else if (s.time_mode == TM_GLOBAL) {
-            double m = 0.0;
-            for (int i = 0; i < (NT >> 5); i++) m = greatest(m, red2[i]);
-            dt_used = s.dt_or_cfl * (m > 0.0 ? dt_of_max(T(m)) : __longlong_as_double(0x7FF0000000000000LL));
+            dt_used = s_dt;
         }
         const bool want_r2 = last_step || steps0 + step == 0;
         r2 = 0.0;
         for (int w = tid; w < (NVAR == 4 ? nb : Bp + nb); w += NT) {
             const int j = NVAR == 4 ? 0 : w >= Bp, c = w - j * Bp;
             if (NVAR != 4 && c >= nb) continue;
-            short cs[8];
-            lds_slots(sSlot + c * a.Wp, a.Wp, cs);
-            if (cs[0] < 0) continue;
+            if (sNbr[c] == kNoFace) continue;
             T u[NVAR], R[NVAR], un[NVAR];
             lds_vars<NVAR>(sU, NL, c, j, u);
-            cell_flux_sum<T, W, COMP, NVAR>(cs, sF, sGeo, nf, 8, j, R, a.err);
+            resident_flux_sum<T, W, COMP, NVAR>(sNbr + c, Bp, sF, sGeo, nf, j, R);
             const T dt = s.time_mode == TM_LOCAL ? sDt[c] : T(dt_used);
             const T Rr = cell_update<NVAR>(u, R, sIv[c], dt, un, bad);
             if (j == 0) {
@@ -384,20 +497,14 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         // ghost refresh (Euler.cpp:96, :138-142): a cell is its ghosts' only neighbour
         for (int c = tid; c < nb; c += NT) {
             if (!(sFlag[c] & kCellHasGhost)) continue;
-            short cs[8];
-            lds_slots(sSlot + c * a.Wp, a.Wp, cs);
             T un[4];
             lds_cell(sU, NL, c, un);
-#pragma unroll
+#pragma unroll 1
             for (int k = 0; k < W; k++) {
-                if (cs[k] < 0 || (cs[k] & 1)) continue;
-                const int e = cs[k] >> 1;
-                if (!index_ok(e < nf, a.err)) continue;
-                const unsigned w = sMeta[e];
-                const int bc = meta_bc(w);
-                if (bc < 0) continue;
-                const int lb = meta_lb(w);
-                if (!index_ok(local_ok(lb, nb, a.B, nh) && bc < MAXBC, a.err)) continue;
+                const unsigned x = sNbr[k * Bp + c];
+                if (x == kNoFace || nbr_right(x)) continue;
+                const int e = nbr_entry(x), lb = nbr_local(x), bc = meta_bc(sMeta[e]);
+                if (bc < 0 || !index_ok(bc < MAXBC, a.err)) continue;
                 T gnx, gny, gA, ug[4];
                 lds_geo3(sGeo, nf, e, 8, gnx, gny, gA);
                 ghost_state(s.bc.type[bc], un, gnx, gny, s.gma, s.bc.UBC[bc], s.bc.QBC[bc], ug);
@@ -413,6 +520,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
             }
         }
         if (last_step) break;
+        wave_speeds();
         if (refetch && tid == 0) {
             // the r vectors back over the fluxes, which every thread has read
             fence_proxy_async();

@@ -102,7 +102,7 @@ struct hcfd_solver {
     // early take more tiles; without, every CTA takes every grid-th tile
     bool queue1 = true, queue2 = false;
     bool tiled = false;
-    // resident steps (hcfd_resident.cuh): tp[0] holds one tile per SM; d_flags marks its cells,
+    // resident steps (hcfd_resident.cuh; in place in d_U[0]): tp[0] holds one tile per SM; d_flags marks its cells,
     // d_ll holds the words tiles exchange (states, gradients, CFL), epoch is the stamp of the
     // next launch's first step
     bool resident = false, refetch = false, pairs = false;
@@ -265,6 +265,8 @@ int launch_resident(hcfd_solver* s, int time_mode, double dt_or_cfl, int nsteps,
     r.llU = s->d_ll;
     r.llG = r.llU + (size_t) s->Nc * (sizeof(hcfd::Cell4<T>) / 8);
     r.llX = r.llG + (size_t) s->Nc * (sizeof(hcfd::Grad8<T>) / 8);
+    // a half step leaves the gradients of all cells to the other half, where whole steps exchange theirs
+    a.s.phiG = (hcfd::Grad8<T>*) r.llG;
     r.epoch = s->epoch;
     r.dtmin = s->d_dtmin;
     r.partial_first = s->d_partial + s->partial_len;
@@ -604,8 +606,9 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
     for (const TiledPass& P : h->tp) niv = std::max(niv, (size_t) P.plan.ntiles * P.plan.B);
     if ((rc = dalloc(&h->d_fc, 2 * (size_t) Nf)) || (rc = dalloc(&h->d_perm, Nc)) ||
         (rc = dalloc(&h->d_geo64, Nf)) || (rc = dalloc((char**) &h->d_iv, tsz * niv)) ||
-        (rc = dalloc((char**) &h->d_U[0], tsz * 4 * Nc)) || (rc = dalloc((char**) &h->d_U[1], tsz * 4 * Nc)) ||
-        (rc = dalloc((char**) &h->d_phiG, tsz * 8 * Nc)) || (rc = dalloc(&h->d_io, 4 * (size_t) Nc)) ||
+        (rc = dalloc((char**) &h->d_U[0], tsz * 4 * Nc)) ||
+        (!h->resident && ((rc = dalloc((char**) &h->d_U[1], tsz * 4 * Nc)) || (rc = dalloc((char**) &h->d_phiG, tsz * 8 * Nc)))) ||
+        (rc = dalloc(&h->d_io, 4 * (size_t) Nc)) ||
         (p.freeze_limiter_after > 0 && (rc = dalloc((char**) &h->d_phiF, tsz * 4 * Nc))) ||
         (rc = dalloc(&h->d_cp, Nf)) || (rc = dalloc(&h->d_dtmin, 2)) || (rc = dalloc(&h->d_partial, 2 * (size_t) h->partial_len)) ||
         (rc = dalloc(&h->d_counter, 4)) || (rc = dalloc(&h->d_err, 1)) || (rc = dalloc(&h->d_stats, 1)) ||
@@ -707,9 +710,9 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
     if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_counter, 0, 4 * sizeof(unsigned int), st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_err, 0, sizeof(unsigned int), st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_stats, 0, sizeof(hcfd::StepStats), st);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_phiG, 0, tsz * 8 * Nc, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_U[0], 0, tsz * 4 * Nc, st);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_U[1], 0, tsz * 4 * Nc, st);
+    if (ce == cudaSuccess && !h->resident) ce = cudaMemsetAsync(h->d_phiG, 0, tsz * 8 * Nc, st);
+    if (ce == cudaSuccess && !h->resident) ce = cudaMemsetAsync(h->d_U[1], 0, tsz * 4 * Nc, st);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
     free_tmp();
     if (ce != cudaSuccess) return bail(fail(HCFD_ECUDA, std::string("gpu_create: ") + cudaGetErrorString(ce)));

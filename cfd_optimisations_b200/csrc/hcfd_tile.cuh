@@ -706,23 +706,32 @@ __device__ __forceinline__ void lds_vars(const Cell4<T>* p, int ps, int i, int j
     }
 }
 
-// Pass 1's face loop of tile cell c (pair j of its variables when NVAR is 2), operands from shared
-// memory: nf entries, nb tile cells and nh halo cells of NL staged.
-template <class T, int W, int NVAR>
-__device__ __forceinline__ void tile_faces(Pass1Cell<T, W, NVAR>& p, const TileArgs<T>& a, const Cell4<T>* sU, const T* sGeo,
-                                           const unsigned* sMeta, const short cs[8], int NL, int nf, int nb, int nh, int c,
-                                           int j, bool with_lam) {
+// Own state of tile cell c (pair j of its variables when NVAR is 2) into p.
+template <class T, int NVAR>
+__device__ __forceinline__ void tile_begin(Pass1Cell<T, NVAR>& p, const Cell4<T>* sU, int NL, int c, int j, bool with_lam, T gma) {
     lds_vars<NVAR>(sU, NL, c, j, p.u);
     if constexpr (NVAR == 4) {
-        p.begin(with_lam, a.s.gma, p.u);
+        p.begin(with_lam, gma, p.u);
     } else {
         T U[4];
         if (with_lam) lds_cell(sU, NL, c, U);
-        p.begin(with_lam, a.s.gma, U);
+        p.begin(with_lam, gma, U);
     }
+}
+
+// Pass 1 of tile cell c up to the limiter's increments, operands from shared memory: nf entries, nb
+// tile cells and nh halo cells of NL staged.  Unrolled: the face loads overlap.
+template <class T, int W>
+__device__ __forceinline__ void tile_faces(Pass1Cell<T>& p, const TileArgs<T>& a, const Cell4<T>* sU, const T* sGeo,
+                                           const unsigned* sMeta, const short cs[8], int NL, int nf, int nb, int nh, int c,
+                                           T iv) {
+    const bool with_lam = a.s.time_mode != TM_FIXED;
+    T ro[W][2];
+    tile_begin(p, sU, NL, c, 0, with_lam, a.s.gma);
 #pragma unroll
     for (int k = 0; k < W; k++) {
-        if (W > 3 && cs[k] < 0) { p.no_face(k); continue; }
+        ro[k][0] = T(0); ro[k][1] = T(0);
+        if (W > 3 && cs[k] < 0) continue;
         // A slot a cell does not use (W = 3: a cell of an open mesh with fewer faces) reads
         // entry 0 with zero length, the cell itself as its neighbour and r = 0, which adds
         // nothing, in place of a branch per face.
@@ -736,12 +745,17 @@ __device__ __forceinline__ void tile_faces(Pass1Cell<T, W, NVAR>& p, const TileA
         int nbl = isL ? meta_lb(sMeta[e]) : meta_la(sMeta[e]);
         if constexpr (kChecked)
             nbl = index_ok(!on || local_ok(nbl, nb, a.B, nh), a.err) ? nbl : 0;
-        T un[NVAR];
-        lds_vars<NVAR>(sU, NL, on ? nbl : c, j, un);
+        T un[4];
+        lds_cell(sU, NL, on ? nbl : c, un);
+        p.face(un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, with_lam);
         // this cell's own centre-to-face vector: one pair, at its side's plane
         const auto rr = ldp(sGeo, nf, isL ? 2 : 3, e);
-        p.face(k, un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, on ? rr.x : T(0), on ? rr.y : T(0), with_lam);
+        ro[k][0] = on ? rr.x : T(0);
+        ro[k][1] = on ? rr.y : T(0);
     }
+    p.gradient(iv);
+#pragma unroll
+    for (int k = 0; k < W; k++) p.increment(ro[k][0], ro[k][1]);
 }
 
 template <class T, int W, bool ARENA>
@@ -756,9 +770,9 @@ __global__ void __launch_bounds__(288) tile_pass1_kernel(const TileArgs<T> a) {
         short cs[8];
         lds_slots(sSlot + c * a.Wp, a.Wp, cs);
         if (cs[0] < 0) continue;
-        Pass1Cell<T, W> p;
+        Pass1Cell<T> p;
         const T iv = sIv[c];
-        tile_faces(p, a, sU, sGeo, sMeta, cs, NL, nfl, nb, si.nh, c, 0, s.time_mode != TM_FIXED);
+        tile_faces<T, W>(p, a, sU, sGeo, sMeta, cs, NL, nfl, nb, si.nh, c, iv);
         T out[8], phis[4];
         if (lmode == LIM_FROZEN) ld_cell(s.phiF, a.ps, base + c, phis);
         p.finish(iv, s.limiter, s.venkat_K, lmode, phis, out);
