@@ -110,15 +110,15 @@ __device__ __forceinline__ void ll_values(ulonglong2* p, int k0, const float* x,
     for (int i = 0; i < n / 2; i++) ll_store(p + k0 / 2 + i, payload(x[2 * i], x[2 * i + 1]), stamp);
 }
 
-// Halo records of a step into chunk planes of stride NL, from local cell B on: one thread per
-// 8 bytes.  Ghosts in the halo (ids stored complemented) are refreshed by this tile itself.
+// Halo records of a step into chunk planes of stride NL, from local cell B on, by threads t of n:
+// 8 bytes a thread.  Ghosts in the halo (ids stored complemented) are refreshed by this tile itself.
 template <class R>
-__device__ __forceinline__ bool halo_receive(R* s, int NL, int B, const ulonglong2* ll, const int* sHalo, int nh, unsigned stamp,
-                                             unsigned polls, unsigned* err) {
+__device__ __forceinline__ bool halo_receive(R* s, int NL, int B, const ulonglong2* ll, const int* sHalo, int nh, int t, int n,
+                                             unsigned stamp, unsigned polls, unsigned* err) {
     constexpr int K = sizeof(R) / 8;
     unsigned long long* d = reinterpret_cast<unsigned long long*>(s);
     bool ok = true;
-    for (int q = threadIdx.x; q < nh * K; q += blockDim.x) {
+    for (int q = t; q < nh * K; q += n) {
         const int h = q / K, k = q % K, ci = sHalo[h];
         if (ci < 0) continue;
         unsigned long long x = 0;
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         xmx = warp_max_pos(xmx);
         if (lane == 0) red[wid] = (double) xmx;
     };
-    wave_speeds();
+    wave_speeds();                                   // (warps without a cell leave 0)
     __syncthreads();
 
     double r2 = 0.0, dt_used = s.dt_or_cfl;
@@ -406,17 +406,6 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         const unsigned stamp = r.epoch + (unsigned) step;
         bool ok = true;
         if (r.phases & 1) {
-            // the tile's smallest step at CFL 1: to every tile under a global CFL number; folded into
-            // one minimum for the statistics under local time stepping
-            const bool fold = r.phases == 1 ? s.time_mode != TM_FIXED : s.time_mode == TM_LOCAL && last_step;
-            if ((s.time_mode == TM_GLOBAL || fold) && wid == 0) {
-                const double m = warp_max_pos(lane < (NT >> 5) ? red[lane] : 0.0);
-                const double d = m > 0.0 ? dt_of_max(T(m)) : __longlong_as_double(0x7FF0000000000000LL);
-                if (lane == 0) {
-                    if (!fold) ll_store(r.llX + (size_t) (step & 1) * gridDim.x + blockIdx.x, payload(d), stamp);
-                    else atomicMin(r.dtmin, payload(d));
-                }
-            }
             const int lmode = limiter_mode(steps0 + step, s.freeze_after);
             for (int w = tid; w < (NVAR == 4 ? nb : Bp + nb); w += NT) {
                 const int j = NVAR == 4 ? 0 : w >= Bp, c = w - j * Bp;
@@ -446,9 +435,21 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
                 }
                 if (r.phases == 3 && (sFlag[c] & kCellExported)) ll_values<2 * NVAR>(r.llG + (size_t) (base + c) * KG, 4 * j, out, stamp);
             }
-            if (r.phases == 1) return;
             __syncthreads();
-            ok = halo_receive(sG, NL, a.B, r.llG, sHalo, nh, stamp, a.polls, a.err);
+            // The last warp posts the tile's smallest step at CFL 1 (to every tile under a global CFL
+            // number; folded into one minimum for the statistics under local time stepping) while
+            // the others receive the halo's gradients.
+            const bool fold = r.phases == 1 ? s.time_mode != TM_FIXED : s.time_mode == TM_LOCAL && last_step;
+            if (wid == (NT >> 5) - 1 && (s.time_mode == TM_GLOBAL || fold)) {
+                const double m = warp_max_pos(lane < (NT >> 5) ? red[lane] : 0.0);
+                const double d = m > 0.0 ? dt_of_max(T(m)) : __longlong_as_double(0x7FF0000000000000LL);
+                if (lane == 0) {
+                    if (!fold) ll_store(r.llX + (size_t) (step & 1) * gridDim.x + blockIdx.x, payload(d), stamp);
+                    else atomicMin(r.dtmin, payload(d));
+                }
+            }
+            if (r.phases == 1) return;
+            if (tid < NT - 32) ok = halo_receive(sG, NL, a.B, r.llG, sHalo, nh, tid, NT - 32, stamp, a.polls, a.err);
             if (!__syncthreads_and(ok)) return;
         }
 #pragma unroll 1
@@ -485,9 +486,12 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
             const T dt = s.time_mode == TM_LOCAL ? sDt[c] : T(dt_used);
             const T Rr = cell_update<NVAR>(u, R, sIv[c], dt, un, bad);
             if (j == 0) {
-                const double q = (double) Rr * (double) Rr;
-                if (want_r2) r2 += q;
-                bad |= !isfinite(q);
+                if (sizeof(T) == 4) bad |= !isfinite(Rr);           // its square fits a double
+                if (sizeof(T) == 8 || want_r2) {
+                    const double q = (double) Rr * (double) Rr;
+                    r2 += q;
+                    bad |= !isfinite(q);
+                }
             }
             if (!last_step && (sFlag[c] & kCellExported)) ll_values<NVAR>(r.llU + (size_t) (base + c) * KU, 2 * j, un, stamp);
             st_vars<NVAR>(sU, NL, c, j, un);
@@ -520,14 +524,17 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
             }
         }
         if (last_step) break;
-        wave_speeds();
         if (refetch && tid == 0) {
             // the r vectors back over the fluxes, which every thread has read
             fence_proxy_async();
             mbar_arrive_expect_tx(full, nf * 4u * (unsigned) sizeof(T));
             if (nf) bulk_g2s(sF, a.tgeo + (size_t) f0 * 8 + 4 * (size_t) nf, nf * 4u * (unsigned) sizeof(T), full);
         }
-        ok = halo_receive(sU, NL, a.B, r.llU, sHalo, nh, stamp, a.polls, a.err);
+        // the halo's states by the second half of the threads while the first forms the wave speeds
+        // (two threads a cell), or by all behind it
+        if (NVAR == 4 || tid < Bp) wave_speeds();
+        if (NVAR == 4) ok = halo_receive(sU, NL, a.B, r.llU, sHalo, nh, tid, NT, stamp, a.polls, a.err);
+        else if (tid >= Bp) ok = halo_receive(sU, NL, a.B, r.llU, sHalo, nh, tid - Bp, NT - Bp, stamp, a.polls, a.err);
         if (refetch && !mbar_wait(full, (unsigned) (step + 1) & 1u, a.polls, a.err, abort_word(smem))) ok = false;
         if (!__syncthreads_and(ok)) {
             if (refetch && tid == 0) mbar_drain(full, (unsigned) (step + 1) & 1u, a.err);

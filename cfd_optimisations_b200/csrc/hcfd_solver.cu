@@ -371,7 +371,7 @@ int setup_resident_w(hcfd_solver* s, bool* fits) {
     const int Bp = (P.B + 31) / 32 * 32;
     s->pairs = 2 * Bp <= hcfd::kResidentThreads;
     s->tp[0].block = s->pairs ? std::min(hcfd::kResidentThreads, std::max(2 * Bp, (P.Fmax + 31) / 32 * 32))
-                              : std::min(Bp, hcfd::kResidentThreads);
+                              : std::min(std::max(Bp, 64), hcfd::kResidentThreads);
     const void* kernel = resident_fn<T, W>(s);
     *fits = false;
     int maxsm = 0;
