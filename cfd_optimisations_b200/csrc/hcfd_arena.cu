@@ -223,7 +223,7 @@ struct hcfd_arena {
     void* phiG = nullptr;
     void* phiF = nullptr;
     void* iv = nullptr;
-    short* cslot = nullptr;
+    unsigned* nbr = nullptr;                // pack_nbr words
     void* tgeo = nullptr;
     unsigned* tmeta = nullptr;              // pack_meta words
     int* halo = nullptr;
@@ -304,7 +304,7 @@ hcfd::TileArgs<T> arena_args(hcfd_arena* A, int cur, int par) {
     a.rec = 8;                             // one plan serves both passes: pass 1 reads If
     a.tmeta = A->tmeta;
     a.halo = A->halo;
-    a.cslot = A->cslot;
+    a.nbr = A->nbr;
     a.ntiles = A->nact_tiles;
     a.B = A->B;
     a.Wp = A->Wp;
@@ -330,16 +330,15 @@ hcfd::TileArgs<T> arena_args(hcfd_arena* A, int cur, int par) {
 template <class T, int W>
 int enqueue_step(hcfd_arena* A, int cur, int par) {
     hcfd::TileArgs<T> a = arena_args<T>(A, cur, par);
-    constexpr bool COMP = std::is_same<T, float>::value;
     // pass 1 takes its tiles from a queue (per-instance dt minima are order-free), and pass 2,
     // which runs between two pass-1 launches, zeroes it; pass 2 takes every grid-th tile
     // (measured faster for it than a queue)
     a.claim = A->queue;
     a.claim_reset = nullptr;
-    hcfd::tile_pass1_kernel<T, W, true><<<A->grid1, A->B + 32, A->smem1, A->stream>>>(a);
+    hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->time_mode)<<<A->grid1, A->B + 32, A->smem1, A->stream>>>(a);
     a.claim = nullptr;
     a.claim_reset = A->queue;
-    hcfd::tile_pass2_kernel<T, W, COMP, true><<<A->grid2, A->B + 32, A->smem2, A->stream>>>(a);
+    hcfd::pass2_variant<T, W, true>(8, A->time_mode)<<<A->grid2, A->B + 32, A->smem2, A->stream>>>(a);
     arena_chunk_kernel<<<A->nchunks, 256, 0, A->stream>>>(A->chunks, A->tile_r2, A->tile_bad, A->chunk_r2, A->chunk_bad);
     arena_finalize_kernel<<<(A->nact + 127) / 128, 128, 0, A->stream>>>(A->nact, A->nchunks, A->act, A->chunk_r2,
                                                                        A->chunk_bad, A->inst_dt, A->inst_dtmin, A->stats,
@@ -355,7 +354,6 @@ int enqueue_step_w(hcfd_arena* A, int cur, int par) {
 
 template <class T, int W>
 int setup_kernels(hcfd_arena* A) {
-    constexpr bool COMP = std::is_same<T, float>::value;
     // the attributes allow the largest staging the arena admits; launches size the shared
     // memory to the active instances (configure_kernels)
     const size_t s1 = hcfd::TileSmem<T>(A->B, A->Hcap, A->Fcap, W, A->Wp, false).total;
@@ -363,8 +361,13 @@ int setup_kernels(hcfd_arena* A) {
     int maxsm = 0;
     CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, A->device));
     if ((int) s2 > maxsm || (int) s1 > maxsm) return fail(HCFD_EINVAL, "arena: tile does not fit in shared memory");
-    CK(cudaFuncSetAttribute(hcfd::tile_pass1_kernel<T, W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) s1));
-    CK(cudaFuncSetAttribute(hcfd::tile_pass2_kernel<T, W, COMP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) s2));
+    // all a block may have: the attribute belongs to the kernel, which arenas of other tile sizes share
+    for (const void* k : {(const void*) hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->time_mode),
+                          (const void*) hcfd::pass2_variant<T, W, true>(8, A->time_mode)}) {
+        cudaFuncAttributes fa;
+        CK(cudaFuncGetAttributes(&fa, k));
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm - (int) fa.sharedSizeBytes));
+    }
     return HCFD_OK;
 }
 
@@ -373,12 +376,11 @@ int setup_kernels(hcfd_arena* A) {
 // an SM.
 template <class T, int W>
 int configure_kernels(hcfd_arena* A) {
-    constexpr bool COMP = std::is_same<T, float>::value;
     A->smem1 = hcfd::TileSmem<T>(A->B, A->Hcur, A->Fcur, W, A->Wp, false).total;
     A->smem2 = hcfd::TileSmem<T>(A->B, A->Hcur, A->Fcur, W, A->Wp, true).total;
     int b1 = 0, b2 = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, hcfd::tile_pass1_kernel<T, W, true>, A->B + 32, A->smem1));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, hcfd::tile_pass2_kernel<T, W, COMP, true>, A->B + 32, A->smem2));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->time_mode), A->B + 32, A->smem1));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, hcfd::pass2_variant<T, W, true>(8, A->time_mode), A->B + 32, A->smem2));
     if (b1 < 1 || b2 < 1) return fail(HCFD_EINVAL, "arena: kernels cannot be resident");
     A->grid1 = b1 * A->nsm;
     A->grid2 = b2 * A->nsm;
@@ -454,7 +456,7 @@ void arena_free(hcfd_arena* A) {
     if (A->admit_ev) cudaEventDestroy(A->admit_ev);
     if (A->list_ev) cudaEventDestroy(A->list_ev);
     if (A->astream) cudaStreamDestroy(A->astream);
-    void* p[] = {A->U[0], A->U[1], A->phiG, A->phiF, A->iv, A->cslot, A->tgeo, A->tmeta, A->halo, A->inst_dt, A->inst_dtmin,
+    void* p[] = {A->U[0], A->U[1], A->phiG, A->phiF, A->iv, A->nbr, A->tgeo, A->tmeta, A->halo, A->inst_dt, A->inst_dtmin,
                  A->inst_bc, A->stats, A->tiles, A->act, A->tile_r2, A->tile_bad, A->err, A->queue, A->chunks,
                  A->chunk_r2, A->chunk_bad};
     for (void* q : p) if (q) cudaFree(q);
@@ -499,7 +501,7 @@ int hcfd_arena_create(const hcfd_arena_params* prm, hcfd_arena** out) {
     const size_t ts = A->tsz;
     // Budget split, bytes per cell: state x2, gradients, iv, slots; ~1.75 face entries per
     // cell (records + metadata) and ~0.6 halo ids per cell, as the wedge meshes need.
-    const double per_cell = 2 * 4 * ts + 8 * ts + ts + A->Wp * 2 + 1.75 * (8 * ts + 8) + 0.6 * 4 +
+    const double per_cell = 2 * 4 * ts + 8 * ts + ts + A->Wp * 4 + 1.75 * (8 * ts + 4) + 0.6 * 4 +
                             (p.freeze_limiter_after > 0 ? 4 * ts : 0);
     size_t budget = p.hbm_budget;
     size_t C = (size_t) (budget / per_cell);
@@ -525,7 +527,7 @@ int hcfd_arena_create(const hcfd_arena_params* prm, hcfd_arena** out) {
     if ((rc = dalloc((char**) &h->U[0], 4 * ts * C)) || (rc = dalloc((char**) &h->U[1], 4 * ts * C)) ||
         (rc = dalloc((char**) &h->phiG, 8 * ts * C)) || (rc = dalloc((char**) &h->iv, ts * C)) ||
         (p.freeze_limiter_after > 0 && (rc = dalloc((char**) &h->phiF, 4 * ts * C))) ||
-        (rc = dalloc(&h->cslot, h->Wp * C)) || (rc = dalloc((char**) &h->tgeo, 8 * ts * h->Ecap)) ||
+        (rc = dalloc(&h->nbr, h->Wp * C)) || (rc = dalloc((char**) &h->tgeo, 8 * ts * h->Ecap)) ||
         (rc = dalloc(&h->tmeta, h->Ecap)) || (rc = dalloc(&h->halo, h->HLcap)) ||
         (rc = dalloc(&h->inst_dt, p.max_instances)) || (rc = dalloc(&h->inst_dtmin, 2 * (size_t) p.max_instances)) ||
         (rc = dalloc(&h->inst_bc, p.max_instances)) || (rc = dalloc(&h->stats, p.max_instances)) ||
@@ -687,9 +689,9 @@ int hcfd_arena_admit_prepared(hcfd_arena* A, const hcfd_admission* D, int* slot_
     up(d_halo, P.halo.data(), 4 * I.nh);
     up(d_nodes, mv->nodes, 16 * (size_t) mv->Nn);
     up(I.d_perm, D->perm.data(), 4 * (size_t) Nc);
-    const std::vector<unsigned> mw = hcfd::packed_meta(P);
+    const std::vector<unsigned> mw = hcfd::packed_meta(P), nw = hcfd::packed_nbr(P);
     up(A->tmeta + I.e0, mw.data(), 4 * mw.size());
-    up(A->cslot + A->Wp * I.c0, P.cslot.data(), 2 * P.cslot.size());
+    up(A->nbr + A->Wp * I.c0, nw.data(), 4 * nw.size());
     if (ce == cudaSuccess) {
         arena_cellmap_kernel<<<nblk(2 * (long long) Nf, 256), 256, 0, st>>>(2 * (long long) Nf, (int) I.c0, d_iperm, d_fcu, d_fcg);
         if (I.nh) arena_offset_kernel<<<nblk((long long) I.nh, 256), 256, 0, st>>>((long long) I.nh, (int) I.c0, d_halo, A->halo + I.h0);

@@ -328,8 +328,16 @@ struct Pass1Cell {
             dn[v] = least(dn[v], d);
         }
     }
-    __device__ __forceinline__ void limit(int limiter, T e2, T* phi) const {
+    // LIM: the limiter, when known at compile time.
+    template <int LIM = -1>
+    __device__ __forceinline__ void limiter_values(T iv, int limiter_, T venkat_K, T* phi) const {
+        const int limiter = LIM >= 0 ? LIM : limiter_;
         const T eps = T(1e-9);
+        T e2 = T(0);
+        if (limiter == LIM_VENKAT) {
+            const T kh = venkat_K * qsqrt(qrcp(iv));
+            e2 = kh * kh * kh;
+        }
         T num[NVAR], den[NVAR];
         bool any = false;
 #pragma unroll
@@ -356,20 +364,12 @@ struct Pass1Cell {
             for (int v = 0; v < NVAR; v++) phi[v] = num[v] < den[v] ? num[v] / den[v] : T(1);
         }
     }
-    // The limited gradient in out; phis holds the limiter values used (given when frozen).
-    __device__ __forceinline__ void finish(T iv, int limiter, T venkat_K, int lmode, T* phis, T* out) const {
-        if (lmode != LIM_FROZEN) {
-            T e2 = T(0);
-            if (limiter == LIM_VENKAT) {
-                const T kh = venkat_K * qsqrt(qrcp(iv));
-                e2 = kh * kh * kh;
-            }
-            limit(limiter, e2, phis);
-        }
+    // The limited gradient.
+    __device__ __forceinline__ void limited(const T* phi, T* out) const {
 #pragma unroll
         for (int v = 0; v < NVAR; v++) {
-            out[2 * v] = phis[v] * G[2 * v];
-            out[2 * v + 1] = phis[v] * G[2 * v + 1];
+            out[2 * v] = phi[v] * G[2 * v];
+            out[2 * v + 1] = phi[v] * G[2 * v + 1];
         }
     }
 };
@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
             const int lmode = limiter_mode(a.stats->steps, a.freeze_after);
             T out[8], phis[4];
             if (lmode == LIM_FROZEN) ld_cell(a.phiF, a.Nc, c, phis);
-            p.finish(iv, a.limiter, a.venkat_K, lmode, phis, out);
+            else p.limiter_values(iv, a.limiter, a.venkat_K, phis);
+            p.limited(phis, out);
             if (lmode == LIM_RECORD) st_cell(a.phiF, a.Nc, c, phis);
             st_grad(a.phiG, a.Nc, c, out);
             if (a.time_mode != TM_FIXED) xmx = iv * p.lam;

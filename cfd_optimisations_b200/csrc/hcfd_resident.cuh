@@ -58,7 +58,7 @@ struct ResidentSmem {
         geo = p;      p += align128((size_t) Fmax * sizeof(FaceGeo<T>));
         flux = p;     p += refetch ? 0 : align128((size_t) Fmax * sizeof(Cell4<T>));
         meta = p;     p += align128((size_t) Fmax * 4);
-        nbr = p;      p += align128((size_t) ((B + 31) & ~31) * Wp * sizeof(unsigned));
+        nbr = p;      p += align128((size_t) B * Wp * sizeof(unsigned));
         iv = p;       p += align128((size_t) B * sizeof(T));
         dt = p;       p += align128((size_t) B * sizeof(T));          // local time steps
         flags = p;    p += align128((size_t) B);
@@ -195,83 +195,14 @@ __device__ __forceinline__ double block_sum(double x, double* sm) {
     return t;
 }
 
-// One face of a tile cell in a word: its entry (bits 0-13), the cell's side (bit 14: right), the
-// local index of the neighbour across it (bits 15-27); kNoFace for an unused slot.  It saves the
-// step loops a trip through the entry's metadata.
-constexpr unsigned kNoFace = 0xFFFFFFFFu;
-__device__ __forceinline__ int nbr_entry(unsigned w) { return (int) (w & 0x3FFFu); }
-__device__ __forceinline__ bool nbr_right(unsigned w) { return (w >> 14) & 1u; }
-__device__ __forceinline__ int nbr_local(unsigned w) { return (int) (w >> 15); }
-
-// Pass 1 of a cell up to the limiter's increments, as tile_faces, its face words at nbr (stride Bp).
-template <class T, int W, int NVAR>
-__device__ __forceinline__ void resident_faces(Pass1Cell<T, NVAR>& p, const Cell4<T>* sU, const T* sGeo, const unsigned* nbr,
-                                               int Bp, int NL, int nf, int c, int j, T iv) {
-    T ro[W][2];
-    unsigned x[W];
-#pragma unroll
-    for (int k = 0; k < W; k++) x[k] = nbr[k * Bp];
-    lds_vars<NVAR>(sU, NL, c, j, p.u);
-    p.begin(false, T(0), nullptr);
-#pragma unroll
-    for (int k = 0; k < W; k++) {
-        ro[k][0] = ro[k][1] = T(0);
-        if (W > 3 && x[k] == kNoFace) continue;
-        const bool on = W > 3 || x[k] != kNoFace;     // (W = 3) an unused slot adds nothing, see tile_faces
-        const int e = on ? nbr_entry(x[k]) : 0;
-        const bool isL = !nbr_right(x[k]);
-        FaceGeo<T> g;
-        lds_geo4(sGeo, nf, e, g);
-        T un[NVAR];
-        lds_vars<NVAR>(sU, NL, on ? nbr_local(x[k]) : c, j, un);
-        p.face(un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, false);
-        const auto rr = ldp(sGeo, nf, isL ? 2 : 3, e);
-        ro[k][0] = on ? rr.x : T(0);
-        ro[k][1] = on ? rr.y : T(0);
-    }
-    p.gradient(iv);
-#pragma unroll
-    for (int k = 0; k < W; k++) p.increment(ro[k][0], ro[k][1]);
-}
-
-// The cell's wave-speed sum (as Pass1Cell and cell_wave_sum form it).
-template <class T, int W>
-__device__ __forceinline__ T resident_wave_sum(const Cell4<T>* sU, const T* sGeo, const unsigned* nbr, int Bp, int NL, int nf,
-                                               int c, T gma) {
-    T u[4], cu, cv, ca, lam = T(0);
-    lds_cell(sU, NL, c, u);
-    cell_speed(u, gma, cu, cv, ca);
-#pragma unroll
-    for (int k = 0; k < W; k++) {
-        const unsigned x = nbr[k * Bp];
-        if (W > 3 && x == kNoFace) continue;
-        const bool on = W > 3 || x != kNoFace;
-        T nx, ny, A;
-        lds_geo3(sGeo, nf, on ? nbr_entry(x) : 0, 8, nx, ny, A);
-        lam += wave(cu, cv, ca, nx, ny, on ? A : T(0));
-    }
-    return lam;
-}
-
-// A_f F over a cell's faces, as cell_flux_sum.
-template <class T, int W, bool COMP, int NVAR>
-__device__ __forceinline__ void resident_flux_sum(const unsigned* nbr, int Bp, const T* sF, const T* sGeo, int nf, int j, T* R) {
-    short cs[8];
-#pragma unroll
-    for (int k = 0; k < W; k++) {
-        const unsigned x = nbr[k * Bp];
-        cs[k] = x == kNoFace ? (short) -1 : (short) ((nbr_entry(x) << 1) | (nbr_right(x) ? 1 : 0));
-    }
-    cell_flux_sum<T, W, COMP, NVAR>(cs, sF, sGeo, nf, 8, j, R, nullptr);
-}
-
 // NVAR 2: two threads per cell, each with one pair of variables (gradient, limiter, flux sum and
 // update are independent per variable), for tiles of at most 256 cells, whose steps are a chain
 // of latencies with one or two warps per scheduler; NVAR 4: a thread per cell.
 // One CTA per SM: the tile takes most of an SM's shared memory at the upper end, and at the lower
 // end more CTAs would only add halo.
-template <class T, int W, bool COMP, int NVAR>
+template <class T, int W, int NVAR>
 __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const TileArgs<T> a, const ResidentArgs r) {
+    constexpr bool COMP = sizeof(T) == 4;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ double red[32], red3[32], s_dt;
     __shared__ int s_bad;
@@ -314,8 +245,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         if ((int) blockIdx.x != a.skip_tile) {       // failure injection for tests: nothing armed
             const unsigned bu = nb * 16u * CU, bg = r.phases == 2 ? nb * 16u * CG : 0u;
             const unsigned bf = nf * 8u * (unsigned) sizeof(T), bm = nf * 4u;
-            const unsigned bi = good ? a.B * (unsigned) sizeof(T) : 0u;
-            mbar_arrive_expect_tx(full, bu + bg + bf + bm + bi);
+            const unsigned bs = good ? a.B * W * 4u : 0u, bi = good ? a.B * (unsigned) sizeof(T) : 0u;
+            mbar_arrive_expect_tx(full, bu + bg + bf + bm + bs + bi);
             if (good) {
 #pragma unroll
                 for (int j = 0; j < CU; j++)
@@ -330,6 +261,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
                     bulk_g2s(sGeo, a.tgeo + (size_t) f0 * 8, bf, full);
                     bulk_g2s(sMeta, a.tmeta + f0, bm, full);
                 }
+                bulk_g2s(sNbr, a.nbr + (size_t) base * W, bs, full);
                 bulk_g2s(sIv, s.iv + base, bi, full);
             }
         }
@@ -355,23 +287,6 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         if (tid == 0 && (int) blockIdx.x != a.skip_tile) mbar_drain(full, 0, a.err);
         return;
     }
-    for (int c = tid; c < nb; c += NT) {
-        short cs[8];
-        lds_slots(a.cslot + (size_t) (base + c) * a.Wp, a.Wp, cs);
-#pragma unroll
-        for (int k = 0; k < W; k++) {
-            unsigned x = kNoFace;
-            if (cs[k] >= 0) {
-                const int e = cs[k] >> 1, side = cs[k] & 1;
-                if (index_ok(e < nf, a.err)) {
-                    const int l = side ? meta_la(sMeta[e]) : meta_lb(sMeta[e]);
-                    if (index_ok(local_ok(l, nb, a.B, nh), a.err)) x = (unsigned) (e | (side << 14) | (l << 15));
-                }
-            }
-            sNbr[k * Bp + c] = x;
-        }
-    }
-    __syncthreads();
     if (r.phases == 2) {
         // no exchange of half 1 stands between these halo reads and the other CTAs' updates: wait for all tiles
         if (tid == 0) ll_store(r.llX + blockIdx.x, 0ULL, r.epoch);
@@ -388,10 +303,14 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         if (s.time_mode == TM_FIXED) return;
         T xmx = T(0);
         for (int c = tid; c < nb; c += NT) {
-            if (sNbr[c] == kNoFace) continue;
-            const T x = sIv[c] * resident_wave_sum<T, W>(sU, sGeo, sNbr + c, Bp, NL, nf, c, s.gma);
-            xmx = fmax(xmx, x);
-            if (s.time_mode == TM_LOCAL) sDt[c] = T(s.dt_or_cfl) * qrcp(x);
+            unsigned x[W];
+            lds_nbr<W>(sNbr + c * W, x);
+            if (x[0] == kNoFace) continue;
+            T u[4];
+            lds_cell(sU, NL, c, u);
+            const T rate = sIv[c] * cell_wave_sum<T, W>(x, sGeo, nf, 8, u, s.gma, a.err);
+            xmx = fmax(xmx, rate);
+            if (s.time_mode == TM_LOCAL) sDt[c] = T(s.dt_or_cfl) * qrcp(rate);
         }
         xmx = warp_max_pos(xmx);
         if (lane == 0) red[wid] = (double) xmx;
@@ -400,7 +319,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
     __syncthreads();
 
     double r2 = 0.0, dt_used = s.dt_or_cfl;
-    int bad = 0;
+    int top = 0;
     for (int step = 0;; step++) {
         const bool last_step = step + 1 == r.nsteps;
         const unsigned stamp = r.epoch + (unsigned) step;
@@ -410,10 +329,12 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
             for (int w = tid; w < (NVAR == 4 ? nb : Bp + nb); w += NT) {
                 const int j = NVAR == 4 ? 0 : w >= Bp, c = w - j * Bp;
                 if (NVAR != 4 && c >= nb) continue;
-                if (sNbr[c] == kNoFace) continue;
+                unsigned x[W];
+                lds_nbr<W>(sNbr + c * W, x);
+                if (x[0] == kNoFace) continue;
                 const T iv = sIv[c];
                 Pass1Cell<T, NVAR> p;
-                resident_faces<T, W, NVAR>(p, sU, sGeo, sNbr + c, Bp, NL, nf, c, j, iv);
+                tile_faces<T, W, NVAR>(p, x, sU, sGeo, NL, nf, c, j, false, s.gma, iv, nb, a.B, nh, a.err);
                 T out[2 * NVAR], phis[NVAR];
                 if (lmode == LIM_FROZEN) {
                     // perhaps written in this launch (by this thread): not through the read-only path
@@ -422,8 +343,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
                         const auto x = __ldcg(pair_at(s.phiF, a.ps, base + c, j + h));
                         phis[2 * h] = x.x; phis[2 * h + 1] = x.y;
                     }
+                } else {
+                    p.limiter_values(iv, s.limiter, s.venkat_K, phis);
                 }
-                p.finish(iv, s.limiter, s.venkat_K, lmode, phis, out);
+                p.limited(phis, out);
 #pragma unroll
                 for (int h = 0; h < NVAR / 2; h++) {
                     if (lmode == LIM_RECORD) {
@@ -479,18 +402,20 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
         for (int w = tid; w < (NVAR == 4 ? nb : Bp + nb); w += NT) {
             const int j = NVAR == 4 ? 0 : w >= Bp, c = w - j * Bp;
             if (NVAR != 4 && c >= nb) continue;
-            if (sNbr[c] == kNoFace) continue;
+            unsigned x[W];
+            lds_nbr<W>(sNbr + c * W, x);
+            if (x[0] == kNoFace) continue;
             T u[NVAR], R[NVAR], un[NVAR];
             lds_vars<NVAR>(sU, NL, c, j, u);
-            resident_flux_sum<T, W, COMP, NVAR>(sNbr + c, Bp, sF, sGeo, nf, j, R);
+            cell_flux_sum<T, W, COMP, NVAR>(x, sF, sGeo, nf, 8, j, R, a.err);
             const T dt = s.time_mode == TM_LOCAL ? sDt[c] : T(dt_used);
-            const T Rr = cell_update<NVAR>(u, R, sIv[c], dt, un, bad);
+            const T Rr = cell_update<NVAR>(u, R, sIv[c], dt, un, top);
             if (j == 0) {
-                if (sizeof(T) == 4) bad |= !isfinite(Rr);           // its square fits a double
+                if (sizeof(T) == 4) top = max(top, exponent_word(Rr));   // its square fits a double
                 if (sizeof(T) == 8 || want_r2) {
                     const double q = (double) Rr * (double) Rr;
                     r2 += q;
-                    bad |= !isfinite(q);
+                    if (sizeof(T) == 8) top = max(top, exponent_word(q));
                 }
             }
             if (!last_step && (sFlag[c] & kCellExported)) ll_values<NVAR>(r.llU + (size_t) (base + c) * KU, 2 * j, un, stamp);
@@ -505,10 +430,12 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
             lds_cell(sU, NL, c, un);
 #pragma unroll 1
             for (int k = 0; k < W; k++) {
-                const unsigned x = sNbr[k * Bp + c];
-                if (x == kNoFace || nbr_right(x)) continue;
-                const int e = nbr_entry(x), lb = nbr_local(x), bc = meta_bc(sMeta[e]);
-                if (bc < 0 || !index_ok(bc < MAXBC, a.err)) continue;
+                const unsigned x = sNbr[c * W + k];
+                if (x == kNoFace || !(x & kBoundaryFace)) continue;
+                const int e = nbr_entry(x), lb = nbr_local(x);
+                if (!index_ok(e < nf && local_ok(lb, nb, a.B, nh), a.err)) continue;
+                const int bc = meta_bc(sMeta[e]);
+                if (!index_ok(bc >= 0 && bc < MAXBC, a.err)) continue;
                 T gnx, gny, gA, ug[4];
                 lds_geo3(sGeo, nf, e, 8, gnx, gny, gA);
                 ghost_state(s.bc.type[bc], un, gnx, gny, s.gma, s.bc.UBC[bc], s.bc.QBC[bc], ug);
@@ -543,7 +470,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
     }
 
     // statistics: the last CTA to arrive sums the partials in CTA order
-    if (bad) s_bad = 1;
+    if (not_finite<T>(top)) s_bad = 1;
     __syncthreads();
     if (tid == 0) {
         if (s_bad) atomicOr(&s.stats->nonfinite, 1);

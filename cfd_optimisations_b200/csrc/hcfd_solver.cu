@@ -62,7 +62,7 @@ struct TiledPass {
     void* d_tgeo = nullptr;              // face records [entries], T
     unsigned* d_tmeta = nullptr;         // pack_meta words [entries]
     int *d_foff = nullptr, *d_hoff = nullptr, *d_halo = nullptr;
-    short* d_cslot = nullptr;
+    unsigned* d_nbr = nullptr;           // pack_nbr words
     int* d_efid = nullptr;               // set-up only
     int block = 0;                       // compute threads per CTA
     int rec = 8;                         // values per face record (7: pass 2 on a plan of its own)
@@ -151,7 +151,7 @@ void free_all(hcfd_solver* s) {
                     s->d_phiG, s->d_phiF, s->d_io, s->d_cp, s->d_dtmin, s->d_partial, s->d_counter, s->d_err, s->d_stats, s->d_flags, s->d_ll};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (TiledPass& P : s->tp) {
-        void* q[] = {P.d_tgeo, P.d_tmeta, P.d_foff, P.d_hoff, P.d_halo, P.d_cslot, P.d_efid};
+        void* q[] = {P.d_tgeo, P.d_tmeta, P.d_foff, P.d_hoff, P.d_halo, P.d_nbr, P.d_efid};
         for (void* p : q) if (p) cudaFree(p);
     }
     if (s->graph) cudaGraphExecDestroy(s->graph);
@@ -203,7 +203,7 @@ hcfd::TileArgs<T> tile_args(hcfd_solver* s, int time_mode, double dt_or_cfl, con
     a.foff = P.d_foff;
     a.hoff = P.d_hoff;
     a.halo = P.d_halo;
-    a.cslot = P.d_cslot;
+    a.nbr = P.d_nbr;
     a.ntiles = P.plan.ntiles;
     a.B = P.plan.B;
     a.Wp = P.plan.Wp;
@@ -248,8 +248,7 @@ int prof_end(hcfd_solver* s, bool rec, Ev& e, std::vector<cudaEvent_t>& into) {
 // The resident kernel of a handle's shape.
 template <class T, int W>
 const void* resident_fn(const hcfd_solver* s) {
-    constexpr bool COMP = std::is_same<T, float>::value;
-    return s->pairs ? (const void*) hcfd::resident_kernel<T, W, COMP, 2> : (const void*) hcfd::resident_kernel<T, W, COMP, 4>;
+    return s->pairs ? (const void*) hcfd::resident_kernel<T, W, 2> : (const void*) hcfd::resident_kernel<T, W, 4>;
 }
 
 // nsteps steps (phases 3), or one half of one step, of the resident kernel.
@@ -307,10 +306,10 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl) {
         const hcfd::TileArgs<T> a1 = tile_args<T>(s, time_mode, dt_or_cfl, s->tp[0], 1);
         const hcfd::TileArgs<T> a2 = tile_args<T>(s, time_mode, dt_or_cfl, P2, 2);
         if ((rc = prof_begin(s, rec, e1))) return rc;
-        hcfd::tile_pass1_kernel<T, W, false><<<s->grid1, s->tp[0].block + 32, s->smem1, s->stream>>>(a1);
+        hcfd::pass1_variant<T, W, false>(s->prm.limiter, time_mode)<<<s->grid1, s->tp[0].block + 32, s->smem1, s->stream>>>(a1);
         if ((rc = prof_end(s, rec, e1, s->ev1))) return rc;
         if ((rc = prof_begin(s, rec, e2))) return rc;
-        hcfd::tile_pass2_kernel<T, W, std::is_same<T, float>::value, false><<<s->grid2, P2.block + 32, s->smem2, s->stream>>>(a2);
+        hcfd::pass2_variant<T, W, false>(P2.rec, time_mode)<<<s->grid2, P2.block + 32, s->smem2, s->stream>>>(a2);
         if ((rc = prof_end(s, rec, e2, s->ev2))) return rc;
     } else {
         const int grid = nblk(s->Nc, s->block);
@@ -336,6 +335,15 @@ int launch_step_w(hcfd_solver* s, int time_mode, double dt_or_cfl) {
     }
 }
 
+// Lets a kernel use all the dynamic shared memory a block may have.  The attribute belongs to the
+// kernel, which handles of other sizes share, so it is never set to one handle's need.
+int allow_smem(const void* kernel, int maxsm) {
+    cudaFuncAttributes fa;
+    CK(cudaFuncGetAttributes(&fa, kernel));
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm - (int) fa.sharedSizeBytes));
+    return HCFD_OK;
+}
+
 // Shared-memory opt-in and persistent grid size of the tiled kernels for one (T, W).
 template <class T, int W>
 int setup_tiled_w(hcfd_solver* s) {
@@ -347,15 +355,19 @@ int setup_tiled_w(hcfd_solver* s) {
     int maxsm = 0;
     CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
     if ((int) s->smem2 > maxsm || (int) s->smem1 > maxsm) return fail(HCFD_EINVAL, "tile does not fit in shared memory");
-    CK(cudaFuncSetAttribute(hcfd::tile_pass1_kernel<T, W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) s->smem1));
-    CK(cudaFuncSetAttribute(hcfd::tile_pass2_kernel<T, W, std::is_same<T, float>::value, false>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int) s->smem2));
+    // every time mode's variants, on one grid: the fewest CTAs an SM holds of any of them
     int b1 = 0, b2 = 0;
-    // blocks of the tiled kernels: `block` compute threads + one producer warp
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, hcfd::tile_pass1_kernel<T, W, false>, s->tp[0].block + 32,
-                                                     s->smem1));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, hcfd::tile_pass2_kernel<T, W, std::is_same<T, float>::value, false>,
-                                                     T2.block + 32, s->smem2));
+    for (int mode : {HCFD_FIXED_DT, HCFD_GLOBAL_CFL, HCFD_LOCAL_CFL}) {
+        const void* k1 = (const void*) hcfd::pass1_variant<T, W, false>(s->prm.limiter, mode);
+        const void* k2 = (const void*) hcfd::pass2_variant<T, W, false>(s->split ? 7 : 8, mode);
+        int n1 = 0, n2 = 0, rc;
+        if ((rc = allow_smem(k1, maxsm)) || (rc = allow_smem(k2, maxsm))) return rc;
+        // blocks of the tiled kernels: `block` compute threads + one producer warp
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n1, k1, s->tp[0].block + 32, s->smem1));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n2, k2, T2.block + 32, s->smem2));
+        b1 = mode == HCFD_FIXED_DT ? n1 : std::min(b1, n1);
+        b2 = mode == HCFD_FIXED_DT ? n2 : std::min(b2, n2);
+    }
     if (b1 < 1 || b2 < 1) return fail(HCFD_EINVAL, "tiled kernels cannot be resident");
     s->grid1 = std::min(P.ntiles, b1 * s->nsm);
     s->grid2 = std::min(Q.ntiles, b2 * s->nsm);
@@ -382,9 +394,8 @@ int setup_resident_w(hcfd_solver* s, bool* fits) {
     s->refetch = hcfd::ResidentSmem<T>(P.B, P.Hmax, P.Fmax, P.Wp, false).total > room;
     s->smem1 = hcfd::ResidentSmem<T>(P.B, P.Hmax, P.Fmax, P.Wp, s->refetch).total;
     if (s->smem1 > room) return HCFD_OK;
-    // the attribute is the kernel's, shared by every handle: the largest any handle may need
-    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) room));
-    int nb = 0;
+    int nb = 0, rc = allow_smem(kernel, maxsm);
+    if (rc) return rc;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, s->tp[0].block, s->smem1));
     s->grid1 = s->grid2 = P.ntiles;
     *fits = nb >= 1 && P.ntiles <= nb * s->nsm;
@@ -626,7 +637,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
             P.rec = k == 1 ? 7 : 8;     // pass 2's own plan leaves out If, which only pass 1 reads
             if ((rc = dalloc((char**) &P.d_tgeo, tsz * P.rec * E)) || (rc = dalloc(&P.d_tmeta, E)) ||
                 (rc = dalloc(&P.d_foff, P.plan.foff.size())) || (rc = dalloc(&P.d_hoff, P.plan.hoff.size())) ||
-                (rc = dalloc(&P.d_halo, P.plan.halo.size())) || (rc = dalloc(&P.d_cslot, P.plan.cslot.size())) ||
+                (rc = dalloc(&P.d_halo, P.plan.halo.size())) || (rc = dalloc(&P.d_nbr, P.plan.cslot.size())) ||
                 (rc = dalloc(&P.d_efid, E))) {
                 free_tmp();
                 return bail(rc);
@@ -661,12 +672,12 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         for (int k = 0; k < (h->split ? 2 : 1); k++) {
             TiledPass& T = h->tp[k];
             const hcfd::TilePlan& P = T.plan;
-            const std::vector<unsigned> mw = hcfd::packed_meta(P);
+            const std::vector<unsigned> mw = hcfd::packed_meta(P), nw = hcfd::packed_nbr(P);
             if (ce == cudaSuccess) ce = up(T.d_tmeta, mw.data(), 4 * mw.size());
             if (ce == cudaSuccess) ce = up(T.d_foff, P.foff.data(), 4 * P.foff.size());
             if (ce == cudaSuccess) ce = up(T.d_hoff, P.hoff.data(), 4 * P.hoff.size());
             if (ce == cudaSuccess) ce = up(T.d_halo, P.halo.data(), 4 * P.halo.size());
-            if (ce == cudaSuccess) ce = up(T.d_cslot, P.cslot.data(), 2 * P.cslot.size());
+            if (ce == cudaSuccess) ce = up(T.d_nbr, nw.data(), 4 * nw.size());
             if (ce == cudaSuccess) ce = up(T.d_efid, P.efid.data(), 4 * P.efid.size());
         }
         if (h->resident) {

@@ -28,7 +28,7 @@ struct TileArgs {
     const int* __restrict__ foff;          // [ntiles + 1], multiples of 4
     const int* __restrict__ hoff;          // [ntiles + 1]
     const int* __restrict__ halo;          // internal cell ids
-    const short* __restrict__ cslot;       // [ntiles * B * Wp]: (entry << 1) | cell-is-right, or -1; Wp = W
+    const unsigned* __restrict__ nbr;      // [ntiles * B * Wp]: a word per cell and face (pack_nbr); Wp = W
     int ntiles, B, Wp, Hmax, Fmax;
     unsigned int* err;                     // bit 0: a bounded wait gave up; bit 1: copies did not drain;
                                            // bit 2: an index out of range (checked build)
@@ -54,7 +54,7 @@ struct TileArgs {
     int* claim;
     int* claim_reset;
     long long nentries, nhalo, ncap;       // lengths of tgeo/tmeta (entries), halo, and of the
-                                           // per-cell arrays iv/cslot (cells): checked build
+                                           // per-cell arrays iv/nbr (cells): checked build
 };
 
 // Metadata of a face entry in one 32-bit word: the local index (tile cell 0..B-1, halo cell
@@ -72,6 +72,42 @@ inline std::vector<unsigned> packed_meta(const TilePlan& P) {
 __device__ __forceinline__ int meta_la(unsigned w) { return (int) (w & 0x1FFFu); }
 __device__ __forceinline__ int meta_lb(unsigned w) { return (int) ((w >> 13) & 0x1FFFu); }
 __device__ __forceinline__ int meta_bc(unsigned w) { return (int) (w >> 26) - 1; }
+
+// One face of a tile cell in one word: its entry (bits 0-13), the cell's side (bit 14: right), the
+// local index of the cell across it (bits 15-27) and whether it is a boundary face (bit 28);
+// kNoFace for a position the cell does not use.  With it a cell's loads of face record and neighbour
+// state both hang on one word, not on the entry's metadata in between (pass 1 reads none).
+constexpr unsigned kNoFace = 0xFFFFFFFFu, kBoundaryFace = 1u << 28;
+__host__ __device__ __forceinline__ unsigned pack_nbr(int e, int side, int l, bool boundary) {
+    return (unsigned) e | ((unsigned) side << 14) | ((unsigned) l << 15) | (boundary ? kBoundaryFace : 0u);
+}
+inline std::vector<unsigned> packed_nbr(const TilePlan& P) {
+    std::vector<unsigned> w(P.cslot.size(), kNoFace);
+    const size_t per = (size_t) P.B * P.Wp;
+    for (int t = 0; t < P.ntiles; t++)
+        for (size_t i = t * per; i < (t + 1) * per; i++) {
+            if (P.cslot[i] < 0) continue;
+            const int e = P.cslot[i] >> 1, side = P.cslot[i] & 1;
+            const short* m = &P.meta[4 * ((size_t) P.foff[t] + e)];
+            w[i] = pack_nbr(e, side, side ? m[0] : m[1], m[2] >= 0);
+        }
+    return w;
+}
+__device__ __forceinline__ int nbr_entry(unsigned w) { return (int) (w & 0x3FFFu); }
+__device__ __forceinline__ bool nbr_right(unsigned w) { return (w >> 14) & 1u; }
+__device__ __forceinline__ int nbr_local(unsigned w) { return (int) ((w >> 15) & 0x1FFFu); }
+template <int W>   // a cell's W words
+__device__ __forceinline__ void lds_nbr(const unsigned* p, unsigned x[W]) {
+    if constexpr (W == 3) {
+        x[0] = p[0]; x[1] = p[1]; x[2] = p[2];
+    } else {
+#pragma unroll
+        for (int k = 0; k < W; k += 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(p + k);
+            x[k] = v.x; x[k + 1] = v.y; x[k + 2] = v.z; x[k + 3] = v.w;
+        }
+    }
+}
 
 // A local cell index of a tile: one of its nb cells, or one of its nh halo cells (B..).
 __device__ __forceinline__ bool local_ok(int l, int nb, int B, int nh) {
@@ -255,19 +291,19 @@ __host__ __device__ constexpr size_t align128(size_t x) { return (x + 127) & ~si
 
 // Shared-memory layout of one CTA: two mbarriers and two staging buffers (double buffering:
 // tile i+1 is in flight while tile i is computed).  One staging buffer holds the tile's and
-// its halo's cells (and limited gradients in pass 2), its face records and metadata, its
-// slot table and its iv.  Pass 2 keeps its fluxes in the staged face records, so a CTA
+// its halo's cells (and limited gradients in pass 2), its face records and metadata
+// (pass 2), its cells' face words and its iv.  Pass 2 keeps its fluxes in the staged face records, so a CTA
 // needs no other scratch (three CTAs of 128 + 32 threads fit an SM at 128-cell tiles).
 template <class T>
 struct TileSmem {
-    size_t u, g, geo, meta, cslot, iv, stage, total;   // byte offsets within a stage
+    size_t u, g, geo, meta, nbr, iv, stage, total;   // byte offsets within a stage
     __host__ __device__ TileSmem(int B, int Hmax, int Fmax, int W, int Wp, bool pass2) {
         size_t p = 0;
         u = p;     p += align128((size_t) (B + Hmax) * sizeof(Cell4<T>));
         g = p;     if (pass2) p += align128((size_t) (B + Hmax) * sizeof(Grad8<T>));
         geo = p;   p += align128((size_t) Fmax * sizeof(FaceGeo<T>));
-        meta = p;  p += align128((size_t) Fmax * 4);
-        cslot = p; p += align128((size_t) B * Wp * sizeof(short));
+        meta = p;  if (pass2) p += align128((size_t) Fmax * 4);
+        nbr = p;   p += align128((size_t) B * Wp * sizeof(unsigned));
         iv = p;    p += align128((size_t) B * sizeof(T));
         stage = p;
         total = kHeader + 2 * stage;
@@ -376,8 +412,8 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
         Grad8<T>* sG = reinterpret_cast<Grad8<T>*>(st + L.g);
         if (lane == 0) {
             const unsigned bu = nb * sizeof(Cell4<T>), bg = PASS2 ? nb * sizeof(Grad8<T>) : 0u;
-            const unsigned bf = nf * a.rec * (unsigned) sizeof(T), bm = nf * 4u;
-            const unsigned bs = a.B * a.Wp * sizeof(short), bi = a.B * sizeof(T);
+            const unsigned bf = nf * a.rec * (unsigned) sizeof(T), bm = PASS2 ? nf * 4u : 0u;
+            const unsigned bs = a.B * a.Wp * sizeof(unsigned), bi = a.B * sizeof(T);
             // the tile's descriptor and instance scalars, published by the release of the
             // arrive below
             StageInfo* si = reinterpret_cast<StageInfo*>(smem + 64) + buf;
@@ -405,9 +441,9 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
             }
             if (bf) {
                 bulk_g2s(st + L.geo, a.tgeo + (size_t) f0 * a.rec, bf, full + buf);
-                bulk_g2s(st + L.meta, a.tmeta + f0, bm, full + buf);
+                if (PASS2) bulk_g2s(st + L.meta, a.tmeta + f0, bm, full + buf);
             }
-            bulk_g2s(st + L.cslot, a.cslot + (size_t) base * a.Wp, bs, full + buf);
+            bulk_g2s(st + L.nbr, a.nbr + (size_t) base * a.Wp, bs, full + buf);
             bulk_g2s(st + L.iv, a.s.iv + base, bi, full + buf);
             }
         }
@@ -481,22 +517,6 @@ __device__ __forceinline__ void finish_step(const StepArgs<T>& a, double r2, int
 
 // ---------------------------------------------------------------------------------------
 
-__device__ __forceinline__ void lds_slots(const short* p, int Wp, short cs[8]) {
-    if (Wp == 3) {
-        cs[0] = p[0]; cs[1] = p[1]; cs[2] = p[2];
-        cs[3] = cs[4] = cs[5] = cs[6] = cs[7] = -1;
-    } else if (Wp == 4) {
-        const short4 a = *reinterpret_cast<const short4*>(p);
-        cs[0] = a.x; cs[1] = a.y; cs[2] = a.z; cs[3] = a.w;
-        cs[4] = cs[5] = cs[6] = cs[7] = -1;
-    } else {
-        const int4 a = *reinterpret_cast<const int4*>(p);
-        const short* q = reinterpret_cast<const short*>(&a);
-#pragma unroll
-        for (int k = 0; k < 8; k++) cs[k] = q[k];
-    }
-}
-
 // One face entry of pass 2: operands gathered from shared memory and reduced at once to the
 // MUSCL states on both sides (Flux.cpp:83-87), then the Rusanov flux in the face's own
 // L -> R orientation.  Only the reconstructed states stay live between load and flux.
@@ -545,41 +565,39 @@ struct FaceIn {
 };
 
 // Sum of A_f F over one cell's faces in increasing face order (Flux.cpp:39-42), F as stored by
-// FaceIn::store at sF; one face's flux leaves its left cell and enters its right one.  NVAR 2: the
-// sums of variable pair j alone.  FP32 sums are compensated; the first term needs no two-sum,
+// FaceIn::store at sF.  NVAR 2: the sums of variable pair j alone.  FP32 sums are compensated; the first term needs no two-sum,
 // 0 + x being exact.
 template <class T, int W, bool COMP, int NVAR>
-__device__ __forceinline__ void cell_flux_sum(const short cs[8], const T* sF, const T* sGeo, int nf, int rec, int j, T* R,
+__device__ __forceinline__ void cell_flux_sum(const unsigned x[W], const T* sF, const T* sGeo, int nf, int rec, int j, T* R,
                                               unsigned int* err) {
     T Rc[NVAR];
 #pragma unroll
     for (int v = 0; v < NVAR; v++) { R[v] = T(0); Rc[v] = T(0); }
 #pragma unroll
     for (int k = 0; k < W; k++) {
-        if (W > 3 && cs[k] < 0) continue;
-        // (W = 3) an unused slot reads entry 0 with weight zero, in place of a branch per face
-        const bool on = W > 3 || cs[k] >= 0;
-        const bool isL = (cs[k] & 1) == 0;
-        int e = on ? cs[k] >> 1 : 0;
+        if (W > 3 && x[k] == kNoFace) continue;
+        // (W = 3) an unused position reads entry 0 with weight zero, in place of a branch per face
+        const bool on = W > 3 || x[k] != kNoFace;
+        int e = on ? nbr_entry(x[k]) : 0;
         if constexpr (kChecked) e = index_ok(e < nf, err) ? e : 0;
         T Fk[NVAR];
 #pragma unroll
         for (int h = 0; h < NVAR / 2; h++) {
-            const auto x = ldp(sF, nf, NVAR == 4 ? h : j, e);
-            Fk[2 * h] = x.x; Fk[2 * h + 1] = x.y;
+            const auto f = ldp(sF, nf, NVAR == 4 ? h : j, e);
+            Fk[2 * h] = f.x; Fk[2 * h + 1] = f.y;
         }
-        if constexpr (COMP) {
+        // one face's flux leaves its left cell and enters its right one; COMP: Fk holds A_f F
+        T w = COMP ? T(1) : lds_area(sGeo, nf, e, rec);
+        w = nbr_right(x[k]) ? w : -w;
+        if (W == 3) w = on ? w : T(0);
 #pragma unroll
-            for (int v = 0; v < NVAR; v++) {                     // Fk holds A_f F here
-                const T x = !on ? T(0) : isL ? -Fk[v] : Fk[v];
-                if (k == 0) R[v] = x;
-                else two_sum(R[v], Rc[v], x);
+        for (int v = 0; v < NVAR; v++) {
+            if constexpr (COMP) {
+                if (k == 0) R[v] = w * Fk[v];
+                else two_sum(R[v], Rc[v], __fmul_rn(w, Fk[v]));
+            } else {
+                R[v] += w * Fk[v];
             }
-        } else {
-            const T Af = lds_area(sGeo, nf, e, rec);
-            const T sA = !on ? T(0) : isL ? -Af : Af;
-#pragma unroll
-            for (int v = 0; v < NVAR; v++) R[v] += sA * Fk[v];
         }
     }
     if constexpr (COMP)
@@ -587,31 +605,37 @@ __device__ __forceinline__ void cell_flux_sum(const short cs[8], const T* sF, co
         for (int v = 0; v < NVAR; v++) R[v] += Rc[v];
 }
 
-// The wave-speed sum of a cell with state u (local time stepping in pass 2).
+// The wave-speed sum of a cell with state u.
 template <class T, int W>
-__device__ __forceinline__ T cell_wave_sum(const short cs[8], const T* sGeo, int nf, int rec, const T u[4], T gma,
+__device__ __forceinline__ T cell_wave_sum(const unsigned x[W], const T* sGeo, int nf, int rec, const T u[4], T gma,
                                            unsigned int* err) {
     T cu, cv, ca, lam = T(0);
     cell_speed(u, gma, cu, cv, ca);
 #pragma unroll
     for (int k = 0; k < W; k++) {
-        if (cs[k] < 0) continue;
-        int e = cs[k] >> 1;
+        if (W > 3 && x[k] == kNoFace) continue;
+        const bool on = W > 3 || x[k] != kNoFace;
+        int e = on ? nbr_entry(x[k]) : 0;
         if constexpr (kChecked) e = index_ok(e < nf, err) ? e : 0;
         T nx, ny, A;
         lds_geo3(sGeo, nf, e, rec, nx, ny, A);
-        lam += wave(cu, cv, ca, nx, ny, A);
+        lam += wave(cu, cv, ca, nx, ny, on ? A : T(0));
     }
     return lam;
 }
 
 // U += dt R (Flux.cpp:45-49, Euler.cpp:107-113); returns the density residual R_rho.
+// `top` keeps the largest exponent word seen, for not_finite.
+__device__ __forceinline__ int exponent_word(double x) { return __double2hiint(x) & 0x7FFFFFFF; }
+__device__ __forceinline__ int exponent_word(float x) { return __float_as_int(x) & 0x7FFFFFFF; }
+template <class T>
+__device__ __forceinline__ bool not_finite(int top) { return top >= (sizeof(T) == 8 ? 0x7FF00000 : 0x7F800000); }
 template <int NVAR, class T>
-__device__ __forceinline__ T cell_update(const T* u, const T* R, T iv, T dt, T* un, int& bad) {
+__device__ __forceinline__ T cell_update(const T* u, const T* R, T iv, T dt, T* un, int& top) {
 #pragma unroll
     for (int v = 0; v < NVAR; v++) {
         un[v] = u[v] + dt * (R[v] * iv);
-        bad |= !isfinite(un[v]);
+        top = max(top, exponent_word(un[v]));
     }
     return R[0] * iv;
 }
@@ -661,8 +685,7 @@ __device__ __forceinline__ T cell_update(const T* u, const T* R, T iv, T dt, T* 
         const Cell4<T>* sU = reinterpret_cast<const Cell4<T>*>(st + L.u);                        \
         const T* sGeo = reinterpret_cast<const T*>(st + L.geo);                                  \
         const int nfl = si.nf;                                                                   \
-        const unsigned* sMeta = reinterpret_cast<const unsigned*>(st + L.meta);                  \
-        const short* sSlot = reinterpret_cast<const short*>(st + L.cslot);                       \
+        const unsigned* sNbr = reinterpret_cast<const unsigned*>(st + L.nbr);                    \
         const T* sIv = reinterpret_cast<const T*>(st + L.iv);
 
 #define HCFD_TILE_LOOP_END                                                                       \
@@ -706,47 +729,34 @@ __device__ __forceinline__ void lds_vars(const Cell4<T>* p, int ps, int i, int j
     }
 }
 
-// Own state of tile cell c (pair j of its variables when NVAR is 2) into p.
-template <class T, int NVAR>
-__device__ __forceinline__ void tile_begin(Pass1Cell<T, NVAR>& p, const Cell4<T>* sU, int NL, int c, int j, bool with_lam, T gma) {
-    lds_vars<NVAR>(sU, NL, c, j, p.u);
-    if constexpr (NVAR == 4) {
-        p.begin(with_lam, gma, p.u);
-    } else {
-        T U[4];
-        if (with_lam) lds_cell(sU, NL, c, U);
-        p.begin(with_lam, gma, U);
-    }
-}
-
-// Pass 1 of tile cell c up to the limiter's increments, operands from shared memory: nf entries, nb
-// tile cells and nh halo cells of NL staged.  Unrolled: the face loads overlap.
-template <class T, int W>
-__device__ __forceinline__ void tile_faces(Pass1Cell<T>& p, const TileArgs<T>& a, const Cell4<T>* sU, const T* sGeo,
-                                           const unsigned* sMeta, const short cs[8], int NL, int nf, int nb, int nh, int c,
-                                           T iv) {
-    const bool with_lam = a.s.time_mode != TM_FIXED;
+// Pass 1 of tile cell c (pair j of its variables when NVAR is 2) up to the limiter's increments,
+// operands from shared memory: its face words in x, nf entries, nb tile cells and nh halo cells of
+// NL staged.  Unrolled: the face loads overlap.
+template <class T, int W, int NVAR>
+__device__ __forceinline__ void tile_faces(Pass1Cell<T, NVAR>& p, const unsigned x[W], const Cell4<T>* sU, const T* sGeo, int NL,
+                                           int nf, int c, int j, bool with_lam, T gma, T iv, int nb, int B, int nh,
+                                           unsigned int* err) {
     T ro[W][2];
-    tile_begin(p, sU, NL, c, 0, with_lam, a.s.gma);
+    lds_vars<NVAR>(sU, NL, c, j, p.u);
+    p.begin(with_lam, gma, p.u);
 #pragma unroll
     for (int k = 0; k < W; k++) {
         ro[k][0] = T(0); ro[k][1] = T(0);
-        if (W > 3 && cs[k] < 0) continue;
-        // A slot a cell does not use (W = 3: a cell of an open mesh with fewer faces) reads
+        if (W > 3 && x[k] == kNoFace) continue;
+        // A position a cell does not use (W = 3: a cell of an open mesh with fewer faces) reads
         // entry 0 with zero length, the cell itself as its neighbour and r = 0, which adds
         // nothing, in place of a branch per face.
-        const bool on = W > 3 || cs[k] >= 0;
-        int e = on ? cs[k] >> 1 : 0;
-        const bool isL = (cs[k] & 1) == 0;
-        if constexpr (kChecked)    // a bad index is replaced by entry 0 / tile cell 0 (no branch)
-            e = index_ok(e < nf, a.err) ? e : 0;
+        const bool on = W > 3 || x[k] != kNoFace;
+        int e = on ? nbr_entry(x[k]) : 0, nbl = on ? nbr_local(x[k]) : c;
+        const bool isL = !nbr_right(x[k]);
+        if constexpr (kChecked) {  // a bad index is replaced by entry 0 / tile cell 0 (no branch)
+            e = index_ok(e < nf, err) ? e : 0;
+            nbl = index_ok(!on || local_ok(nbl, nb, B, nh), err) ? nbl : 0;
+        }
         FaceGeo<T> g;
         lds_geo4(sGeo, nf, e, g);
-        int nbl = isL ? meta_lb(sMeta[e]) : meta_la(sMeta[e]);
-        if constexpr (kChecked)
-            nbl = index_ok(!on || local_ok(nbl, nb, a.B, nh), a.err) ? nbl : 0;
-        T un[4];
-        lds_cell(sU, NL, on ? nbl : c, un);
+        T un[NVAR];
+        lds_vars<NVAR>(sU, NL, nbl, j, un);
         p.face(un, isL, g.nx, g.ny, on ? g.Af : T(0), g.If, with_lam);
         // this cell's own centre-to-face vector: one pair, at its side's plane
         const auto rr = ldp(sGeo, nf, isL ? 2 : 3, e);
@@ -758,34 +768,39 @@ __device__ __forceinline__ void tile_faces(Pass1Cell<T>& p, const TileArgs<T>& a
     for (int k = 0; k < W; k++) p.increment(ro[k][0], ro[k][1]);
 }
 
-template <class T, int W, bool ARENA>
-__global__ void __launch_bounds__(288) tile_pass1_kernel(const TileArgs<T> a) {
+// LIM and LAM: the limiter and whether the CFL sums are wanted, fixed at compile time (the branches
+// on them, eight a cell, and the register moves where their sides meet were a tenth of the kernel's
+// instructions); -1: read from the arguments (W = 8, meshes no workload has).
+template <class T, int W, bool ARENA, int LIM, int LAM>
+__global__ void __maxnreg__(sizeof(T) == 8 ? 128 : W == 3 ? 56 : 72) tile_pass1_kernel(const TileArgs<T> a) {
     extern __shared__ __align__(128) unsigned char smem[];
     const TileSmem<T> L(a.B, a.Hmax, a.Fmax, W, a.Wp, false);
     const StepArgs<T>& s = a.s;
     T xmx = T(0);                        // largest iv * lam (see dt_of_max)
     HCFD_TILE_LOOP_BEGIN(false, ARENA)
     const int lmode = limiter_mode(si.steps, s.freeze_after);
+    const bool with_lam = LAM >= 0 ? LAM != 0 : s.time_mode != TM_FIXED;
     for (int c = threadIdx.x; c < nb; c += NT) {
-        short cs[8];
-        lds_slots(sSlot + c * a.Wp, a.Wp, cs);
-        if (cs[0] < 0) continue;
+        unsigned x[W];
+        lds_nbr<W>(sNbr + c * W, x);
+        if (x[0] == kNoFace) continue;
         Pass1Cell<T> p;
         const T iv = sIv[c];
-        tile_faces<T, W>(p, a, sU, sGeo, sMeta, cs, NL, nfl, nb, si.nh, c, iv);
+        tile_faces<T, W, 4>(p, x, sU, sGeo, NL, nfl, c, 0, with_lam, s.gma, iv, nb, a.B, si.nh, a.err);
         T out[8], phis[4];
         if (lmode == LIM_FROZEN) ld_cell(s.phiF, a.ps, base + c, phis);
-        p.finish(iv, s.limiter, s.venkat_K, lmode, phis, out);
+        else p.template limiter_values<LIM>(iv, s.limiter, s.venkat_K, phis);
+        p.limited(phis, out);
         if (lmode == LIM_RECORD) st_cell(s.phiF, a.ps, base + c, phis);
         st_grad(s.phiG, a.ps, base + c, out);
-        if (s.time_mode != TM_FIXED) xmx = fmax(xmx, iv * p.lam);
+        if (with_lam) xmx = fmax(xmx, iv * p.lam);
     }
     if constexpr (ARENA) {
         // per-instance minimum (exact and order-free): each warp carries its minimum across
         // this CTA's consecutive tiles of one instance and posts it with one atomic when the
         // next tile belongs to another instance, so a large instance sees a few atomics per
         // CTA rather than one per warp and tile on a single address
-        if (s.time_mode != TM_FIXED) {
+        if (with_lam) {
             if (si.next_inst != inst) {
                 const double m = dt_of_max(warp_max(xmx));
                 if ((threadIdx.x & 31) == 0 && m < 1e300)
@@ -795,7 +810,7 @@ __global__ void __launch_bounds__(288) tile_pass1_kernel(const TileArgs<T> a) {
         }
     }
     HCFD_TILE_LOOP_END
-    if (!ARENA && s.time_mode != TM_FIXED) {
+    if (!ARENA && (LAM >= 0 ? LAM != 0 : s.time_mode != TM_FIXED)) {
         __shared__ T sm[32];
         T m = warp_max(xmx);
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -809,15 +824,21 @@ __global__ void __launch_bounds__(288) tile_pass1_kernel(const TileArgs<T> a) {
     }
 }
 
-template <class T, int W, bool COMP, bool ARENA>
+// REC and LOCAL: the record length and local time stepping, fixed at compile time as in pass 1
+// (-1: read from the arguments).
+template <class T, int W, bool ARENA, int REC, int LOCAL>
 __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
+    constexpr bool COMP = sizeof(T) == 4;
     extern __shared__ __align__(128) unsigned char smem[];
     const TileSmem<T> L(a.B, a.Hmax, a.Fmax, W, a.Wp, true);
     const StepArgs<T>& s = a.s;
     double dt_used = 0.0;
     double r2 = 0.0;
-    int bad = 0;
+    int top = 0;
+    const int rec = REC >= 0 ? REC : a.rec;
+    const bool local = LOCAL >= 0 ? LOCAL != 0 : s.time_mode == TM_LOCAL;
     HCFD_TILE_LOOP_BEGIN(true, ARENA)
+    const unsigned* sMeta = reinterpret_cast<const unsigned*>(st + L.meta);
     const T cfl_or_dt = T(si.dt_or_cfl);
     if (staged && !fin) dt_used = (s.time_mode == TM_FIXED) ? si.dt_or_cfl : si.dt_or_cfl * si.dtmin;
     const Grad8<T>* sG = reinterpret_cast<const Grad8<T>*>(st + L.g);
@@ -834,7 +855,7 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
     // B200 the split costs more than it saves.
     // The fluxes go over the r pairs of the staged records, which only the entry's own thread
     // reads in pass 2, and has read by then.
-    T* sF = reinterpret_cast<T*>(st + L.geo) + 2 * rplane(a.rec) * nf;
+    T* sF = reinterpret_cast<T*>(st + L.geo) + 2 * rplane(rec) * nf;
     for (int e = threadIdx.x; e < nf; e += 2 * NT) {
         const int base2 = e - (int) threadIdx.x;                 // first entry of this round
         const int pairs = min(NT, max(0, nf - base2 - NT));      // threads with a second entry
@@ -843,8 +864,8 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
             if constexpr (kChecked)
                 if (!entry_ok(sMeta[e], nb, a.B, si.nh, a.err) || !entry_ok(sMeta[eB], nb, a.B, si.nh, a.err)) continue;
             FaceIn<T> A, Bq;
-            A.load(sU, sG, NL, sGeo, sMeta, nf, a.rec, e);
-            Bq.load(sU, sG, NL, sGeo, sMeta, nf, a.rec, eB);
+            A.load(sU, sG, NL, sGeo, sMeta, nf, rec, e);
+            Bq.load(sU, sG, NL, sGeo, sMeta, nf, rec, eB);
             T FA[4], FB[4];
             A.flux(s.gma, FA);
             Bq.flux(s.gma, FB);
@@ -854,7 +875,7 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
             if constexpr (kChecked)
                 if (!entry_ok(sMeta[e], nb, a.B, si.nh, a.err)) continue;
             FaceIn<T> A;
-            A.load(sU, sG, NL, sGeo, sMeta, nf, a.rec, e);
+            A.load(sU, sG, NL, sGeo, sMeta, nf, rec, e);
             T FA[4];
             A.flux(s.gma, FA);
             A.template store<COMP>(sF, nf, FA);
@@ -866,34 +887,36 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
     if (*compute_abort_word(smem) || fin) break;
     // cell phase: slots in increasing face order, update, ghost refresh
     for (int c = threadIdx.x; c < nb; c += NT) {
-        short cs[8];
-        lds_slots(sSlot + c * a.Wp, a.Wp, cs);
-        if (cs[0] < 0) continue;
+        unsigned x[W];
+        lds_nbr<W>(sNbr + c * W, x);
+        if (x[0] == kNoFace) continue;
         T u[4];
         lds_cell(sU, NL, c, u);
         const T iv = sIv[c];
         T R[4], un_[4];
-        cell_flux_sum<T, W, COMP, 4>(cs, sF, sGeo, nf, a.rec, 0, R, a.err);
+        cell_flux_sum<T, W, COMP, 4>(x, sF, sGeo, nf, rec, 0, R, a.err);
         T dt = T(dt_used);
-        if (s.time_mode == TM_LOCAL)
-            dt = cfl_or_dt * qrcp(iv * cell_wave_sum<T, W>(cs, sGeo, nf, a.rec, u, s.gma, a.err));
-        const T Rr = cell_update<4>(u, R, iv, dt, un_, bad);
+        if (local) dt = cfl_or_dt * qrcp(iv * cell_wave_sum<T, W>(x, sGeo, nf, rec, u, s.gma, a.err));
+        const T Rr = cell_update<4>(u, R, iv, dt, un_, top);
         r2 += (double) Rr * (double) Rr;
         st_cell(s.Unew, a.ps, base + c, un_);
         // ghost refresh (Euler.cpp:96, :138-142): this cell is its ghosts' only neighbour
+        bool any = false;
 #pragma unroll
+        for (int k = 0; k < W; k++) any |= x[k] != kNoFace && (x[k] & kBoundaryFace);
+        if (!any) continue;
+#pragma unroll 1
         for (int k = 0; k < W; k++) {
-            if (cs[k] < 0 || (cs[k] & 1)) continue;
-            const int e = cs[k] >> 1;
-            const unsigned w = sMeta[e];
-            const int bc = meta_bc(w);
-            if (bc < 0) continue;
-            const int lb = meta_lb(w);
-            if (!index_ok(local_ok(lb, nb, a.B, si.nh) && bc < MAXBC, a.err)) continue;
+            const unsigned xk = sNbr[c * W + k];
+            if (xk == kNoFace || !(xk & kBoundaryFace)) continue;
+            const int e = nbr_entry(xk), lb = nbr_local(xk);
+            if (!index_ok(e < nf && local_ok(lb, nb, a.B, si.nh), a.err)) continue;
+            const int bc = meta_bc(sMeta[e]);
+            if (!index_ok(bc >= 0 && bc < MAXBC, a.err)) continue;
             const int gi = lb < a.B ? base + lb : __ldg(a.halo + si.h0 + lb - a.B);
             if (!index_ok(gi >= 0 && gi < a.ps, a.err)) continue;
             T gnx, gny, gA;
-            lds_geo3(sGeo, nf, e, a.rec, gnx, gny, gA);
+            lds_geo3(sGeo, nf, e, rec, gnx, gny, gA);
             T ug[4];
             const BCTable* bt = ARENA ? a.inst_bc + inst : &s.bc;
             ghost_state(bt->type[bc], un_, gnx, gny, s.gma, bt->UBC[bc], bt->QBC[bc], ug);
@@ -904,17 +927,42 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
         // per-tile residual: one partial per warp (fixed order, no barrier); the finalize
         // kernel sums an instance's partials in order
         const double w = warp_sum(r2);
-        const int wb = __any_sync(0xffffffffu, bad);
+        const int wb = __any_sync(0xffffffffu, not_finite<T>(top));
         if ((threadIdx.x & 31) == 0) {
             const int k = t * (NT >> 5) + (int) (threadIdx.x >> 5);
             a.tile_r2[k] = w;
             a.tile_bad[k] = wb;
         }
         r2 = 0.0;
-        bad = 0;
+        top = 0;
     }
     HCFD_TILE_LOOP_END
-    if constexpr (!ARENA) finish_step(s, r2, bad, dt_used);
+    if constexpr (!ARENA) finish_step(s, r2, not_finite<T>(top), dt_used);
+}
+
+// The variants of a handle's shape.
+template <class T>
+using TileKernel = void (*)(const TileArgs<T>);
+template <class T, int W, bool ARENA>
+TileKernel<T> pass1_variant(int limiter, int time_mode) {
+    if constexpr (W == 8) {
+        return tile_pass1_kernel<T, W, ARENA, -1, -1>;
+    } else {
+        const bool lam = time_mode != TM_FIXED;
+        if (limiter == LIM_BJ) return lam ? tile_pass1_kernel<T, W, ARENA, LIM_BJ, 1> : tile_pass1_kernel<T, W, ARENA, LIM_BJ, 0>;
+        return lam ? tile_pass1_kernel<T, W, ARENA, LIM_VENKAT, 1> : tile_pass1_kernel<T, W, ARENA, LIM_VENKAT, 0>;
+    }
+}
+template <class T, int W, bool ARENA>
+TileKernel<T> pass2_variant(int rec, int time_mode) {
+    if constexpr (W == 8) {
+        return tile_pass2_kernel<T, W, ARENA, -1, -1>;
+    } else {
+        const bool local = time_mode == TM_LOCAL;
+        if constexpr (!ARENA)
+            if (rec == 7) return local ? tile_pass2_kernel<T, W, ARENA, 7, 1> : tile_pass2_kernel<T, W, ARENA, 7, 0>;
+        return local ? tile_pass2_kernel<T, W, ARENA, 8, 1> : tile_pass2_kernel<T, W, ARENA, 8, 0>;
+    }
 }
 
 // Face records in tile order, pair-major per tile, rec values each (8 or 7; see rplane):
