@@ -133,6 +133,10 @@ __device__ __forceinline__ void tile_info(const TileArgs<T>& a, int t, int& base
     }
 }
 
+struct TileDesc {
+    int base, nb, f0, nf, h0, nh, inst;
+};
+
 // What the compute warps need of a tile besides its data, written by the producer into the
 // stage header with the tile's copies (published by the same mbarrier), so that the compute
 // warps start a tile without dependent global loads: its descriptor, and for its instance
@@ -333,41 +337,85 @@ __device__ __forceinline__ void compute_sync(int nthreads) {
 // Once any wait of the CTA has given up, the producer issues nothing more; before it
 // returns it waits for the copies it has issued (the last armed phase of each buffer; earlier
 // ones completed before their buffer was re-armed), so no copy lands after the CTA exits.
-// Tile queue: lane 0 of the producer warp issues the claim of a tile at the top of an
-// iteration (claim_issue) and the warp takes its result at the end (claim_take), so that the
-// atomic's round trip overlaps the iteration's staging.
-template <class T>
-__device__ __forceinline__ int claim_issue(const TileArgs<T>& a, int lane) {
-    return (a.claim && lane == 0) ? atomicAdd(a.claim, 1) : 0;
-}
-template <class T>
-__device__ __forceinline__ int claim_take(const TileArgs<T>& a, int t, int pending) {
-    if (!a.claim) return t + (int) gridDim.x;
-    return (int) gridDim.x + __shfl_sync(0xffffffffu, pending, 0);
+template <class T>   // within the arrays and the staging capacity
+__device__ __forceinline__ bool desc_ok(const TileArgs<T>& a, const TileDesc& d) {
+    return d.base >= 0 && d.nb >= 0 && d.nb <= a.B && d.base + d.nb <= a.ps && d.base + a.B <= a.ncap && d.f0 >= 0 &&
+           d.nf >= 0 && d.nf <= a.Fmax && d.f0 + d.nf <= a.nentries && d.h0 >= 0 && d.nh >= 0 && d.nh <= a.Hmax &&
+           d.h0 + d.nh <= a.nhalo;
 }
 
+// The producer's own latencies are pipelined over tiles: while tile t0 is staged, the halo ids and
+// instance scalars of t1, the descriptor of t2 and the claim of the tile after it are on their way.
+// Done one after the other for each tile they made the producer the slower side (5,200 cycles a
+// tile in FP64 pass 1 and 4,700-5,500 in the FP32 passes, where computing one takes 3,500 and
+// 1,700-2,000).
 template <class T, bool PASS2, bool ARENA>
 __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned char* smem, unsigned long long* full,
                                               unsigned long long* empty, const TileSmem<T>& L) {
     const int lane = threadIdx.x & 31;
     constexpr int CU = sizeof(Cell4<T>) / 16, CG = PASS2 ? sizeof(Grad8<T>) / 16 : 0;
+    constexpr int KH = 4;          // halo ids a lane holds for the next tile (128 a tile; the rest are loaded late)
     const int NL = a.B + a.Hmax;   // plane stride of the staged cells
     volatile int* abort = abort_word(smem);
     int armed[2] = {-1, -1};       // last iteration whose copies were issued into each buffer
-    unsigned iter = 0;
-    // the current tile t and the next tn are known at the top of an iteration; the tile after
-    // tn is claimed during the iteration
-    int t = blockIdx.x;
-    int tn = claim_take(a, t, claim_issue(a, lane));
-    int pending = 0;
-    for (;; iter++, t = tn, tn = t < a.ntiles ? claim_take(a, t, pending) : t) {
+    // dt or CFL number, dt minimum (pass 2) and step count of the tile's instance; none of them changes
+    // during the kernel in a way the kernel reads (dt minima and step counts come from earlier kernels)
+    struct Scalars {
+        double dt, dtmin;
+        long long steps;
+    };
+    auto load_scalars = [&](int inst, Scalars& v) {
+        if constexpr (ARENA) {
+            v.dt = __ldg(a.inst_dt + inst);
+            v.dtmin = PASS2 ? __longlong_as_double((long long) a.inst_dtmin[2 * inst + a.par]) : 0.0;
+            v.steps = PASS2 ? 0 : a.inst_stats[inst].steps;
+        } else {
+            v.dt = a.s.dt_or_cfl;
+            v.dtmin = PASS2 ? __longlong_as_double((long long) *a.s.dtmin) : 0.0;
+            v.steps = PASS2 ? 0 : a.s.stats->steps;
+        }
+    };
+    auto describe = [&](int tile, TileDesc& d) {
+        if (tile < a.ntiles) tile_info<ARENA>(a, tile, d.base, d.nb, d.f0, d.nf, d.h0, d.nh, d.inst);
+        if constexpr (kChecked)
+            if (tile < a.ntiles && !index_ok(desc_ok<T>(a, d), a.err)) d.nb = d.nf = d.nh = -1;   // staged empty
+    };
+    auto load_ids = [&](int tile, const TileDesc& d, int id[KH]) {
+        if (tile >= a.ntiles) return;
+#pragma unroll
+        for (int k = 0; k < KH; k++) {
+            const int h = lane + 32 * k;
+            if (h < d.nh) id[k] = __ldg(a.halo + d.h0 + h);
+        }
+    };
+    int t0 = blockIdx.x, t1, t2;
+    if (a.claim) {
+        const int v = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(a.claim, 2) : 0, 0);
+        t1 = (int) gridDim.x + v;
+        t2 = t1 + 1;
+    } else {
+        t1 = t0 + (int) gridDim.x;
+        t2 = t1 + (int) gridDim.x;
+    }
+    TileDesc d0{}, d1{}, d2{};
+    Scalars v0{}, v1{};
+    int id0[KH], id1[KH];
+    describe(t0, d0);
+    describe(t1, d1);
+    load_ids(t0, d0, id0);
+    load_scalars(d0.inst, v0);
+    v1 = v0;
+    for (unsigned iter = 0;; iter++) {
         const int buf = iter & 1;
-        if (tn < a.ntiles) pending = claim_issue(a, lane);
+        describe(t2, d2);
+        load_ids(t1, d1, id1);
+        if (ARENA && t1 < a.ntiles) load_scalars(d1.inst, v1);
+        const int pending = (a.claim && lane == 0 && t2 < a.ntiles) ? atomicAdd(a.claim, 1) : 0;
         if (__any_sync(0xffffffffu, *abort)) break;
-        if (t >= a.ntiles) {
+        if (iter >= 2 && !__all_sync(0xffffffffu, mbar_wait(empty + buf, ((iter >> 1) - 1) & 1, a.polls, a.err, abort)))
+            break;
+        if (t0 >= a.ntiles) {
             // no more tiles: a stage with tile -1 and nothing copied ends the compute warps' loop
-            if (iter >= 2 && !__all_sync(0xffffffffu, mbar_wait(empty + buf, ((iter >> 1) - 1) & 1, a.polls, a.err, abort)))
-                break;
             if (lane == 0) {
                 reinterpret_cast<StageInfo*>(smem + 64)[buf].t = -1;
                 mbar_arrive_expect_tx(full + buf, 0u);
@@ -376,91 +424,73 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
             armed[buf] = (int) iter;
             break;
         }
-        // the tile's descriptor and its instance's scalars are loaded before the wait for the
-        // stage, so that their latency hides behind it (none of them changes during the kernel
-        // in a way the kernel reads: dt minima and step counts come from earlier kernels)
-        int base, nb, f0, nf, h0, nh, inst;
-        tile_info<ARENA>(a, t, base, nb, f0, nf, h0, nh, inst);
-        double v_dt = 0.0, v_dtmin = 0.0;
-        long long v_steps = 0;
-        int v_next = -1;
-        if (lane == 0) {
-            if constexpr (ARENA) {
-                v_dt = __ldg(a.inst_dt + inst);
-                v_dtmin = __longlong_as_double((long long) a.inst_dtmin[2 * inst + a.par]);
-                v_steps = a.inst_stats[inst].steps;
-                if (!PASS2 && tn < a.ntiles) v_next = __ldg(&a.tiles[2 * tn].w);
-            } else {
-                v_dt = a.s.dt_or_cfl;
-                v_dtmin = __longlong_as_double((long long) *a.s.dtmin);
-                v_steps = a.s.stats->steps;
-            }
-        }
-        if (iter >= 2 && !__all_sync(0xffffffffu, mbar_wait(empty + buf, ((iter >> 1) - 1) & 1, a.polls, a.err, abort)))
-            break;
-        if (t == a.skip_tile) continue;      // failure injection: nothing armed, nothing in flight
-        bool good = true;
-        if constexpr (kChecked) {
-            // a descriptor outside the arrays or the staging capacity: the tile is staged empty
-            good = index_ok(base >= 0 && nb >= 0 && nb <= a.B && base + nb <= a.ps && base + a.B <= a.ncap &&
-                            f0 >= 0 && nf >= 0 && nf <= a.Fmax && f0 + nf <= a.nentries &&
-                            h0 >= 0 && nh >= 0 && nh <= a.Hmax && h0 + nh <= a.nhalo, a.err);
-            if (!good) nb = nf = nh = 0;
-        }
-        unsigned char* st = smem + kHeader + buf * L.stage;
-        Cell4<T>* sU = reinterpret_cast<Cell4<T>*>(st + L.u);
-        Grad8<T>* sG = reinterpret_cast<Grad8<T>*>(st + L.g);
-        if (lane == 0) {
-            const unsigned bu = nb * sizeof(Cell4<T>), bg = PASS2 ? nb * sizeof(Grad8<T>) : 0u;
-            const unsigned bf = nf * a.rec * (unsigned) sizeof(T), bm = PASS2 ? nf * 4u : 0u;
-            const unsigned bs = a.B * a.Wp * sizeof(unsigned), bi = a.B * sizeof(T);
-            // the tile's descriptor and instance scalars, published by the release of the
-            // arrive below
-            StageInfo* si = reinterpret_cast<StageInfo*>(smem + 64) + buf;
-            si->base = base; si->nb = nb; si->f0 = f0; si->nf = nf; si->h0 = h0; si->nh = nh; si->inst = inst;
-            si->t = t;
-            si->next_inst = v_next;                  // pass 1 in arena mode only
-            si->dt_or_cfl = v_dt;
-            si->dtmin = v_dtmin;
-            si->steps = v_steps;
-            if (!good) {
-                mbar_arrive_expect_tx(full + buf, 0u);   // nothing copied (checked build)
-            } else {
-            mbar_arrive_expect_tx(full + buf, bu + bg + bf + bm + bs + bi);
-            // one bulk copy per 16-byte chunk plane of the tile's cell range
+        if (t0 != a.skip_tile) {             // failure injection: nothing armed, nothing in flight
+            const bool good = !kChecked || d0.nb >= 0;
+            const int base = d0.base, nb = good ? d0.nb : 0, nf = good ? d0.nf : 0, nh = good ? d0.nh : 0;
+            unsigned char* st = smem + kHeader + buf * L.stage;
+            Cell4<T>* sU = reinterpret_cast<Cell4<T>*>(st + L.u);
+            Grad8<T>* sG = reinterpret_cast<Grad8<T>*>(st + L.g);
+            if (lane == 0) {
+                const unsigned bu = nb * sizeof(Cell4<T>), bg = PASS2 ? nb * sizeof(Grad8<T>) : 0u;
+                const unsigned bf = nf * a.rec * (unsigned) sizeof(T), bm = PASS2 ? nf * 4u : 0u;
+                const unsigned bs = a.B * a.Wp * sizeof(unsigned), bi = a.B * sizeof(T);
+                // the tile's descriptor and instance scalars, published by the release of the
+                // arrive below
+                StageInfo* si = reinterpret_cast<StageInfo*>(smem + 64) + buf;
+                si->base = base; si->nb = nb; si->f0 = d0.f0; si->nf = nf; si->h0 = d0.h0; si->nh = nh; si->inst = d0.inst;
+                si->t = t0;
+                si->next_inst = (ARENA && !PASS2 && t1 < a.ntiles) ? d1.inst : -1;
+                si->dt_or_cfl = v0.dt;
+                si->dtmin = v0.dtmin;
+                si->steps = v0.steps;
+                if (!good) {
+                    mbar_arrive_expect_tx(full + buf, 0u);   // nothing copied (checked build)
+                } else {
+                    mbar_arrive_expect_tx(full + buf, bu + bg + bf + bm + bs + bi);
+                    // one bulk copy per 16-byte chunk plane of the tile's cell range
 #pragma unroll
-            for (int j = 0; j < CU; j++)
-                bulk_g2s(reinterpret_cast<char*>(sU) + (size_t) 16 * j * NL,
-                         reinterpret_cast<const char*>(a.s.U) + 16 * ((size_t) j * a.ps + base), nb * 16u, full + buf);
-            if (PASS2) {
+                    for (int j = 0; j < CU; j++)
+                        bulk_g2s(reinterpret_cast<char*>(sU) + (size_t) 16 * j * NL,
+                                 reinterpret_cast<const char*>(a.s.U) + 16 * ((size_t) j * a.ps + base), nb * 16u, full + buf);
+                    if (PASS2) {
+#pragma unroll
+                        for (int j = 0; j < CG; j++)
+                            bulk_g2s(reinterpret_cast<char*>(sG) + (size_t) 16 * j * NL,
+                                     reinterpret_cast<const char*>(a.s.phiG) + 16 * ((size_t) j * a.ps + base), nb * 16u,
+                                     full + buf);
+                    }
+                    if (bf) {
+                        bulk_g2s(st + L.geo, a.tgeo + (size_t) d0.f0 * a.rec, bf, full + buf);
+                        if (PASS2) bulk_g2s(st + L.meta, a.tmeta + d0.f0, bm, full + buf);
+                    }
+                    bulk_g2s(st + L.nbr, a.nbr + (size_t) base * a.Wp, bs, full + buf);
+                    bulk_g2s(st + L.iv, a.s.iv + base, bi, full + buf);
+                }
+            }
+            auto gather = [&](int h, int ci) {
+                if (!index_ok(ci >= 0 && ci < a.ps, a.err)) return;
+#pragma unroll
+                for (int j = 0; j < CU; j++)
+                    cp_async16(reinterpret_cast<char*>(sU) + 16 * ((size_t) j * NL + a.B + h),
+                               reinterpret_cast<const char*>(a.s.U) + 16 * ((size_t) j * a.ps + ci));
 #pragma unroll
                 for (int j = 0; j < CG; j++)
-                    bulk_g2s(reinterpret_cast<char*>(sG) + (size_t) 16 * j * NL,
-                             reinterpret_cast<const char*>(a.s.phiG) + 16 * ((size_t) j * a.ps + base), nb * 16u,
-                             full + buf);
-            }
-            if (bf) {
-                bulk_g2s(st + L.geo, a.tgeo + (size_t) f0 * a.rec, bf, full + buf);
-                if (PASS2) bulk_g2s(st + L.meta, a.tmeta + f0, bm, full + buf);
-            }
-            bulk_g2s(st + L.nbr, a.nbr + (size_t) base * a.Wp, bs, full + buf);
-            bulk_g2s(st + L.iv, a.s.iv + base, bi, full + buf);
-            }
-        }
-        for (int h = lane; h < nh; h += 32) {
-            const int ci = __ldg(a.halo + h0 + h);
-            if (!index_ok(ci >= 0 && ci < a.ps, a.err)) continue;
+                    cp_async16(reinterpret_cast<char*>(sG) + 16 * ((size_t) j * NL + a.B + h),
+                               reinterpret_cast<const char*>(a.s.phiG) + 16 * ((size_t) j * a.ps + ci));
+            };
 #pragma unroll
-            for (int j = 0; j < CU; j++)
-                cp_async16(reinterpret_cast<char*>(sU) + 16 * ((size_t) j * NL + a.B + h),
-                           reinterpret_cast<const char*>(a.s.U) + 16 * ((size_t) j * a.ps + ci));
-#pragma unroll
-            for (int j = 0; j < CG; j++)
-                cp_async16(reinterpret_cast<char*>(sG) + 16 * ((size_t) j * NL + a.B + h),
-                           reinterpret_cast<const char*>(a.s.phiG) + 16 * ((size_t) j * a.ps + ci));
+            for (int k = 0; k < KH; k++)
+                if (lane + 32 * k < nh) gather(lane + 32 * k, id0[k]);
+            for (int h = lane + 32 * KH; h < nh; h += 32) gather(h, __ldg(a.halo + d0.h0 + h));
+            cp_async_arrive_noinc(full + buf);
+            armed[buf] = (int) iter;
         }
-        cp_async_arrive_noinc(full + buf);
-        armed[buf] = (int) iter;
+        t0 = t1; d0 = d1; v0 = v1;
+#pragma unroll
+        for (int k = 0; k < KH; k++) id0[k] = id1[k];
+        t1 = t2; d1 = d2;
+        if (t2 < a.ntiles)
+            t2 = a.claim ? (int) gridDim.x + __shfl_sync(0xffffffffu, pending, 0) : t2 + (int) gridDim.x;
     }
     cp_async_wait_all();
     for (int b = 0; b < 2; b++)
