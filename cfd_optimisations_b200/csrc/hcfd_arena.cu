@@ -250,8 +250,7 @@ struct hcfd_arena {
     int time_mode = HCFD_GLOBAL_CFL;
     size_t smem1 = 0, smem2 = 0;
     int grid1 = 0, grid2 = 0;
-    cudaGraphExec_t graph = nullptr;
-    int graph_steps = 0;
+    bool first_res = true;               // the next step's residual is wanted (see hcfd_arena_step)
     long long steps_done = 0;
     bool fp32() const { return prm.precision == HCFD_FP32; }
 };
@@ -270,10 +269,6 @@ struct hcfd_admission {
 };
 
 namespace {
-
-void free_graph(hcfd_arena* a) {
-    if (a->graph) { cudaGraphExecDestroy(a->graph); a->graph = nullptr; a->graph_steps = 0; }
-}
 
 // Orders the step stream after every admission enqueued so far (device-side wait).
 int wait_admissions(hcfd_arena* A) {
@@ -328,17 +323,20 @@ hcfd::TileArgs<T> arena_args(hcfd_arena* A, int cur, int par) {
 }
 
 template <class T, int W>
-int enqueue_step(hcfd_arena* A, int cur, int par) {
+int enqueue_step(hcfd_arena* A, int cur, int par, bool want_res) {
     hcfd::TileArgs<T> a = arena_args<T>(A, cur, par);
+    a.want_res = want_res ? 1 : 0;
     // pass 1 takes its tiles from a queue (per-instance dt minima are order-free), and pass 2,
     // which runs between two pass-1 launches, zeroes it; pass 2 takes every grid-th tile
     // (measured faster for it than a queue)
     a.claim = A->queue;
     a.claim_reset = nullptr;
-    hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->time_mode)<<<A->grid1, A->B + 32, A->smem1, A->stream>>>(a);
+    CK(hcfd::launch_dependent(hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->time_mode), A->grid1, A->B + 32, A->smem1,
+                              A->stream, a));
     a.claim = nullptr;
     a.claim_reset = A->queue;
-    hcfd::pass2_variant<T, W, true>(8, A->time_mode)<<<A->grid2, A->B + 32, A->smem2, A->stream>>>(a);
+    CK(hcfd::launch_dependent(hcfd::pass2_variant<T, W, true>(8, A->time_mode), A->grid2, A->B + 32, A->smem2, A->stream, a));
+    if (!want_res) return HCFD_OK;
     arena_chunk_kernel<<<A->nchunks, 256, 0, A->stream>>>(A->chunks, A->tile_r2, A->tile_bad, A->chunk_r2, A->chunk_bad);
     arena_finalize_kernel<<<(A->nact + 127) / 128, 128, 0, A->stream>>>(A->nact, A->nchunks, A->act, A->chunk_r2,
                                                                        A->chunk_bad, A->inst_dt, A->inst_dtmin, A->stats,
@@ -348,8 +346,8 @@ int enqueue_step(hcfd_arena* A, int cur, int par) {
 }
 
 template <class T>
-int enqueue_step_w(hcfd_arena* A, int cur, int par) {
-    return A->W == 3 ? enqueue_step<T, 3>(A, cur, par) : enqueue_step<T, 4>(A, cur, par);
+int enqueue_step_w(hcfd_arena* A, int cur, int par, bool want_res) {
+    return A->W == 3 ? enqueue_step<T, 3>(A, cur, par, want_res) : enqueue_step<T, 4>(A, cur, par, want_res);
 }
 
 template <class T, int W>
@@ -429,7 +427,7 @@ int rebuild_active(hcfd_arena* A) {
     if (!chk.empty()) CK(cudaMemcpyAsync(A->chunks, chk.data(), sizeof(int4) * chk.size(), cudaMemcpyHostToDevice, A->stream));
     CK(cudaEventRecord(A->list_ev, A->stream));
     A->list_pending = true;
-    free_graph(A);
+    A->first_res = true;
     A->Hcur = hmax;
     A->Fcur = fmax;
     A->dirty = false;
@@ -451,7 +449,6 @@ void arena_free(hcfd_arena* A) {
     cudaSetDevice(A->device);
     if (A->astream) cudaStreamSynchronize(A->astream);
     if (A->stream) cudaStreamSynchronize(A->stream);
-    free_graph(A);
     for (auto& I : A->inst) if (I.d_perm) cudaFree(I.d_perm);
     if (A->admit_ev) cudaEventDestroy(A->admit_ev);
     if (A->list_ev) cudaEventDestroy(A->list_ev);
@@ -528,7 +525,7 @@ int hcfd_arena_create(const hcfd_arena_params* prm, hcfd_arena** out) {
         (rc = dalloc((char**) &h->phiG, 8 * ts * C)) || (rc = dalloc((char**) &h->iv, ts * C)) ||
         (p.freeze_limiter_after > 0 && (rc = dalloc((char**) &h->phiF, 4 * ts * C))) ||
         (rc = dalloc(&h->nbr, h->Wp * C)) || (rc = dalloc((char**) &h->tgeo, 8 * ts * h->Ecap)) ||
-        (rc = dalloc(&h->tmeta, h->Ecap)) || (rc = dalloc(&h->halo, h->HLcap)) ||
+        (rc = dalloc(&h->tmeta, h->Ecap)) || (rc = dalloc(&h->halo, h->HLcap + 1)) ||
         (rc = dalloc(&h->inst_dt, p.max_instances)) || (rc = dalloc(&h->inst_dtmin, 2 * (size_t) p.max_instances)) ||
         (rc = dalloc(&h->inst_bc, p.max_instances)) || (rc = dalloc(&h->stats, p.max_instances)) ||
         (rc = dalloc(&h->tiles, 2 * h->tiles_cap)) || (rc = dalloc(&h->act, p.max_instances)) ||
@@ -643,7 +640,8 @@ int hcfd_arena_admit_prepared(hcfd_arena* A, const hcfd_admission* D, int* slot_
         d[3] = slot;
         d[4] = (int) (I.h0 + P.hoff[t]);
         d[5] = P.hoff[t + 1] - P.hoff[t];
-        d[6] = d[7] = 0;
+        d[6] = t == 0;
+        d[7] = 0;
     }
     // device work: geometry of this mesh (stream-ordered temporaries), then the arena ranges
     cudaStream_t st = A->astream;
@@ -767,32 +765,16 @@ int hcfd_arena_step(hcfd_arena* A, int nsteps) {
         if (rc) return rc;
     }
     if (A->nact == 0 || nsteps == 0) return HCFD_OK;
-    // one graph holds two steps (the ping-pong buffers and dt slots return to their start)
-    if (!A->graph) {
-        cudaGraph_t g;
-        CK(cudaStreamBeginCapture(A->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = HCFD_OK;
-        for (int k = 0; k < 2 && rc == HCFD_OK; k++)
-            rc = A->fp32() ? enqueue_step_w<float>(A, A->cur ^ k, A->par ^ k) : enqueue_step_w<double>(A, A->cur ^ k, A->par ^ k);
-        cudaError_t e = cudaStreamEndCapture(A->stream, &g);
+    // A residual is formed in the first step after the active list changed (it may be an instance's
+    // first) and in the call's last; the others are two launches, each started under the tail of
+    // the one before.
+    for (int k = 0; k < nsteps; k++) {
+        const bool want_res = k == nsteps - 1 || A->first_res;
+        const int rc = A->fp32() ? enqueue_step_w<float>(A, A->cur, A->par, want_res) : enqueue_step_w<double>(A, A->cur, A->par, want_res);
         if (rc) return rc;
-        if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("arena_step: capture: ") + cudaGetErrorString(e));
-        e = cudaGraphInstantiate(&A->graph, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("arena_step: instantiate: ") + cudaGetErrorString(e));
-        A->graph_steps = 2;
-    }
-    int n = nsteps;
-    while (n >= 2) {
-        CK(cudaGraphLaunch(A->graph, A->stream));
-        n -= 2;
-    }
-    if (n == 1) {
-        int rc = A->fp32() ? enqueue_step_w<float>(A, A->cur, A->par) : enqueue_step_w<double>(A, A->cur, A->par);
-        if (rc) return rc;
+        A->first_res = false;
         A->cur ^= 1;
         A->par ^= 1;
-        free_graph(A);   // the graph was captured for the other parity
     }
     A->steps_done += nsteps;
     return HCFD_OK;
@@ -940,6 +922,7 @@ int hcfd_arena_restore(hcfd_arena* A, int slot, const char* path) {
     st.steps = h.steps;
     st.nonfinite = h.nonfinite;
     if (e == cudaSuccess) e = cudaMemcpyAsync(A->stats + slot, &st, sizeof(st), cudaMemcpyHostToDevice, A->stream);
+    A->first_res = true;
     cudaFreeAsync(d_in, A->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(A->stream);
     if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("arena_restore: ") + cudaGetErrorString(e));

@@ -125,6 +125,7 @@ struct hcfd_solver {
     cudaGraphExec_t graph = nullptr;
     int g_mode = -1, g_cur = -1;
     double g_value = 0.0;
+    bool first_res = true;               // the next step may be a solve's first: its residual is wanted
     bool prof = false;
     int prof_every = 1;                  // record every prof_every-th step
     long long prof_count = 0;
@@ -190,7 +191,7 @@ hcfd::StepArgs<T> step_args(hcfd_solver* s, int time_mode, double dt_or_cfl) {
 }
 
 template <class T>
-hcfd::TileArgs<T> tile_args(hcfd_solver* s, int time_mode, double dt_or_cfl, const TiledPass& P, int pass) {
+hcfd::TileArgs<T> tile_args(hcfd_solver* s, int time_mode, double dt_or_cfl, const TiledPass& P, int pass, bool want_res = true) {
     hcfd::TileArgs<T> a;
     int* q1 = s->queue1 ? (int*) s->d_counter + 1 : nullptr;
     int* q2 = s->queue2 ? (int*) s->d_counter + 2 : nullptr;
@@ -220,9 +221,11 @@ hcfd::TileArgs<T> tile_args(hcfd_solver* s, int time_mode, double dt_or_cfl, con
     a.inst_dt = nullptr;
     a.inst_dtmin = nullptr;
     a.inst_bc = nullptr;
+    a.inst_stats = nullptr;
     a.tile_r2 = nullptr;
     a.tile_bad = nullptr;
     a.par = 0;
+    a.want_res = want_res ? 1 : 0;
     return a;
 }
 
@@ -288,7 +291,7 @@ int launch_resident_w(hcfd_solver* s, int time_mode, double dt_or_cfl, int nstep
 }
 
 template <class T, int W>
-int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl) {
+int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl, bool want_res) {
     Ev e1, e2;
     int rc;
     const bool rec = s->prof && (s->prof_count++ % s->prof_every == 0);
@@ -304,12 +307,14 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl) {
     if (s->tiled) {
         const TiledPass& P2 = s->split ? s->tp[1] : s->tp[0];
         const hcfd::TileArgs<T> a1 = tile_args<T>(s, time_mode, dt_or_cfl, s->tp[0], 1);
-        const hcfd::TileArgs<T> a2 = tile_args<T>(s, time_mode, dt_or_cfl, P2, 2);
+        const hcfd::TileArgs<T> a2 = tile_args<T>(s, time_mode, dt_or_cfl, P2, 2, want_res);
         if ((rc = prof_begin(s, rec, e1))) return rc;
-        hcfd::pass1_variant<T, W, false>(s->prm.limiter, time_mode)<<<s->grid1, s->tp[0].block + 32, s->smem1, s->stream>>>(a1);
+        CK(hcfd::launch_dependent(hcfd::pass1_variant<T, W, false>(s->prm.limiter, time_mode), s->grid1, s->tp[0].block + 32,
+                                  s->smem1, s->stream, a1));
         if ((rc = prof_end(s, rec, e1, s->ev1))) return rc;
         if ((rc = prof_begin(s, rec, e2))) return rc;
-        hcfd::pass2_variant<T, W, false>(P2.rec, time_mode)<<<s->grid2, P2.block + 32, s->smem2, s->stream>>>(a2);
+        CK(hcfd::launch_dependent(hcfd::pass2_variant<T, W, false>(P2.rec, time_mode), s->grid2, P2.block + 32, s->smem2,
+                                  s->stream, a2));
         if ((rc = prof_end(s, rec, e2, s->ev2))) return rc;
     } else {
         const int grid = nblk(s->Nc, s->block);
@@ -327,11 +332,11 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl) {
 }
 
 template <class T>
-int launch_step_w(hcfd_solver* s, int time_mode, double dt_or_cfl) {
+int launch_step_w(hcfd_solver* s, int time_mode, double dt_or_cfl, bool want_res = true) {
     switch (s->W) {
-    case 3: return launch_step<T, 3>(s, time_mode, dt_or_cfl);
-    case 4: return launch_step<T, 4>(s, time_mode, dt_or_cfl);
-    default: return launch_step<T, 8>(s, time_mode, dt_or_cfl);
+    case 3: return launch_step<T, 3>(s, time_mode, dt_or_cfl, want_res);
+    case 4: return launch_step<T, 4>(s, time_mode, dt_or_cfl, want_res);
+    default: return launch_step<T, 8>(s, time_mode, dt_or_cfl, want_res);
     }
 }
 
@@ -779,6 +784,7 @@ int hcfd_gpu_initialise(hcfd_solver* s, const double* qic) {
     CK(cudaMemcpyAsync(s->d_dtmin, inf2, sizeof(inf2), cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     s->initialised = true;
+    s->first_res = true;
     return HCFD_OK;
 }
 
@@ -812,9 +818,11 @@ int hcfd_gpu_step(hcfd_solver* s, int nsteps, int time_mode, double dt_or_cfl, h
         n -= k;
     }
     while (n > 0) {
-        // pairs of steps without per-kernel events run as the graph; profiled steps run eagerly
+        // Per-cell kernels: pairs of steps without per-kernel events run as the graph, profiled steps
+        // eagerly.  The tiled kernels, whose launches take less host time than they run, each start
+        // under the tail of the one before (launch_dependent), which a graph would end every two steps.
         const bool rec = s->prof && (s->prof_count % s->prof_every == 0 || (s->prof_count + 1) % s->prof_every == 0);
-        if (n >= 2 && !rec && !s->resident) {
+        if (n >= 2 && !rec && !s->tiled) {
             if (s->graph && (s->g_mode != time_mode || s->g_value != dt_or_cfl || s->g_cur != s->cur)) {
                 cudaGraphExecDestroy(s->graph);
                 s->graph = nullptr;
@@ -845,8 +853,11 @@ int hcfd_gpu_step(hcfd_solver* s, int nsteps, int time_mode, double dt_or_cfl, h
             if (s->prof) s->prof_count += 2;
             n -= 2;
         } else {
-            rc = s->fp32() ? launch_step_w<float>(s, time_mode, dt_or_cfl) : launch_step_w<double>(s, time_mode, dt_or_cfl);
+            const bool want_res = n == 1 || s->first_res;
+            rc = s->fp32() ? launch_step_w<float>(s, time_mode, dt_or_cfl, want_res)
+                           : launch_step_w<double>(s, time_mode, dt_or_cfl, want_res);
             if (rc) return rc;
+            s->first_res = false;
             n -= 1;
         }
     }
@@ -1055,6 +1066,7 @@ int hcfd_gpu_restore(hcfd_solver* s, const char* path) {
     st.nonfinite = h.nonfinite;
     CK(cudaMemcpyAsync(s->d_stats, &st, sizeof(st), cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));
+    s->first_res = true;
     s->initialised = true;
     return HCFD_OK;
 }

@@ -38,21 +38,24 @@ struct TileArgs {
     int ps;                                // plane stride of the cell planes (Nc, or the arena's capacity)
     // Arena mode (many meshes in one flat arena; see hcfd_arena.cu).  Tile i of the active
     // list is described by tiles[2i] = {first cell, first entry, entries, instance} and
-    // tiles[2i+1] = {first halo id, halo count, -, -}; every arena tile holds B cells.
+    // tiles[2i+1] = {first halo id, halo count, instance's first tile, -}; every arena tile holds B cells.
     const int4* __restrict__ tiles;
     const double* __restrict__ inst_dt;    // per instance: dt (fixed mode) or CFL number
     unsigned long long* inst_dtmin;        // per instance, two parity slots (double bits)
     const BCTable* __restrict__ inst_bc;   // per instance
-    const StepStats* inst_stats;           // per instance (step counts for limiter freezing)
+    StepStats* inst_stats;                 // per instance
     double* tile_r2;                       // per active tile and compute warp (t * B/32 + warp): sum of R_rho^2
     int* tile_bad;                         // same layout: a NaN/Inf appeared
     int par;                               // which dtmin slot this step uses
-    // Tile queue: each CTA takes tile blockIdx.x first, then, with `claim` set, the tile
-    // gridDim.x + atomicAdd(claim, 1) (CTAs that finish early take more tiles), else every
-    // gridDim.x-th tile.  `claim_reset` (the other pass's queue) is zeroed by this kernel:
+    // Tile queue: each CTA takes three tiles by position first (every gridDim.x-th from blockIdx.x),
+    // then, with `claim` set, the tile 3 gridDim.x + atomicAdd(claim, 1) (CTAs that finish early take more
+    // tiles), else every gridDim.x-th tile.  `claim_reset` (the other pass's queue) is zeroed by this kernel:
     // the other pass runs before and after it in stream order, never during it.
     int* claim;
     int* claim_reset;
+    // Pass 2: whether this step's residual is wanted (the first of a solve, for res2_first, and
+    // the last of a call, for whoever asks); steps without it skip the squares and their sums.
+    int want_res;
     long long nentries, nhalo, ncap;       // lengths of tgeo/tmeta (entries), halo, and of the
                                            // per-cell arrays iv/nbr (cells): checked build
 };
@@ -134,7 +137,7 @@ __device__ __forceinline__ void tile_info(const TileArgs<T>& a, int t, int& base
 }
 
 struct TileDesc {
-    int base, nb, f0, nf, h0, nh, inst;
+    int base, nb, f0, nf, h0, nh, inst, first;
 };
 
 // What the compute warps need of a tile besides its data, written by the producer into the
@@ -147,7 +150,7 @@ struct StageInfo {
     double dtmin;
     long long steps;
     int t;                                            // the tile, or -1: the CTA has no more tiles
-    int pad2;
+    int first;                                        // (arena) the instance's first tile
 };
 static_assert(sizeof(StageInfo) == 64, "stage info is 64 bytes");
 // Header of a CTA's shared memory: full[2] and empty[2] mbarriers (bytes 0-31), the abort
@@ -167,6 +170,17 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned coun
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// Programmatic dependent launch: lets the next kernel of the stream start once every CTA of this one
+// has called it or left; waits for the kernel before it (its writes included).  A kernel launched without the attribute
+// passes both at once.
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
@@ -315,9 +329,6 @@ struct TileSmem {
     }
 };
 
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 // Arrival on `bar` once all cp.async operations issued so far by this thread have landed;
 // counts as one of the barrier's expected arrivals (.noinc).
 __device__ __forceinline__ void cp_async_arrive_noinc(unsigned long long* bar) {
@@ -344,11 +355,19 @@ __device__ __forceinline__ bool desc_ok(const TileArgs<T>& a, const TileDesc& d)
            d.h0 + d.nh <= a.nhalo;
 }
 
+// The next tile of the queue, a predicated atomic: with a branch around it the warp would wait for
+// the result where the branch ends, not where the tile is needed.
+__device__ __forceinline__ void claim_tile(int* queue, bool on, int& tile) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p atom.global.add.u32 %0, [%1], 1;\n\t}"
+                 : "+r"(tile) : "l"(queue), "r"((int) on) : "memory");
+}
+
 // The producer's own latencies are pipelined over tiles: while tile t0 is staged, the halo ids and
 // instance scalars of t1, the descriptor of t2 and the claim of the tile after it are on their way.
 // Done one after the other for each tile they made the producer the slower side (5,200 cycles a
 // tile in FP64 pass 1 and 4,700-5,500 in the FP32 passes, where computing one takes 3,500 and
-// 1,700-2,000).
+// 1,700-2,000).  A deeper pipeline of claims (five tiles by position, results taken up an iteration
+// later) cost FP64 2 % at 2001x1001: tiles claimed early are tiles the CTAs that end first cannot take.
 template <class T, bool PASS2, bool ARENA>
 __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned char* smem, unsigned long long* full,
                                               unsigned long long* empty, const TileSmem<T>& L) {
@@ -375,47 +394,94 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
             v.steps = PASS2 ? 0 : a.s.stats->steps;
         }
     };
-    auto describe = [&](int tile, TileDesc& d) {
-        if (tile < a.ntiles) tile_info<ARENA>(a, tile, d.base, d.nb, d.f0, d.nf, d.h0, d.nh, d.inst);
-        if constexpr (kChecked)
-            if (tile < a.ntiles && !index_ok(desc_ok<T>(a, d), a.err)) d.nb = d.nf = d.nh = -1;   // staged empty
+    // A descriptor as loaded (nothing computed from it until it is needed, a tile later).
+    struct Raw {
+        int x, y, z, w, u, v, first;
     };
-    auto load_ids = [&](int tile, const TileDesc& d, int id[KH]) {
-        if (tile >= a.ntiles) return;
-#pragma unroll
-        for (int k = 0; k < KH; k++) {
-            const int h = lane + 32 * k;
-            if (h < d.nh) id[k] = __ldg(a.halo + d.h0 + h);
+    // (Not inside a branch, past the end the last tile's is read again: where a branch's sides meet,
+    // the warp would wait for what one of them loaded.)
+    const int last = a.ntiles - 1;
+    auto load_raw = [&](int tile, Raw& q) {
+        tile = min(tile, last);
+        if constexpr (ARENA) {
+            const int4 e0 = __ldg(a.tiles + 2 * tile);
+            const int4 e1 = __ldg(a.tiles + 2 * tile + 1);
+            q = Raw{e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z};
+        } else {
+            q = Raw{__ldg(a.foff + tile), __ldg(a.foff + tile + 1), __ldg(a.hoff + tile), __ldg(a.hoff + tile + 1), 0, 0, 0};
         }
     };
-    int t0 = blockIdx.x, t1, t2;
-    if (a.claim) {
-        const int v = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(a.claim, 2) : 0, 0);
-        t1 = (int) gridDim.x + v;
-        t2 = t1 + 1;
-    } else {
-        t1 = t0 + (int) gridDim.x;
-        t2 = t1 + (int) gridDim.x;
-    }
-    TileDesc d0{}, d1{}, d2{};
+    auto describe = [&](int tile, const Raw& q) {
+        TileDesc d;
+        tile = min(tile, last);
+        if constexpr (ARENA) {
+            d = TileDesc{q.x, a.B, q.y, q.z, q.u, q.v, q.w, q.first};
+        } else {
+            const int base = tile * a.B;
+            d = TileDesc{base, min(a.B, a.s.Nc - base), q.x, q.y - q.x, q.z, q.w - q.z, 0, 0};
+        }
+        if constexpr (kChecked)
+            if (!index_ok(desc_ok<T>(a, d), a.err)) d.nb = d.nf = d.nh = -1;   // staged empty
+        return d;
+    };
+    auto load_ids = [&](int tile, const TileDesc& d, int id[KH]) {
+        // Arena: never inside a branch either (an empty halo reads one past its place, where the list is
+        // padded): its steps took 129 us with the branch, 116 without.  Single mesh, where descriptors
+        // need no instance: only the ids there are (FP32 pass 2 40 us against 35).
+        if (!ARENA && tile >= a.ntiles) return;
+        const int top = max(d.nh - 1, 0);
+#pragma unroll
+        for (int k = 0; k < KH; k++)
+            if (ARENA || lane + 32 * k < d.nh) id[k] = __ldg(a.halo + d.h0 + min(lane + 32 * k, top));
+    };
+    // the first three tiles are the CTA's by position; the queue hands out the rest
+    int t0 = blockIdx.x, t1 = t0 + (int) gridDim.x, t2 = t1 + (int) gridDim.x;
+    TileDesc d0, d1;
+    Raw q0{}, q1{}, q2{};
     Scalars v0{}, v1{};
     int id0[KH], id1[KH];
-    describe(t0, d0);
-    describe(t1, d1);
+    load_raw(t0, q0);
+    load_raw(t1, q1);
+    d0 = describe(t0, q0);
     load_ids(t0, d0, id0);
+    d1 = describe(t1, q1);
+    // Arms stage `buf` for a tile and copies what no kernel writes: its face records and metadata, face
+    // words and 1 / areas.
+    auto stage_static = [&](const TileDesc& d, bool good, int buf) {
+        if (lane != 0) return;
+        const unsigned nb = good ? d.nb : 0, nf = good ? d.nf : 0;
+        const unsigned bu = nb * sizeof(Cell4<T>), bg = PASS2 ? nb * sizeof(Grad8<T>) : 0u;
+        const unsigned bf = nf * a.rec * (unsigned) sizeof(T), bm = PASS2 ? nf * 4u : 0u;
+        const unsigned bs = good ? a.B * a.Wp * sizeof(unsigned) : 0u, bi = good ? a.B * sizeof(T) : 0u;
+        unsigned char* st = smem + kHeader + buf * L.stage;
+        mbar_expect_tx(full + buf, bu + bg + bf + bm + bs + bi);
+        if (bf) {
+            bulk_g2s(st + L.geo, a.tgeo + (size_t) d.f0 * a.rec, bf, full + buf);
+            if (PASS2) bulk_g2s(st + L.meta, a.tmeta + d.f0, bm, full + buf);
+        }
+        if (bs) {
+            bulk_g2s(st + L.nbr, a.nbr + (size_t) d.base * a.Wp, bs, full + buf);
+            bulk_g2s(st + L.iv, a.s.iv + d.base, bi, full + buf);
+        }
+    };
+    // the first tile's while the kernel before this one ends; everything else waits for it
+    if (t0 < a.ntiles && t0 != a.skip_tile) stage_static(d0, !kChecked || d0.nb >= 0, 0);
+    grid_wait_previous();
     load_scalars(d0.inst, v0);
     v1 = v0;
     for (unsigned iter = 0;; iter++) {
         const int buf = iter & 1;
-        describe(t2, d2);
+        load_raw(t2, q2);
         load_ids(t1, d1, id1);
-        if (ARENA && t1 < a.ntiles) load_scalars(d1.inst, v1);
-        const int pending = (a.claim && lane == 0 && t2 < a.ntiles) ? atomicAdd(a.claim, 1) : 0;
+        int pending = 0;
+        if (ARENA) load_scalars(d1.inst, v1);
+        claim_tile(a.claim, a.claim && lane == 0 && t2 < a.ntiles, pending);
         if (__any_sync(0xffffffffu, *abort)) break;
         if (iter >= 2 && !__all_sync(0xffffffffu, mbar_wait(empty + buf, ((iter >> 1) - 1) & 1, a.polls, a.err, abort)))
             break;
         if (t0 >= a.ntiles) {
             // no more tiles: a stage with tile -1 and nothing copied ends the compute warps' loop
+            grid_launch_next();      // this CTA's place falls free soon
             if (lane == 0) {
                 reinterpret_cast<StageInfo*>(smem + 64)[buf].t = -1;
                 mbar_arrive_expect_tx(full + buf, 0u);
@@ -430,41 +496,29 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
             unsigned char* st = smem + kHeader + buf * L.stage;
             Cell4<T>* sU = reinterpret_cast<Cell4<T>*>(st + L.u);
             Grad8<T>* sG = reinterpret_cast<Grad8<T>*>(st + L.g);
+            if (iter) stage_static(d0, good, buf);
             if (lane == 0) {
-                const unsigned bu = nb * sizeof(Cell4<T>), bg = PASS2 ? nb * sizeof(Grad8<T>) : 0u;
-                const unsigned bf = nf * a.rec * (unsigned) sizeof(T), bm = PASS2 ? nf * 4u : 0u;
-                const unsigned bs = a.B * a.Wp * sizeof(unsigned), bi = a.B * sizeof(T);
-                // the tile's descriptor and instance scalars, published by the release of the
-                // arrive below
+                // the tile's descriptor and instance scalars, published by the release of the arrive
                 StageInfo* si = reinterpret_cast<StageInfo*>(smem + 64) + buf;
                 si->base = base; si->nb = nb; si->f0 = d0.f0; si->nf = nf; si->h0 = d0.h0; si->nh = nh; si->inst = d0.inst;
                 si->t = t0;
+                si->first = d0.first;
                 si->next_inst = (ARENA && !PASS2 && t1 < a.ntiles) ? d1.inst : -1;
                 si->dt_or_cfl = v0.dt;
                 si->dtmin = v0.dtmin;
                 si->steps = v0.steps;
-                if (!good) {
-                    mbar_arrive_expect_tx(full + buf, 0u);   // nothing copied (checked build)
-                } else {
-                    mbar_arrive_expect_tx(full + buf, bu + bg + bf + bm + bs + bi);
+                mbar_arrive(full + buf);
+                if (nb) {
                     // one bulk copy per 16-byte chunk plane of the tile's cell range
 #pragma unroll
                     for (int j = 0; j < CU; j++)
                         bulk_g2s(reinterpret_cast<char*>(sU) + (size_t) 16 * j * NL,
                                  reinterpret_cast<const char*>(a.s.U) + 16 * ((size_t) j * a.ps + base), nb * 16u, full + buf);
-                    if (PASS2) {
 #pragma unroll
-                        for (int j = 0; j < CG; j++)
-                            bulk_g2s(reinterpret_cast<char*>(sG) + (size_t) 16 * j * NL,
-                                     reinterpret_cast<const char*>(a.s.phiG) + 16 * ((size_t) j * a.ps + base), nb * 16u,
-                                     full + buf);
-                    }
-                    if (bf) {
-                        bulk_g2s(st + L.geo, a.tgeo + (size_t) d0.f0 * a.rec, bf, full + buf);
-                        if (PASS2) bulk_g2s(st + L.meta, a.tmeta + d0.f0, bm, full + buf);
-                    }
-                    bulk_g2s(st + L.nbr, a.nbr + (size_t) base * a.Wp, bs, full + buf);
-                    bulk_g2s(st + L.iv, a.s.iv + base, bi, full + buf);
+                    for (int j = 0; j < CG; j++)
+                        bulk_g2s(reinterpret_cast<char*>(sG) + (size_t) 16 * j * NL,
+                                 reinterpret_cast<const char*>(a.s.phiG) + 16 * ((size_t) j * a.ps + base), nb * 16u,
+                                 full + buf);
                 }
             }
             auto gather = [&](int h, int ci) {
@@ -488,9 +542,10 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
         t0 = t1; d0 = d1; v0 = v1;
 #pragma unroll
         for (int k = 0; k < KH; k++) id0[k] = id1[k];
-        t1 = t2; d1 = d2;
+        t1 = t2;
+        d1 = describe(t2, q2);
         if (t2 < a.ntiles)
-            t2 = a.claim ? (int) gridDim.x + __shfl_sync(0xffffffffu, pending, 0) : t2 + (int) gridDim.x;
+            t2 = a.claim ? 3 * (int) gridDim.x + __shfl_sync(0xffffffffu, pending, 0) : t2 + (int) gridDim.x;
     }
     cp_async_wait_all();
     for (int b = 0; b < 2; b++)
@@ -698,6 +753,7 @@ __device__ __forceinline__ T cell_update(const T* u, const T* R, T iv, T dt, T* 
     if ((int) threadIdx.x >= NT) {                                                               \
         producer_loop<T, PASS2, ARENA>(a, smem, full, empty, L);                                 \
     } else {                                                                                     \
+    grid_wait_previous();                                                                        \
     if (a.claim_reset && blockIdx.x == 0 && threadIdx.x == 0) *a.claim_reset = 0;               \
     for (unsigned iter = 0;; iter++) {                                                           \
         const int buf = iter & 1;                                                                \
@@ -928,7 +984,7 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
         T dt = T(dt_used);
         if (local) dt = cfl_or_dt * qrcp(iv * cell_wave_sum<T, W>(x, sGeo, nf, rec, u, s.gma, a.err));
         const T Rr = cell_update<4>(u, R, iv, dt, un_, top);
-        r2 += (double) Rr * (double) Rr;
+        if (a.want_res) r2 += (double) Rr * (double) Rr;
         st_cell(s.Unew, a.ps, base + c, un_);
         // ghost refresh (Euler.cpp:96, :138-142): this cell is its ghosts' only neighbour
         bool any = false;
@@ -954,25 +1010,60 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
         }
     }
     if constexpr (ARENA) {
-        // per-tile residual: one partial per warp (fixed order, no barrier); the finalize
-        // kernel sums an instance's partials in order
-        const double w = warp_sum(r2);
         const int wb = __any_sync(0xffffffffu, not_finite<T>(top));
-        if ((threadIdx.x & 31) == 0) {
-            const int k = t * (NT >> 5) + (int) (threadIdx.x >> 5);
-            a.tile_r2[k] = w;
-            a.tile_bad[k] = wb;
+        if (a.want_res) {
+            // per-tile residual: one partial per warp (fixed order, no barrier); the finalize
+            // kernel sums an instance's partials in order and does the step's bookkeeping
+            const double w = warp_sum(r2);
+            if ((threadIdx.x & 31) == 0) {
+                const int k = t * (NT >> 5) + (int) (threadIdx.x >> 5);
+                a.tile_r2[k] = w;
+                a.tile_bad[k] = wb;
+            }
+        } else {
+            if (wb && (threadIdx.x & 31) == 0) atomicOr(&a.inst_stats[inst].nonfinite, 1);
+            if (si.first && threadIdx.x == 0) {
+                a.inst_stats[inst].steps += 1;
+                a.inst_dtmin[2 * inst + (1 - a.par)] = 0x7FF0000000000000ULL;
+            }
         }
         r2 = 0.0;
         top = 0;
     }
     HCFD_TILE_LOOP_END
-    if constexpr (!ARENA) finish_step(s, r2, not_finite<T>(top), dt_used);
+    if constexpr (!ARENA) {
+        if (a.want_res) {
+            finish_step(s, r2, not_finite<T>(top), dt_used);
+        } else {
+            if (not_finite<T>(top)) atomicOr(&s.stats->nonfinite, 1);
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                s.stats->steps += 1;
+                if (s.time_mode != TM_FIXED) *s.dtmin_next = 0x7FF0000000000000ULL;
+            }
+        }
+    }
 }
 
 // The variants of a handle's shape.
 template <class T>
 using TileKernel = void (*)(const TileArgs<T>);
+// Launches a tiled kernel so that it may start while the stream's kernel before it still runs: its
+// CTAs take the places of those that have left, fetch what no kernel writes and wait for the rest
+// in grid_wait_previous.
+template <class T>
+cudaError_t launch_dependent(TileKernel<T> kernel, int grid, int block, size_t smem, cudaStream_t stream, const TileArgs<T>& a) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
 template <class T, int W, bool ARENA>
 TileKernel<T> pass1_variant(int limiter, int time_mode) {
     if constexpr (W == 8) {
