@@ -42,6 +42,15 @@ def _iptr(a):
     return a.ctypes.data_as(ct.POINTER(ct.c_int))
 
 
+def _rows(a):
+    """The addresses of a (4, n) array's rows, as the native library takes them (a[v].ctypes for
+    each row costs several microseconds, as much as a small solve's step)."""
+    if isinstance(a, np.ndarray) and a.ndim == 2 and a.shape[0] >= 4:
+        base, stride = a.__array_interface__["data"][0], a.strides[0]
+        return ct.cast((ct.c_void_p * 4)(base, base + stride, base + 2 * stride, base + 3 * stride), ct.POINTER(_n._dp))
+    return (ct.POINTER(ct.c_double) * 4)(*[_dptr(a[v]) for v in range(4)])
+
+
 class Mesh:
     """A host mesh owned by the native library (the reference's Mesh, src/Mesh.cpp)."""
 
@@ -186,8 +195,7 @@ class Solver:
 
     def download(self, prims: bool = False, out: np.ndarray | None = None) -> np.ndarray:
         out = np.empty((4, self.Nc)) if out is None else out
-        ptrs = (ct.POINTER(ct.c_double) * 4)(*[_dptr(out[v]) for v in range(4)])
-        _n.check(_n.lib().hcfd_gpu_download(self._h, 1 if prims else 0, ptrs))
+        _n.check(_n.lib().hcfd_gpu_download(self._h, 1 if prims else 0, _rows(out)))
         return out
 
     def U(self) -> np.ndarray:
@@ -198,8 +206,7 @@ class Solver:
 
     def upload(self, U: np.ndarray) -> None:
         U = np.ascontiguousarray(U, dtype=np.float64).reshape(4, self.Nc)
-        ptrs = (ct.POINTER(ct.c_double) * 4)(*[_dptr(U[v]) for v in range(4)])
-        _n.check(_n.lib().hcfd_gpu_upload(self._h, ptrs))
+        _n.check(_n.lib().hcfd_gpu_upload(self._h, _rows(U)))
 
     def snapshot(self, out: np.ndarray, prims: bool = True) -> "Snapshot":
         """Starts copying the current state into `out` (4 x Nc float64, C order; pin it with

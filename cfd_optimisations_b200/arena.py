@@ -8,7 +8,7 @@ import os
 import numpy as np
 
 from . import native as _n
-from . import FP32, GLOBAL_CFL, LIMITER_BJ, Mesh
+from . import FP32, GLOBAL_CFL, LIMITER_BJ, Mesh, _rows
 
 
 class Arena:
@@ -88,8 +88,7 @@ class Arena:
 
     def fetch(self, slot: int, prims: bool = False) -> np.ndarray:
         out = np.empty((4, self._nc[slot]))
-        ptrs = (ct.POINTER(ct.c_double) * 4)(*[out[v].ctypes.data_as(_n._dp) for v in range(4)])
-        _n.check(_n.lib().hcfd_arena_fetch(self._h, slot, 1 if prims else 0, ptrs))
+        _n.check(_n.lib().hcfd_arena_fetch(self._h, slot, 1 if prims else 0, _rows(out)))
         return out
 
     def checkpoint(self, slot: int, path: str) -> None:

@@ -454,7 +454,7 @@ void arena_free(hcfd_arena* A) {
     if (A->list_ev) cudaEventDestroy(A->list_ev);
     if (A->astream) cudaStreamDestroy(A->astream);
     void* p[] = {A->U[0], A->U[1], A->phiG, A->phiF, A->iv, A->nbr, A->tgeo, A->tmeta, A->halo, A->inst_dt, A->inst_dtmin,
-                 A->inst_bc, A->stats, A->tiles, A->act, A->tile_r2, A->tile_bad, A->err, A->queue, A->chunks,
+                 A->inst_bc, A->stats, A->tiles, A->act, A->tile_r2, A->tile_bad, A->queue, A->chunks,
                  A->chunk_r2, A->chunk_bad};
     for (void* q : p) if (q) cudaFree(q);
     if (A->stream) cudaStreamDestroy(A->stream);
@@ -527,13 +527,14 @@ int hcfd_arena_create(const hcfd_arena_params* prm, hcfd_arena** out) {
         (rc = dalloc(&h->nbr, h->Wp * C)) || (rc = dalloc((char**) &h->tgeo, 8 * ts * h->Ecap)) ||
         (rc = dalloc(&h->tmeta, h->Ecap)) || (rc = dalloc(&h->halo, h->HLcap + 1)) ||
         (rc = dalloc(&h->inst_dt, p.max_instances)) || (rc = dalloc(&h->inst_dtmin, 2 * (size_t) p.max_instances)) ||
-        (rc = dalloc(&h->inst_bc, p.max_instances)) || (rc = dalloc(&h->stats, p.max_instances)) ||
+        (rc = dalloc(&h->inst_bc, p.max_instances)) || (rc = dalloc(&h->stats, p.max_instances + 1)) ||
         (rc = dalloc(&h->tiles, 2 * h->tiles_cap)) || (rc = dalloc(&h->act, p.max_instances)) ||
         (rc = dalloc(&h->tile_r2, h->tiles_cap * (h->B / 32))) || (rc = dalloc(&h->tile_bad, h->tiles_cap * (h->B / 32))) ||
-        (rc = dalloc(&h->err, 1)) || (rc = dalloc(&h->queue, 1)) || (rc = dalloc(&h->chunks, h->chunks_cap)) ||
+        (rc = dalloc(&h->queue, 1)) || (rc = dalloc(&h->chunks, h->chunks_cap)) ||
         (rc = dalloc(&h->chunk_r2, h->chunks_cap)) || (rc = dalloc(&h->chunk_bad, h->chunks_cap)))
         return bail(rc);
-    cudaError_t ce = cudaMemsetAsync(h->err, 0, sizeof(unsigned int), h->stream);
+    h->err = (unsigned int*) (h->stats + p.max_instances);
+    cudaError_t ce = cudaMemsetAsync(h->err, 0, sizeof(hcfd::StepStats), h->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(h->queue, 0, sizeof(int), h->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(h->U[0], 0, 4 * ts * C, h->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(h->U[1], 0, 4 * ts * C, h->stream);
@@ -788,11 +789,11 @@ int hcfd_arena_poll(hcfd_arena* A, int max, int* slots, hcfd_step_stats* stats, 
         const int rc_ = wait_admissions(A);
         if (rc_) return rc_;
     }
-    std::vector<hcfd::StepStats> st(A->inst.size());
-    unsigned int err = 0;
+    std::vector<hcfd::StepStats> st(A->inst.size() + 1);     // the error word is in the last one's place
     CK(cudaMemcpyAsync(st.data(), A->stats, sizeof(hcfd::StepStats) * st.size(), cudaMemcpyDeviceToHost, A->stream));
-    CK(cudaMemcpyAsync(&err, A->err, sizeof(err), cudaMemcpyDeviceToHost, A->stream));
     CK(cudaStreamSynchronize(A->stream));
+    unsigned int err = 0;
+    std::memcpy(&err, &st.back(), sizeof(err));
     int k = 0;
     for (size_t i = 0; i < A->inst.size() && k < max; i++) {
         const Inst& I = A->inst[i];
@@ -828,8 +829,9 @@ int hcfd_arena_fetch(hcfd_arena* A, int slot, int prims, double* const* out) {
     else
         arena_out_kernel<double><<<nblk(I.Nc, 256), 256, 0, A->stream>>>(A->Ccap, I.c0, I.Nc, (const Cell4<double>*) A->U[A->cur], I.d_perm, A->prm.gma, prims, d_out);
     cudaError_t e = cudaGetLastError();
-    for (int v = 0; v < 4 && e == cudaSuccess; v++)
-        e = cudaMemcpyAsync(out[v], d_out + (size_t) v * I.Nc, sizeof(double) * I.Nc, cudaMemcpyDeviceToHost, A->stream);
+    const int blocks = hcfd::one_block(out, I.Nc) ? 1 : 4;
+    for (int v = 0; v < blocks && e == cudaSuccess; v++)
+        e = cudaMemcpyAsync(out[v], d_out + (size_t) v * I.Nc, sizeof(double) * 4 / blocks * I.Nc, cudaMemcpyDeviceToHost, A->stream);
     cudaFreeAsync(d_out, A->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(A->stream);
     if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("arena_fetch: ") + cudaGetErrorString(e));

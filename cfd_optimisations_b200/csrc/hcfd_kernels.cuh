@@ -101,7 +101,14 @@ struct StepArgs {
     // reused by every later step (freeze_after = 0: never).  Steps are counted on the device.
     Cell4<T>* phiF;
     long long freeze_after;
+    StepStats* clear_stats;              // per-cell pass 1: statistics to start over with this step (or null)
 };
+
+// Programmatic dependent launch: lets the next kernel of the stream start once every CTA of this one
+// has called it or left; waits for the kernel before this one (its writes included).  A kernel
+// launched without the attribute passes the wait at once.
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 enum { LIM_NORMAL = 0, LIM_RECORD = 1, LIM_FROZEN = 2 };
 // How pass 1 treats the limiter in the step after `steps_before` steps.
@@ -155,6 +162,15 @@ __device__ __forceinline__ void ld_grad(const Grad8<float>* p, size_t ps, int i,
     const float4* q = reinterpret_cast<const float4*>(p);
     const float4 a = __ldg(q + i), b = __ldg(q + ps + i);
     g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w; g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
+}
+template <class T>
+__device__ __forceinline__ void ld_grad_l2(const Grad8<T>* p, size_t ps, int i, T g[8]) {
+    constexpr int C = sizeof(Grad8<T>) / 16;
+    const uint4* q = reinterpret_cast<const uint4*>(p);
+    uint4 x[C];
+#pragma unroll
+    for (int k = 0; k < C; k++) x[k] = __ldcg(q + k * ps + i);
+    memcpy(g, x, sizeof(x));
 }
 __device__ __forceinline__ void st_grad(Grad8<double>* p, size_t ps, int i, const double g[8]) {
     double2* q = reinterpret_cast<double2*>(p);
@@ -471,6 +487,7 @@ template <class T, int W>
 __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     T xmx = T(0);                        // largest iv * lam (see dt_of_max)
+    if (a.clear_stats && c == 0) *a.clear_stats = StepStats{};
     if (c < a.Nc) {
         int2 s[W];
 #pragma unroll
@@ -509,6 +526,7 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
             if (a.time_mode != TM_FIXED) xmx = iv * p.lam;
         }
     }
+    grid_launch_next();                  // pass 2 fetches its tables meanwhile
     if (a.time_mode != TM_FIXED) {
         __shared__ T sm[32];
         T m = warp_max(xmx);
@@ -532,17 +550,25 @@ __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
     double r2 = 0.0;
     int bad = 0;
     double dt_used = 0.0;
+    int2 s[W];
+#pragma unroll
+    for (int k = 0; k < W; k++) s[k] = make_int2(-1, -1);
+    T iv = T(0);
+    if (c < a.Nc) {
+#pragma unroll
+        for (int k = 0; k < W; k++) s[k] = __ldg(a.slot + (size_t) k * a.Nc + c);
+        iv = __ldg(a.iv + c);
+    }
+    grid_wait_previous();                // pass 1's gradients and dt
     if (a.time_mode == TM_FIXED) dt_used = a.dt_or_cfl;
     else dt_used = a.dt_or_cfl * __longlong_as_double((long long) *a.dtmin);
     if (c < a.Nc) {
-        int2 s[W];
-#pragma unroll
-        for (int k = 0; k < W; k++) s[k] = __ldg(a.slot + (size_t) k * a.Nc + c);
         if (s[0].y >= 0) {
             T u[4], pg[8];
             ld_cell(a.U, a.Nc, c, u);
-            ld_grad(a.phiG, a.Nc, c, pg);
-            const T iv = __ldg(a.iv + c);
+            // written by the kernel before, perhaps while this one was starting: not through the
+            // read-only path
+            ld_grad_l2(a.phiG, a.Nc, c, pg);
             T R[4], Rc[4];
 #pragma unroll
             for (int v = 0; v < 4; v++) { R[v] = T(0); Rc[v] = T(0); }
@@ -572,7 +598,7 @@ __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
                     }
                 } else {
                     T pn[8];
-                    ld_grad(a.phiG, a.Nc, s[k].y, pn);
+                    ld_grad_l2(a.phiG, a.Nc, s[k].y, pn);
 #pragma unroll
                     for (int v = 0; v < 4; v++) {
                         uo[v] = u[v] + (pg[2 * v] * ro0 + pg[2 * v + 1] * ro1);

@@ -25,7 +25,9 @@ using hcfd::fail;
 
 namespace {
 
-constexpr int kBlock = 256;
+// 128 threads: a mesh of the size limit fills the SMs in small steps (58,000 cells are 227 blocks of
+// 256, one and a half an SM).
+constexpr int kBlock = 128;
 constexpr int kMaxBlocks = (HCFD_NOALLOC_MAX_CELLS + kBlock - 1) / kBlock;
 
 // Byte layout of the scratch array (offsets are multiples of 256).
@@ -49,7 +51,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 // so the library needs no link against libcuda.
 constexpr int kMaxDevices = 64;
 struct ScratchAddr {
-    unsigned long long ctx_id;   // 0: not looked up yet
+    unsigned long long ctx_id;   // 0: not looked up yet, or a call left the scratch unsettled
     unsigned char* addr;
 };
 ScratchAddr g_addr[kMaxDevices] = {};
@@ -79,7 +81,9 @@ unsigned long long current_ctx_id() {
     return id;
 }
 
-// Clears what must start at zero (and the dt minimum at +inf) on every call.
+// Clears what must start at zero (and the dt minimum at +inf): before the first step in a context.
+// Every step leaves the minimum and the counter as it found them (its last block resets both) and
+// clears the statistics it is about to write.
 __global__ void noalloc_reset_kernel(unsigned long long* dtmin, unsigned int* counter, unsigned int* err,
                                      hcfd::StepStats* stats) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
@@ -92,11 +96,22 @@ __global__ void noalloc_reset_kernel(unsigned long long* dtmin, unsigned int* co
     }
 }
 
+// Pass 2 starts under the tail of pass 1 (it fetches its slots and waits), except in a stream being
+// captured, whose graph is the caller's.
 template <int W>
-void launch(const hcfd::StepArgs<double>& a, cudaStream_t st) {
+cudaError_t launch(const hcfd::StepArgs<double>& a, cudaStream_t st, bool overlap) {
     const int grid = (a.Nc + kBlock - 1) / kBlock;
     hcfd::pass1_kernel<double, W><<<grid, kBlock, 0, st>>>(a);
-    hcfd::pass2_kernel<double, W, false><<<grid, kBlock, 0, st>>>(a);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kBlock);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, hcfd::pass2_kernel<double, W, false>, a);
 }
 
 }  // namespace
@@ -133,6 +148,7 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
     if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("step_noalloc: ") + cudaGetErrorString(e));
     if (dev < 0 || dev >= kMaxDevices) return fail(HCFD_EINVAL, "step_noalloc: device index too large");
     unsigned char* base;
+    bool fresh = false;          // the scratch of this context has not been settled by a step yet
     {
         // Once per device and context, with that device current: the device address of the
         // scratch.  Where the context id cannot be read, the address is looked up on every
@@ -146,6 +162,7 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
                 return fail(HCFD_ECUDA, std::string("step_noalloc: cudaGetSymbolAddress: ") + cudaGetErrorString(e));
             // the lookup makes the device's context current if none was: take its id now
             g_addr[dev].ctx_id = current_ctx_id();
+            fresh = true;
             g_addr[dev].addr = static_cast<unsigned char*>(p);
         }
         base = g_addr[dev].addr;
@@ -174,7 +191,7 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
     a.slot = reinterpret_cast<const int2*>(m->slot);
     a.iv = m->iv;
     a.dtmin = reinterpret_cast<unsigned long long*>(base + kDtmin);
-    a.dtmin_next = a.dtmin + 1;
+    a.dtmin_next = a.dtmin;  // reset by pass 2's last block, when every block has read it
     a.partial = reinterpret_cast<double*>(base + kPartial);
     a.counter = reinterpret_cast<unsigned int*>(base + kCounter);
     a.stats = reinterpret_cast<hcfd::StepStats*>(base + kStats);
@@ -188,10 +205,13 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
     a.bc = bc;
     a.phiF = nullptr;        // no limiter freezing here
     a.freeze_after = 0;
+    a.clear_stats = a.stats;
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned int* d_err = reinterpret_cast<unsigned int*>(base + kErr);
-    noalloc_reset_kernel<<<1, 32, 0, st>>>(a.dtmin, a.counter, d_err, a.stats);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) capture = cudaStreamCaptureStatusActive;
+    if (fresh || hcfd::kChecked) noalloc_reset_kernel<<<1, 32, 0, st>>>(a.dtmin, a.counter, d_err, a.stats);
     if constexpr (hcfd::kChecked) {
         // checked build: the caller's slot table is checked on the device before the step,
         // which is not launched when an id is out of range
@@ -205,12 +225,18 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
         if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("step_noalloc: ") + cudaGetErrorString(e));
         if (err & 4u) return fail(HCFD_EINVAL, "step_noalloc, checked build: a face or neighbour id was out of range");
     }
+    const bool overlap = capture == cudaStreamCaptureStatusNone;
     switch (m->slots) {
-    case 3: launch<3>(a, st); break;
-    case 4: launch<4>(a, st); break;
-    default: launch<8>(a, st); break;
+    case 3: e = launch<3>(a, st, overlap); break;
+    case 4: e = launch<4>(a, st, overlap); break;
+    default: e = launch<8>(a, st, overlap); break;
     }
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        // a step that may have run in part: the next call starts the scratch over
+        std::lock_guard<std::mutex> lk(g_addr_mu);
+        g_addr[dev].ctx_id = 0;
+    }
     if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("step_noalloc: launch: ") + cudaGetErrorString(e));
     if (dt_used || res_l2) {
         hcfd::StepStats h{};

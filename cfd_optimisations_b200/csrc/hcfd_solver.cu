@@ -149,7 +149,7 @@ void free_all(hcfd_solver* s) {
     for (auto e : s->ev1) cudaEventDestroy(e);
     for (auto e : s->ev2) cudaEventDestroy(e);
     void* ptrs[] = {s->d_fc, s->d_perm, s->d_slot, s->d_geo64, s->d_geoT, s->d_iv, s->d_U[0], s->d_U[1],
-                    s->d_phiG, s->d_phiF, s->d_io, s->d_cp, s->d_dtmin, s->d_partial, s->d_counter, s->d_err, s->d_stats, s->d_flags, s->d_ll};
+                    s->d_phiG, s->d_phiF, s->d_io, s->d_cp, s->d_dtmin, s->d_partial, s->d_counter, s->d_stats, s->d_flags, s->d_ll};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (TiledPass& P : s->tp) {
         void* q[] = {P.d_tgeo, P.d_tmeta, P.d_foff, P.d_hoff, P.d_halo, P.d_nbr, P.d_efid};
@@ -187,6 +187,7 @@ hcfd::StepArgs<T> step_args(hcfd_solver* s, int time_mode, double dt_or_cfl) {
     a.bc = s->bc;
     a.phiF = (hcfd::Cell4<T>*) s->d_phiF;
     a.freeze_after = s->prm.freeze_limiter_after;
+    a.clear_stats = nullptr;
     return a;
 }
 
@@ -441,12 +442,18 @@ int check_handle(hcfd_solver* s) {
     return HCFD_OK;
 }
 
-int read_stats(hcfd_solver* s, hcfd_step_stats* out) {
+// The statistics and the error word, side by side on the device: one copy reads both.
+struct StatsAndErr {
     hcfd::StepStats st;
-    unsigned int err = 0;
-    CK(cudaMemcpyAsync(&st, s->d_stats, sizeof(st), cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaMemcpyAsync(&err, s->d_err, sizeof(err), cudaMemcpyDeviceToHost, s->stream));
+    unsigned int err, pad;
+};
+
+int read_stats(hcfd_solver* s, hcfd_step_stats* out) {
+    StatsAndErr se{};
+    CK(cudaMemcpyAsync(&se, s->d_stats, sizeof(se), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
+    const hcfd::StepStats& st = se.st;
+    const unsigned int err = se.err;
     if (out) {
         out->dt = st.dt_last;
         out->res_l2 = s->Nreal > 0 ? std::sqrt(st.res2_last / s->Nreal) : 0.0;
@@ -627,7 +634,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         (rc = dalloc(&h->d_io, 4 * (size_t) Nc)) ||
         (p.freeze_limiter_after > 0 && (rc = dalloc((char**) &h->d_phiF, tsz * 4 * Nc))) ||
         (rc = dalloc(&h->d_cp, Nf)) || (rc = dalloc(&h->d_dtmin, 2)) || (rc = dalloc(&h->d_partial, 2 * (size_t) h->partial_len)) ||
-        (rc = dalloc(&h->d_counter, 4)) || (rc = dalloc(&h->d_err, 1)) || (rc = dalloc(&h->d_stats, 1)) ||
+        (rc = dalloc(&h->d_counter, 4)) || (rc = dalloc((StatsAndErr**) &h->d_stats, 1)) ||
         (rc = dalloc(&d_fn, 2 * (size_t) Nf)) || (rc = dalloc(&d_fcu, 2 * (size_t) Nf)) ||
         (rc = dalloc(&d_cnoff, Nc + 1)) || (rc = dalloc(&d_cncon, ncn)) || (rc = dalloc(&d_cfoff, Nc + 1)) ||
         (rc = dalloc(&d_cfcon, cf_con.size())) || (rc = dalloc(&d_nodes, 2 * (size_t) h->Nn)) ||
@@ -635,6 +642,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         free_tmp();
         return bail(rc);
     }
+    h->d_err = &((StatsAndErr*) h->d_stats)->err;
     if (h->tiled) {
         for (int k = 0; k < (h->split ? 2 : 1); k++) {
             TiledPass& P = h->tp[k];
@@ -904,8 +912,10 @@ int hcfd_gpu_download(hcfd_solver* s, int prims, double* const* out) {
     if (s->fp32()) hcfd::out_kernel<float><<<nblk(s->Nc, 256), 256, 0, s->stream>>>(s->Nc, (const hcfd::Cell4<float>*) s->d_U[s->cur], s->d_perm, s->prm.gma, prims, s->d_io);
     else hcfd::out_kernel<double><<<nblk(s->Nc, 256), 256, 0, s->stream>>>(s->Nc, (const hcfd::Cell4<double>*) s->d_U[s->cur], s->d_perm, s->prm.gma, prims, s->d_io);
     CK(cudaGetLastError());
-    for (int v = 0; v < 4; v++)
-        CK(cudaMemcpyAsync(out[v], s->d_io + (size_t) v * s->Nc, sizeof(double) * s->Nc, cudaMemcpyDeviceToHost, s->stream));
+    const int blocks = hcfd::one_block(out, s->Nc) ? 1 : 4;
+    for (int v = 0; v < blocks; v++)
+        CK(cudaMemcpyAsync(out[v], s->d_io + (size_t) v * s->Nc, sizeof(double) * 4 / blocks * s->Nc, cudaMemcpyDeviceToHost,
+                           s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return HCFD_OK;
 }
@@ -915,10 +925,11 @@ int hcfd_gpu_upload(hcfd_solver* s, const double* const* in) {
     int rc = check_handle(s);
     if (rc) return rc;
     if (!in) return fail(HCFD_EINVAL, "upload: null input");
-    for (int v = 0; v < 4; v++) {
-        if (!in[v]) return fail(HCFD_EINVAL, "upload: null input array");
-        CK(cudaMemcpyAsync(s->d_io + (size_t) v * s->Nc, in[v], sizeof(double) * s->Nc, cudaMemcpyHostToDevice, s->stream));
-    }
+    for (int v = 0; v < 4; v++) if (!in[v]) return fail(HCFD_EINVAL, "upload: null input array");
+    const int blocks = hcfd::one_block(in, s->Nc) ? 1 : 4;
+    for (int v = 0; v < blocks; v++)
+        CK(cudaMemcpyAsync(s->d_io + (size_t) v * s->Nc, in[v], sizeof(double) * 4 / blocks * s->Nc, cudaMemcpyHostToDevice,
+                           s->stream));
     if (s->fp32()) hcfd::in_kernel<float><<<nblk(s->Nc, 256), 256, 0, s->stream>>>(s->Nc, s->d_io, s->d_perm, (hcfd::Cell4<float>*) s->d_U[s->cur]);
     else hcfd::in_kernel<double><<<nblk(s->Nc, 256), 256, 0, s->stream>>>(s->Nc, s->d_io, s->d_perm, (hcfd::Cell4<double>*) s->d_U[s->cur]);
     CK(cudaGetLastError());
