@@ -205,20 +205,34 @@ __device__ __forceinline__ float qsqrt<float>(float x) { return x == 0.0f ? 0.0f
 // flux arithmetic, written with the reference's expression trees
 
 // One side of the Rusanov flux: Euler flux along n (Flux::EulerFlux, src/Base/Flux.cpp:89-97)
-// and the side's wave speed |u.n| + a.  The reference expands every component over n0 and n1;
-// with m = n.(rho u) and u.n = m / rho formed once, F = (m, u.n rho u + P n0, u.n rho v + P n1,
-// (E + P) u.n): 9 operations in place of 22, equal up to rounding.
+// and the side's wave speed |u.n| + a (:60-73).  FP64 keeps the reference's expression trees, so
+// that a solve frozen or cycling at its limiter, which amplifies a difference of one rounding 10^7
+// times, stays where it was.  In FP32, with m = n.(rho u) and u.n = m / rho formed once, F =
+// (m, u.n rho u + P n0, u.n rho v + P n1, (E + P) u.n): 9 operations in place of 22.
 template <class T>
 __device__ __forceinline__ void euler_side(const T U[4], T n0, T n1, T gma, T F[4], T& speed) {
+    const T gmo = gma - T(1);
     const T ir = qrcp(U[0]);
-    const T m = n0 * U[1] + n1 * U[2];
-    const T vn = m * ir;
-    const T P = (gma - T(1)) * (U[3] - T(0.5) * ir * (U[1] * U[1] + U[2] * U[2]));
-    F[0] = m;
-    F[1] = vn * U[1] + n0 * P;
-    F[2] = vn * U[2] + n1 * P;
-    F[3] = vn * (U[3] + P);
-    speed = fabs(vn) + qsqrt(gma * P * ir);
+    if constexpr (sizeof(T) == 4) {
+        const T m = n0 * U[1] + n1 * U[2];
+        const T vn = m * ir;
+        const T P = gmo * (U[3] - T(0.5) * ir * (U[1] * U[1] + U[2] * U[2]));
+        F[0] = m;
+        F[1] = vn * U[1] + n0 * P;
+        F[2] = vn * U[2] + n1 * P;
+        F[3] = vn * (U[3] + P);
+        speed = fabs(vn) + qsqrt(gma * P * ir);
+    } else {
+        const T nv = (n0 * U[1] + n1 * U[2]) * ir;
+        const T qq = T(0.5) * (U[1] * U[1] + U[2] * U[2]) * ir;
+        const T p = gmo * (U[3] - qq);
+        speed = fabs(nv) + qsqrt(gma * p * ir);
+        const T P = gmo * (U[3] - T(0.5) * ir * (U[1] * U[1] + U[2] * U[2]));
+        F[0] = n0 * U[1] + n1 * U[2];
+        F[1] = n0 * (U[1] * U[1] * ir + P) + n1 * U[2] * U[1] * ir;
+        F[2] = n0 * U[1] * U[2] * ir + n1 * (U[2] * U[2] * ir + P);
+        F[3] = n0 * (U[3] + P) * U[1] * ir + n1 * (U[3] + P) * U[2] * ir;
+    }
 }
 
 // Flux::Rusanov (src/Base/Flux.cpp:52-81).  The reference takes the largest of |u.n -+ a| over
