@@ -163,6 +163,17 @@ __device__ __forceinline__ void ld_grad(const Grad8<float>* p, size_t ps, int i,
     const float4 a = __ldg(q + i), b = __ldg(q + ps + i);
     g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w; g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
 }
+// The same from L2, past the read-only path: values that an earlier kernel may have written while
+// this one was starting.
+template <class T>
+__device__ __forceinline__ void ld_cell_l2(const Cell4<T>* p, size_t ps, int i, T u[4]) {
+    constexpr int C = sizeof(Cell4<T>) / 16;
+    const uint4* q = reinterpret_cast<const uint4*>(p);
+    uint4 x[C];
+#pragma unroll
+    for (int k = 0; k < C; k++) x[k] = __ldcg(q + k * ps + i);
+    memcpy(u, x, sizeof(x));
+}
 template <class T>
 __device__ __forceinline__ void ld_grad_l2(const Grad8<T>* p, size_t ps, int i, T g[8]) {
     constexpr int C = sizeof(Grad8<T>) / 16;
@@ -580,8 +591,6 @@ __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
         if (s[0].y >= 0) {
             T u[4], pg[8];
             ld_cell(a.U, a.Nc, c, u);
-            // written by the kernel before, perhaps while this one was starting: not through the
-            // read-only path
             ld_grad_l2(a.phiG, a.Nc, c, pg);
             T R[4], Rc[4];
 #pragma unroll

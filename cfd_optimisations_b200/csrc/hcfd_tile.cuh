@@ -280,12 +280,6 @@ __device__ __forceinline__ T lds_area(const T* p, int nf, int e, int rec) {
     return rec == 7 ? p[6 * nf + e] : p[2 * (nf + e)];
 }
 
-template <class T>
-__device__ __forceinline__ void lds_geo(const T* p, int nf, int e, FaceGeo<T>& g) {
-    const auto a = ldp(p, nf, 0, e), b = ldp(p, nf, 1, e), c = ldp(p, nf, 2, e), d = ldp(p, nf, 3, e);
-    g.nx = a.x; g.ny = a.y; g.Af = b.x; g.If = b.y; g.rLx = c.x; g.rLy = c.y; g.rRx = d.x; g.rRy = d.y;
-}
-
 // Normal, length and interpolation weight (pass 1 reads the r vector of one side apart).
 template <class T>
 __device__ __forceinline__ void lds_geo4(const T* p, int nf, int e, FaceGeo<T>& g) {
@@ -378,16 +372,12 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
         double dt, dtmin;
         long long steps;
     };
-    auto load_scalars = [&](int inst, Scalars& v) {
-        if constexpr (ARENA) {
-            v.dt = __ldg(a.inst_dt + inst);
-            v.dtmin = PASS2 ? __longlong_as_double((long long) a.inst_dtmin[2 * inst + a.par]) : 0.0;
-            v.steps = PASS2 ? 0 : a.inst_stats[inst].steps;
-        } else {
-            v.dt = a.s.dt_or_cfl;
-            v.dtmin = PASS2 ? __longlong_as_double((long long) *a.s.dtmin) : 0.0;
-            v.steps = PASS2 ? 0 : a.s.stats->steps;
-        }
+    auto load_scalars = [&](int inst, Scalars& v) {      // (from L2: the kernel before may still run)
+        v.dt = ARENA ? __ldg(a.inst_dt + inst) : a.s.dt_or_cfl;
+        if constexpr (PASS2)
+            v.dtmin = __longlong_as_double((long long) __ldcg(ARENA ? a.inst_dtmin + 2 * inst + a.par : a.s.dtmin));
+        else
+            v.steps = __ldcg(ARENA ? &a.inst_stats[inst].steps : &a.s.stats->steps);
     };
     // A descriptor as loaded (nothing computed from it until it is needed, a tile later).
     struct Raw {
@@ -869,7 +859,7 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : W == 3 ? 56 : 72) tile_pass1_
         const T iv = sIv[c];
         tile_faces<T, W, 4>(p, x, sU, sGeo, NL, nfl, c, 0, with_lam, s.gma, iv, nb, a.B, si.nh, a.err);
         T out[8], phis[4];
-        if (lmode == LIM_FROZEN) ld_cell(s.phiF, a.ps, base + c, phis);
+        if (lmode == LIM_FROZEN) ld_cell_l2(s.phiF, a.ps, base + c, phis);
         else p.template limiter_values<LIM>(iv, s.limiter, s.venkat_K, phis);
         p.limited(phis, out);
         if (lmode == LIM_RECORD) st_cell(s.phiF, a.ps, base + c, phis);

@@ -137,3 +137,37 @@ def test_handles_of_different_sizes_take_turns():
                 s.step(2, H.GLOBAL_CFL, 0.4, wait=False)
         for s, t in zip(alone, turns):
             assert np.array_equal(s.U(), t.U())
+
+
+def test_handles_on_threads_of_their_own_step_at_the_same_time():
+    """Each handle has its stream, and ctypes calls release the GIL: resident kernels that fill every
+    SM, smaller ones and tiled steps at once give what they give alone (the resident
+    kernel's CTAs wait for one another, so its launch is cooperative: all of them or none)."""
+    import threading
+    case = H.wedge_case(2.5)
+    shapes = [(333, 178, {}), (333, 178, {}), (161, 81, {}), (41, 21, {}), (241, 121, dict(tile=128)), (17, 9, {})]
+    meshes = [H.Mesh.wedge(nx, ny, seed=8, numbering=H.NUMBER_RANDOM) for nx, ny, _ in shapes]
+    alone = []
+    for m, (_, _, kw) in zip(meshes, shapes):
+        s = _solver(m, case, **kw)
+        st = [s.step(25, H.GLOBAL_CFL, 0.4) for _ in range(8)][-1]
+        alone.append((s.U(), st))
+        del s
+    together = [_solver(m, case, **kw) for m, (_, _, kw) in zip(meshes, shapes)]
+    got, errors = [None] * len(shapes), []
+
+    def run(i):
+        try:
+            st = [together[i].step(25, H.GLOBAL_CFL, 0.4) for _ in range(8)][-1]
+            got[i] = (together[i].U(), st)
+        except Exception as e:                       # reported by the assertion below
+            errors.append((i, e))
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(len(shapes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for (U, s), (V, t) in zip(alone, got):
+        assert np.array_equal(U, V) and s == t
