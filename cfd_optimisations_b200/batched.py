@@ -107,7 +107,7 @@ def run(instances: int = 512, steps: int = 2000, seed: int = 2024, loop: bool = 
     """Config-4 batched solves: the FP32 arena against the plain FP64 loop on the same instances.
 
     Both sides are timed on the device over steps 3..`steps` of every instance (the first two
-    steps, which build the CUDA graphs, stay out); mesh generation and admission are reported
+    steps, which load the kernels, stay out); mesh generation and admission are reported
     apart.  Every `spread_every`-th instance is also solved in FP64 from an initial density one
     rounding step larger (x (1 + 2^-52)): that solve's distance from the unperturbed FP64 solve
     is the spread rounding alone produces, reported beside the FP32 error of the same instance."""

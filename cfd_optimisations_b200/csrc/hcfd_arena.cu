@@ -9,8 +9,8 @@
 // all active tiles; a finalize kernel then forms each instance's residual from its tiles in
 // tile order.  An instance's arithmetic is exactly that of the single-mesh solver with the
 // same tile size, whatever else is in the arena, so a result is the same alone and in the
-// mix.  A chunk of steps is captured once as a CUDA graph and replayed until the set of
-// instances changes.
+// mix.  A step is two launches (each under the tail of the one before); the residual kernels run
+// in the first step after the set of instances changed and in the last of a call.
 #include "hcfd_internal.hpp"
 #include "hcfd_kernels.cuh"
 #include "hcfd_tile.cuh"

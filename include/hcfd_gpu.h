@@ -222,7 +222,8 @@ int  hcfd_gpu_stats(hcfd_solver* s, hcfd_step_stats* stats);
 /* Failure injection for tests of the bounded waits (no reference counterpart: the reference
  * has no device and no waits).  Every wait of the tiled step kernels gives up after `polls`
  * polls (0 restores the default, 2^22; at most 2^30); with skip_tile >= 0 the staging warp
- * arms and copies nothing for that tile, so the wait for it runs out with no copy in flight.
+ * (in the resident kernel, that tile's CTA) arms and copies nothing for that tile, so the wait
+ * for it runs out with no copy in flight.
  * The next step then returns HCFD_ETIMEOUT with the state partly stepped; the kernels leave
  * no copy in flight and the context stays usable: hcfd_gpu_initialise clears the error, and
  * with the hook reset (polls 0, skip_tile -1) the handle steps normally again. */
@@ -237,7 +238,7 @@ int  hcfd_gpu_info(hcfd_solver* s, int* Nc, int* Nf, int* Nreal, int* slots);
 /* Per-kernel timing with CUDA events on the handle's stream (the reference times only whole
  * runs, with clock(), src/Test.cpp:72-74).  enable = N > 0 starts
  * recording the two step kernels' launches of every N-th step (N > 1 keeps the events'
- * own cost out of most steps); 0 stops.  hcfd_gpu_profile_read returns the summed
+ * own cost out of most steps; the resident kernel's two halves are launched apart for it); 0 stops.  hcfd_gpu_profile_read returns the summed
  * milliseconds and launch counts of the recorded launches since enabling. */
 int  hcfd_gpu_profile(hcfd_solver* s, int enable);
 int  hcfd_gpu_profile_read(hcfd_solver* s, double* ms_pass1, long long* n_pass1,
@@ -246,7 +247,9 @@ int  hcfd_gpu_profile_read(hcfd_solver* s, double* ms_pass1, long long* n_pass1,
  * CUDA events recorded on the handle's stream before the first and after the last launch.
  * No reference counterpart (the reference times whole runs with clock(), src/Test.cpp:72-74). */
 int  hcfd_gpu_step_timed(hcfd_solver* s, int nsteps, int time_mode, double dt_or_cfl, double* ms);
-/* Number of kernel launches one step issues (the two passes; no reference counterpart). */
+/* Number of kernel launches one step issues at most: 2 (the two passes), or 1 where the mesh is
+ * stepped by the resident kernel, whose launch takes up to 1024 steps of a call (no reference
+ * counterpart). */
 int  hcfd_gpu_launches_per_step(hcfd_solver* s);
 /* Replaces the Euler destructor (src/Base/Euler.cpp:27-40) and those of the objects
  * hcfd_gpu_create stands in for: frees the handle's device memory, stream and graphs. */
@@ -272,7 +275,7 @@ int  hcfd_plan_check(const hcfd_mesh_view* mesh, int tile, int keep_numbering, l
  * meshes (instances) into one flat set of device arrays sized from an HBM budget; each
  * admitted mesh gets contiguous ranges (per-instance offsets), its own BC table, dt or CFL
  * number and statistics, and all active instances advance together through the tiled step
- * kernels, a chunk of steps replayed as one CUDA graph.  An instance's arithmetic does not
+ * kernels.  An instance's arithmetic does not
  * depend on what else is in the arena: its state is the same alone and in the mix. */
 typedef struct hcfd_arena hcfd_arena;
 typedef struct hcfd_arena_params {
