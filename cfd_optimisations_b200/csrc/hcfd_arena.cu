@@ -223,7 +223,7 @@ struct hcfd_arena {
     void* phiG = nullptr;
     void* phiF = nullptr;
     void* iv = nullptr;
-    unsigned* nbr = nullptr;                // pack_nbr words
+    unsigned* nbr = nullptr;                // pack_nbr_kernel's words
     void* tgeo = nullptr;
     unsigned* tmeta = nullptr;              // pack_meta words
     int* halo = nullptr;
@@ -648,6 +648,7 @@ int hcfd_arena_admit_prepared(hcfd_arena* A, const hcfd_admission* D, int* slot_
     cudaStream_t st = A->astream;
     int *d_fn = nullptr, *d_fcu = nullptr, *d_fcg = nullptr, *d_cnoff = nullptr, *d_cncon = nullptr, *d_cfoff = nullptr,
         *d_cfcon = nullptr, *d_efid = nullptr, *d_foff = nullptr, *d_iperm = nullptr, *d_halo = nullptr;
+    short* d_cslot = nullptr;
     double *d_nodes = nullptr, *d_xc = nullptr, *d_ivu = nullptr;
     hcfd::FaceGeo<double>* d_geo = nullptr;
     const int ncn = mv->cn_off[Nc];
@@ -657,11 +658,11 @@ int hcfd_arena_admit_prepared(hcfd_arena* A, const hcfd_admission* D, int* slot_
     };
     tmp(&d_fn, 2 * (size_t) Nf); tmp(&d_fcu, 2 * (size_t) Nf); tmp(&d_fcg, 2 * (size_t) Nf);
     tmp(&d_cnoff, Nc + 1); tmp(&d_cncon, ncn); tmp(&d_cfoff, Nc + 1); tmp(&d_cfcon, D->cf_con.size());
-    tmp(&d_efid, I.ne); tmp(&d_foff, P.foff.size()); tmp(&d_iperm, Nc); tmp(&d_halo, I.nh);
+    tmp(&d_efid, I.ne); tmp(&d_foff, P.foff.size()); tmp(&d_iperm, Nc); tmp(&d_halo, I.nh); tmp(&d_cslot, P.cslot.size());
     tmp(&d_nodes, 2 * (size_t) mv->Nn); tmp(&d_xc, 2 * (size_t) Nc); tmp(&d_ivu, Nc); tmp(&d_geo, Nf);
     auto tmp_free = [&]() {
         void* t[] = {d_fn, d_fcu, d_fcg, d_cnoff, d_cncon, d_cfoff, d_cfcon, d_efid, d_foff, d_iperm, d_halo,
-                     d_nodes, d_xc, d_ivu, d_geo};
+                     d_cslot, d_nodes, d_xc, d_ivu, d_geo};
         for (void* q : t) if (q) cudaFreeAsync(q, st);
     };
     if (ce == cudaSuccess) ce = cudaMallocAsync((void**) &I.d_perm, sizeof(int) * (size_t) Nc, st);
@@ -688,10 +689,11 @@ int hcfd_arena_admit_prepared(hcfd_arena* A, const hcfd_admission* D, int* slot_
     up(d_halo, P.halo.data(), 4 * I.nh);
     up(d_nodes, mv->nodes, 16 * (size_t) mv->Nn);
     up(I.d_perm, D->perm.data(), 4 * (size_t) Nc);
-    const std::vector<unsigned> mw = hcfd::packed_meta(P), nw = hcfd::packed_nbr(P);
+    const std::vector<unsigned> mw = hcfd::packed_meta(P);
     up(A->tmeta + I.e0, mw.data(), 4 * mw.size());
-    up(A->nbr + A->Wp * I.c0, nw.data(), 4 * nw.size());
+    up(d_cslot, P.cslot.data(), 2 * P.cslot.size());
     if (ce == cudaSuccess) {
+        hcfd::pack_nbr_kernel<<<P.ntiles, 128, 0, st>>>(P.B * P.Wp, d_foff, A->tmeta + I.e0, d_cslot, A->nbr + A->Wp * I.c0);
         arena_cellmap_kernel<<<nblk(2 * (long long) Nf, 256), 256, 0, st>>>(2 * (long long) Nf, (int) I.c0, d_iperm, d_fcu, d_fcg);
         if (I.nh) arena_offset_kernel<<<nblk((long long) I.nh, 256), 256, 0, st>>>((long long) I.nh, (int) I.c0, d_halo, A->halo + I.h0);
         hcfd::geom_xc_kernel<<<nblk(Nc, 256), 256, 0, st>>>(Nc, d_cnoff, d_cncon, d_nodes, d_xc);

