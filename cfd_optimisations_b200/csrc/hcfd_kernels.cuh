@@ -101,7 +101,7 @@ struct StepArgs {
     // reused by every later step (freeze_after = 0: never).  Steps are counted on the device.
     Cell4<T>* phiF;
     long long freeze_after;
-    StepStats* clear_stats;              // per-cell pass 1: statistics to start over with this step (or null)
+    double* block_dt;                    // per-cell kernels, OWN: smallest CFL-1 step of each block of pass 1
 };
 
 // Programmatic dependent launch: lets the next kernel of the stream start once every CTA of this one
@@ -479,6 +479,13 @@ __device__ __forceinline__ T warp_max(T x) {
     for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
     return x;
 }
+// Smallest of a warp's values >= 0 (their bit patterns order them).
+__device__ __forceinline__ double warp_min_pos(double x) {
+    const unsigned long long b = (unsigned long long) __double_as_longlong(x);
+    const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned) (b >> 32));
+    const unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned) (b >> 32) == hi ? (unsigned) b : 0xffffffffu);
+    return __longlong_as_double((long long) (((unsigned long long) hi << 32) | lo));
+}
 // The CFL time-step minimum of a set of cells, min_i 1 / x_i with x_i = iv_i lam_i > 0: a
 // correctly rounded reciprocal (FP64) does not grow as x grows, so the minimum equals
 // 1 / max_i x_i bit for bit, and the cells keep a running maximum, one reciprocal being formed
@@ -510,11 +517,18 @@ static __global__ void check_slots_kernel(const int2* __restrict__ slot, int W, 
     }
 }
 
-template <class T, int W>
+// Block minima that a thread of the allocation-free step's pass 2 reduces.
+constexpr int kOwnBlocksPerThread = 4;
+// OWN (the allocation-free step, both passes): a step that takes nothing from the steps before it.
+// Pass 1 starts statistics and block counter over and leaves each block's smallest CFL step in
+// block_dt, which every block of pass 2 reduces, in place of a minimum that must be found at +inf:
+// whatever an earlier call left behind (refused, captured or raced against another), this one is
+// right, without a launch that resets the scratch.  Pass 2 starts under the tail of pass 1.
+template <class T, int W, bool OWN>
 __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     T xmx = T(0);                        // largest iv * lam (see dt_of_max)
-    if (a.clear_stats && c == 0) *a.clear_stats = StepStats{};
+    if (OWN && c == 0) { *a.stats = StepStats{}; *a.counter = 0u; }
     if (c < a.Nc) {
         int2 s[W];
 #pragma unroll
@@ -543,7 +557,7 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
             p.gradient(iv);
 #pragma unroll
             for (int k = 0; k < W; k++) p.increment(ro[k][0], ro[k][1]);
-            const int lmode = limiter_mode(a.stats->steps, a.freeze_after);
+            const int lmode = OWN ? LIM_NORMAL : limiter_mode(a.stats->steps, a.freeze_after);
             T out[8], phis[4];
             if (lmode == LIM_FROZEN) ld_cell(a.phiF, a.Nc, c, phis);
             else p.limiter_values(iv, a.limiter, a.venkat_K, phis);
@@ -553,7 +567,7 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
             if (a.time_mode != TM_FIXED) xmx = iv * p.lam;
         }
     }
-    grid_launch_next();                  // pass 2 fetches its tables meanwhile
+    if (OWN) grid_launch_next();         // pass 2 fetches its tables meanwhile
     if (a.time_mode != TM_FIXED) {
         __shared__ T sm[32];
         T m = warp_max(xmx);
@@ -563,7 +577,11 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
         if (wid == 0) {
             m = lane < (int) (blockDim.x >> 5) ? sm[lane] : T(0);
             const double d = dt_of_max(warp_max(m));
-            if (lane == 0 && d < 1e300) atomicMin(a.dtmin, (unsigned long long) __double_as_longlong(d));
+            if (OWN) {
+                if (lane == 0) a.block_dt[blockIdx.x] = d < 1e300 ? d : __longlong_as_double(0x7FF0000000000000LL);
+            } else if (lane == 0 && d < 1e300) {
+                atomicMin(a.dtmin, (unsigned long long) __double_as_longlong(d));
+            }
         }
     }
 }
@@ -571,7 +589,7 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
 // ---------------------------------------------------------------------------------------
 // pass 2: reconstruction + flux + gather + update + ghost refresh (+ residual)
 
-template <class T, int W, bool COMP>
+template <class T, int W, bool COMP, bool OWN>
 __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double r2 = 0.0;
@@ -586,14 +604,39 @@ __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
         for (int k = 0; k < W; k++) s[k] = __ldg(a.slot + (size_t) k * a.Nc + c);
         iv = __ldg(a.iv + c);
     }
-    grid_wait_previous();                // pass 1's gradients and dt
-    if (a.time_mode == TM_FIXED) dt_used = a.dt_or_cfl;
-    else dt_used = a.dt_or_cfl * __longlong_as_double((long long) *a.dtmin);
+    if (OWN) grid_wait_previous();       // pass 1's gradients and dt
+    // OWN: pass 1's block minima, fetched with the cell's state and reduced while that travels
+    constexpr int MB = OWN ? kOwnBlocksPerThread : 1;
+    double md[MB];
+    if (OWN && a.time_mode != TM_FIXED) {
+#pragma unroll
+        for (int k = 0; k < MB; k++) {
+            const int i = threadIdx.x + k * blockDim.x;
+            md[k] = i < (int) gridDim.x ? __ldcg(a.block_dt + i) : __longlong_as_double(0x7FF0000000000000LL);
+        }
+    }
+    T u[4], pg[8];
+    if (c < a.Nc && s[0].y >= 0) {
+        ld_cell(a.U, a.Nc, c, u);
+        ld_grad_l2(a.phiG, a.Nc, c, pg);
+    }
+    if (a.time_mode == TM_FIXED) {
+        dt_used = a.dt_or_cfl;
+    } else if constexpr (OWN) {
+        __shared__ double smin[32];
+        double m = md[0];
+#pragma unroll
+        for (int k = 1; k < MB; k++) m = least(m, md[k]);
+        m = warp_min_pos(m);
+        if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = m;
+        __syncthreads();
+        for (int i = 0; i < (int) (blockDim.x >> 5); i++) m = least(m, smin[i]);
+        dt_used = a.dt_or_cfl * m;
+    } else {
+        dt_used = a.dt_or_cfl * __longlong_as_double((long long) *a.dtmin);
+    }
     if (c < a.Nc) {
         if (s[0].y >= 0) {
-            T u[4], pg[8];
-            ld_cell(a.U, a.Nc, c, u);
-            ld_grad_l2(a.phiG, a.Nc, c, pg);
             T R[4], Rc[4];
 #pragma unroll
             for (int v = 0; v < 4; v++) { R[v] = T(0); Rc[v] = T(0); }
@@ -715,7 +758,7 @@ __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
             st->dt_last = dt_used;
             if (!(tot == tot) || tot > 1.7e308) st->nonfinite = 1;
             *a.counter = 0u;
-            if (a.time_mode != TM_FIXED) *a.dtmin_next = 0x7FF0000000000000ULL;   // +inf
+            if (!OWN && a.time_mode != TM_FIXED) *a.dtmin_next = 0x7FF0000000000000ULL;   // +inf
         }
     }
 }

@@ -9,7 +9,9 @@
 // adds no allocation of any kind.  The one buffer the step needs besides them — the limited
 // gradients that pass 1 writes and pass 2 reads, plus the reduction slots — is the static
 // device array below, sized for at most HCFD_NOALLOC_MAX_CELLS cells.  Every GPU that loads
-// the library holds that array (about 4 MiB) until the process exits.
+// the library holds that array (about 4 MiB) until the process exits.  A call reads nothing of it
+// that it has not written itself (the kernels' OWN), so no call depends on the ones before it:
+// not on one that was refused, that sits in a graph yet to run, or that raced another.
 #include "hcfd_internal.hpp"
 #include "hcfd_kernels.cuh"
 
@@ -29,12 +31,14 @@ namespace {
 // 256, one and a half an SM).
 constexpr int kBlock = 128;
 constexpr int kMaxBlocks = (HCFD_NOALLOC_MAX_CELLS + kBlock - 1) / kBlock;
+static_assert(kMaxBlocks <= hcfd::kOwnBlocksPerThread * kBlock, "pass 2 reduces every block's minimum");
 
 // Byte layout of the scratch array (offsets are multiples of 256).
+constexpr size_t kBlockBytes = (sizeof(double) * kMaxBlocks + 255) & ~(size_t) 255;
 constexpr size_t kPhiG = 0;                                                   // Grad8<double> planes
 constexpr size_t kPartial = kPhiG + (size_t) 64 * HCFD_NOALLOC_MAX_CELLS;     // double[kMaxBlocks]
-constexpr size_t kDtmin = kPartial + ((sizeof(double) * kMaxBlocks + 255) & ~(size_t) 255);  // u64[2]
-constexpr size_t kCounter = kDtmin + 256;                                     // unsigned int
+constexpr size_t kBlockDt = kPartial + kBlockBytes;                           // double[kMaxBlocks]
+constexpr size_t kCounter = kBlockDt + kBlockBytes;                           // unsigned int
 constexpr size_t kErr = kCounter + 128;                                       // unsigned int (checked build)
 constexpr size_t kStats = kCounter + 256;                                     // StepStats
 constexpr size_t kScratchBytes = kStats + 256;
@@ -51,7 +55,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 // so the library needs no link against libcuda.
 constexpr int kMaxDevices = 64;
 struct ScratchAddr {
-    unsigned long long ctx_id;   // 0: not looked up yet, or a call left the scratch unsettled
+    unsigned long long ctx_id;   // 0: not looked up yet
     unsigned char* addr;
 };
 ScratchAddr g_addr[kMaxDevices] = {};
@@ -81,27 +85,12 @@ unsigned long long current_ctx_id() {
     return id;
 }
 
-// Clears what must start at zero (and the dt minimum at +inf): before the first step in a context.
-// Every step leaves the minimum and the counter as it found them (its last block resets both) and
-// clears the statistics it is about to write.
-__global__ void noalloc_reset_kernel(unsigned long long* dtmin, unsigned int* counter, unsigned int* err,
-                                     hcfd::StepStats* stats) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        dtmin[0] = 0x7FF0000000000000ULL;
-        dtmin[1] = 0x7FF0000000000000ULL;
-        *counter = 0u;
-        *err = 0u;
-        hcfd::StepStats z{};
-        *stats = z;
-    }
-}
-
 // Pass 2 starts under the tail of pass 1 (it fetches its slots and waits), except in a stream being
 // captured, whose graph is the caller's.
 template <int W>
 cudaError_t launch(const hcfd::StepArgs<double>& a, cudaStream_t st, bool overlap) {
     const int grid = (a.Nc + kBlock - 1) / kBlock;
-    hcfd::pass1_kernel<double, W><<<grid, kBlock, 0, st>>>(a);
+    hcfd::pass1_kernel<double, W, true><<<grid, kBlock, 0, st>>>(a);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kBlock);
@@ -111,7 +100,7 @@ cudaError_t launch(const hcfd::StepArgs<double>& a, cudaStream_t st, bool overla
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
     cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, hcfd::pass2_kernel<double, W, false>, a);
+    return cudaLaunchKernelEx(&cfg, hcfd::pass2_kernel<double, W, false, true>, a);
 }
 
 }  // namespace
@@ -148,7 +137,6 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
     if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("step_noalloc: ") + cudaGetErrorString(e));
     if (dev < 0 || dev >= kMaxDevices) return fail(HCFD_EINVAL, "step_noalloc: device index too large");
     unsigned char* base;
-    bool fresh = false;          // the scratch of this context has not been settled by a step yet
     {
         // Once per device and context, with that device current: the device address of the
         // scratch.  Where the context id cannot be read, the address is looked up on every
@@ -162,7 +150,6 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
                 return fail(HCFD_ECUDA, std::string("step_noalloc: cudaGetSymbolAddress: ") + cudaGetErrorString(e));
             // the lookup makes the device's context current if none was: take its id now
             g_addr[dev].ctx_id = current_ctx_id();
-            fresh = true;
             g_addr[dev].addr = static_cast<unsigned char*>(p);
         }
         base = g_addr[dev].addr;
@@ -190,8 +177,8 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
     a.geo = reinterpret_cast<const hcfd::FaceGeo<double>*>(m->geo);
     a.slot = reinterpret_cast<const int2*>(m->slot);
     a.iv = m->iv;
-    a.dtmin = reinterpret_cast<unsigned long long*>(base + kDtmin);
-    a.dtmin_next = a.dtmin;  // reset by pass 2's last block, when every block has read it
+    a.dtmin = a.dtmin_next = nullptr;      // the step's own block minima in their place
+    a.block_dt = reinterpret_cast<double*>(base + kBlockDt);
     a.partial = reinterpret_cast<double*>(base + kPartial);
     a.counter = reinterpret_cast<unsigned int*>(base + kCounter);
     a.stats = reinterpret_cast<hcfd::StepStats*>(base + kStats);
@@ -205,17 +192,17 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
     a.bc = bc;
     a.phiF = nullptr;        // no limiter freezing here
     a.freeze_after = 0;
-    a.clear_stats = a.stats;
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    unsigned int* d_err = reinterpret_cast<unsigned int*>(base + kErr);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) capture = cudaStreamCaptureStatusActive;
-    if (fresh || hcfd::kChecked) noalloc_reset_kernel<<<1, 32, 0, st>>>(a.dtmin, a.counter, d_err, a.stats);
     if constexpr (hcfd::kChecked) {
         // checked build: the caller's slot table is checked on the device before the step,
         // which is not launched when an id is out of range
         const long long n = (long long) m->slots * m->Nc;
+        unsigned int* d_err = reinterpret_cast<unsigned int*>(base + kErr);
+        e = cudaMemsetAsync(d_err, 0, sizeof(unsigned int), st);
+        if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("step_noalloc: ") + cudaGetErrorString(e));
         hcfd::check_slots_kernel<<<(int) std::min<long long>((n + 255) / 256, 1184), 256, 0, st>>>(
             a.slot, m->slots, m->Nc, m->Nf, d_err);
         unsigned int err = 0;
@@ -232,11 +219,6 @@ extern "C" int hcfd_step_noalloc(const hcfd_noalloc_mesh* m, const double* U_in,
     default: e = launch<8>(a, st, overlap); break;
     }
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        // a step that may have run in part: the next call starts the scratch over
-        std::lock_guard<std::mutex> lk(g_addr_mu);
-        g_addr[dev].ctx_id = 0;
-    }
     if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("step_noalloc: launch: ") + cudaGetErrorString(e));
     if (dt_used || res_l2) {
         hcfd::StepStats h{};

@@ -149,14 +149,6 @@ __device__ __forceinline__ double warp_max_pos(double x) {
     return __longlong_as_double((long long) (((unsigned long long) hi << 32) | lo));
 }
 
-// Smallest of a warp's values >= 0.
-__device__ __forceinline__ double warp_min_pos(double x) {
-    const unsigned long long b = (unsigned long long) __double_as_longlong(x);
-    const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned) (b >> 32));
-    const unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned) (b >> 32) == hi ? (unsigned) b : 0xffffffffu);
-    return __longlong_as_double((long long) (((unsigned long long) hi << 32) | lo));
-}
-
 // Smallest of n stamped doubles >= 0, by one warp, up to five words a lane in flight at once.
 __device__ __forceinline__ bool ll_least(const ulonglong2* p, int n, unsigned stamp, double& least_out, unsigned polls,
                                          unsigned* err) {

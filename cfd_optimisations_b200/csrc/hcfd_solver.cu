@@ -187,7 +187,7 @@ hcfd::StepArgs<T> step_args(hcfd_solver* s, int time_mode, double dt_or_cfl) {
     a.bc = s->bc;
     a.phiF = (hcfd::Cell4<T>*) s->d_phiF;
     a.freeze_after = s->prm.freeze_limiter_after;
-    a.clear_stats = nullptr;
+    a.block_dt = nullptr;
     return a;
 }
 
@@ -321,10 +321,10 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl, bool want_res) 
         const int grid = nblk(s->Nc, s->block);
         hcfd::StepArgs<T> a = step_args<T>(s, time_mode, dt_or_cfl);
         if ((rc = prof_begin(s, rec, e1))) return rc;
-        hcfd::pass1_kernel<T, W><<<grid, s->block, 0, s->stream>>>(a);
+        hcfd::pass1_kernel<T, W, false><<<grid, s->block, 0, s->stream>>>(a);
         if ((rc = prof_end(s, rec, e1, s->ev1))) return rc;
         if ((rc = prof_begin(s, rec, e2))) return rc;
-        hcfd::pass2_kernel<T, W, std::is_same<T, float>::value><<<grid, s->block, 0, s->stream>>>(a);
+        hcfd::pass2_kernel<T, W, std::is_same<T, float>::value, false><<<grid, s->block, 0, s->stream>>>(a);
         if ((rc = prof_end(s, rec, e2, s->ev2))) return rc;
     }
     CK(cudaGetLastError());
