@@ -589,6 +589,14 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
 // ---------------------------------------------------------------------------------------
 // pass 2: reconstruction + flux + gather + update + ghost refresh (+ residual)
 
+// Pass 1's limited gradient of a cell: through the read-only path, whose lines a block's cells share,
+// unless pass 1 may still be writing when this kernel starts (OWN).
+template <bool OWN, class T>
+__device__ __forceinline__ void ld_phig(const StepArgs<T>& a, int i, T g[8]) {
+    if (OWN) ld_grad_l2(a.phiG, a.Nc, i, g);
+    else ld_grad(a.phiG, a.Nc, i, g);
+}
+
 template <class T, int W, bool COMP, bool OWN>
 __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -618,7 +626,7 @@ __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
     T u[4], pg[8];
     if (c < a.Nc && s[0].y >= 0) {
         ld_cell(a.U, a.Nc, c, u);
-        ld_grad_l2(a.phiG, a.Nc, c, pg);
+        ld_phig<OWN>(a, c, pg);
     }
     if (a.time_mode == TM_FIXED) {
         dt_used = a.dt_or_cfl;
@@ -666,7 +674,7 @@ __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
                     }
                 } else {
                     T pn[8];
-                    ld_grad_l2(a.phiG, a.Nc, s[k].y, pn);
+                    ld_phig<OWN>(a, s[k].y, pn);
 #pragma unroll
                     for (int v = 0; v < 4; v++) {
                         uo[v] = u[v] + (pg[2 * v] * ro0 + pg[2 * v + 1] * ro1);
