@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(256) pass2_kernel(const StepArgs<T> a) {
             st->dt_last = dt_used;
             if (!(tot == tot) || tot > 1.7e308) st->nonfinite = 1;
             *a.counter = 0u;
-            if (!OWN && a.time_mode != TM_FIXED) *a.dtmin_next = 0x7FF0000000000000ULL;   // +inf
+            if (!OWN) *a.dtmin_next = 0x7FF0000000000000ULL;   // +inf (in every mode, as finish_step)
         }
     }
 }

@@ -588,7 +588,9 @@ __device__ __forceinline__ void finish_step(const StepArgs<T>& a, double r2, int
             st->dt_last = dt_used;
             if (!(tot == tot) || tot > 1.7e308) st->nonfinite = 1;
             *a.counter = 0u;
-            if (a.time_mode != TM_FIXED) *a.dtmin_next = 0x7FF0000000000000ULL;
+            // after a fixed step too: the next call may step under a CFL number, and the other slot
+            // holds the minimum of the step before
+            *a.dtmin_next = 0x7FF0000000000000ULL;
         }
     }
 }
@@ -1031,7 +1033,7 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
             if (not_finite<T>(top)) atomicOr(&s.stats->nonfinite, 1);
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 s.stats->steps += 1;
-                if (s.time_mode != TM_FIXED) *s.dtmin_next = 0x7FF0000000000000ULL;
+                *s.dtmin_next = 0x7FF0000000000000ULL;
             }
         }
     }
