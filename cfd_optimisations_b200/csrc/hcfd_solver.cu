@@ -303,6 +303,9 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl, bool want_res) 
             (rc = prof_end(s, rec, e1, s->ev1)) || (rc = prof_begin(s, rec, e2)) ||
             (rc = launch_resident<T, W>(s, time_mode, dt_or_cfl, 1, 2)) || (rc = prof_end(s, rec, e2, s->ev2)))
             return rc;
+        // The halves passed unstamped gradients through the words' memory: a value whose upper halves
+        // are a coming step's stamp would be taken for that step's word.
+        CK(cudaMemsetAsync(s->d_ll, 0, sizeof(ulonglong2) * s->ll_words, s->stream));
         return HCFD_OK;
     }
     if (s->tiled) {
