@@ -300,6 +300,7 @@ hcfd::TileArgs<T> arena_args(hcfd_arena* A, int cur, int par) {
     a.tmeta = A->tmeta;
     a.halo = A->halo;
     a.nbr = A->nbr;
+    a.cslot = nullptr;
     a.ntiles = A->nact_tiles;
     a.B = A->B;
     a.Wp = A->Wp;

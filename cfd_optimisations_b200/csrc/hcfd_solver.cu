@@ -63,6 +63,7 @@ struct TiledPass {
     unsigned* d_tmeta = nullptr;         // pack_meta words [entries]
     int *d_foff = nullptr, *d_hoff = nullptr, *d_halo = nullptr;
     unsigned* d_nbr = nullptr;           // pack_nbr_kernel's words
+    short* d_cslot = nullptr;            // the plan's 16-bit words: kept for a pass with short words, else set-up only
     int* d_efid = nullptr;               // set-up only
     int block = 0;                       // compute threads per CTA
     int rec = 8;                         // values per face record (7: pass 2 on a plan of its own)
@@ -96,6 +97,7 @@ struct hcfd_solver {
     // tiled kernels
     TiledPass tp[2];                     // pass 1; pass 2 when it has its own tiling
     bool split = false;                  // pass 2 uses tp[1]
+    bool short1 = false, short2 = false; // the pass stages 16-bit face words: its tiles do not fit with 32-bit ones
     size_t smem1 = 0, smem2 = 0;
     int grid1 = 0, grid2 = 0;
     // tile queues (d_counter[1] for pass 1, d_counter[2] for pass 2): CTAs that finish
@@ -152,7 +154,7 @@ void free_all(hcfd_solver* s) {
                     s->d_phiG, s->d_phiF, s->d_io, s->d_cp, s->d_dtmin, s->d_partial, s->d_counter, s->d_stats, s->d_flags, s->d_ll};
     for (void* p : ptrs) if (p) cudaFree(p);
     for (TiledPass& P : s->tp) {
-        void* q[] = {P.d_tgeo, P.d_tmeta, P.d_foff, P.d_hoff, P.d_halo, P.d_nbr, P.d_efid};
+        void* q[] = {P.d_tgeo, P.d_tmeta, P.d_foff, P.d_hoff, P.d_halo, P.d_nbr, P.d_cslot, P.d_efid};
         for (void* p : q) if (p) cudaFree(p);
     }
     if (s->graph) cudaGraphExecDestroy(s->graph);
@@ -206,6 +208,7 @@ hcfd::TileArgs<T> tile_args(hcfd_solver* s, int time_mode, double dt_or_cfl, con
     a.hoff = P.d_hoff;
     a.halo = P.d_halo;
     a.nbr = P.d_nbr;
+    a.cslot = (pass == 1 ? s->short1 : s->short2) ? P.d_cslot : nullptr;
     a.ntiles = P.plan.ntiles;
     a.B = P.plan.B;
     a.Wp = P.plan.Wp;
@@ -317,7 +320,7 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl, bool want_res) 
                                   s->smem1, s->stream, a1));
         if ((rc = prof_end(s, rec, e1, s->ev1))) return rc;
         if ((rc = prof_begin(s, rec, e2))) return rc;
-        CK(hcfd::launch_dependent(hcfd::pass2_variant<T, W, false>(P2.rec, time_mode), s->grid2, P2.block + 32, s->smem2,
+        CK(hcfd::launch_dependent(hcfd::pass2_variant<T, W, false>(P2.rec, time_mode, s->short2), s->grid2, P2.block + 32, s->smem2,
                                   s->stream, a2));
         if ((rc = prof_end(s, rec, e2, s->ev2))) return rc;
     } else {
@@ -359,8 +362,8 @@ int setup_tiled_w(hcfd_solver* s) {
     const hcfd::TilePlan& P = s->tp[0].plan;
     const TiledPass& T2 = s->split ? s->tp[1] : s->tp[0];
     const hcfd::TilePlan& Q = T2.plan;
-    s->smem1 = hcfd::TileSmem<T>(P.B, P.Hmax, P.Fmax, W, P.Wp, false).total;
-    s->smem2 = hcfd::TileSmem<T>(Q.B, Q.Hmax, Q.Fmax, W, Q.Wp, true).total;
+    s->smem1 = hcfd::TileSmem<T>(P.B, P.Hmax, P.Fmax, W, P.Wp, false, s->short1).total;
+    s->smem2 = hcfd::TileSmem<T>(Q.B, Q.Hmax, Q.Fmax, W, Q.Wp, true, s->short2).total;
     int maxsm = 0;
     CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
     if ((int) s->smem2 > maxsm || (int) s->smem1 > maxsm) return fail(HCFD_EINVAL, "tile does not fit in shared memory");
@@ -368,7 +371,7 @@ int setup_tiled_w(hcfd_solver* s) {
     int b1 = 0, b2 = 0;
     for (int mode : {HCFD_FIXED_DT, HCFD_GLOBAL_CFL, HCFD_LOCAL_CFL}) {
         const void* k1 = (const void*) hcfd::pass1_variant<T, W, false>(s->prm.limiter, mode);
-        const void* k2 = (const void*) hcfd::pass2_variant<T, W, false>(s->split ? 7 : 8, mode);
+        const void* k2 = (const void*) hcfd::pass2_variant<T, W, false>(s->split ? 7 : 8, mode, s->short2);
         int n1 = 0, n2 = 0, rc;
         if ((rc = allow_smem(k1, maxsm)) || (rc = allow_smem(k2, maxsm))) return rc;
         // blocks of the tiled kernels: `block` compute threads + one producer warp
@@ -558,9 +561,18 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         const bool f64 = p.precision == HCFD_FP64;
         int maxsm = 0;
         CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
-        auto need = [&](const hcfd::TilePlan& Q, bool pass2) {
-            return f64 ? hcfd::TileSmem<double>(Q.B, Q.Hmax, Q.Fmax, s->W, Q.Wp, pass2).total
-                       : hcfd::TileSmem<float>(Q.B, Q.Hmax, Q.Fmax, s->W, Q.Wp, pass2).total;
+        // With 32-bit face words, or where only that makes them fit with the plan's 16-bit ones, which a
+        // kernel variant widens as it reads them (pass 1 with three or four faces a cell, which stages no
+        // metadata then, is never the larger for the 32-bit words where it is near the limit).
+        auto fits = [&](const hcfd::TilePlan& Q, bool pass2, bool& short_words) {
+            for (int k = 0; k < (pass2 || s->W == 8 ? 2 : 1); k++) {
+                short_words = k == 1;
+                const size_t need = f64 ? hcfd::TileSmem<double>(Q.B, Q.Hmax, Q.Fmax, s->W, Q.Wp, pass2, short_words).total
+                                        : hcfd::TileSmem<float>(Q.B, Q.Hmax, Q.Fmax, s->W, Q.Wp, pass2, short_words).total;
+                // beside the kernels' static shared memory: pass 1's sums of a warp, finish_step's in pass 2
+                if (need + (pass2 ? 512 : 32 * (f64 ? sizeof(double) : sizeof(float))) <= (size_t) maxsm) return true;
+            }
+            return false;
         };
         std::vector<int> c1 = p.tile ? std::vector<int>{p.tile} : std::vector<int>{f64 ? 224 : 256, 128, 64};
         std::vector<int> c2 = p.tile2 ? std::vector<int>{p.tile2}
@@ -569,7 +581,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         for (int t : c1) {
             rc = hcfd::build_tile_plan(*mv, cf_off, cf_con, ghost, perm, s->F_BC, bc_first, t, s->W, s->tp[0].plan);
             if (rc != HCFD_OK) return rc;
-            if (need(s->tp[0].plan, false) <= (size_t) maxsm) { ok = true; break; }
+            if (fits(s->tp[0].plan, false, s->short1)) { ok = true; break; }
         }
         if (!ok) return fail(HCFD_EINVAL, "tile does not fit in shared memory");
         const int tile1 = s->tp[0].plan.B;
@@ -577,13 +589,13 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         ok = false;
         for (int t : c2) {
             if (t == tile1) {
-                if (need(s->tp[0].plan, true) <= (size_t) maxsm) { s->split = false; ok = true; break; }
+                if (fits(s->tp[0].plan, true, s->short2)) { s->split = false; ok = true; break; }
                 continue;
             }
             rc = hcfd::build_tile_plan(*mv, cf_off, cf_con, ghost, perm, s->F_BC, bc_first, t, s->W, s->tp[1].plan,
                                        true);
             if (rc != HCFD_OK) return rc;
-            if (need(s->tp[1].plan, true) <= (size_t) maxsm) {
+            if (fits(s->tp[1].plan, true, s->short2)) {
                 s->split = true;
                 s->tp[1].block = p.block ? p.block : std::min(t, 256);
                 ok = true;
@@ -622,12 +634,16 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
     int* d_fn = nullptr; int* d_fcu = nullptr; int* d_cnoff = nullptr; int* d_cncon = nullptr;
     int* d_cfoff = nullptr; int* d_cfcon = nullptr;
     double* d_nodes = nullptr; double* d_xc = nullptr; double* d_ivu = nullptr;
-    short* d_cslot[2] = {nullptr, nullptr};
     auto free_tmp = [&]() {
         cudaStreamSynchronize(h->stream);
-        void* t[] = {d_fn, d_fcu, d_cnoff, d_cncon, d_cfoff, d_cfcon, d_nodes, d_xc, d_ivu, h->tp[0].d_efid, h->tp[1].d_efid, d_cslot[0], d_cslot[1]};
+        void* t[] = {d_fn, d_fcu, d_cnoff, d_cncon, d_cfoff, d_cfcon, d_nodes, d_xc, d_ivu, h->tp[0].d_efid, h->tp[1].d_efid};
         for (void* q : t) if (q) cudaFree(q);
         h->tp[0].d_efid = h->tp[1].d_efid = nullptr;
+        for (int k = 0; k < 2; k++) {
+            if ((k == 0 && h->short1) || (h->short2 && k == (h->split ? 1 : 0))) continue;
+            if (h->tp[k].d_cslot) cudaFree(h->tp[k].d_cslot);
+            h->tp[k].d_cslot = nullptr;
+        }
     };
     const int ncn = mv->cn_off[Nc];
     // iv is read one whole tile at a time by the tiled kernels: pad it to full tiles.
@@ -657,7 +673,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
             if ((rc = dalloc((char**) &P.d_tgeo, tsz * P.rec * E)) || (rc = dalloc(&P.d_tmeta, E)) ||
                 (rc = dalloc(&P.d_foff, P.plan.foff.size())) || (rc = dalloc(&P.d_hoff, P.plan.hoff.size())) ||
                 (rc = dalloc(&P.d_halo, P.plan.halo.size())) || (rc = dalloc(&P.d_nbr, P.plan.cslot.size())) ||
-                (rc = dalloc(&d_cslot[k], P.plan.cslot.size())) || (rc = dalloc(&P.d_efid, E))) {
+                (rc = dalloc(&P.d_cslot, P.plan.cslot.size())) || (rc = dalloc(&P.d_efid, E))) {
                 free_tmp();
                 return bail(rc);
             }
@@ -696,7 +712,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
             if (ce == cudaSuccess) ce = up(T.d_foff, P.foff.data(), 4 * P.foff.size());
             if (ce == cudaSuccess) ce = up(T.d_hoff, P.hoff.data(), 4 * P.hoff.size());
             if (ce == cudaSuccess) ce = up(T.d_halo, P.halo.data(), 4 * P.halo.size());
-            if (ce == cudaSuccess) ce = up(d_cslot[k], P.cslot.data(), 2 * P.cslot.size());
+            if (ce == cudaSuccess) ce = up(T.d_cslot, P.cslot.data(), 2 * P.cslot.size());
             if (ce == cudaSuccess) ce = up(T.d_efid, P.efid.data(), 4 * P.efid.size());
         }
         if (h->resident) {
@@ -725,7 +741,7 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
         for (int k = 0; h->tiled && k < (h->split ? 2 : 1); k++) {
             TiledPass& T = h->tp[k];
             const int nt = T.plan.ntiles;
-            hcfd::pack_nbr_kernel<<<nt, 128, 0, st>>>(T.plan.B * T.plan.Wp, T.d_foff, T.d_tmeta, d_cslot[k], T.d_nbr);
+            hcfd::pack_nbr_kernel<<<nt, 128, 0, st>>>(T.plan.B * T.plan.Wp, T.d_foff, T.d_tmeta, T.d_cslot, T.d_nbr);
             if (T.plan.efid.empty()) continue;
             if (f32) hcfd::gather_geo_kernel<float><<<nt, 128, 0, st>>>(nt, T.d_foff, T.d_efid, h->d_geo64, (float*) T.d_tgeo, T.rec);
             else hcfd::gather_geo_kernel<double><<<nt, 128, 0, st>>>(nt, T.d_foff, T.d_efid, h->d_geo64, (double*) T.d_tgeo, T.rec);

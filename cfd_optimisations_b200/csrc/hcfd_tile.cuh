@@ -35,6 +35,8 @@ struct TileArgs {
     const int* __restrict__ hoff;          // [ntiles + 1]
     const int* __restrict__ halo;          // internal cell ids
     const unsigned* __restrict__ nbr;      // [ntiles * B * Wp]: a word per cell and face (pack_nbr_kernel); Wp = W
+    const short* __restrict__ cslot;       // the same as the plan's 16-bit {entry, side}, staged in their place by the
+                                           // variants of arguments read at run time; null: the words are staged
     int ntiles, B, Wp, Hmax, Fmax;
     unsigned int* err;                     // bit 0: a bounded wait gave up; bit 1: copies did not drain;
                                            // bit 2: an index out of range (checked build)
@@ -87,6 +89,12 @@ __device__ __forceinline__ int meta_bc(unsigned w) { return (int) (w >> 26) - 1;
 // kNoFace for a position the cell does not use.  With it a cell's loads of face record and neighbour
 // state both hang on one word, not on the entry's metadata in between (pass 1 reads none).
 constexpr unsigned kNoFace = 0xFFFFFFFFu, kBoundaryFace = 1u << 28;
+// The word of the plan's {entry, side} (-1: none), m the packed metadata of the tile's entries.
+__device__ __forceinline__ unsigned nbr_word(int s, const unsigned* m) {
+    if (s < 0) return kNoFace;
+    const unsigned e = (unsigned) s >> 1, side = s & 1, x = m[e];
+    return e | (side << 14) | ((side ? x & 0x1FFFu : (x >> 13) & 0x1FFFu) << 15) | (x >> 26 ? kBoundaryFace : 0u);
+}
 // A block per tile: the words of its cells, from the plan's {entry, side} table (cslot, -1: none) and the
 // packed metadata of the tile's entries.  Packed on the host, creating a solver of 1025x513 nodes took
 // 1,171 ms (FP64) and 1,195 (FP32), packed here 1,123 and 1,165 (the quickest of 14).
@@ -94,15 +102,7 @@ static __global__ void pack_nbr_kernel(int per, const int* __restrict__ foff, co
                                 const short* __restrict__ cslot, unsigned* __restrict__ nbr) {
     const size_t t0 = (size_t) blockIdx.x * per;
     const unsigned* m = meta + foff[blockIdx.x];
-    for (int i = threadIdx.x; i < per; i += blockDim.x) {
-        const int s = cslot[t0 + i];
-        unsigned w = kNoFace;
-        if (s >= 0) {
-            const unsigned e = (unsigned) s >> 1, side = s & 1, x = m[e];
-            w = e | (side << 14) | ((side ? x & 0x1FFFu : (x >> 13) & 0x1FFFu) << 15) | (x >> 26 ? kBoundaryFace : 0u);
-        }
-        nbr[t0 + i] = w;
-    }
+    for (int i = threadIdx.x; i < per; i += blockDim.x) nbr[t0 + i] = nbr_word(cslot[t0 + i], m);
 }
 __device__ __forceinline__ int nbr_entry(unsigned w) { return (int) (w & 0x3FFFu); }
 __device__ __forceinline__ bool nbr_right(unsigned w) { return (w >> 14) & 1u; }
@@ -117,6 +117,18 @@ __device__ __forceinline__ void lds_nbr(const unsigned* p, unsigned x[W]) {
             const uint4 v = *reinterpret_cast<const uint4*>(p + k);
             x[k] = v.x; x[k + 1] = v.y; x[k + 2] = v.z; x[k + 3] = v.w;
         }
+    }
+}
+
+// GEN: the variant may have 16-bit words staged (sNbr then points at them), which are widened here.
+template <int W, bool GEN>
+__device__ __forceinline__ void cell_words(const unsigned* sNbr, bool short_words, const unsigned* sMeta, int c, unsigned x[W]) {
+    if (GEN && short_words) {
+        const short* q = reinterpret_cast<const short*>(sNbr) + c * W;
+#pragma unroll
+        for (int k = 0; k < W; k++) x[k] = nbr_word(q[k], sMeta);
+    } else {
+        lds_nbr<W>(sNbr + c * W, x);
     }
 }
 
@@ -312,13 +324,14 @@ __host__ __device__ constexpr size_t align128(size_t x) { return (x + 127) & ~si
 template <class T>
 struct TileSmem {
     size_t u, g, geo, meta, nbr, iv, stage, total;   // byte offsets within a stage
-    __host__ __device__ TileSmem(int B, int Hmax, int Fmax, int W, int Wp, bool pass2) {
+    // short_words: the plan's 16-bit face words and the metadata they need, in place of the 32-bit words
+    __host__ __device__ TileSmem(int B, int Hmax, int Fmax, int W, int Wp, bool pass2, bool short_words = false) {
         size_t p = 0;
         u = p;     p += align128((size_t) (B + Hmax) * sizeof(Cell4<T>));
         g = p;     if (pass2) p += align128((size_t) (B + Hmax) * sizeof(Grad8<T>));
         geo = p;   p += align128((size_t) Fmax * sizeof(FaceGeo<T>));
-        meta = p;  if (pass2) p += align128((size_t) Fmax * 4);
-        nbr = p;   p += align128((size_t) B * Wp * sizeof(unsigned));
+        meta = p;  if (pass2 || short_words) p += align128((size_t) Fmax * 4);
+        nbr = p;   p += align128((size_t) B * Wp * (short_words ? sizeof(short) : sizeof(unsigned)));
         iv = p;    p += align128((size_t) B * sizeof(T));
         stage = p;
         total = kHeader + 2 * stage;
@@ -365,7 +378,7 @@ __device__ __forceinline__ void claim_tile(int* queue, bool on, int& tile) {
 // tile in FP64 pass 1 and 4,700-5,500 in the FP32 passes, where computing one takes 3,500 and
 // 1,700-2,000).  A deeper pipeline of claims (five tiles by position, results taken up an iteration
 // later) cost FP64 2 % at 2001x1001: tiles claimed early are tiles the CTAs that end first cannot take.
-template <class T, bool PASS2, bool ARENA>
+template <class T, bool PASS2, bool ARENA, bool GEN>
 __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned char* smem, unsigned long long* full,
                                               unsigned long long* empty, const TileSmem<T>& L) {
     const int lane = threadIdx.x & 31;
@@ -444,16 +457,19 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
         if (lane != 0) return;
         const unsigned nb = good ? d.nb : 0, nf = good ? d.nf : 0;
         const unsigned bu = nb * sizeof(Cell4<T>), bg = PASS2 ? nb * sizeof(Grad8<T>) : 0u;
-        const unsigned bf = nf * a.rec * (unsigned) sizeof(T), bm = PASS2 ? nf * 4u : 0u;
-        const unsigned bs = good ? a.B * a.Wp * sizeof(unsigned) : 0u, bi = good ? a.B * sizeof(T) : 0u;
+        const bool short_words = GEN && a.cslot;
+        const unsigned bf = nf * a.rec * (unsigned) sizeof(T), bm = PASS2 || short_words ? nf * 4u : 0u;
+        const unsigned bs = good ? a.B * a.Wp * (short_words ? sizeof(short) : sizeof(unsigned)) : 0u;
+        const unsigned bi = good ? a.B * sizeof(T) : 0u;
         unsigned char* st = smem + kHeader + buf * L.stage;
         mbar_expect_tx(full + buf, bu + bg + bf + bm + bs + bi);
         if (bf) {
             bulk_g2s(st + L.geo, a.tgeo + (size_t) d.f0 * a.rec, bf, full + buf);
-            if (PASS2) bulk_g2s(st + L.meta, a.tmeta + d.f0, bm, full + buf);
+            if (bm) bulk_g2s(st + L.meta, a.tmeta + d.f0, bm, full + buf);
         }
         if (bs) {
-            bulk_g2s(st + L.nbr, a.nbr + (size_t) d.base * a.Wp, bs, full + buf);
+            bulk_g2s(st + L.nbr, short_words ? (const void*) (a.cslot + (size_t) d.base * a.Wp) : a.nbr + (size_t) d.base * a.Wp,
+                     bs, full + buf);
             bulk_g2s(st + L.iv, a.s.iv + d.base, bi, full + buf);
         }
     };
@@ -732,7 +748,7 @@ __device__ __forceinline__ T cell_update(const T* u, const T* R, T iv, T dt, T* 
 // it marks the compute abort word and skips the face phase (`staged` false); every compute
 // warp then meets at the compute barrier that ends the face phase and leaves the loop
 // there if any of them gave up, so none is left waiting at that barrier.
-#define HCFD_TILE_LOOP_BEGIN(PASS2, ARENA)                                                       \
+#define HCFD_TILE_LOOP_BEGIN(PASS2, ARENA, GEN)                                                  \
     const int NT = blockDim.x - 32;                                                              \
     const int NL = a.B + a.Hmax;                                                                 \
     unsigned long long* full = reinterpret_cast<unsigned long long*>(smem);                      \
@@ -746,7 +762,7 @@ __device__ __forceinline__ T cell_update(const T* u, const T* R, T iv, T dt, T* 
     }                                                                                            \
     __syncthreads();                                                                             \
     if ((int) threadIdx.x >= NT) {                                                               \
-        producer_loop<T, PASS2, ARENA>(a, smem, full, empty, L);                                 \
+        producer_loop<T, PASS2, ARENA, GEN>(a, smem, full, empty, L);                            \
     } else {                                                                                     \
     grid_wait_previous();                                                                        \
     if (a.claim_reset && blockIdx.x == 0 && threadIdx.x == 0) *a.claim_reset = 0;               \
@@ -767,6 +783,7 @@ __device__ __forceinline__ T cell_update(const T* u, const T* R, T iv, T dt, T* 
         const T* sGeo = reinterpret_cast<const T*>(st + L.geo);                                  \
         const int nfl = si.nf;                                                                   \
         const unsigned* sNbr = reinterpret_cast<const unsigned*>(st + L.nbr);                    \
+        const unsigned* sMeta = reinterpret_cast<const unsigned*>(st + L.meta);                  \
         const T* sIv = reinterpret_cast<const T*>(st + L.iv);
 
 #define HCFD_TILE_LOOP_END                                                                       \
@@ -855,15 +872,16 @@ __device__ __forceinline__ void tile_faces(Pass1Cell<T, NVAR>& p, const unsigned
 template <class T, int W, bool ARENA, int LIM, int LAM>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : W == 3 ? 56 : 72) tile_pass1_kernel(const TileArgs<T> a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const TileSmem<T> L(a.B, a.Hmax, a.Fmax, W, a.Wp, false);
+    constexpr bool GEN = LIM < 0;
+    const TileSmem<T> L(a.B, a.Hmax, a.Fmax, W, a.Wp, false, GEN && a.cslot);
     const StepArgs<T>& s = a.s;
     T xmx = T(0);                        // largest iv * lam (see dt_of_max)
-    HCFD_TILE_LOOP_BEGIN(false, ARENA)
+    HCFD_TILE_LOOP_BEGIN(false, ARENA, GEN)
     const int lmode = limiter_mode(si.steps, s.freeze_after);
     const bool with_lam = LAM >= 0 ? LAM != 0 : s.time_mode != TM_FIXED;
     for (int c = threadIdx.x; c < nb; c += NT) {
         unsigned x[W];
-        lds_nbr<W>(sNbr + c * W, x);
+        cell_words<W, GEN>(sNbr, a.cslot, sMeta, c, x);
         if (x[0] == kNoFace) continue;
         Pass1Cell<T> p;
         const T iv = sIv[c];
@@ -911,15 +929,15 @@ template <class T, int W, bool ARENA, int REC, int LOCAL>
 __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
     constexpr bool COMP = sizeof(T) == 4;
     extern __shared__ __align__(128) unsigned char smem[];
-    const TileSmem<T> L(a.B, a.Hmax, a.Fmax, W, a.Wp, true);
+    constexpr bool GEN = REC < 0;
+    const TileSmem<T> L(a.B, a.Hmax, a.Fmax, W, a.Wp, true, GEN && a.cslot);
     const StepArgs<T>& s = a.s;
     double dt_used = 0.0;
     double r2 = 0.0;
     int top = 0;
     const int rec = REC >= 0 ? REC : a.rec;
     const bool local = LOCAL >= 0 ? LOCAL != 0 : s.time_mode == TM_LOCAL;
-    HCFD_TILE_LOOP_BEGIN(true, ARENA)
-    const unsigned* sMeta = reinterpret_cast<const unsigned*>(st + L.meta);
+    HCFD_TILE_LOOP_BEGIN(true, ARENA, GEN)
     const T cfl_or_dt = T(si.dt_or_cfl);
     if (staged && !fin) dt_used = (s.time_mode == TM_FIXED) ? si.dt_or_cfl : si.dt_or_cfl * si.dtmin;
     const Grad8<T>* sG = reinterpret_cast<const Grad8<T>*>(st + L.g);
@@ -969,7 +987,7 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
     // cell phase: slots in increasing face order, update, ghost refresh
     for (int c = threadIdx.x; c < nb; c += NT) {
         unsigned x[W];
-        lds_nbr<W>(sNbr + c * W, x);
+        cell_words<W, GEN>(sNbr, a.cslot, sMeta, c, x);
         if (x[0] == kNoFace) continue;
         T u[4];
         lds_cell(sU, NL, c, u);
@@ -988,7 +1006,7 @@ __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
         if (!any) continue;
 #pragma unroll 1
         for (int k = 0; k < W; k++) {
-            const unsigned xk = sNbr[c * W + k];
+            const unsigned xk = GEN && a.cslot ? nbr_word(reinterpret_cast<const short*>(sNbr)[c * W + k], sMeta) : sNbr[c * W + k];
             if (xk == kNoFace || !(xk & kBoundaryFace)) continue;
             const int e = nbr_entry(xk), lb = nbr_local(xk);
             if (!index_ok(e < nf && local_ok(lb, nb, a.B, si.nh), a.err)) continue;
@@ -1070,11 +1088,13 @@ TileKernel<T> pass1_variant(int limiter, int time_mode) {
     }
 }
 template <class T, int W, bool ARENA>
-TileKernel<T> pass2_variant(int rec, int time_mode) {
+TileKernel<T> pass2_variant(int rec, int time_mode, bool short_words = false) {
     if constexpr (W == 8) {
         return tile_pass2_kernel<T, W, ARENA, -1, -1>;
     } else {
         const bool local = time_mode == TM_LOCAL;
+        if constexpr (!ARENA)
+            if (short_words) return tile_pass2_kernel<T, W, ARENA, -1, -1>;
         if constexpr (!ARENA)
             if (rec == 7) return local ? tile_pass2_kernel<T, W, ARENA, 7, 1> : tile_pass2_kernel<T, W, ARENA, 7, 0>;
         return local ? tile_pass2_kernel<T, W, ARENA, 8, 1> : tile_pass2_kernel<T, W, ARENA, 8, 0>;
