@@ -350,8 +350,8 @@ __device__ __forceinline__ void compute_sync(int nthreads) {
 }
 
 // Producer warp: for each of this CTA's tiles, waits until the compute warps have released
-// the staging buffer, then lane 0 arms the buffer's `full` mbarrier with the byte count of
-// the bulk copies and issues them, and every lane gathers its share of the halo cells with
+// the staging buffer, then lane 0 arms the buffer's `full` mbarrier with the byte counts of
+// the bulk copies and issues them (those of the first tile that no kernel writes ahead of the rest), and every lane gathers its share of the halo cells with
 // cp.async and signals their completion on the same mbarrier.  The `full` barrier therefore
 // completes when all of the tile's data has landed: 1 expect-tx arrival + 32 cp.async
 // arrivals + the transaction bytes.
@@ -451,18 +451,17 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
     d0 = describe(t0, q0);
     load_ids(t0, d0, id0);
     d1 = describe(t1, q1);
-    // Arms stage `buf` for a tile and copies what no kernel writes: its face records and metadata, face
-    // words and 1 / areas.
+    // Copies into stage `buf` what no kernel writes of a tile, its face records and metadata, face words
+    // and 1 / areas, and adds their bytes to the stage's phase.
     auto stage_static = [&](const TileDesc& d, bool good, int buf) {
         if (lane != 0) return;
-        const unsigned nb = good ? d.nb : 0, nf = good ? d.nf : 0;
-        const unsigned bu = nb * sizeof(Cell4<T>), bg = PASS2 ? nb * sizeof(Grad8<T>) : 0u;
+        const unsigned nf = good ? d.nf : 0;
         const bool short_words = GEN && a.cslot;
         const unsigned bf = nf * a.rec * (unsigned) sizeof(T), bm = PASS2 || short_words ? nf * 4u : 0u;
         const unsigned bs = good ? a.B * a.Wp * (short_words ? sizeof(short) : sizeof(unsigned)) : 0u;
         const unsigned bi = good ? a.B * sizeof(T) : 0u;
         unsigned char* st = smem + kHeader + buf * L.stage;
-        mbar_expect_tx(full + buf, bu + bg + bf + bm + bs + bi);
+        mbar_expect_tx(full + buf, bf + bm + bs + bi);
         if (bf) {
             bulk_g2s(st + L.geo, a.tgeo + (size_t) d.f0 * a.rec, bf, full + buf);
             if (bm) bulk_g2s(st + L.meta, a.tmeta + d.f0, bm, full + buf);
@@ -474,7 +473,8 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
         }
     };
     // the first tile's while the kernel before this one ends; everything else waits for it
-    if (t0 < a.ntiles && t0 != a.skip_tile) stage_static(d0, !kChecked || d0.nb >= 0, 0);
+    const bool ahead = t0 < a.ntiles && t0 != a.skip_tile;
+    if (ahead) stage_static(d0, !kChecked || d0.nb >= 0, 0);
     grid_wait_previous();
     load_scalars(d0.inst, v0);
     v1 = v0;
@@ -516,7 +516,7 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
                 si->dt_or_cfl = v0.dt;
                 si->dtmin = v0.dtmin;
                 si->steps = v0.steps;
-                mbar_arrive(full + buf);
+                mbar_arrive_expect_tx(full + buf, nb * (unsigned) (sizeof(Cell4<T>) + (PASS2 ? sizeof(Grad8<T>) : 0)));
                 if (nb) {
                     // one bulk copy per 16-byte chunk plane of the tile's cell range
 #pragma unroll
@@ -557,6 +557,17 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
             t2 = a.claim ? 3 * (int) gridDim.x + __shfl_sync(0xffffffffu, pending, 0) : t2 + (int) gridDim.x;
     }
     cp_async_wait_all();
+    if (ahead && armed[0] < 0) {
+        // The CTA gave up before the first tile's stage was armed in full, with its static copies in flight:
+        // the stage is closed as at the end, with tile -1 and the arrivals it lacks, and completes when
+        // they have landed.
+        if (lane == 0) {
+            reinterpret_cast<StageInfo*>(smem + 64)[0].t = -1;
+            mbar_arrive(full);
+        }
+        cp_async_arrive_noinc(full);
+        armed[0] = 0;
+    }
     for (int b = 0; b < 2; b++)
         if (armed[b] >= 0) mbar_drain(full + b, ((unsigned) armed[b] >> 1) & 1, a.err);
 }
