@@ -832,9 +832,10 @@ int hcfd_arena_fetch(hcfd_arena* A, int slot, int prims, double* const* out) {
     else
         arena_out_kernel<double><<<nblk(I.Nc, 256), 256, 0, A->stream>>>(A->Ccap, I.c0, I.Nc, (const Cell4<double>*) A->U[A->cur], I.d_perm, A->prm.gma, prims, d_out);
     cudaError_t e = cudaGetLastError();
-    const int blocks = hcfd::one_block(out, I.Nc) ? 1 : 4;
-    for (int v = 0; v < blocks && e == cudaSuccess; v++)
-        e = cudaMemcpyAsync(out[v], d_out + (size_t) v * I.Nc, sizeof(double) * 4 / blocks * I.Nc, cudaMemcpyDeviceToHost, A->stream);
+    if (e == cudaSuccess)
+        e = hcfd::copy_rows(out, I.Nc, [&](int v, size_t n) {
+            return cudaMemcpyAsync(out[v], d_out + (size_t) v * I.Nc, sizeof(double) * n, cudaMemcpyDeviceToHost, A->stream);
+        });
     cudaFreeAsync(d_out, A->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(A->stream);
     if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("arena_fetch: ") + cudaGetErrorString(e));

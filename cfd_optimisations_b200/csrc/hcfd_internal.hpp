@@ -52,13 +52,6 @@ int build_tile_plan(const hcfd_mesh_view& v, const std::vector<int>& cf_off, con
 }  // namespace hcfd
 
 namespace hcfd {
-// Whether four host arrays of n doubles follow one another (a C-contiguous 4 x n array): one copy
-// moves them, where four cost a call and a wait each.
-template <class P>
-inline bool one_block(P const* a, size_t n) { return a[1] == a[0] + n && a[2] == a[1] + n && a[3] == a[2] + n; }
-}  // namespace hcfd
-
-namespace hcfd {
 // Checkpoint file of one solve (hcfd_gpu_checkpoint / hcfd_arena_checkpoint): this header,
 // then the conservative state of every cell, variable-major, in the input numbering, as
 // doubles (FP32 values widen exactly), then, with limiter freezing, the recorded limiter

@@ -937,4 +937,21 @@ __global__ void wall_cp_kernel(int Nc, int F1, int F2, const int* __restrict__ f
     out[f - F1] = (p - p_inf) / qinf;
 }
 
+// Moves four host arrays a of n doubles by copy(v, count), which copies count doubles from array v on:
+// in one copy where they follow one another (a C-contiguous 4 x n array), saving three calls and
+// waits.  CUDA refuses that one where they are page-locked row by row, a registration each
+// (cudaErrorInvalidValue, nothing copied); then, as where they lie apart, each is copied by itself.
+// (Asking cudaPointerGetAttributes of each row first took 10 us of the 53 of a one-step call.)
+template <class P, class Copy>
+cudaError_t copy_rows(P const* a, size_t n, Copy copy) {
+    if (a[1] == a[0] + n && a[2] == a[1] + n && a[3] == a[2] + n) {
+        const cudaError_t e = copy(0, 4 * n);
+        if (e != cudaErrorInvalidValue) return e;
+        cudaGetLastError();
+    }
+    cudaError_t e = cudaSuccess;
+    for (int v = 0; v < 4 && e == cudaSuccess; v++) e = copy(v, n);
+    return e;
+}
+
 }  // namespace hcfd

@@ -935,10 +935,10 @@ int hcfd_gpu_download(hcfd_solver* s, int prims, double* const* out) {
     if (s->fp32()) hcfd::out_kernel<float><<<nblk(s->Nc, 256), 256, 0, s->stream>>>(s->Nc, (const hcfd::Cell4<float>*) s->d_U[s->cur], s->d_perm, s->prm.gma, prims, s->d_io);
     else hcfd::out_kernel<double><<<nblk(s->Nc, 256), 256, 0, s->stream>>>(s->Nc, (const hcfd::Cell4<double>*) s->d_U[s->cur], s->d_perm, s->prm.gma, prims, s->d_io);
     CK(cudaGetLastError());
-    const int blocks = hcfd::one_block(out, s->Nc) ? 1 : 4;
-    for (int v = 0; v < blocks; v++)
-        CK(cudaMemcpyAsync(out[v], s->d_io + (size_t) v * s->Nc, sizeof(double) * 4 / blocks * s->Nc, cudaMemcpyDeviceToHost,
-                           s->stream));
+    const cudaError_t e = hcfd::copy_rows(out, s->Nc, [&](int v, size_t n) {
+        return cudaMemcpyAsync(out[v], s->d_io + (size_t) v * s->Nc, sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream);
+    });
+    if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("download: ") + cudaGetErrorString(e));
     CK(cudaStreamSynchronize(s->stream));
     return HCFD_OK;
 }
@@ -949,10 +949,10 @@ int hcfd_gpu_upload(hcfd_solver* s, const double* const* in) {
     if (rc) return rc;
     if (!in) return fail(HCFD_EINVAL, "upload: null input");
     for (int v = 0; v < 4; v++) if (!in[v]) return fail(HCFD_EINVAL, "upload: null input array");
-    const int blocks = hcfd::one_block(in, s->Nc) ? 1 : 4;
-    for (int v = 0; v < blocks; v++)
-        CK(cudaMemcpyAsync(s->d_io + (size_t) v * s->Nc, in[v], sizeof(double) * 4 / blocks * s->Nc, cudaMemcpyHostToDevice,
-                           s->stream));
+    const cudaError_t e = hcfd::copy_rows(in, s->Nc, [&](int v, size_t n) {
+        return cudaMemcpyAsync(s->d_io + (size_t) v * s->Nc, in[v], sizeof(double) * n, cudaMemcpyHostToDevice, s->stream);
+    });
+    if (e != cudaSuccess) return fail(HCFD_ECUDA, std::string("upload: ") + cudaGetErrorString(e));
     if (s->fp32()) hcfd::in_kernel<float><<<nblk(s->Nc, 256), 256, 0, s->stream>>>(s->Nc, s->d_io, s->d_perm, (hcfd::Cell4<float>*) s->d_U[s->cur]);
     else hcfd::in_kernel<double><<<nblk(s->Nc, 256), 256, 0, s->stream>>>(s->Nc, s->d_io, s->d_perm, (hcfd::Cell4<double>*) s->d_U[s->cur]);
     CK(cudaGetLastError());
