@@ -12,18 +12,22 @@ Two tunings:
     an arena holding copies of a wedge of the size class, about 2 million cells in all, so
     that the timing is that of a full device and not of one launch-bound instance.
 A size class is round(log2(real cells)), clamped to [10, 24].  The winners are stored in a
-JSON cache ($HCFD_AUTOTUNE_CACHE, default ~/.cache/hcfd_b200/autotune.json).
+JSON cache ($HCFD_AUTOTUNE_CACHE, default ~/.cache/hcfd_b200/autotune.json), under the GPU's
+name and the library's contents: a winner among other kernels' timings says nothing of these.
 
     python -m cfd_optimisations_b200.autotune --cells N [--fp32] [--arena]
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import math
 import os
 import subprocess
 import time
 
+from . import native
 from . import (FP64, GLOBAL_CFL, KERNEL_CELL, KERNEL_TILED, LIMITER_BJ, NUMBER_RANDOM, Mesh, Solver, device_sync,
                wedge_case)
 
@@ -65,8 +69,17 @@ def class_mesh(cls: int) -> Mesh:
     return Mesh.wedge(2 * ny1 + 1, ny1 + 1, seed=4321, numbering=NUMBER_RANDOM)
 
 
+@functools.lru_cache(maxsize=None)
+def library_id(path: str) -> str:
+    """A digest of the native library's contents (about 10 ms, once a process)."""
+    h = hashlib.blake2b(digest_size=6)
+    with open(path, "rb") as fh:
+        h.update(fh.read())
+    return h.hexdigest()
+
+
 def _key(kind: str, cls: int, precision: int, limiter: int) -> str:
-    return f"{gpu_name()}|{kind}|{'fp64' if precision == FP64 else 'fp32'}|lim{limiter}|c{cls}"
+    return f"{gpu_name()}|lib{library_id(native.LIB_PATH)}|{kind}|{'fp64' if precision == FP64 else 'fp32'}|lim{limiter}|c{cls}"
 
 
 def _load() -> dict:
