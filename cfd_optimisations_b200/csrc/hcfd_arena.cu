@@ -332,7 +332,7 @@ int enqueue_step(hcfd_arena* A, int cur, int par, bool want_res) {
     // (measured faster for it than a queue)
     a.claim = A->queue;
     a.claim_reset = nullptr;
-    CK(hcfd::launch_dependent(hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->time_mode), A->grid1, A->B + 32, A->smem1,
+    CK(hcfd::launch_dependent(hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->prm.venkat_K, A->time_mode), A->grid1, A->B + 32, A->smem1,
                               A->stream, a));
     a.claim = nullptr;
     a.claim_reset = A->queue;
@@ -361,7 +361,7 @@ int setup_kernels(hcfd_arena* A) {
     CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, A->device));
     if ((int) s2 > maxsm || (int) s1 > maxsm) return fail(HCFD_EINVAL, "arena: tile does not fit in shared memory");
     // all a block may have: the attribute belongs to the kernel, which arenas of other tile sizes share
-    for (const void* k : {(const void*) hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->time_mode),
+    for (const void* k : {(const void*) hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->prm.venkat_K, A->time_mode),
                           (const void*) hcfd::pass2_variant<T, W, true>(8, A->time_mode)}) {
         cudaFuncAttributes fa;
         CK(cudaFuncGetAttributes(&fa, k));
@@ -378,7 +378,7 @@ int configure_kernels(hcfd_arena* A) {
     A->smem1 = hcfd::TileSmem<T>(A->B, A->Hcur, A->Fcur, W, A->Wp, false).total;
     A->smem2 = hcfd::TileSmem<T>(A->B, A->Hcur, A->Fcur, W, A->Wp, true).total;
     int b1 = 0, b2 = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->time_mode), A->B + 32, A->smem1));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, hcfd::pass1_variant<T, W, true>(A->prm.limiter, A->prm.venkat_K, A->time_mode), A->B + 32, A->smem1));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, hcfd::pass2_variant<T, W, true>(8, A->time_mode), A->B + 32, A->smem2));
     if (b1 < 1 || b2 < 1) return fail(HCFD_EINVAL, "arena: kernels cannot be resident");
     A->grid1 = b1 * A->nsm;

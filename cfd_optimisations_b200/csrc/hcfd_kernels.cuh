@@ -289,6 +289,10 @@ __device__ __forceinline__ void cell_speed(const T U[4], T gma, T& u, T& v, T& a
     a = qsqrt(gma * p * ir);
 }
 
+// Whether the limiter's values need every face's quotient (see Pass1Cell::limiter_by_face).
+template <class T>
+__host__ __device__ __forceinline__ bool by_face(int limiter, T venkat_K) { return limiter == LIM_VENKAT && venkat_K < T(0); }
+
 // Running extremes.  FP64 has no min/max instruction: fmin and fmax, with their NaN rules, cost
 // several times a compare and a select.  A NaN x leaves acc as it is, as fmin and fmax do.
 __device__ __forceinline__ double least(double acc, double x) { return x < acc ? x : acc; }
@@ -405,6 +409,27 @@ struct Pass1Cell {
         if (sizeof(T) == 8 && any) {
 #pragma unroll
             for (int v = 0; v < NVAR; v++) phi[v] = num[v] < den[v] ? num[v] / den[v] : T(1);
+        }
+    }
+    // The same face by face, r the cell's centre-to-face vectors (zero: no face), with Limiter.cpp:50-74's
+    // signed room D1: for Venkatakrishnan with a negative constant, whose e2 < 0 makes num / den
+    // rise again with |d| and change sign, so that the largest |d| decides nothing.
+    template <int W>
+    __device__ __forceinline__ void limiter_by_face(T iv, T venkat_K, const T (&r)[W][2], T* phi) const {
+        const T eps = T(1e-9);
+        const T kh = venkat_K * qsqrt(qrcp(iv));
+        const T e2 = kh * kh * kh;
+#pragma unroll
+        for (int v = 0; v < NVAR; v++) {
+            phi[v] = T(1);
+#pragma unroll 1
+            for (int k = 0; k < W; k++) {
+                const T d = G[2 * v] * r[k][0] + G[2 * v + 1] * r[k][1];
+                if (!(d > eps || d < -eps)) continue;
+                const T D1 = d > eps ? umax[v] - u[v] : umin[v] - u[v];
+                const T num = D1 * D1 + e2 + T(2) * D1 * d, den = D1 * D1 + T(2) * d * d + D1 * d + e2;
+                phi[v] = fmin(phi[v], fmin(T(1), qdiv(num, den)));
+            }
         }
     }
     // The limited gradient.
@@ -524,7 +549,8 @@ constexpr int kOwnBlocksPerThread = 4;
 // block_dt, which every block of pass 2 reduces, in place of a minimum that must be found at +inf:
 // whatever an earlier call left behind (refused, captured or raced against another), this one is
 // right, without a launch that resets the scratch.  Pass 2 starts under the tail of pass 1.
-template <class T, int W, bool OWN>
+// BYFACE: the limiter face by face (limiter_by_face).
+template <class T, int W, bool OWN, bool BYFACE>
 __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     T xmx = T(0);                        // largest iv * lam (see dt_of_max)
@@ -560,6 +586,7 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
             const int lmode = OWN ? LIM_NORMAL : limiter_mode(a.stats->steps, a.freeze_after);
             T out[8], phis[4];
             if (lmode == LIM_FROZEN) ld_cell(a.phiF, a.Nc, c, phis);
+            else if (BYFACE) p.limiter_by_face(iv, a.venkat_K, ro, phis);
             else p.limiter_values(iv, a.limiter, a.venkat_K, phis);
             p.limited(phis, out);
             if (lmode == LIM_RECORD) st_cell(a.phiF, a.Nc, c, phis);
@@ -584,6 +611,12 @@ __global__ void __launch_bounds__(256) pass1_kernel(const StepArgs<T> a) {
             }
         }
     }
+}
+
+// The pass 1 of a limiter and its constant.
+template <class T, int W, bool OWN>
+auto pass1_of(int limiter, double venkat_K) {
+    return by_face(limiter, T(venkat_K)) ? pass1_kernel<T, W, OWN, true> : pass1_kernel<T, W, OWN, false>;
 }
 
 // ---------------------------------------------------------------------------------------

@@ -90,7 +90,7 @@ unsigned long long current_ctx_id() {
 template <int W>
 cudaError_t launch(const hcfd::StepArgs<double>& a, cudaStream_t st, bool overlap) {
     const int grid = (a.Nc + kBlock - 1) / kBlock;
-    hcfd::pass1_kernel<double, W, true><<<grid, kBlock, 0, st>>>(a);
+    hcfd::pass1_of<double, W, true>(a.limiter, a.venkat_K)<<<grid, kBlock, 0, st>>>(a);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kBlock);

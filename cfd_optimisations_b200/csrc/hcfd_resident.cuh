@@ -337,7 +337,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Til
                 if (x[0] == kNoFace) continue;
                 const T iv = sIv[c];
                 Pass1Cell<T, NVAR> p;
-                tile_faces<T, W, NVAR>(p, x, sU, sGeo, NL, nf, c, j, false, s.gma, iv, nb, a.B, nh, a.err);
+                T ro[W][2];
+                tile_faces<T, W, NVAR>(p, x, sU, sGeo, NL, nf, c, j, false, s.gma, iv, nb, a.B, nh, a.err, ro);
                 T out[2 * NVAR], phis[NVAR];
                 if (lmode == LIM_FROZEN) {
                     // perhaps written in this launch (by this thread): not through the read-only path

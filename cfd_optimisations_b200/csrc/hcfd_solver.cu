@@ -316,7 +316,7 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl, bool want_res) 
         const hcfd::TileArgs<T> a1 = tile_args<T>(s, time_mode, dt_or_cfl, s->tp[0], 1);
         const hcfd::TileArgs<T> a2 = tile_args<T>(s, time_mode, dt_or_cfl, P2, 2, want_res);
         if ((rc = prof_begin(s, rec, e1))) return rc;
-        CK(hcfd::launch_dependent(hcfd::pass1_variant<T, W, false>(s->prm.limiter, time_mode), s->grid1, s->tp[0].block + 32,
+        CK(hcfd::launch_dependent(hcfd::pass1_variant<T, W, false>(s->prm.limiter, s->prm.venkat_K, time_mode), s->grid1, s->tp[0].block + 32,
                                   s->smem1, s->stream, a1));
         if ((rc = prof_end(s, rec, e1, s->ev1))) return rc;
         if ((rc = prof_begin(s, rec, e2))) return rc;
@@ -327,7 +327,7 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl, bool want_res) 
         const int grid = nblk(s->Nc, s->block);
         hcfd::StepArgs<T> a = step_args<T>(s, time_mode, dt_or_cfl);
         if ((rc = prof_begin(s, rec, e1))) return rc;
-        hcfd::pass1_kernel<T, W, false><<<grid, s->block, 0, s->stream>>>(a);
+        hcfd::pass1_of<T, W, false>(s->prm.limiter, s->prm.venkat_K)<<<grid, s->block, 0, s->stream>>>(a);
         if ((rc = prof_end(s, rec, e1, s->ev1))) return rc;
         if ((rc = prof_begin(s, rec, e2))) return rc;
         hcfd::pass2_kernel<T, W, std::is_same<T, float>::value, false><<<grid, s->block, 0, s->stream>>>(a);
@@ -370,7 +370,7 @@ int setup_tiled_w(hcfd_solver* s) {
     // every time mode's variants, on one grid: the fewest CTAs an SM holds of any of them
     int b1 = 0, b2 = 0;
     for (int mode : {HCFD_FIXED_DT, HCFD_GLOBAL_CFL, HCFD_LOCAL_CFL}) {
-        const void* k1 = (const void*) hcfd::pass1_variant<T, W, false>(s->prm.limiter, mode);
+        const void* k1 = (const void*) hcfd::pass1_variant<T, W, false>(s->prm.limiter, s->prm.venkat_K, mode);
         const void* k2 = (const void*) hcfd::pass2_variant<T, W, false>(s->split ? 7 : 8, mode, s->short2);
         int n1 = 0, n2 = 0, rc;
         if ((rc = allow_smem(k1, maxsm)) || (rc = allow_smem(k2, maxsm))) return rc;
@@ -531,9 +531,9 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
 
     s->tiled = (p.kernel == HCFD_KERNEL_TILED);
     std::vector<int2> slot;
-    if (s->tiled && !p.tile && !p.tile2 && !p.block) {
+    if (s->tiled && !p.tile && !p.tile2 && !p.block && !hcfd::by_face(p.limiter, p.venkat_K)) {
         // Resident steps where the whole mesh fits in the SMs' shared memory, one tile per SM
-        // (no explicit tile or block): faster than the tiled kernels at every size that fits, up to the
+        // (no explicit tile or block, and a limiter that the deciding faces give): faster than the tiled kernels at every size that fits, up to the
         // last (361x181 nodes in FP64 15.5 us a step against 20.1, 501x251 in FP32 13.4 against 17.1), so
         // capacity draws the line.  The plan is built only where the cells' own arrays fit.
         const bool f64 = p.precision == HCFD_FP64;

@@ -839,13 +839,12 @@ __device__ __forceinline__ void lds_vars(const Cell4<T>* p, int ps, int i, int j
 }
 
 // Pass 1 of tile cell c (pair j of its variables when NVAR is 2) up to the limiter's increments,
-// operands from shared memory: its face words in x, nf entries, nb tile cells and nh halo cells of
+// operands from shared memory (its centre-to-face vectors stay in ro): its face words in x, nf entries, nb tile cells and nh halo cells of
 // NL staged.  Unrolled: the face loads overlap.
 template <class T, int W, int NVAR>
 __device__ __forceinline__ void tile_faces(Pass1Cell<T, NVAR>& p, const unsigned x[W], const Cell4<T>* sU, const T* sGeo, int NL,
                                            int nf, int c, int j, bool with_lam, T gma, T iv, int nb, int B, int nh,
-                                           unsigned int* err) {
-    T ro[W][2];
+                                           unsigned int* err, T (&ro)[W][2]) {
     lds_vars<NVAR>(sU, NL, c, j, p.u);
     p.begin(with_lam, gma, p.u);
 #pragma unroll
@@ -879,7 +878,7 @@ __device__ __forceinline__ void tile_faces(Pass1Cell<T, NVAR>& p, const unsigned
 
 // LIM and LAM: the limiter and whether the CFL sums are wanted, fixed at compile time (the branches
 // on them, eight a cell, and the register moves where their sides meet were a tenth of the kernel's
-// instructions); -1: read from the arguments (W = 8, meshes no workload has).
+// instructions); -1: read from the arguments (W = 8, meshes no workload has, and a limiter by_face).
 template <class T, int W, bool ARENA, int LIM, int LAM>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : W == 3 ? 56 : 72) tile_pass1_kernel(const TileArgs<T> a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -896,9 +895,11 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : W == 3 ? 56 : 72) tile_pass1_
         if (x[0] == kNoFace) continue;
         Pass1Cell<T> p;
         const T iv = sIv[c];
-        tile_faces<T, W, 4>(p, x, sU, sGeo, NL, nfl, c, 0, with_lam, s.gma, iv, nb, a.B, si.nh, a.err);
+        T ro[W][2];
+        tile_faces<T, W, 4>(p, x, sU, sGeo, NL, nfl, c, 0, with_lam, s.gma, iv, nb, a.B, si.nh, a.err, ro);
         T out[8], phis[4];
         if (lmode == LIM_FROZEN) ld_cell_l2(s.phiF, a.ps, base + c, phis);
+        else if (LIM < 0 && by_face(s.limiter, s.venkat_K)) p.limiter_by_face(iv, s.venkat_K, ro, phis);
         else p.template limiter_values<LIM>(iv, s.limiter, s.venkat_K, phis);
         p.limited(phis, out);
         if (lmode == LIM_RECORD) st_cell(s.phiF, a.ps, base + c, phis);
@@ -1089,10 +1090,11 @@ cudaError_t launch_dependent(TileKernel<T> kernel, int grid, int block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 template <class T, int W, bool ARENA>
-TileKernel<T> pass1_variant(int limiter, int time_mode) {
+TileKernel<T> pass1_variant(int limiter, double venkat_K, int time_mode) {
     if constexpr (W == 8) {
         return tile_pass1_kernel<T, W, ARENA, -1, -1>;
     } else {
+        if (by_face(limiter, T(venkat_K))) return tile_pass1_kernel<T, W, ARENA, -1, -1>;
         const bool lam = time_mode != TM_FIXED;
         if (limiter == LIM_BJ) return lam ? tile_pass1_kernel<T, W, ARENA, LIM_BJ, 1> : tile_pass1_kernel<T, W, ARENA, LIM_BJ, 0>;
         return lam ? tile_pass1_kernel<T, W, ARENA, LIM_VENKAT, 1> : tile_pass1_kernel<T, W, ARENA, LIM_VENKAT, 0>;
