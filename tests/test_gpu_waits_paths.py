@@ -51,3 +51,23 @@ def test_a_poll_limit_of_one(precision, launches, nx, ny, kw):
         except H.HcfdError as e:
             assert e.code == N.ETIMEOUT
     _recovers(s, m, precision, kw)
+
+
+@pytest.mark.parametrize("skip", [0, 1])
+@pytest.mark.parametrize("mode,value", [(H.GLOBAL_CFL, 0.5), (H.FIXED_DT, 1e-5)])
+@pytest.mark.parametrize("precision,launches,nx,ny,kw", CASES)
+def test_a_tile_that_never_arrives(precision, launches, nx, ny, kw, mode, value, skip):
+    """In the resident kernel a fixed step holds no tile back but a neighbour, so tiles far from the
+    missing one give up some steps later, with their r vectors' copies of the next step in flight
+    where fluxes take those vectors' room."""
+    m = H.Mesh.wedge(nx, ny, seed=9, numbering=H.NUMBER_RCM)
+    s = _solver(m, precision, kw)
+    assert s.launches_per_step() == launches
+    s.step(2, H.GLOBAL_CFL, 0.5)
+    N.check(N.lib().hcfd_gpu_test_waits(s._h, 1 << 14, skip))
+    with pytest.raises(H.HcfdError) as e:
+        s.step(40 if launches == 1 else 2, mode, value)
+    assert e.value.code == N.ETIMEOUT
+    with pytest.raises(H.HcfdError):
+        s.sync()
+    _recovers(s, m, precision, kw)
