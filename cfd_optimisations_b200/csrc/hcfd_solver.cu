@@ -316,7 +316,7 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl, bool want_res) 
         const hcfd::TileArgs<T> a1 = tile_args<T>(s, time_mode, dt_or_cfl, s->tp[0], 1);
         const hcfd::TileArgs<T> a2 = tile_args<T>(s, time_mode, dt_or_cfl, P2, 2, want_res);
         if ((rc = prof_begin(s, rec, e1))) return rc;
-        CK(hcfd::launch_dependent(hcfd::pass1_variant<T, W, false>(s->prm.limiter, s->prm.venkat_K, time_mode), s->grid1, s->tp[0].block + 32,
+        CK(hcfd::launch_dependent(hcfd::pass1_variant<T, W, false>(s->prm.limiter, s->prm.venkat_K, time_mode, s->short1), s->grid1, s->tp[0].block + 32,
                                   s->smem1, s->stream, a1));
         if ((rc = prof_end(s, rec, e1, s->ev1))) return rc;
         if ((rc = prof_begin(s, rec, e2))) return rc;
@@ -370,7 +370,7 @@ int setup_tiled_w(hcfd_solver* s) {
     // every time mode's variants, on one grid: the fewest CTAs an SM holds of any of them
     int b1 = 0, b2 = 0;
     for (int mode : {HCFD_FIXED_DT, HCFD_GLOBAL_CFL, HCFD_LOCAL_CFL}) {
-        const void* k1 = (const void*) hcfd::pass1_variant<T, W, false>(s->prm.limiter, s->prm.venkat_K, mode);
+        const void* k1 = (const void*) hcfd::pass1_variant<T, W, false>(s->prm.limiter, s->prm.venkat_K, mode, s->short1);
         const void* k2 = (const void*) hcfd::pass2_variant<T, W, false>(s->split ? 7 : 8, mode, s->short2);
         int n1 = 0, n2 = 0, rc;
         if ((rc = allow_smem(k1, maxsm)) || (rc = allow_smem(k2, maxsm))) return rc;

@@ -36,7 +36,7 @@ struct TileArgs {
     const int* __restrict__ halo;          // internal cell ids
     const unsigned* __restrict__ nbr;      // [ntiles * B * Wp]: a word per cell and face (pack_nbr_kernel); Wp = W
     const short* __restrict__ cslot;       // the same as the plan's 16-bit {entry, side}, staged in their place by the
-                                           // variants of arguments read at run time; null: the words are staged
+                                           // kRareToo variants; null: the words are staged
     int ntiles, B, Wp, Hmax, Fmax;
     unsigned int* err;                     // bit 0: a bounded wait gave up; bit 1: copies did not drain;
                                            // bit 2: an index out of range (checked build)
@@ -119,6 +119,12 @@ __device__ __forceinline__ void lds_nbr(const unsigned* p, unsigned x[W]) {
         }
     }
 }
+
+// Values of a kernel's template arguments beside those fixed at compile time: read from the arguments
+// (W = 8, meshes no workload has); the same with what few handles need on top, 16-bit face words
+// (GEN) and a limiter by_face.  On W = 8, whose other handles took the same variant at first, these cost
+// 6-7 % (260,000 cells of three to eight faces, FP64 52.2 us a step without them and 55.7 with, FP32 31.9 and 33.8).
+constexpr int kRunTime = -1, kRareToo = -2;
 
 // GEN: the variant may have 16-bit words staged (sNbr then points at them), which are widened here.
 template <int W, bool GEN>
@@ -878,11 +884,11 @@ __device__ __forceinline__ void tile_faces(Pass1Cell<T, NVAR>& p, const unsigned
 
 // LIM and LAM: the limiter and whether the CFL sums are wanted, fixed at compile time (the branches
 // on them, eight a cell, and the register moves where their sides meet were a tenth of the kernel's
-// instructions); -1: read from the arguments (W = 8, meshes no workload has, and a limiter by_face).
+// instructions), or kRunTime or kRareToo.
 template <class T, int W, bool ARENA, int LIM, int LAM>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : W == 3 ? 56 : 72) tile_pass1_kernel(const TileArgs<T> a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr bool GEN = LIM < 0;
+    constexpr bool GEN = LIM == kRareToo;
     const TileSmem<T> L(a.B, a.Hmax, a.Fmax, W, a.Wp, false, GEN && a.cslot);
     const StepArgs<T>& s = a.s;
     T xmx = T(0);                        // largest iv * lam (see dt_of_max)
@@ -899,7 +905,7 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : W == 3 ? 56 : 72) tile_pass1_
         tile_faces<T, W, 4>(p, x, sU, sGeo, NL, nfl, c, 0, with_lam, s.gma, iv, nb, a.B, si.nh, a.err, ro);
         T out[8], phis[4];
         if (lmode == LIM_FROZEN) ld_cell_l2(s.phiF, a.ps, base + c, phis);
-        else if (LIM < 0 && by_face(s.limiter, s.venkat_K)) p.limiter_by_face(iv, s.venkat_K, ro, phis);
+        else if (LIM == kRareToo && by_face(s.limiter, s.venkat_K)) p.limiter_by_face(iv, s.venkat_K, ro, phis);
         else p.template limiter_values<LIM>(iv, s.limiter, s.venkat_K, phis);
         p.limited(phis, out);
         if (lmode == LIM_RECORD) st_cell(s.phiF, a.ps, base + c, phis);
@@ -936,12 +942,12 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : W == 3 ? 56 : 72) tile_pass1_
 }
 
 // REC and LOCAL: the record length and local time stepping, fixed at compile time as in pass 1
-// (-1: read from the arguments).
+// (or kRunTime or kRareToo).
 template <class T, int W, bool ARENA, int REC, int LOCAL>
 __global__ void __maxnreg__(128) tile_pass2_kernel(const TileArgs<T> a) {
     constexpr bool COMP = sizeof(T) == 4;
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr bool GEN = REC < 0;
+    constexpr bool GEN = REC == kRareToo;
     const TileSmem<T> L(a.B, a.Hmax, a.Fmax, W, a.Wp, true, GEN && a.cslot);
     const StepArgs<T>& s = a.s;
     double dt_used = 0.0;
@@ -1090,11 +1096,11 @@ cudaError_t launch_dependent(TileKernel<T> kernel, int grid, int block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 template <class T, int W, bool ARENA>
-TileKernel<T> pass1_variant(int limiter, double venkat_K, int time_mode) {
+TileKernel<T> pass1_variant(int limiter, double venkat_K, int time_mode, bool short_words = false) {
+    if (by_face(limiter, T(venkat_K)) || short_words) return tile_pass1_kernel<T, W, ARENA, kRareToo, -1>;
     if constexpr (W == 8) {
-        return tile_pass1_kernel<T, W, ARENA, -1, -1>;
+        return tile_pass1_kernel<T, W, ARENA, kRunTime, -1>;
     } else {
-        if (by_face(limiter, T(venkat_K))) return tile_pass1_kernel<T, W, ARENA, -1, -1>;
         const bool lam = time_mode != TM_FIXED;
         if (limiter == LIM_BJ) return lam ? tile_pass1_kernel<T, W, ARENA, LIM_BJ, 1> : tile_pass1_kernel<T, W, ARENA, LIM_BJ, 0>;
         return lam ? tile_pass1_kernel<T, W, ARENA, LIM_VENKAT, 1> : tile_pass1_kernel<T, W, ARENA, LIM_VENKAT, 0>;
@@ -1102,12 +1108,12 @@ TileKernel<T> pass1_variant(int limiter, double venkat_K, int time_mode) {
 }
 template <class T, int W, bool ARENA>
 TileKernel<T> pass2_variant(int rec, int time_mode, bool short_words = false) {
+    if constexpr (!ARENA)
+        if (short_words) return tile_pass2_kernel<T, W, ARENA, kRareToo, -1>;
     if constexpr (W == 8) {
-        return tile_pass2_kernel<T, W, ARENA, -1, -1>;
+        return tile_pass2_kernel<T, W, ARENA, kRunTime, -1>;
     } else {
         const bool local = time_mode == TM_LOCAL;
-        if constexpr (!ARENA)
-            if (short_words) return tile_pass2_kernel<T, W, ARENA, -1, -1>;
         if constexpr (!ARENA)
             if (rec == 7) return local ? tile_pass2_kernel<T, W, ARENA, 7, 1> : tile_pass2_kernel<T, W, ARENA, 7, 0>;
         return local ? tile_pass2_kernel<T, W, ARENA, 8, 1> : tile_pass2_kernel<T, W, ARENA, 8, 0>;
