@@ -85,7 +85,7 @@ struct hcfd_solver {
     void* d_geoT = nullptr;              // per-cell kernels in float: FaceGeo<float> [Nf]
     void* d_iv = nullptr;                // T [Nc]
     void* d_U[2] = {nullptr, nullptr};   // Cell4<T> [Nc]
-    void* d_phiG = nullptr;              // Grad8<T> [Nc]
+    void* d_phiG = nullptr;              // Grad8<T> [Nc] (resident: from the first profiled step on)
     void* d_phiF = nullptr;              // Cell4<T> [Nc]: frozen limiter values
     double* d_io = nullptr;              // 4 Nc doubles staging for upload/download
     double* d_cp = nullptr;              // Nf doubles for the wall Cp
@@ -271,8 +271,6 @@ int launch_resident(hcfd_solver* s, int time_mode, double dt_or_cfl, int nsteps,
     r.llU = s->d_ll;
     r.llG = r.llU + (size_t) s->Nc * (sizeof(hcfd::Cell4<T>) / 8);
     r.llX = r.llG + (size_t) s->Nc * (sizeof(hcfd::Grad8<T>) / 8);
-    // a half step leaves the gradients of all cells to the other half, where whole steps exchange theirs
-    a.s.phiG = (hcfd::Grad8<T>*) r.llG;
     r.epoch = s->epoch;
     r.dtmin = s->d_dtmin;
     r.partial_first = s->d_partial + s->partial_len;
@@ -306,9 +304,6 @@ int launch_step(hcfd_solver* s, int time_mode, double dt_or_cfl, bool want_res) 
             (rc = prof_end(s, rec, e1, s->ev1)) || (rc = prof_begin(s, rec, e2)) ||
             (rc = launch_resident<T, W>(s, time_mode, dt_or_cfl, 1, 2)) || (rc = prof_end(s, rec, e2, s->ev2)))
             return rc;
-        // The halves passed unstamped gradients through the words' memory: a value whose upper halves
-        // are a coming step's stamp would be taken for that step's word.
-        CK(cudaMemsetAsync(s->d_ll, 0, sizeof(ulonglong2) * s->ll_words, s->stream));
         return HCFD_OK;
     }
     if (s->tiled) {
@@ -1140,6 +1135,14 @@ int hcfd_gpu_profile(hcfd_solver* s, int enable) {
     s->ev1.clear(); s->ev2.clear();
     s->ms1 = s->ms2 = 0; s->n1 = s->n2 = 0;
     if (enable < 0) return fail(HCFD_EINVAL, "profile: negative sampling period");
+    if (enable && s->resident && !s->d_phiG) {
+        // Half steps of the resident kernel leave the gradients of all cells to each other; whole steps
+        // exchange theirs as stamped words, whose memory plain values must stay out of (one whose upper
+        // halves are a coming step's stamp would be taken for that step's word).
+        const size_t bytes = (s->fp32() ? sizeof(hcfd::Grad8<float>) : sizeof(hcfd::Grad8<double>)) * (size_t) s->Nc;
+        if ((rc = dalloc((char**) &s->d_phiG, bytes))) return rc;
+        CK(cudaMemsetAsync(s->d_phiG, 0, bytes, s->stream));
+    }
     s->prof = enable != 0;
     s->prof_every = enable > 0 ? enable : 1;
     s->prof_count = 0;
