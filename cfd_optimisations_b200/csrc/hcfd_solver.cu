@@ -528,8 +528,8 @@ int hcfd_gpu_create(const hcfd_mesh_view* mv, const hcfd_params* prm, hcfd_solve
     std::vector<int2> slot;
     if (s->tiled && !p.tile && !p.tile2 && !p.block && !hcfd::by_face(p.limiter, p.venkat_K)) {
         // Resident steps where the whole mesh fits in the SMs' shared memory, one tile per SM
-        // (no explicit tile or block, and a limiter that the deciding faces give): faster than the tiled kernels at every size that fits, up to the
-        // last (361x181 nodes in FP64 15.5 us a step against 20.1, 501x251 in FP32 13.4 against 17.1), so
+        // (no explicit tile or block, and a limiter that the deciding faces give): faster than the tiled
+        // kernels at every size that fits, up to the last (361x181 nodes in FP64 15.5 us a step against 20.1, 501x251 in FP32 13.4 against 17.1), so
         // capacity draws the line.  The plan is built only where the cells' own arrays fit.
         const bool f64 = p.precision == HCFD_FP64;
         int maxsm = 0, coop = 0;

@@ -357,8 +357,8 @@ __device__ __forceinline__ void compute_sync(int nthreads) {
 
 // Producer warp: for each of this CTA's tiles, waits until the compute warps have released
 // the staging buffer, then lane 0 arms the buffer's `full` mbarrier with the byte counts of
-// the bulk copies and issues them (those of the first tile that no kernel writes ahead of the rest), and every lane gathers its share of the halo cells with
-// cp.async and signals their completion on the same mbarrier.  The `full` barrier therefore
+// the bulk copies and issues them (those of the first tile that no kernel writes ahead of the rest), and
+// every lane gathers its share of the halo cells with cp.async and signals their completion on the same mbarrier.  The `full` barrier therefore
 // completes when all of the tile's data has landed: 1 expect-tx arrival + 32 cp.async
 // arrivals + the transaction bytes.
 // Once any wait of the CTA has given up, the producer issues nothing more; before it
@@ -845,8 +845,8 @@ __device__ __forceinline__ void lds_vars(const Cell4<T>* p, int ps, int i, int j
 }
 
 // Pass 1 of tile cell c (pair j of its variables when NVAR is 2) up to the limiter's increments,
-// operands from shared memory (its centre-to-face vectors stay in ro): its face words in x, nf entries, nb tile cells and nh halo cells of
-// NL staged.  Unrolled: the face loads overlap.
+// operands from shared memory (its centre-to-face vectors stay in ro): its face words in x, nf entries,
+// nb tile cells and nh halo cells of NL staged.  Unrolled: the face loads overlap.
 template <class T, int W, int NVAR>
 __device__ __forceinline__ void tile_faces(Pass1Cell<T, NVAR>& p, const unsigned x[W], const Cell4<T>* sU, const T* sGeo, int NL,
                                            int nf, int c, int j, bool with_lam, T gma, T iv, int nb, int B, int nh,
