@@ -71,10 +71,13 @@ def class_mesh(cls: int) -> Mesh:
 
 @functools.lru_cache(maxsize=None)
 def library_id(path: str) -> str:
-    """A digest of the native library's contents (about 10 ms, once a process)."""
+    """A digest of the native library's contents (about 10 ms, once a process); "none" where it is not built."""
     h = hashlib.blake2b(digest_size=6)
-    with open(path, "rb") as fh:
-        h.update(fh.read())
+    try:
+        with open(path, "rb") as fh:
+            h.update(fh.read())
+    except OSError:
+        return "none"
     return h.hexdigest()
 
 

@@ -39,3 +39,11 @@ def test_winners_without_a_library_count_as_missing(tmp_path, monkeypatch):
     monkeypatch.setattr(A, "gpu_name", lambda: "B200")
     cache.write_text(json.dumps({"B200|solver|fp64|lim0|c15": {"best": TILE_64}}))
     assert A.best_solver_shape(25_600, tune=False) == A.DEFAULT_SHAPE
+
+
+def test_without_a_library_the_default_shape(tmp_path, monkeypatch):
+    monkeypatch.setenv("HCFD_AUTOTUNE_CACHE", str(tmp_path / "autotune.json"))
+    monkeypatch.setattr(A, "gpu_name", lambda: "B200")
+    monkeypatch.setattr(A.native, "LIB_PATH", str(tmp_path / "not_built.so"))
+    assert A.best_solver_shape(25_600, tune=False) == A.DEFAULT_SHAPE
+    assert A.best_arena_tile(25_600, H.FP32, tune=False) == 128
