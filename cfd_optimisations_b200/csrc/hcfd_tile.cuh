@@ -479,8 +479,7 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
         }
     };
     // the first tile's while the kernel before this one ends; everything else waits for it
-    const bool ahead = t0 < a.ntiles && t0 != a.skip_tile;
-    if (ahead) stage_static(d0, !kChecked || d0.nb >= 0, 0);
+    if (t0 < a.ntiles && t0 != a.skip_tile) stage_static(d0, !kChecked || d0.nb >= 0, 0);
     grid_wait_previous();
     load_scalars(d0.inst, v0);
     v1 = v0;
@@ -563,10 +562,11 @@ __device__ __forceinline__ void producer_loop(const TileArgs<T>& a, unsigned cha
             t2 = a.claim ? 3 * (int) gridDim.x + __shfl_sync(0xffffffffu, pending, 0) : t2 + (int) gridDim.x;
     }
     cp_async_wait_all();
-    if (ahead && armed[0] < 0) {
+    if ((int) blockIdx.x < a.ntiles && (int) blockIdx.x != a.skip_tile && armed[0] < 0) {
         // The CTA gave up before the first tile's stage was armed in full, with its static copies in flight:
         // the stage is closed as at the end, with tile -1 and the arrivals it lacks, and completes when
-        // they have landed.
+        // they have landed.  (The test is formed anew: kept in a register through the loop, it cost the FP32
+        // arena's step 0.2 %.)
         if (lane == 0) {
             reinterpret_cast<StageInfo*>(smem + 64)[0].t = -1;
             mbar_arrive(full);
